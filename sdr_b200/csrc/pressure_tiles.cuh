@@ -6,37 +6,52 @@
 // thread per line. A tile walks the levels L = i+j+k of its cells in order;
 // within a level every line has at most one cell (i = L - j - k), whose -x
 // predecessor is the thread's own previous cell (a register) and whose -y and
-// -z predecessors are the neighbouring lines' cells of level L-1 (shared
-// memory, double-buffered by level), or, on the tile's low faces, cells of
-// the neighbouring tiles. So a level costs one barrier of the tile's threads,
-// and tiles synchronise only with their two upstream neighbours through
-// exchange entries that mark their own readiness: a tile runs as soon as its
-// neighbours are one level ahead, and a sweep takes about (levels x the level step) + (tile hops
-// x the hand-off latency) instead of one grid-wide barrier per level. The
-// backward sweep mirrors it (tiles wait on their +y / +z neighbours, levels in
-// decreasing order).
+// -z predecessors are the neighbouring lines' cells of level L-1. Those live
+// in a shared-memory window of kTwRing levels, one slot per line plus a halo
+// row and column for the cells of the neighbouring tiles. So a level costs one
+// barrier of the tile's threads, and tiles synchronise only with their two
+// upstream neighbours through exchange entries that mark their own readiness:
+// a tile runs as soon as its neighbours are one level ahead, and a sweep takes
+// about (levels x the level step) + (tile hops x the hand-off latency) instead
+// of one grid-wide barrier per level. The backward sweep mirrors it (tiles
+// wait on their +y / +z neighbours, levels in decreasing order): thread t then
+// takes line 255 - t, so both sweeps read the same two slots.
+//
+// The level step is a chain of latencies (cycles on a B200: shared load 29,
+// add 12, multiply 8, barrier of 8 warps 40; 132 for a bare step) and of issue
+// slots (two warps per scheduler), so it holds as few instructions as it can.
+// A branch per neighbour, 64-bit addresses and the operands' arrival took it to
+// about 1,400 cycles. The step now has no branch: a line without a fluid cell
+// at a level leaves -0.0 in its slot, and t + (-0.0) is t for every t, so each
+// cell adds its three predecessors unconditionally and no neighbour mask is
+// read. The operands (residual or forward result, factor, z's places) are rows
+// brought to shared memory by the bulk-copy engine, four levels to a copy, and
+// each thread reads its own of level s+1 while it computes level s. The loop is
+// unrolled over a copy's four levels, so most addresses are a constant away
+// from a register (unrolled over the whole window, a step took 700 cycles on
+// sweeps of 15 levels: the instructions themselves had to be fetched).
 //
 // Per cell the arithmetic is that of k_pcg / k_pcg_cluster (the same operands
 // in the same order), so the factor and both sweeps give the same bits, and so
 // does the solve: the matvec, the updates and the dots run in the wavefront
 // order and tiling of the other kernels, spread over the grid. The sweeps'
 // operands live in rows: per tile one row of kTwLines entries per level of its
-// range, so the lines of a level are contiguous and every copy and store of a
-// level is coalesced (the lines' cells lie some 70 cells apart in cell order,
-// which made each warp access touch 32 cache lines). The update phase writes
-// the residual into the rows and the dots read z back through the wavefront
-// index -> row map. Each compute thread keeps its next kTwDepth levels'
-// operands in flight to shared memory (cp.async), so a level's step never
-// waits on a global load.
+// range, so a level is contiguous. The update phase writes the residual into
+// its row; z goes straight to its place in wavefront order (the cells of a
+// tile row are neighbours there too, so a level's stores are runs of 128 bytes).
 //
 // Synchronisation: one cooperative launch (every CTA resident). Phases are
 // separated by a grid barrier (an arrival counter and a generation word,
 // release/acquire at GPU scope). In a sweep the 8 compute warps of a CTA share
-// a named barrier per level; a ninth warp polls the upstream tiles' exchange
-// entries and copies their boundary values into a shared-memory ring, so
-// compute threads never wait on a global load. Every wait gives up after about a
-// second (2^31 SM cycles) or as soon as another CTA has given up, sets an
-// error bit and lets the kernel wind down.
+// a named barrier per level; two more warps, one per upstream face, poll the
+// upstream tiles' exchange entries and copy their values into the window's
+// halo, and one issues the operand copies, so compute threads never wait on a
+// global load. Only tiles with fluid cells take a CTA. Every wait gives up
+// after about a second (2^31 SM cycles) or as soon as another CTA has given
+// up, sets an error bit and lets the kernel wind down. The waits of a level (y
+// values, z values, operands) and the published progress belong to three clerk
+// warps that join its barrier: one release store or one try_wait on a compute
+// warp cost 90 cycles of every other level.
 #pragma once
 #include "pressure.cuh"
 
@@ -45,36 +60,47 @@ namespace sdr {
 constexpr int kTwJ = 16;                     // lines per tile along y
 constexpr int kTwK = 16;                     // lines per tile along z
 constexpr int kTwLines = kTwJ * kTwK;        // compute threads: one per line
-constexpr int kTwBS = kTwLines + 32;         // plus the progress warp
+// Threads: the compute warps, a progress warp per upstream face, the operand
+// warp, three clerk warps (kTwBarrier threads share a level's barrier), and
+// more for the grid-wide phases (24 warps per SM keep enough loads in
+// flight; one CTA per SM makes the grid barrier half of what two cost).
+constexpr int kTwBS = 768;
+constexpr int kTwBarrier = kTwLines + 96;
 constexpr int kTwWarps = kTwBS / 32;
-constexpr int kTwRing = 32;                  // levels of neighbour boundary values staged ahead
-constexpr int kTwDepth = 6;                  // cells of each line whose operands are in flight to shared memory
+constexpr int kTwRing = 16;                  // levels the window holds (a power of two)
+constexpr int kTwPitch = kTwJ + 1;           // window slots per line row: the halo, then the tile's lines
+constexpr int kTwSlots = (kTwK + 1) * kTwPitch;  // window slots per level
+constexpr int kTwDepth = kTwRing;            // levels of operands in shared memory
+constexpr int kTwGroup = 4;                  // levels per bulk copy
+constexpr int kTwGroups = kTwDepth / kTwGroup;
 constexpr long long kTwWaitCycles = 1ll << 31;  // ~1.1 s at 1965 MHz
 constexpr uint32_t kTwErrWait = 16u;         // error bit: a sweep or barrier wait gave up
-constexpr uint32_t kTwNoCell = 0xFFFFFFFFu;  // a row entry without a fluid cell
+constexpr uint16_t kTwNoCell = 0xFFFFu;      // a row entry without a fluid cell
 constexpr int kTwFace = 16;                  // lines of a tile face (either face)
-// Levels a progress-warp poll loads at once: more loads in flight per poll
-// slow the compute warps' shared-memory accesses on the same SM (pool solve
-// at 0.2 mm: 76.3 ms with 2, 77.1 with 4, 79.7 with 8).
-constexpr int kTwPoll = 2;
+// Levels a progress-warp poll covers: two per load (the half-warps take
+// neighbouring levels), kTwPoll loads in flight.
+constexpr int kTwPoll = 3;
+constexpr int kTwThirds = kTwBS / kTwLines;  // 256-thread groups of a CTA in the matvec
+constexpr int kTwBatch = 2 * kTwThirds;      // 256-cell dot tiles of the matvec a CTA has in flight
 static_assert(kTwJ == kTwFace && kTwK == kTwFace, "both tile faces hold kTwFace lines");
+static_assert((kTwRing & (kTwRing - 1)) == 0, "the window's level is taken by a mask");
+static_assert(kTile == kTwLines, "the matvec takes one cell of a dot tile per compute thread");
+static_assert(kTwRing * kTwSlots >= kTwBatch * kTile, "the grid-wide phases use the window as scratch");
 
 struct TwArgs {
     PcgArgs a;                   // wavefront-order vectors, tables and dots (as k_pcg)
     int nx, ny, nz;
     int tj, tk, ntiles;          // tiles along y and z
-    const uint32_t* coff;        // dense cell -> cell-order index of its fluid cell (exclusive scan, ncell + 1)
-    uint32_t* icm_c;             // cell order: i | fluid-neighbour bits (NB_*) << 16 | non-solid count << 24
-    // The sweeps' operands in rows: per tile, one row of kTwLines entries per
-    // level of its range (entry = rbase[tile] + (L - tlo[tile]) * kTwLines +
-    // line), so the lines of a level are contiguous and every access of a
-    // level is coalesced. Entries without a fluid cell hold kTwNoCell in icm.
-    uint32_t* icm;               // rows: the (i, mask, count) word, or kTwNoCell
-    double2* rp;                 // rows: (residual, MIC(0) factor), the forward sweep's operands
-    double2* qp;                 // rows: (forward sweep result, MIC(0) factor), the backward sweep's
-    double* zr;                  // rows: backward sweep result
+    // Rows: per tile, one row of kTwLines entries per level of its range
+    // (entry = rbase[tile] + (L - tlo[tile]) * kTwLines + line).
+    uint16_t* word;              // rows: fluid-neighbour bits (NB_*) | non-solid count << 8, or kTwNoCell
+    uint32_t* idx;               // rows: the cell's wavefront index (cells only)
+    double* rr;                  // rows: residual (cells only)
+    double* pc;                  // rows: MIC(0) factor; -0.0, which no factor is, where there is no cell
+    double* qr;                  // rows: forward sweep result (cells only)
     uint32_t* tpos;              // wavefront index -> row entry of its cell
     uint32_t* rbase;             // per tile: its first row entry (ntiles + 1 entries)
+    int* tlist;                  // the tiles with fluid cells in increasing order, after their number
     size_t rows_cap;             // row entries allocated
     // Exchange planes, level-major like the rows: a tile's boundary values of
     // its q-th level (sweep order) at rbase[tile] / kTwFace + q * kTwFace + l,
@@ -113,32 +139,48 @@ __device__ __forceinline__ void st_relaxed_gpu_f64(double* p, double v) {
 __device__ __forceinline__ void st_relaxed_gpu_u64(double* p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-// 4-byte asynchronous copy into shared memory (cp_async16 and cp_commit are
-// pressure.cuh's), and a wait until at most N of this thread's groups are pending.
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+// Shared-memory accesses at a constant offset from a 32-bit address, in program
+// order with the barriers around them.
+template <int OFF>
+__device__ __forceinline__ double lds_f64(uint32_t a) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1+%2];" : "=d"(v) : "r"(a), "n"(OFF));
+    return v;
 }
-template <int N>
-__device__ __forceinline__ void cp_wait_n() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+template <int OFF>
+__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+__device__ __forceinline__ void sts_f64(uint32_t a, double v) {
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
 __device__ __forceinline__ bool tw_failed(const TwArgs& t) { return *(volatile uint32_t*)t.err != 0u; }
-// Barrier of the compute warps (named barrier 1).
-__device__ __forceinline__ void tw_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kTwLines) : "memory"); }
+// Barrier of the compute and clerk warps (named barrier 1).
+__device__ __forceinline__ void tw_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kTwBarrier) : "memory"); }
 
 struct TwShared {
-    double v[2][kTwLines];            // this tile's values of the last two levels, by line
-    uint8_t m[2][kTwLines];           // the factorisation's neighbour masks, by line
-    double ring[2][kTwRing][16];      // upstream neighbours' boundary values by level ([0] y face, [1] z face)
-    uint8_t ringm[2][kTwRing][16];    // their masks (factorisation)
-    double2 rec[kTwDepth][kTwLines];  // each line's next cells: (r or q, factor), by cell ordinal mod kTwDepth
-    uint32_t icm[kTwDepth][kTwLines]; // and their (i, mask, count) words
-    unsigned long long mine;          // levels this tile has completed (sweep order), for the progress warp
-    unsigned long long avail[2];      // levels whose y / z neighbour values are in the ring
-    int ok;
+    double win[kTwRing * kTwSlots];   // the last levels' values by window slot; scratch of the grid-wide phases
+    // operand rows by level of the sweep mod kTwDepth (backward: the levels of a
+    // group in decreasing place, as they lie in memory):
+    double op_a[kTwDepth][kTwLines];  // residual or forward result,
+    double op_b[kTwDepth][kTwLines];  // factor,
+    uint32_t op_i[kTwDepth][kTwLines];  // and wavefront index (backward)
+    uint64_t op_full[kTwGroups];      // mbarriers: the group's rows have arrived
+    unsigned long long avail[2];      // levels (of the sweep) whose y / z neighbour values are in the window
+    long long mine;                   // the last level (of the sweep, from 0) whose barrier this tile has passed
     double red[kTwWarps];
+    int ok;
+    uint8_t m[2][kTwSlots];           // the factorisation's neighbour masks of the last two levels, by window slot
+    uint8_t ringm[2][kTwRing][kTwFace];  // the upstream neighbours' masks by level (factorisation)
 };
+constexpr size_t kTwSmem = sizeof(TwShared);
+extern __shared__ __align__(128) unsigned char tw_smem[];
+#define TW_SH (*reinterpret_cast<TwShared*>(tw_smem))
 
 // Grid barrier; false if the wait gave up or another CTA has (the error bit is set).
-__device__ bool tw_grid_sync(const TwArgs& t, TwShared& sh) {
+__device__ bool tw_grid_sync(const TwArgs& t) {
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
@@ -162,52 +204,67 @@ __device__ bool tw_grid_sync(const TwArgs& t, TwShared& sh) {
             }
         }
         if (ok && tw_failed(t)) ok = 0;  // another CTA gave up: wind down
-        sh.ok = ok;
+        TW_SH.ok = ok;
     }
     __syncthreads();
-    return sh.ok != 0;
+    return TW_SH.ok != 0;
 }
 
-__device__ __forceinline__ double tw_block_max(double v, TwShared& sh) {
+__device__ __forceinline__ double tw_block_max(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = v;
+    if ((threadIdx.x & 31) == 0) TW_SH.red[threadIdx.x >> 5] = v;
     __syncthreads();
-    double m = sh.red[0];
-    for (int w = 1; w < kTwWarps; ++w) m = fmax(m, sh.red[w]);
+    double m = TW_SH.red[0];
+    for (int w = 1; w < kTwWarps; ++w) m = fmax(m, TW_SH.red[w]);
     __syncthreads();
     return m;
 }
 
 // Maximum over the grid (order-free): CTA maxima through a double-buffered slot array.
-__device__ bool tw_grid_max(const TwArgs& t, TwShared& sh, double v, int& parity, double& out) {
-    const double bm = tw_block_max(v, sh);
+__device__ bool tw_grid_max(const TwArgs& t, double v, int& parity, double& out) {
+    const double bm = tw_block_max(v);
     double* sl = t.gslots + (size_t)parity * gridDim.x;
     parity ^= 1;
     if (threadIdx.x == 0) sl[blockIdx.x] = bm;
-    if (!tw_grid_sync(t, sh)) return false;
+    if (!tw_grid_sync(t)) return false;
     if (threadIdx.x < 32) {
         double m = 0.0;
         for (unsigned q = threadIdx.x; q < gridDim.x; q += 32) m = fmax(m, __ldcg(sl + q));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (threadIdx.x == 0) sh.red[0] = m;
+        if (threadIdx.x == 0) TW_SH.red[0] = m;
     }
     __syncthreads();
-    out = sh.red[0];
+    out = TW_SH.red[0];
     __syncthreads();
     return true;
 }
 
 // Total of the tree-order tile sums (the lane pattern and xor tree of
-// pcg_tile_total), formed by warp 0 and handed to the CTA.
-__device__ double tw_tile_total(const TwArgs& t, uint32_t ntile, TwShared& sh) {
+// pcg_tile_total): the CTA brings them to shared memory, warp 0 adds them.
+// One warp loading them from L2 itself took 7 us for the 4,650 sums of a
+// 1.19 M-cell pool, twice per iteration.
+__device__ double tw_tile_total(const TwArgs& t, uint32_t ntile) {
+    double* const scratch = TW_SH.win;
+    constexpr uint32_t kChunk = kTwRing * kTwSlots / 32 * 32;
+    double s = 0.0;
+    for (uint32_t c0 = 0; c0 < ntile; c0 += kChunk) {
+        const uint32_t n = min(kChunk, ntile - c0);
+        __syncthreads();
+        for (uint32_t q = threadIdx.x; q < n; q += kTwBS) scratch[q] = __ldcg(t.a.tpart + c0 + q);
+        __syncthreads();
+        if (threadIdx.x < 32) {
+#pragma unroll 8
+            for (uint32_t q = threadIdx.x; q < n; q += 32) s = dadd(s, scratch[q]);
+        }
+    }
     if (threadIdx.x < 32) {
-        const double s = pcg_tile_total(t.a, ntile);
-        if (threadIdx.x == 0) sh.red[0] = s;
+        s = warp_tree_sum(s);
+        if (threadIdx.x == 0) TW_SH.red[0] = s;
     }
     __syncthreads();
-    const double r = sh.red[0];
+    const double r = TW_SH.red[0];
     __syncthreads();
     return r;
 }
@@ -215,9 +272,9 @@ __device__ double tw_tile_total(const TwArgs& t, uint32_t ntile, TwShared& sh) {
 // The reference's chunked dot (pressure.rs:588-603) over `prod` in cell
 // order: one warp per 4096-cell chunk across the grid, then the chunk sums in
 // chunk order (as pcg_exact_dot).
-__device__ bool tw_exact_dot(const TwArgs& t, TwShared& sh, double& out) {
+__device__ bool tw_exact_dot(const TwArgs& t, double& out) {
     const PcgArgs& a = t.a;
-    if (!tw_grid_sync(t, sh)) return false;  // products complete
+    if (!tw_grid_sync(t)) return false;  // products complete
     const int lane = threadIdx.x & 31;
     const int gw = blockIdx.x * kTwWarps + (threadIdx.x >> 5), nw = gridDim.x * kTwWarps;
     for (int ch = gw; ch < a.nchunks; ch += nw) {
@@ -243,14 +300,14 @@ __device__ bool tw_exact_dot(const TwArgs& t, TwShared& sh, double& out) {
         }
         if (lane == 0) a.partials[ch] = acc;
     }
-    if (!tw_grid_sync(t, sh)) return false;
+    if (!tw_grid_sync(t)) return false;
     if (threadIdx.x == 0) {
         double s = -0.0;
         for (int ch = 0; ch < a.nchunks; ++ch) s = dadd(s, __ldcg(a.partials + ch));
-        sh.red[0] = s;
+        TW_SH.red[0] = s;
     }
     __syncthreads();
-    out = sh.red[0];
+    out = TW_SH.red[0];
     __syncthreads();
     return true;
 }
@@ -258,140 +315,255 @@ __device__ bool tw_exact_dot(const TwArgs& t, TwShared& sh, double& out) {
 // ---------------------------------------------------------------- the tile sweeps
 enum { TW_BUILD = 0, TW_FORWARD = 1, TW_BACKWARD = 2 };
 
-// The progress warp of one tile's sweep: it stages the upstream tiles'
-// boundary values into the shared ring, lanes 0-15 the y face (line
-// (jb, k0 + l)), lanes 16-31 the z face (line (j0 + l, kb)), and publishes per
-// face how many levels are staged. The values carry their own readiness: every
+// Line of window slot order `l` of a face: the backward sweep runs mirrored.
+__device__ __forceinline__ int tw_mirror(bool fwd, int l) { return fwd ? l : kTwFace - 1 - l; }
+// Window slots of the sweep's level q.
+__device__ __forceinline__ double* tw_win(int q) { return TW_SH.win + (q & (kTwRing - 1)) * kTwSlots; }
+
+// The progress warp of one face (0: y, 1: z) of a tile's sweep: it brings the
+// upstream tile's boundary values into the window's halo and publishes how
+// many levels are there. The values carry their own readiness: every
 // entry of an exchange plane holds kTwEmpty until its producer writes it (the
-// planes are filled when the solve lays out its rows), a lane polls the entries its
-// next levels need (relaxed loads, kTwPoll levels at a time), and resets
-// each entry it staged to kTwEmpty (the producer writes it again only in the
-// next sweep of this direction, after a grid barrier). So a hand-off costs
-// the producer's store reaching L2 and one poll, with no progress flags and no
-// GPU-scope fences. A level needs no entry where the producer tile has no
-// level before it (its range is in tlo/thi) or the cell lies outside the grid:
-// the ring gets 0 there. The factorisation also stages the upstream cell's
-// neighbour mask, read from the static cell tables.
+// planes are filled when the solve lays out its rows), a lane polls the entries
+// the next levels need (relaxed loads; lane l takes line l % 16, the upper
+// half-warp one level further), and resets each entry it staged to kTwEmpty
+// (the producer writes it again only in the next sweep of this direction,
+// after a grid barrier). So a hand-off costs the producer's store reaching L2
+// and one poll, with no progress flags and no GPU-scope fences. A level needs
+// no entry where the producer tile has no level before it (its range is in
+// tlo/thi) or the line lies outside the grid: the halo gets -0.0 there. The
+// factorisation also stages the upstream cell's neighbour mask from its row.
 template <int MODE>
-__device__ void tw_progress_warp(const TwArgs& t, TwShared& sh, int tile, int nby, int nbz, int s_first,
-                                 int s_last, int nlevels) {
+__device__ void tw_progress_warp(const TwArgs& t, int face, int tile, int nb, int s_first, int nlev, int nlevels) {
     constexpr bool fwd = MODE != TW_BACKWARD;
     const int lane = threadIdx.x & 31;
     const int J = tile % t.tj, K = tile / t.tj;
-    const int j0 = J * kTwJ, k0 = K * kTwK, nx = t.nx;
-    const int face = lane >> 4, l = lane & 15;
-    const int nb = face == 0 ? nby : nbz;
-    // this tile's boundary line and the producer's line beside it
+    const int j0 = J * kTwJ, k0 = K * kTwK;
+    const int l = lane & 15, half = lane >> 4;
+    // this tile's boundary line
     const int jl = face == 0 ? (fwd ? j0 : j0 + kTwJ - 1) : j0 + l;
     const int kl = face == 0 ? k0 + l : (fwd ? k0 : k0 + kTwK - 1);
-    const int jp = face == 0 ? (fwd ? jl - 1 : jl + 1) : jl;
-    const int kp = face == 0 ? kl : (fwd ? kl - 1 : kl + 1);
-    const bool line_ok = nb >= 0 && (face == 0 ? l < kTwK : l < kTwJ) && jl < t.ny && kl < t.nz;
+    const bool line_ok = jl < t.ny && kl < t.nz;
+    const int lm = tw_mirror(fwd, l);
+    const int slot = face == 0 ? (lm + 1) * kTwPitch : lm + 1;
     // the producer's entries of this line: level q of its sweep at src + q * kTwFace
-    double* src = nb >= 0 ? (fwd ? t.exf : t.exb) + (face == 0 ? 0 : t.rows_cap / kTwFace) +
-                                (size_t)__ldcg(t.rbase + nb) / kTwFace + (size_t)l
-                          : nullptr;
-    // the producer's levels in sweep order
-    int pf = 1, pl = 0;
+    double* src = (fwd ? t.exf : t.exb) + (face == 0 ? 0 : t.rows_cap / kTwFace) +
+                  (size_t)__ldcg(t.rbase + nb) / kTwFace + (size_t)l;
+    // the producer's levels before this tile's level q: its level q - 1 + shift, if within [0, np)
+    int np = 0, shift = 0;
     if (line_ok) {
         const int lo = __ldcg(t.tlo + nb), hi = __ldcg(t.thi + nb);
         if (hi >= lo) {
-            pf = fwd ? lo : nlevels - 1 - hi;
-            pl = fwd ? hi : nlevels - 1 - lo;
+            np = hi - lo + 1;
+            shift = s_first - (fwd ? lo : nlevels - 1 - hi);
         }
     }
-    int next = line_ok ? s_first : s_last + 1;  // next level (sweep order) this lane stages
-    int staged_face = -1;                       // levels of this face published so far
+    src += (ptrdiff_t)(shift - 1) * kTwFace;  // level q's entry: src + q * kTwFace
+    // and the upstream cell's word (forward: the producer's last line row or column)
+    const uint16_t* const words = t.word + (size_t)__ldcg(t.rbase + nb) + (ptrdiff_t)(shift - 1) * kTwLines +
+                                  (face == 0 ? l * kTwJ + kTwJ - 1 : (kTwK - 1) * kTwJ + l);
+    int next = 0;  // next level to stage
     const long long t0 = clock64();
-    for (unsigned polls = 1;; ++polls) {
-        const int mine = (int)ld_acquire_cta_sh(&sh.mine);
-        const int lim = min(s_last, mine + kTwRing - 1);  // ring room
-        if (next <= lim) {
-            // up to kTwPoll levels: an entry per level that needs one, loaded at once
-            double v[kTwPoll];
-            bool need[kTwPoll];
+    for (unsigned polls = 1; next < nlev; ++polls) {
+        const int mine = (int)(long long)ld_acquire_cta_sh(reinterpret_cast<unsigned long long*>(&TW_SH.mine));
+        const int lim = min(nlev, mine + kTwRing);  // window room: levels below lim
+        // entries of levels next + half, next + 2 + half, ..., loaded at once
+        double v[kTwPoll];
+        uint16_t mk[kTwPoll];
+        bool need[kTwPoll];
 #pragma unroll
-            for (int u = 0; u < kTwPoll; ++u) {
-                const int sq = next + u;
-                const int L = fwd ? sq : nlevels - 1 - sq;
-                const int i = L - jl - kl;
-                need[u] = sq <= lim && sq - 1 >= pf && sq - 1 <= pl && i >= 0 && i < nx;
-                v[u] = need[u] ? ld_relaxed_gpu_f64(src + (size_t)(sq - 1 - pf) * kTwFace) : 0.0;
-            }
-            int u = 0;
-            for (; u < kTwPoll && next + u <= lim; ++u) {
-                if (need[u] && __double_as_longlong(v[u]) == (long long)kTwEmpty) break;  // not written yet
-                const int sq = next + u;
-                const int L = fwd ? sq : nlevels - 1 - sq;
-                const int i = L - jl - kl;
-                sh.ring[face][sq % kTwRing][l] = need[u] ? v[u] : 0.0;
-                if (MODE == TW_BUILD) {
-                    uint8_t m = 0;
-                    if (need[u]) {
-                        const size_t d = ((size_t)kp * t.ny + jp) * (size_t)nx + i;
-                        const uint32_t c0 = __ldcg(t.coff + d), c1 = __ldcg(t.coff + d + 1);
-                        if (c1 != c0) m = (uint8_t)(__ldcg(t.icm_c + c0) >> 16);
-                    }
-                    sh.ringm[face][sq % kTwRing][l] = m;
-                }
-                if (need[u]) st_relaxed_gpu_u64(src + (size_t)(sq - 1 - pf) * kTwFace, kTwEmpty);
-            }
-            next += u;
+        for (int u = 0; u < kTwPoll; ++u) {
+            const int q = next + 2 * u + half;
+            need[u] = q < lim && (unsigned)(q - 1 + shift) < (unsigned)np;
+            if (MODE == TW_BUILD) mk[u] = need[u] ? __ldcg(words + (ptrdiff_t)q * kTwLines) : (uint16_t)0;
+            v[u] = need[u] ? ld_relaxed_gpu_f64(src + (ptrdiff_t)q * kTwFace) : -0.0;
         }
-        // a face's levels are staged up to the least of its lanes
-        int fm = next;
+        int nr = 0;  // levels that are ready, in order: all 16 lines of each
+        bool open = true;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) fm = min(fm, __shfl_xor_sync(0xffffffffu, fm, o));
-        __syncwarp();
-        if ((lane == 0 || lane == 16) && fm > staged_face) {
-            st_release_cta_sh(&sh.avail[face], (unsigned long long)fm);
-            staged_face = fm;
+        for (int u = 0; u < kTwPoll; ++u) {
+            const bool ok = next + 2 * u + half < lim &&
+                            !(need[u] && __double_as_longlong(v[u]) == (long long)kTwEmpty);
+            const unsigned b = __ballot_sync(0xffffffffu, ok);
+            if (open && (b & 0xffffu) == 0xffffu) {
+                ++nr;
+                open = (b >> 16) == 0xffffu;
+                nr += open ? 1 : 0;
+            } else {
+                open = false;
+            }
         }
-        if (__all_sync(0xffffffffu, next > s_last)) break;
+#pragma unroll
+        for (int u = 0; u < kTwPoll; ++u) {
+            if (2 * u + half < nr) {
+                const int q = next + 2 * u + half;
+                tw_win(q - 1)[slot] = v[u];
+                if (MODE == TW_BUILD) TW_SH.ringm[face][q & (kTwRing - 1)][l] = (uint8_t)mk[u];
+            }
+        }
+        if (nr) {
+            __syncwarp();
+            if (lane == 0) st_release_cta_sh(&TW_SH.avail[face], (unsigned long long)(next + nr));
+#pragma unroll
+            for (int u = 0; u < kTwPoll; ++u)
+                if (2 * u + half < nr && need[u])
+                    st_relaxed_gpu_u64(src + (ptrdiff_t)(next + 2 * u + half) * kTwFace, kTwEmpty);
+            next += nr;
+        }
         if ((polls & 63u) == 0u && __shfl_sync(0xffffffffu, (int)(tw_failed(t) || clock64() - t0 > kTwWaitCycles), 0)) {
             if (lane == 0) {
                 atomicOr(t.err, kTwErrWait);
-                st_release_cta_sh(&sh.avail[0], ~0ull >> 1);  // release this tile's compute warps
-                st_release_cta_sh(&sh.avail[1], ~0ull >> 1);
+                st_release_cta_sh(&TW_SH.avail[face], ~0ull >> 1);  // release this tile's compute warps
             }
             break;
         }
     }
 }
 
-// Compute-thread wait until the ring holds neighbour values for level s.
-__device__ __forceinline__ void tw_wait(const TwArgs& t, TwShared& sh, int which, unsigned long long s) {
-    if (ld_acquire_cta_sh(&sh.avail[which]) > s) return;
+// The operand warp (one lane): the rows of the sweep's levels, a group per
+// bulk copy, completing on the group's mbarrier. A group's place is free once
+// the barrier of its old last level has been passed (those operands were read
+// before it). Every group is issued even while the kernel winds down (groups
+// past the last level arrive without a copy, so that every sweep uses each
+// mbarrier equally often), and the compute threads wait for every group, so no
+// copy is in flight when the sweep ends.
+template <int MODE>
+__device__ void tw_operand_warp(const TwArgs& t, size_t row0, int nlev) {
+    asm volatile("fence.proxy.async;" ::: "memory");  // the rows were written by ordinary stores
+    constexpr bool fwd = MODE != TW_BACKWARD;
     const long long t0 = clock64();
-    for (unsigned spin = 0; ld_acquire_cta_sh(&sh.avail[which]) <= s; ++spin) {
-        if ((spin & 255u) == 255u && (tw_failed(t) || clock64() - t0 > kTwWaitCycles)) {
+    int passed = -1;
+    for (int q = 0; q < nlev || (q & (kTwDepth - 1)) != 0; q += kTwGroup) {
+        const uint32_t bar = smem_addr(&TW_SH.op_full[(q / kTwGroup) % kTwGroups]);
+        // a group past the last level only waits until its old use has been seen
+        const int until = q - kTwDepth + (q < nlev ? kTwGroup - 1 : 0);
+        for (unsigned spin = 1; passed < until; ++spin) {
+            passed = (int)(long long)ld_acquire_cta_sh(reinterpret_cast<unsigned long long*>(&TW_SH.mine));
+            if ((spin & 255u) == 0u && clock64() - t0 > 2 * kTwWaitCycles) {  // cannot happen: every level is passed
+                atomicOr(t.err, kTwErrWait);
+                return;
+            }
+        }
+        if (q >= nlev) {
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+            continue;
+        }
+        const int n = min(kTwGroup, nlev - q);
+        const int at = (q & (kTwDepth - 1)) + (fwd ? 0 : kTwGroup - n);
+        const size_t e = row0 + (size_t)(fwd ? q : nlev - q - n) * kTwLines;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                     "r"((uint32_t)(n * kTwLines * (fwd ? 16 : 20)))
+                     : "memory");
+        auto copy = [&](void* dst, const void* src, uint32_t bytes) {
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                    smem_addr(dst)),
+                "l"(src), "r"(bytes), "r"(bar)
+                : "memory");
+        };
+        copy(TW_SH.op_a[at], (fwd ? t.rr : t.qr) + e, (uint32_t)(n * kTwLines * 8));
+        copy(TW_SH.op_b[at], t.pc + e, (uint32_t)(n * kTwLines * 8));
+        if (!fwd) copy(TW_SH.op_i[at], t.idx + e, (uint32_t)(n * kTwLines * 4));
+    }
+}
+
+// Wait until group g of the operands has arrived; parity: of the group's use (bounded).
+__device__ __forceinline__ void tw_op_wait(const TwArgs& t, int g, uint32_t parity) {
+    const uint32_t bar = smem_addr(&TW_SH.op_full[g]);
+    long long t0 = 0;
+    for (unsigned spin = 0;; ++spin) {
+        uint32_t done;
+        asm volatile(
+            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return;
+        if (spin == 0) t0 = clock64();
+        else if (clock64() - t0 > 2 * kTwWaitCycles) {
             atomicOr(t.err, kTwErrWait);
             return;
         }
     }
 }
 
-// Operands of this line's entry of the q-th level of the sweep into shared
-// slot q mod kTwDepth, as one cp.async group: the (i, mask, count) word, and
-// for the solves the 16-byte (r, factor) or (q, factor) record through L2 (r
-// is written by other CTAs in the update phase). The row layout makes each of
-// a warp's copies one contiguous stretch. Levels past the sweep's end commit
-// an empty group, so every level commits exactly one.
-template <int MODE>
-__device__ __forceinline__ void tw_stage(const TwArgs& t, TwShared& sh, int tid, size_t e, bool live, int q) {
-    if (live) {
-        const int slot = q % kTwDepth;
-        cp_async4(&sh.icm[slot][tid], t.icm + e);
-        if (MODE != TW_BUILD) cp_async16(&sh.rec[slot][tid], (MODE == TW_FORWARD ? t.rp : t.qp) + e);
+// A clerk's wait until the window holds the neighbour values of level s;
+// returns the levels it holds.
+__device__ __forceinline__ int tw_wait(const TwArgs& t, int which, int s) {
+    unsigned long long have = ld_acquire_cta_sh(&TW_SH.avail[which]);
+    if (have <= (unsigned long long)s) {
+        const long long t0 = clock64();
+        for (unsigned spin = 1; (have = ld_acquire_cta_sh(&TW_SH.avail[which])) <= (unsigned long long)s; ++spin) {
+            if ((spin & 255u) == 0u && (tw_failed(t) || clock64() - t0 > kTwWaitCycles)) {
+                atomicOr(t.err, kTwErrWait);
+                return INT32_MAX;
+            }
+        }
     }
-    cp_commit();
+    return (int)min(have, (unsigned long long)INT32_MAX);
 }
 
-// One tile's sweep. BUILD: the MIC(0) factor into rp.y and qp.y (forward
-// order). FORWARD: q = L^-1 r into qp.x. BACKWARD: z = L^-T q, plus the z*r products in cell
-// order for the reference dot order.
+// A clerk warp: it joins the barrier of every level once the level may begin.
+// Clerk 0 waits for the y neighbour's values, clerk 1 for the z neighbour's
+// and publishes the level passed, clerk 2 waits for the operand group of the
+// level after.
 template <int MODE>
-__device__ void tw_sweep(const TwArgs& t, TwShared& sh, int tile, int nlevels) {
+__device__ void tw_clerk_warp(const TwArgs& t, int clerk, int nb, int nlev, uint32_t parity0) {
+    int have = nb >= 0 ? 0 : INT32_MAX;
+    for (int q = 0; q < nlev; ++q) {
+        if (clerk < 2) {
+            if (have <= q) have = tw_wait(t, clerk, q);
+        } else if (MODE != TW_BUILD && (q + 1) % kTwGroup == 0 && q + 1 < nlev) {
+            tw_op_wait(t, (q + 1) / kTwGroup % kTwGroups, (parity0 + (uint32_t)(q + 1) / kTwDepth) & 1u);
+        }
+        tw_bar();
+        if (clerk == 1 && (threadIdx.x & 31) == 0)
+            st_release_cta_sh(reinterpret_cast<unsigned long long*>(&TW_SH.mine), (unsigned long long)(long long)q);
+    }
+}
+
+// The factor of one cell (build_mic0, pressure.rs:442-513).
+__device__ __forceinline__ double tw_factor(uint8_t m, double diag, double pxi, uint8_t mx_, double pyj, uint8_t my_,
+                                            double pzk, uint8_t mz_) {
+    const double TAU = 0.97, SIGMA = 0.25;
+    double axi = 0, axi_y = 0, axi_z = 0, ayj = 0, ayj_x = 0, ayj_z = 0, azk = 0, azk_x = 0, azk_y = 0;
+    if (m >> NB_MX & 1) {
+        axi = -1.0;
+        axi_y = (mx_ >> NB_PY & 1) ? -1.0 : 0.0;
+        axi_z = (mx_ >> NB_PZ & 1) ? -1.0 : 0.0;
+    } else {
+        pxi = 0.0;
+    }
+    if (m >> NB_MY & 1) {
+        ayj = -1.0;
+        ayj_x = (my_ >> NB_PX & 1) ? -1.0 : 0.0;
+        ayj_z = (my_ >> NB_PZ & 1) ? -1.0 : 0.0;
+    } else {
+        pyj = 0.0;
+    }
+    if (m >> NB_MZ & 1) {
+        azk = -1.0;
+        azk_x = (mz_ >> NB_PX & 1) ? -1.0 : 0.0;
+        azk_y = (mz_ >> NB_PY & 1) ? -1.0 : 0.0;
+    } else {
+        pzk = 0.0;
+    }
+    const double tx = dmul(axi, pxi), ty = dmul(ayj, pyj), tz = dmul(azk, pzk);
+    const double mx = dmul(dmul(dmul(axi, dadd(axi_y, axi_z)), pxi), pxi);
+    const double my = dmul(dmul(dmul(ayj, dadd(ayj_x, ayj_z)), pyj), pyj);
+    const double mz = dmul(dmul(dmul(azk, dadd(azk_x, azk_y)), pzk), pzk);
+    double e = dsub(dsub(dsub(dsub(diag, dmul(tx, tx)), dmul(ty, ty)), dmul(tz, tz)),
+                    dmul(TAU, dadd(dadd(mx, my), mz)));
+    if (e < dmul(SIGMA, diag)) e = diag;
+    return e > 0.0 ? ddiv(1.0, __dsqrt_rn(e)) : 0.0;
+}
+
+// One tile's sweep. BUILD: the MIC(0) factor into pc (forward order). FORWARD:
+// q = L^-1 r into qr. BACKWARD: z = L^-T q, plus the z*r products in cell
+// order for the reference dot order. `uses` counts the rounds of the operand
+// ring this CTA has consumed (the same in every thread).
+template <int MODE>
+__device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, int nlevels, uint32_t& uses) {
     const PcgArgs& a = t.a;
     const int tid = threadIdx.x;
     const int J = tile % t.tj, K = tile / t.tj;
@@ -400,210 +572,301 @@ __device__ void tw_sweep(const TwArgs& t, TwShared& sh, int tile, int nlevels) {
     const int nby = fwd ? (J > 0 ? tile - 1 : -1) : (J + 1 < t.tj ? tile + 1 : -1);
     const int nbz = fwd ? (K > 0 ? tile - t.tj : -1) : (K + 1 < t.tk ? tile + t.tj : -1);
     const int lo = __ldcg(t.tlo + tile), hi = __ldcg(t.thi + tile);
-    const int s_first = hi < lo ? nlevels : (fwd ? lo : nlevels - 1 - hi);
-    const int s_last = hi < lo ? nlevels - 1 : (fwd ? hi : nlevels - 1 - lo);
+    const int s_first = fwd ? lo : nlevels - 1 - hi;  // the sweep's level 0
+    const int nlev = hi - lo + 1;
+    // window slot of this thread's line; its predecessors are at slot - 1 and slot - kTwPitch
+    const int lj = tid % kTwJ, lk = (tid / kTwJ) & (kTwK - 1);
+    const int slot = (lk + 1) * kTwPitch + lj + 1;
     if (tid == 0) {
-        sh.mine = (unsigned long long)s_first;
-        sh.avail[0] = sh.avail[1] = (unsigned long long)s_first;
+        TW_SH.mine = -1;
+        TW_SH.avail[0] = TW_SH.avail[1] = 0ull;
+    }
+    if (tid < kTwLines) {  // no value before the first level, nor beyond the grid's edge
+        tw_win(-1)[slot] = -0.0;
+        if (MODE == TW_BUILD) TW_SH.m[1][slot] = 0;
+        if (nby < 0)
+            TW_SH.win[lj * kTwSlots + (lk + 1) * kTwPitch] = -0.0;  // (level, line) of kTwRing x kTwK
+        if (nbz < 0)
+            TW_SH.win[lk * kTwSlots + lj + 1] = -0.0;
     }
     __syncthreads();
+    const size_t row0 = (size_t)__ldcg(t.rbase + tile);
+    const uint32_t parity0 = uses & 1u;
+    if (MODE != TW_BUILD) uses += (uint32_t)(nlev + kTwDepth - 1) / kTwDepth;
     if (tid >= kTwLines) {
-        tw_progress_warp<MODE>(t, sh, tile, nby, nbz, s_first, s_last, nlevels);
+        const int w = (tid - kTwLines) >> 5;
+        if (w < 2) {
+            const int nb = w == 0 ? nby : nbz;
+            if (nb >= 0) tw_progress_warp<MODE>(t, w, tile, nb, s_first, nlev, nlevels);
+        } else if (w == 2) {
+            if (MODE != TW_BUILD && tid == kTwLines + 64) tw_operand_warp<MODE>(t, row0, nlev);
+        } else if (w < 6) {
+            tw_clerk_warp<MODE>(t, w - 3, w == 3 ? nby : w == 4 ? nbz : -1, nlev, parity0);
+        }
         __syncthreads();
         return;
     }
-    const int lj = tid % kTwJ, lk = tid / kTwJ;
-    const int j = J * kTwJ + lj, k = K * kTwK + lk;
-    const int nx = t.nx;
-    const int jk = j + k;
-    // This line's row entries, level q of the sweep (q = s - s_first) at
-    // row0 + (fwd ? q : nlev - 1 - q) * kTwLines + tid. The operands of the
-    // next kTwDepth levels are in flight to shared memory at all times: level
-    // q stages q + kTwDepth, one cp.async group per level, so when level q is
-    // read the group that staged it has kTwDepth - 1 groups after it.
-    const int nlev = s_last - s_first + 1;
-    const size_t row0 = nlev > 0 ? (size_t)__ldcg(t.rbase + tile) : 0;
+    const int line = fwd ? tid : kTwLines - 1 - tid;  // the line this thread takes
+    const int j = J * kTwJ + line % kTwJ, k = K * kTwK + line / kTwJ;
     // the lines on the downstream faces write an exchange entry at every level
-    // of the sweep where their cell lies in the grid (0 where the line has no
-    // fluid cell), so the downstream tile's progress warp finds every entry it
-    // polls written; level q's entry of face line l is ex + q * kTwFace
+    // (-0.0 where the line has no fluid cell), so the downstream tile's
+    // progress warp finds every entry it polls written; level q's entry of
+    // face line l is ex + q * kTwFace
     double* const ex_own = (fwd ? t.exf : t.exb) + row0 / kTwFace;
     const bool in_grid = j < t.ny && k < t.nz;
-    double* const ex_y = in_grid && (fwd ? lj == kTwJ - 1 : lj == 0) ? ex_own + (size_t)lk : nullptr;
-    double* const ex_z = in_grid && (fwd ? lk == kTwK - 1 : lk == 0) ? ex_own + t.rows_cap / kTwFace + (size_t)lj
-                                                                      : nullptr;
-    auto entry = [&](int q) -> size_t {
-        return row0 + (size_t)(fwd ? q : nlev - 1 - q) * kTwLines + (size_t)tid;
-    };
-    for (int q = 0; q < kTwDepth; ++q) tw_stage<MODE>(t, sh, tid, q < nlev ? entry(q) : 0, q < nlev, q);
-    double carry = 0.0;   // the value of this line's previous cell (the -x / +x predecessor)
-    uint8_t carry_m = 0;  // its neighbour mask (factorisation)
-    const double TAU = 0.97, SIGMA = 0.25;
-    const bool yb = fwd ? lj == 0 : lj == kTwJ - 1;  // this line reads the y neighbour tile
-    const bool zb = fwd ? lk == 0 : lk == kTwK - 1;
-    unsigned long long* const timing = a.timing;  // optional section timers (thread 0)
-    long long t_loop = 0, t_wait = 0;
-    if (timing && (tid == 0 || tid == 32)) t_loop = clock64();
-    for (int s = s_first; s <= s_last; ++s) {
-        const int L = fwd ? s : nlevels - 1 - s;
-        const int q = s - s_first;
-        const int slot = q % kTwDepth;
-        cp_wait_n<kTwDepth - 1>();
-        const uint32_t word = sh.icm[slot][tid];
-        if (timing && tid == 0 && nby >= 0) {
-            const long long w0 = clock64();
-            tw_wait(t, sh, 0, (unsigned long long)s);
-            t_wait += clock64() - w0;
-        } else if (tid == 0 && nby >= 0) {
-            tw_wait(t, sh, 0, (unsigned long long)s);
+    const bool on_y = in_grid && lj == kTwJ - 1, on_z = in_grid && lk == kTwK - 1;
+    double* ex_y = ex_own + (size_t)(line / kTwJ);
+    double* ex_z = ex_own + t.rows_cap / kTwFace + (size_t)(line % kTwJ);
+    double carry = -0.0;  // the value of this line's previous cell (the -x / +x predecessor)
+    const long long t_loop = a.timing && tid == 0 ? clock64() : 0;
+    // Shared-memory addresses: this line's place in the window by level of the
+    // ring, as byte offsets from one register.
+    constexpr uint32_t kLevel = kTwSlots * 8;
+    const uint32_t w_first = smem_addr(TW_SH.win) + (uint32_t)slot * 8;
+    uint32_t w = w_first, w_prev = w_first + (kTwRing - 1) * kLevel;
+    if (MODE == TW_BUILD) {
+        uint8_t carry_m = 0;
+        const uint16_t* words = t.word + row0 + line;
+        double* pout = t.pc + row0 + line;
+        uint16_t wd[kTwGroup], wn[kTwGroup];
+#pragma unroll
+        for (int u = 0; u < kTwGroup; ++u) wd[u] = u < nlev ? __ldcg(words + u * kTwLines) : kTwNoCell;
+        for (int q0 = 0; q0 < nlev; q0 += kTwGroup) {
+            words += kTwGroup * kTwLines;
+#pragma unroll
+            for (int u = 0; u < kTwGroup; ++u)
+                wn[u] = q0 + kTwGroup + u < nlev ? __ldcg(words + u * kTwLines) : kTwNoCell;
+#pragma unroll
+            for (int u = 0; u < kTwGroup; ++u) {
+                const int q = q0 + u;
+                if (q >= nlev) break;  // the same in every thread
+                const uint8_t m = (uint8_t)wd[u];
+                tw_bar();
+                const double vy = lds_f64<-8>(w_prev), vz = lds_f64<-8 * kTwPitch>(w_prev);
+                double pc = -0.0;
+                if (wd[u] != kTwNoCell) {
+                    const uint8_t my = lj == 0 ? TW_SH.ringm[0][q & (kTwRing - 1)][lk] : TW_SH.m[(u + 1) & 1][slot - 1];
+                    const uint8_t mz =
+                        lk == 0 ? TW_SH.ringm[1][q & (kTwRing - 1)][lj] : TW_SH.m[(u + 1) & 1][slot - kTwPitch];
+                    pc = tw_factor(m, (double)(wd[u] >> 8), carry, carry_m, vy, my, vz, mz);
+                }
+                sts_f64(w, pc);
+                TW_SH.m[u & 1][slot] = wd[u] != kTwNoCell ? m : (uint8_t)0;
+                if (on_y) st_relaxed_gpu_f64(ex_y + u * kTwFace, pc);
+                if (on_z) st_relaxed_gpu_f64(ex_z + u * kTwFace, pc);
+                pout[u * kTwLines] = pc;
+                carry = pc;
+                carry_m = m;
+                w_prev = w;
+                w += kLevel;
+                if (u == kTwGroup - 1 && w == w_first + kTwRing * kLevel) w = w_first;
+            }
+#pragma unroll
+            for (int u = 0; u < kTwGroup; ++u) wd[u] = wn[u];
+            pout += kTwGroup * kTwLines;
+            ex_y += kTwGroup * kTwFace;
+            ex_z += kTwGroup * kTwFace;
         }
-        if (timing && tid == 32 && nbz >= 0) {
-            const long long w0 = clock64();
-            tw_wait(t, sh, 1, (unsigned long long)s);
-            t_wait += clock64() - w0;
-        } else if (tid == 32 && nbz >= 0) {
-            tw_wait(t, sh, 1, (unsigned long long)s);
+    } else {
+        tw_op_wait(t, 0, parity0);
+        // place of level u's operands within its group (backward: decreasing)
+        constexpr int kRev = fwd ? 0 : kTwGroup - 1;
+        constexpr uint32_t kRow = kTwLines * 8;  // bytes of a level's row; op_b follows op_a
+        const uint32_t o_first = smem_addr(TW_SH.op_a) + (uint32_t)line * 8;
+        const uint32_t oi_first = smem_addr(TW_SH.op_i) + (uint32_t)line * 4;
+        uint32_t o = o_first, oi = oi_first;
+        double ra = lds_f64<kRev * kRow>(o), pc = lds_f64<kRev * kRow + kTwDepth * kRow>(o);
+        uint32_t at = fwd ? 0u : lds_u32<kRev * kRow / 2>(oi);
+        double* qout = t.qr + row0 + line;
+        double result = 0.0;  // the level before's q or z,
+        bool owed = false;    // if the line had a cell there,
+        uint32_t at_p = 0u;   // and z's place
+        for (int q0 = 0; q0 < nlev; q0 += kTwGroup) {
+            // the next group's operands
+            const uint32_t gn = (uint32_t)(q0 / kTwGroup + 1) & (kTwGroups - 1);
+            const uint32_t on = o_first + gn * (kTwGroup * kRow), oin = oi_first + gn * (kTwGroup * kRow / 2);
+            const int left = nlev - q0;
+#pragma unroll
+            for (int u = 0; u < kTwGroup; ++u) {
+                if (u > 0 && u >= left) break;  // the same in every thread
+                tw_bar();
+                const double vy = lds_f64<-8>(w_prev), vz = lds_f64<-8 * kTwPitch>(w_prev);
+                // level q + 1's operands (past the last level: values nobody uses)
+                constexpr int kM = kTwGroup - 1;
+                const uint32_t os = (u < kM ? o : on) + (uint32_t)(((u + 1) & kM) ^ kRev) * kRow;
+                const double ra_n = lds_f64<0>(os), pc_n = lds_f64<kTwDepth * kRow>(os);
+                const uint32_t at_n =
+                    fwd ? 0u : lds_u32<0>((u < kM ? oi : oin) + (uint32_t)(((u + 1) & kM) ^ kRev) * (kRow / 2));
+                // the level before's result goes out while these loads run
+                if (MODE == TW_FORWARD) {
+                    if (owed) qout[(u - 1) * kTwLines] = result;
+                } else if (owed) {
+                    a.z[at_p] = result;
+                    if (a.exact_dots)  // the reference dot order is over cells in cell order
+                        a.prod[a.cinv[at_p]] = dmul(result, __ldcg(a.r + at_p));
+                }
+                const bool cell = __double2hiint(pc) >= 0;
+                double out;
+                if (MODE == TW_FORWARD) {
+                    // t = r + pq[-x] + pq[-y] + pq[-z]; q = t * pc (pcg_apply_mic0, forward)
+                    const double qv = dmul(dadd(dadd(dadd(ra, carry), vy), vz), pc);
+                    out = cell ? dmul(pc, qv) : -0.0;
+                    result = qv;
+                } else {
+                    // t = q + pc z[+x] + pc z[+y] + pc z[+z]; z = t * pc (pcg_apply_mic0, backward)
+                    const double zv = dmul(dadd(dadd(dadd(ra, dmul(pc, carry)), dmul(pc, vy)), dmul(pc, vz)), pc);
+                    out = cell ? zv : -0.0;
+                    result = zv;
+                    at_p = at;
+                }
+                sts_f64(w, out);
+                owed = cell;
+                if (on_y) st_relaxed_gpu_f64(ex_y + u * kTwFace, out);
+                if (on_z) st_relaxed_gpu_f64(ex_z + u * kTwFace, out);
+                w_prev = w;
+                w += kLevel;
+                if (u == kTwGroup - 1 && w == w_first + kTwRing * kLevel) w = w_first;
+                carry = out;
+                ra = ra_n;
+                pc = pc_n;
+                at = at_n;
+            }
+            o = on;
+            oi = oin;
+            qout += kTwGroup * kTwLines;
+            ex_y += kTwGroup * kTwFace;
+            ex_z += kTwGroup * kTwFace;
         }
-        tw_bar();
-        // levels before s are complete (every eighth level: the progress warp
-        // only needs it to reuse ring slots, 32 levels deep)
-        if (tid == 0 && ((s - s_first) & 7) == 0) st_release_cta_sh(&sh.mine, (unsigned long long)s);
-        const int wp = (s - 1) & 1, wc = s & 1, rs = s % kTwRing;
-        const int i = L - jk;
-        const size_t ent = entry(q);
-        if (word == kTwNoCell) {
-            if (i >= 0 && i < nx) {  // no cell here: the downstream entry still gets written
-                if (ex_y) st_relaxed_gpu_f64(ex_y + (size_t)q * kTwFace, 0.0);
-                if (ex_z) st_relaxed_gpu_f64(ex_z + (size_t)q * kTwFace, 0.0);
-            }
-            tw_stage<MODE>(t, sh, tid, q + kTwDepth < nlev ? entry(q + kTwDepth) : 0, q + kTwDepth < nlev, q + kTwDepth);
-            continue;
-        }
-        const uint8_t m = (uint8_t)(word >> 16);
-        const double2 rec = MODE == TW_BUILD ? make_double2(0.0, 0.0) : sh.rec[slot][tid];
-        const double a0 = MODE == TW_BUILD ? (double)(word >> 24) : rec.x;  // diag, r or q
-        const double b0 = rec.y;                                              // the factor
-        if (MODE == TW_BUILD) {
-            double axi = 0, pxi = 0, axi_y = 0, axi_z = 0;
-            double ayj = 0, pyj = 0, ayj_x = 0, ayj_z = 0;
-            double azk = 0, pzk = 0, azk_x = 0, azk_y = 0;
-            if (m >> NB_MX & 1) {
-                axi = -1.0;
-                pxi = carry;
-                axi_y = (carry_m >> NB_PY & 1) ? -1.0 : 0.0;
-                axi_z = (carry_m >> NB_PZ & 1) ? -1.0 : 0.0;
-            }
-            if (m >> NB_MY & 1) {
-                const uint8_t mk = yb ? sh.ringm[0][rs][lk] : sh.m[wp][tid - 1];
-                pyj = yb ? sh.ring[0][rs][lk] : sh.v[wp][tid - 1];
-                ayj = -1.0;
-                ayj_x = (mk >> NB_PX & 1) ? -1.0 : 0.0;
-                ayj_z = (mk >> NB_PZ & 1) ? -1.0 : 0.0;
-            }
-            if (m >> NB_MZ & 1) {
-                const uint8_t mk = zb ? sh.ringm[1][rs][lj] : sh.m[wp][tid - kTwJ];
-                pzk = zb ? sh.ring[1][rs][lj] : sh.v[wp][tid - kTwJ];
-                azk = -1.0;
-                azk_x = (mk >> NB_PX & 1) ? -1.0 : 0.0;
-                azk_y = (mk >> NB_PY & 1) ? -1.0 : 0.0;
-            }
-            const double tx = dmul(axi, pxi), ty = dmul(ayj, pyj), tz = dmul(azk, pzk);
-            const double diag = a0;
-            const double mx = dmul(dmul(dmul(axi, dadd(axi_y, axi_z)), pxi), pxi);
-            const double my = dmul(dmul(dmul(ayj, dadd(ayj_x, ayj_z)), pyj), pyj);
-            const double mz = dmul(dmul(dmul(azk, dadd(azk_x, azk_y)), pzk), pzk);
-            double e = dsub(dsub(dsub(dsub(diag, dmul(tx, tx)), dmul(ty, ty)), dmul(tz, tz)),
-                            dmul(TAU, dadd(dadd(mx, my), mz)));
-            if (e < dmul(SIGMA, diag)) e = diag;
-            const double pc = e > 0.0 ? ddiv(1.0, __dsqrt_rn(e)) : 0.0;
-            t.rp[ent].y = pc;
-            t.qp[ent].y = pc;
-            sh.v[wc][tid] = pc;
-            sh.m[wc][tid] = m;
-            carry = pc;
-            carry_m = m;
-            if (ex_y) st_relaxed_gpu_f64(ex_y + (size_t)q * kTwFace, pc);
-            if (ex_z) st_relaxed_gpu_f64(ex_z + (size_t)q * kTwFace, pc);
-        } else if (MODE == TW_FORWARD) {
-            // t = r + pq[-x] + pq[-y] + pq[-z]; q = t * pc (pcg_apply_mic0, forward)
-            double tt = a0;
-            if (m >> NB_MX & 1) tt = dadd(tt, carry);
-            if (m >> NB_MY & 1) tt = dadd(tt, yb ? sh.ring[0][rs][lk] : sh.v[wp][tid - 1]);
-            if (m >> NB_MZ & 1) tt = dadd(tt, zb ? sh.ring[1][rs][lj] : sh.v[wp][tid - kTwJ]);
-            const double qv = dmul(tt, b0);
-            const double pqv = dmul(b0, qv);
-            t.qp[ent].x = qv;
-            sh.v[wc][tid] = pqv;
-            carry = pqv;
-            if (ex_y) st_relaxed_gpu_f64(ex_y + (size_t)q * kTwFace, pqv);
-            if (ex_z) st_relaxed_gpu_f64(ex_z + (size_t)q * kTwFace, pqv);
-        } else {
-            // t = q + pc z[+x] + pc z[+y] + pc z[+z]; z = t * pc (pcg_apply_mic0, backward)
-            const double pc = b0;
-            double tt = a0;
-            if (m >> NB_PX & 1) tt = dadd(tt, dmul(pc, carry));
-            if (m >> NB_PY & 1) tt = dadd(tt, dmul(pc, yb ? sh.ring[0][rs][lk] : sh.v[wp][tid + 1]));
-            if (m >> NB_PZ & 1) tt = dadd(tt, dmul(pc, zb ? sh.ring[1][rs][lj] : sh.v[wp][tid + kTwJ]));
-            const double zv = dmul(tt, pc);
-            t.zr[ent] = zv;
-            if (a.exact_dots)  // the reference dot order is over cells in cell order
-                a.prod[__ldcg(t.coff + ((size_t)k * t.ny + j) * (size_t)nx + i)] = dmul(zv, __ldcg(&t.rp[ent].x));
-            sh.v[wc][tid] = zv;
-            carry = zv;
-            if (ex_y) st_relaxed_gpu_f64(ex_y + (size_t)q * kTwFace, zv);
-            if (ex_z) st_relaxed_gpu_f64(ex_z + (size_t)q * kTwFace, zv);
-        }
-        // the slot's values are in registers: it takes the level kTwDepth ahead
-        tw_stage<MODE>(t, sh, tid, q + kTwDepth < nlev ? entry(q + kTwDepth) : 0, q + kTwDepth < nlev, q + kTwDepth);
-    }
-    cp_wait_n<0>();  // nothing in flight into the slots the next sweep reuses
-    tw_bar();
-    if (tid == 0) {
-        if (timing && s_last >= s_first) {  // per tile: level-loop cycles, y waits, levels, sweeps
-            const unsigned long long loop = (unsigned long long)(clock64() - t_loop);
-            atomicAdd(timing + 9, loop);
-            atomicAdd(timing + 8, (unsigned long long)t_wait);
-            atomicAdd(timing + 10, (unsigned long long)(s_last - s_first + 1));
-            atomicAdd(timing + 11, 1ull);
-            if (nby < 0 && nbz < 0) {  // a tile that never waits: the bare level step
-                atomicAdd(timing + 12, loop);
-                atomicAdd(timing + 13, (unsigned long long)(s_last - s_first + 1));
-            }
+        const int last = (nlev - 1) % kTwGroup - kTwGroup;  // qout is a group past the last level's
+        if (owed && MODE == TW_FORWARD) qout[last * kTwLines] = result;
+        if (owed && MODE == TW_BACKWARD) {
+            a.z[at_p] = result;
+            if (a.exact_dots) a.prod[a.cinv[at_p]] = dmul(result, __ldcg(a.r + at_p));
         }
     }
-    if (timing && tid == 32 && s_last >= s_first) atomicAdd(timing + 15, (unsigned long long)t_wait);  // z waits
-    __syncthreads();  // the progress warp has published the final count and left
+    if (MODE != TW_BUILD && a.timing && tid == 0) {  // per tile: level-loop cycles, levels, sweeps
+        const unsigned long long loop = (unsigned long long)(clock64() - t_loop);
+        atomicAdd(a.timing + 9, loop);
+        atomicAdd(a.timing + 10, (unsigned long long)nlev);
+        atomicAdd(a.timing + 11, 1ull);
+        if (nby < 0 && nbz < 0) {  // a tile that never waits: the bare level step
+            atomicAdd(a.timing + 12, loop);
+            atomicAdd(a.timing + 13, (unsigned long long)nlev);
+        }
+    }
+    __syncthreads();  // the progress warps have published the final counts and left
 }
 
-// Every tile of this CTA: tiles blockIdx.x, blockIdx.x + gridDim.x, ... in
-// increasing order forward (each tile after its -y and -z neighbours) and in
-// decreasing order backward, so waits always point to tiles earlier in some
-// CTA's order and the earliest unfinished tile can always run.
+// Every tile of this CTA: entries blockIdx.x, blockIdx.x + gridDim.x, ... of
+// the tile list, in increasing order forward (each tile after its -y and -z
+// neighbours) and in decreasing order backward, so waits always point to tiles
+// earlier in some CTA's order and the earliest unfinished tile can always run.
 template <int MODE>
-__device__ bool tw_sweep_all(const TwArgs& t, TwShared& sh, int nlevels) {
-    const int G = (int)gridDim.x, b = (int)blockIdx.x;
+__device__ bool tw_sweep_all(const TwArgs& t, int nlevels, uint32_t& uses) {
+    const int G = (int)gridDim.x, b = (int)blockIdx.x, n = __ldcg(t.tlist);
     if (MODE == TW_BACKWARD) {
-        if (b < t.ntiles)
-            for (int tile = b + ((t.ntiles - 1 - b) / G) * G; tile >= 0; tile -= G) tw_sweep<MODE>(t, sh, tile, nlevels);
+        if (b < n)
+            for (int q = b + ((n - 1 - b) / G) * G; q >= 0; q -= G) tw_sweep<MODE>(t, __ldcg(t.tlist + 1 + q), nlevels, uses);
     } else {
-        for (int tile = b; tile < t.ntiles; tile += G) tw_sweep<MODE>(t, sh, tile, nlevels);
+        for (int q = b; q < n; q += G) tw_sweep<MODE>(t, __ldcg(t.tlist + 1 + q), nlevels, uses);
     }
     return !tw_failed(t);
 }
 
 // ---------------------------------------------------------------- the solve
+// s*As and As (apply_a, pressure.rs:400-439) of the dot tiles of this CTA: a
+// contiguous share, kTwBatch tiles at a time. Each third of the CTA takes
+// kTwBatch / 3 of them, a thread one cell of each (their loads are
+// independent); the products meet in shared memory and a warp per tile adds
+// them in the tree order (lane l: cells l, l+32, ...; then the xor tree).
+__device__ void tw_matvec(const TwArgs& t, uint32_t nf, uint32_t ntile) {
+    constexpr int kPer = kTwBatch / kTwThirds;
+    const PcgArgs& a = t.a;
+    double* const scratch = TW_SH.win;
+    const uint32_t per = (ntile + gridDim.x - 1) / gridDim.x;
+    const uint32_t t0 = min(blockIdx.x * per, ntile), t1 = min(t0 + per, ntile);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int third = threadIdx.x / kTile, tc = threadIdx.x % kTile;
+    for (uint32_t tb = t0; tb < t1; tb += kTwBatch) {
+        int2 nb[kPer][3];
+        double sv[kPer], dg[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const uint32_t tl = tb + third + q * kTwThirds, i = tl * kTile + tc;
+            const bool live = tl < t1 && i < nf;
+            const int2* nb2 = reinterpret_cast<const int2*>(a.nbr + (size_t)(live ? i : 0) * 6);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) nb[q][d] = live ? nb2[d] : make_int2(-1, -1);
+            sv[q] = live ? __ldcg(a.s + i) : 0.0;
+            dg[q] = live ? (double)a.diag[i] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const uint32_t tl = tb + third + q * kTwThirds, i = tl * kTile + tc;
+            const int nbv[6] = {nb[q][0].x, nb[q][0].y, nb[q][1].x, nb[q][1].y, nb[q][2].x, nb[q][2].y};
+            double nsv[6];
+#pragma unroll
+            for (int d = 0; d < 6; ++d) nsv[d] = nbv[d] >= 0 ? __ldcg(a.s + nbv[d]) : 0.0;
+            double v = dmul(dg[q], sv[q]);
+            v = nbv[NB_PX] >= 0 ? dsub(v, nsv[NB_PX]) : v;
+            v = nbv[NB_MX] >= 0 ? dsub(v, nsv[NB_MX]) : v;
+            v = nbv[NB_PY] >= 0 ? dsub(v, nsv[NB_PY]) : v;
+            v = nbv[NB_MY] >= 0 ? dsub(v, nsv[NB_MY]) : v;
+            v = nbv[NB_PZ] >= 0 ? dsub(v, nsv[NB_PZ]) : v;
+            v = nbv[NB_MZ] >= 0 ? dsub(v, nsv[NB_MZ]) : v;
+            if (tl < t1 && i < nf) {
+                a.as[i] = v;
+                if (a.exact_dots) a.prod[a.cinv[i]] = dmul(sv[q], v);
+            }
+            scratch[(tl - tb) * kTile + tc] = dmul(sv[q], v);
+        }
+        if (a.exact_dots) continue;
+        __syncthreads();
+        if (w < kTwBatch && tb + w < t1) {
+            double acc = 0.0;
+#pragma unroll
+            for (int u = 0; u < kTile / 32; ++u)
+                if ((tb + w) * kTile + u * 32 + lane < nf) acc = dadd(acc, scratch[w * kTile + u * 32 + lane]);
+            acc = warp_tree_sum(acc);
+            if (lane == 0) a.tpart[tb + w] = acc;
+        }
+        __syncthreads();
+    }
+}
+
+// dot(z, r) by the tiles of the tree order, a warp per tile.
+__device__ __forceinline__ void tw_dot_zr(const TwArgs& t, uint32_t nf, uint32_t ntile) {
+    const PcgArgs& a = t.a;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t tl = blockIdx.x * kTwWarps + (threadIdx.x >> 5); tl < ntile; tl += gridDim.x * kTwWarps) {
+        double zv[kTile / 32], rv[kTile / 32];
+#pragma unroll
+        for (int u = 0; u < kTile / 32; ++u) {
+            const uint32_t i = tl * kTile + lane + 32u * u;
+            zv[u] = i < nf ? __ldcg(a.z + i) : 0.0;
+            rv[u] = i < nf ? __ldcg(a.r + i) : 0.0;
+        }
+        double acc = 0.0;
+#pragma unroll
+        for (int u = 0; u < kTile / 32; ++u)
+            if (tl * kTile + lane + 32u * u < nf) acc = dadd(acc, dmul(zv[u], rv[u]));
+        acc = warp_tree_sum(acc);
+        if (lane == 0) a.tpart[tl] = acc;
+    }
+}
+
 // Launched cooperatively (every CTA resident at once).
-__global__ void __launch_bounds__(kTwBS, 2) k_pcg_tiles(TwArgs t) {
-    __shared__ TwShared sh;
+__global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) {
     const PcgArgs& a = t.a;
     const uint32_t nf = *a.nf;
     const uint32_t ntile = (nf + kTile - 1) / kTile;
     const uint32_t G = gridDim.x * kTwBS, gt = blockIdx.x * kTwBS + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const int gw = blockIdx.x * kTwWarps + (threadIdx.x >> 5), nw = gridDim.x * kTwWarps;
     const int nlevels = a.nlevels;
+    constexpr int kU = 4;  // cells a thread of the elementwise phases has in flight
     int parity = 0;
-    double residual = 0.0, sigma = 0.0;
+    double residual = 0.0, sigma = 0.0, alpha = 0.0;
+    bool owed = false;  // p has not had the last step's alpha * s
     // phase timers of CTA 0 (between grid barriers every CTA passes together)
     const bool timed = a.timing != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
     long long tck = timed ? clock64() : 0;
@@ -616,30 +879,34 @@ __global__ void __launch_bounds__(kTwBS, 2) k_pcg_tiles(TwArgs t) {
         }                                                            \
     } while (0)
     int iters = 0;
+    uint32_t uses = 0;  // rounds of the operand ring consumed (phases of op_full)
+    if (threadIdx.x < kTwGroups)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&TW_SH.op_full[threadIdx.x])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");  // before the first barrier below
     double mx = 0.0;
     for (uint32_t i = gt; i < nf; i += G) mx = fmax(mx, fabs(a.b[i]));
     for (uint32_t q = gt; q < (uint32_t)t.ntiles; q += G) {
         t.tlo[q] = INT32_MAX;
         t.thi[q] = -1;
     }
-    if (!tw_grid_max(t, sh, mx, parity, residual)) goto out;
+    if (!tw_grid_max(t, mx, parity, residual)) goto out;
     if (residual > a.tol) {
-        // r and p, the cell-order words, and the tiles' level ranges
+        // r and p, and the tiles' level ranges
         for (uint32_t i = gt; i < nf; i += G) {
             const uint32_t cell = a.lv_cell[i];
             const int ii = (int)(cell % (uint32_t)t.nx), jj = (int)((cell / (uint32_t)t.nx) % (uint32_t)t.ny),
                       kk = (int)(cell / ((uint32_t)t.nx * (uint32_t)t.ny));
-            t.icm_c[a.cinv[i]] = (uint32_t)ii | (uint32_t)a.nmask[i] << 16 | (uint32_t)a.diag[i] << 24;
             a.r[i] = a.b[i];
             a.p[i] = 0.0;
             const int tile = jj / kTwJ + (kk / kTwK) * t.tj;
             atomicMin(t.tlo + tile, ii + jj + kk);
             atomicMax(t.thi + tile, ii + jj + kk);
         }
-        if (!tw_grid_sync(t, sh)) goto out;
+        if (!tw_grid_sync(t)) goto out;
         // each tile's first row entry: a prefix over the tiles' level counts (one warp)
         if (blockIdx.x == 0 && threadIdx.x < 32) {
             unsigned long long run = 0;
+            int listed = 0;
             for (int b0 = 0; b0 < t.ntiles; b0 += 32) {
                 const int q = b0 + lane;
                 unsigned long long n = 0;
@@ -654,17 +921,24 @@ __global__ void __launch_bounds__(kTwBS, 2) k_pcg_tiles(TwArgs t) {
                     if (lane >= o) x += y;
                 }
                 if (q < t.ntiles) t.rbase[q] = (uint32_t)(run + x - n);
+                const unsigned some = __ballot_sync(0xffffffffu, n > 0);
+                if (n > 0) t.tlist[1 + listed + __popc(some & ((1u << lane) - 1u))] = q;
+                listed += __popc(some);
                 run += __shfl_sync(0xffffffffu, x, 31);
             }
             if (lane == 0) {
+                t.tlist[0] = listed;
                 t.rbase[t.ntiles] = (uint32_t)min(run, (unsigned long long)t.rows_cap);
                 if (run > (unsigned long long)t.rows_cap) atomicOr(t.err, kTwErrWait);  // cannot happen: sized per tile
             }
         }
-        if (!tw_grid_sync(t, sh)) goto out;
+        if (!tw_grid_sync(t)) goto out;
         {  // rows: every entry without a cell, then every cell's entry; every exchange entry unwritten
             const size_t nrow = __ldcg(t.rbase + t.ntiles);
-            for (size_t q = gt; q < nrow; q += G) t.icm[q] = kTwNoCell;
+            {
+                uint32_t* w2 = reinterpret_cast<uint32_t*>(t.word);  // two entries a store; nrow is a multiple of 256
+                for (size_t q = gt; q < nrow / 2; q += G) w2[q] = kTwNoCell | (uint32_t)kTwNoCell << 16;
+            }
             const size_t nex = nrow / kTwFace, xf = t.rows_cap / kTwFace;
             unsigned long long* ef = reinterpret_cast<unsigned long long*>(t.exf);
             unsigned long long* eb = reinterpret_cast<unsigned long long*>(t.exb);
@@ -675,7 +949,7 @@ __global__ void __launch_bounds__(kTwBS, 2) k_pcg_tiles(TwArgs t) {
                 eb[xf + q] = kTwEmpty;
             }
         }
-        if (!tw_grid_sync(t, sh)) goto out;
+        if (!tw_grid_sync(t)) goto out;
         for (uint32_t i = gt; i < nf; i += G) {
             const uint32_t cell = a.lv_cell[i];
             const int ii = (int)(cell % (uint32_t)t.nx), jj = (int)((cell / (uint32_t)t.nx) % (uint32_t)t.ny),
@@ -685,112 +959,104 @@ __global__ void __launch_bounds__(kTwBS, 2) k_pcg_tiles(TwArgs t) {
                              (size_t)(ii + jj + kk - __ldcg(t.tlo + tile)) * kTwLines +
                              (size_t)((kk % kTwK) * kTwJ + jj % kTwJ);
             if (e >= t.rows_cap) continue;  // cannot happen: the ranges were sized above
-            t.icm[e] = (uint32_t)ii | (uint32_t)a.nmask[i] << 16 | (uint32_t)a.diag[i] << 24;
-            t.rp[e].x = a.b[i];
+            t.word[e] = (uint16_t)(a.nmask[i] | a.diag[i] << 8);
+            t.idx[e] = i;
+            t.rr[e] = a.b[i];
             t.tpos[i] = (uint32_t)e;
         }
-        if (!tw_grid_sync(t, sh)) goto out;
-        if (!tw_sweep_all<TW_BUILD>(t, sh, nlevels)) goto out;
-        if (!tw_grid_sync(t, sh)) goto out;  // the factor's exchange planes are reused by the sweeps
+        if (!tw_grid_sync(t)) goto out;
+        if (!tw_sweep_all<TW_BUILD>(t, nlevels, uses)) goto out;
+        if (!tw_grid_sync(t)) goto out;  // the factor's exchange planes are reused by the sweeps
         TW_SECTION(0);
-        if (!tw_sweep_all<TW_FORWARD>(t, sh, nlevels)) goto out;
-        if (!tw_sweep_all<TW_BACKWARD>(t, sh, nlevels)) goto out;
+        if (!tw_sweep_all<TW_FORWARD>(t, nlevels, uses)) goto out;
+        if (!tw_sweep_all<TW_BACKWARD>(t, nlevels, uses)) goto out;
         // dot(z, r)
         if (a.exact_dots) {
-            if (!tw_exact_dot(t, sh, sigma)) goto out;
+            if (!tw_exact_dot(t, sigma)) goto out;
         } else {
-            if (!tw_grid_sync(t, sh)) goto out;
-            for (uint32_t tl = (uint32_t)gw; tl < ntile; tl += (uint32_t)nw) {
-                double acc = 0.0;
-                const uint32_t e = min((tl + 1) * kTile, nf);
-                for (uint32_t i = tl * kTile + lane; i < e; i += 32)
-                    acc = dadd(acc, dmul(__ldcg(t.zr + t.tpos[i]), __ldcg(a.r + i)));
-                acc = warp_tree_sum(acc);
-                if (lane == 0) a.tpart[tl] = acc;
-            }
-            if (!tw_grid_sync(t, sh)) goto out;
-            sigma = tw_tile_total(t, ntile, sh);
+            if (!tw_grid_sync(t)) goto out;
+            tw_dot_zr(t, nf, ntile);
+            if (!tw_grid_sync(t)) goto out;
+            sigma = tw_tile_total(t, ntile);
         }
-        for (uint32_t i = gt; i < nf; i += G) a.s[i] = __ldcg(t.zr + t.tpos[i]);
-        if (!tw_grid_sync(t, sh)) goto out;
+        for (uint32_t i = gt; i < nf; i += G) a.s[i] = __ldcg(a.z + i);
+        if (!tw_grid_sync(t)) goto out;
         for (int it = 0; it < a.max_iters; ++it) {
             iters = it + 1;
-            // apply_a (pressure.rs:400-439) and s*As, by the tiles of the tree dot
-            for (uint32_t tl = (uint32_t)gw; tl < ntile; tl += (uint32_t)nw) {
-                double acc = 0.0;
-                for (int u = 0; u < kTile / 32; ++u) {
-                    const uint32_t i = tl * kTile + lane + 32u * u;
-                    if (i >= nf) break;
-                    const int2* nb2 = reinterpret_cast<const int2*>(a.nbr + (size_t)i * 6);
-                    const int2 x0 = nb2[0], x1 = nb2[1], x2 = nb2[2];
-                    const int nbv[6] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y};
-                    const double sv = __ldcg(a.s + i);
-                    double nsv[6];
-#pragma unroll
-                    for (int d = 0; d < 6; ++d) nsv[d] = nbv[d] >= 0 ? __ldcg(a.s + nbv[d]) : 0.0;
-                    double v = dmul((double)a.diag[i], sv);
-                    if (nbv[NB_PX] >= 0) v = dsub(v, nsv[NB_PX]);
-                    if (nbv[NB_MX] >= 0) v = dsub(v, nsv[NB_MX]);
-                    if (nbv[NB_PY] >= 0) v = dsub(v, nsv[NB_PY]);
-                    if (nbv[NB_MY] >= 0) v = dsub(v, nsv[NB_MY]);
-                    if (nbv[NB_PZ] >= 0) v = dsub(v, nsv[NB_PZ]);
-                    if (nbv[NB_MZ] >= 0) v = dsub(v, nsv[NB_MZ]);
-                    a.as[i] = v;
-                    if (a.exact_dots) a.prod[a.cinv[i]] = dmul(sv, v);
-                    else acc = dadd(acc, dmul(sv, v));
-                }
-                if (!a.exact_dots) {
-                    acc = warp_tree_sum(acc);
-                    if (lane == 0) a.tpart[tl] = acc;
-                }
-            }
+            tw_matvec(t, nf, ntile);
             double denom;  // dot(s, As)
             if (a.exact_dots) {
-                if (!tw_exact_dot(t, sh, denom)) goto out;
+                if (!tw_exact_dot(t, denom)) goto out;
             } else {
-                if (!tw_grid_sync(t, sh)) goto out;
-                denom = tw_tile_total(t, ntile, sh);
+                if (!tw_grid_sync(t)) goto out;
+                denom = tw_tile_total(t, ntile);
             }
             TW_SECTION(3);
             if (fabs(denom) < 1e-30) break;
-            const double alpha = ddiv(sigma, denom);
+            alpha = ddiv(sigma, denom);
             double mr = 0.0;
-            for (uint32_t i = gt; i < nf; i += G) {
-                a.p[i] = dadd(a.p[i], dmul(alpha, __ldcg(a.s + i)));
-                const double rv = dsub(a.r[i], dmul(alpha, __ldcg(a.as + i)));
-                a.r[i] = rv;
-                t.rp[t.tpos[i]].x = rv;
-                mr = fmax(mr, fabs(rv));
+            for (uint32_t i0 = gt; i0 < nf; i0 += kU * G) {
+                double rv[kU], av[kU];
+                uint32_t e[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const uint32_t i = i0 + u * G;
+                    rv[u] = i < nf ? a.r[i] : 0.0;  // this thread's own store
+                    av[u] = i < nf ? __ldcg(a.as + i) : 0.0;
+                    e[u] = i < nf ? t.tpos[i] : 0u;
+                }
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const uint32_t i = i0 + u * G;
+                    if (i >= nf) break;
+                    const double nr = dsub(rv[u], dmul(alpha, av[u]));
+                    a.r[i] = nr;
+                    t.rr[e[u]] = nr;
+                    mr = fmax(mr, fabs(nr));
+                }
             }
-            if (!tw_grid_max(t, sh, mr, parity, residual)) goto out;  // also publishes r and rp.x
+            owed = true;  // p takes alpha * s with the next direction, which reads s too
+            if (!tw_grid_max(t, mr, parity, residual)) goto out;  // also publishes the residual rows
             TW_SECTION(5);
             if (residual <= a.tol) break;
-            if (!tw_sweep_all<TW_FORWARD>(t, sh, nlevels)) goto out;
-            if (!tw_sweep_all<TW_BACKWARD>(t, sh, nlevels)) goto out;
+            if (!tw_sweep_all<TW_FORWARD>(t, nlevels, uses)) goto out;
+            if (!tw_sweep_all<TW_BACKWARD>(t, nlevels, uses)) goto out;
             double sigma_new;  // dot(z, r)
             if (a.exact_dots) {
-                if (!tw_exact_dot(t, sh, sigma_new)) goto out;
+                if (!tw_exact_dot(t, sigma_new)) goto out;
             } else {
-                if (!tw_grid_sync(t, sh)) goto out;
-                for (uint32_t tl = (uint32_t)gw; tl < ntile; tl += (uint32_t)nw) {
-                    double acc = 0.0;
-                    const uint32_t e = min((tl + 1) * kTile, nf);
-                    for (uint32_t i = tl * kTile + lane; i < e; i += 32)
-                        acc = dadd(acc, dmul(__ldcg(t.zr + t.tpos[i]), __ldcg(a.r + i)));
-                    acc = warp_tree_sum(acc);
-                    if (lane == 0) a.tpart[tl] = acc;
-                }
-                if (!tw_grid_sync(t, sh)) goto out;
+                if (!tw_grid_sync(t)) goto out;
                 TW_SECTION(1);  // the sweeps end at this barrier
-                sigma_new = tw_tile_total(t, ntile, sh);
+                tw_dot_zr(t, nf, ntile);
+                if (!tw_grid_sync(t)) goto out;
+                sigma_new = tw_tile_total(t, ntile);
+                TW_SECTION(4);
             }
             const double beta = ddiv(sigma_new, sigma);
-            for (uint32_t i = gt; i < nf; i += G) a.s[i] = dadd(__ldcg(t.zr + t.tpos[i]), dmul(beta, a.s[i]));
-            if (!tw_grid_sync(t, sh)) goto out;  // s complete before the next matvec reads neighbours
+            for (uint32_t i0 = gt; i0 < nf; i0 += kU * G) {
+                double sv[kU], pv[kU], zv[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const uint32_t i = i0 + u * G;
+                    sv[u] = i < nf ? a.s[i] : 0.0;
+                    pv[u] = i < nf ? a.p[i] : 0.0;
+                    zv[u] = i < nf ? __ldcg(a.z + i) : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const uint32_t i = i0 + u * G;
+                    if (i >= nf) break;
+                    a.p[i] = dadd(pv[u], dmul(alpha, sv[u]));
+                    a.s[i] = dadd(zv[u], dmul(beta, sv[u]));
+                }
+            }
+            owed = false;
+            if (!tw_grid_sync(t)) goto out;  // s complete before the next matvec reads neighbours
             TW_SECTION(6);
             sigma = sigma_new;
         }
-        for (uint32_t i = gt; i < nf; i += G) a.p_dense[a.lv_cell[i]] = a.p[i];
+        for (uint32_t i = gt; i < nf; i += G)
+            a.p_dense[a.lv_cell[i]] = owed ? dadd(a.p[i], dmul(alpha, a.s[i])) : a.p[i];
     }
 out:
     TW_SECTION(7);

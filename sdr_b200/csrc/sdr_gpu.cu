@@ -455,11 +455,11 @@ struct sdr_solver {
     uint32_t last_nf = 0;           // fluid cells of the last solve (picks the kernel under SDR_PCG_AUTO)
     double* cl_slots = nullptr;     // CTA partials of the cluster kernels
     // whole-GPU tiled solve (k_pcg_tiles), allocated on first use
-    uint32_t *tw_icm = nullptr, *tw_icm_c = nullptr, *tw_tpos = nullptr, *tw_rbase = nullptr;
-    double2 *tw_rp = nullptr, *tw_qp = nullptr;
+    uint32_t *tw_idx = nullptr, *tw_tpos = nullptr, *tw_rbase = nullptr;
+    int* tw_list = nullptr;
+    uint16_t* tw_word = nullptr;
     size_t tw_rows = 0;  // row entries of the sweeps' operand rows
-    double *tw_z = nullptr, *tw_exf = nullptr, *tw_exb = nullptr,
-           *tw_slots = nullptr;
+    double *tw_r = nullptr, *tw_pc = nullptr, *tw_q = nullptr, *tw_exf = nullptr, *tw_exb = nullptr, *tw_slots = nullptr;
     int *tw_lo = nullptr, *tw_hi = nullptr;
     unsigned* tw_bar = nullptr;
     int tw_tj = 0, tw_tk = 0, tw_grid = 0;  // tiles along y and z; CTAs of the cooperative launch (0: not set up)
@@ -643,7 +643,7 @@ struct sdr_solver {
         dfree(lines_cnt, st); dfree(lv_cell, st); dfree(cflag, st); dfree(coff, st); dfree(level_start, st); dfree(pos_of_cell, st);
         dfree(nbr, st); dfree(corder, st); dfree(cinv, st); dfree(prod, st); dfree(frec, st); dfree(brec, st); dfree(chunk_start, st); dfree(diag, st); dfree(nmask, st);
         dfree(b, st); dfree(precon, st); dfree(p, st); dfree(r, st); dfree(z, st); dfree(s, st); dfree(as, st); dfree(q, st); dfree(pq, st);
-        dfree(tw_icm, st); dfree(tw_icm_c, st); dfree(tw_tpos, st); dfree(tw_rbase, st); dfree(tw_rp, st); dfree(tw_qp, st); dfree(tw_z, st); dfree(tw_exf, st); dfree(tw_exb, st); dfree(tw_slots, st); dfree(tw_lo, st);
+        dfree(tw_idx, st); dfree(tw_tpos, st); dfree(tw_list, st); dfree(tw_r, st); dfree(tw_word, st); dfree(tw_rbase, st); dfree(tw_pc, st); dfree(tw_q, st); dfree(tw_exf, st); dfree(tw_exb, st); dfree(tw_slots, st); dfree(tw_lo, st);
         dfree(tw_hi, st); dfree(tw_bar, st);
         dfree(rp_slots, st); dfree(rp_bar, st);
         dfree(partials, st); dfree(p_dense, st); dfree(cl_slots, st); dfree(rclaim, st); dfree(tpart, st); dfree(p2g_list, st);
@@ -914,15 +914,16 @@ struct sdr_solver {
         int coop = 0, nsm = 0, occ = 0;
         CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pcg_tiles, kTwBS, 0) != cudaSuccess) {
+        CK(cudaFuncSetAttribute(k_pcg_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTwSmem));
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pcg_tiles, kTwBS, kTwSmem) != cudaSuccess) {
             cudaGetLastError();
             occ = 0;
         }
-        if (!coop || occ < 1 || g.nx > INT16_MAX) {  // the sweeps keep i in 16 bits
+        if (!coop || occ < 1) {
             tw_grid = -1;
             return false;
         }
-        tw_grid = nsm * std::min(occ, 2);
+        tw_grid = nsm;
         tw_tj = (g.ny + kTwJ - 1) / kTwJ;
         tw_tk = (g.nz + kTwK - 1) / kTwK;
         const size_t nt = (size_t)tw_tj * tw_tk;
@@ -932,8 +933,9 @@ struct sdr_solver {
             tw_grid = -1;
             return false;
         }
-        dalloc(tw_icm, tw_rows, st); dalloc(tw_rp, tw_rows, st); dalloc(tw_qp, tw_rows, st); dalloc(tw_z, tw_rows, st);
-        dalloc(tw_icm_c, ncell, st); dalloc(tw_tpos, ncell, st); dalloc(tw_rbase, nt + 1, st);
+        dalloc(tw_idx, tw_rows, st); dalloc(tw_pc, tw_rows, st); dalloc(tw_q, tw_rows, st);
+        dalloc(tw_r, tw_rows, st); dalloc(tw_tpos, ncell, st); dalloc(tw_list, nt + 1, st);
+        dalloc(tw_word, tw_rows, st); dalloc(tw_rbase, nt + 1, st);
         // exchange planes: two faces of one entry per line and row level
         dalloc(tw_exf, 2 * (tw_rows / kTwFace), st); dalloc(tw_exb, 2 * (tw_rows / kTwFace), st);
         dalloc(tw_lo, nt, st); dalloc(tw_hi, nt, st);
@@ -947,9 +949,8 @@ struct sdr_solver {
         t.a = a;  // a.timing: the section timers of profiling level 2
         t.nx = g.nx; t.ny = g.ny; t.nz = g.nz;
         t.tj = tw_tj; t.tk = tw_tk; t.ntiles = tw_tj * tw_tk;
-        t.coff = coff;
-        t.icm = tw_icm; t.rp = tw_rp; t.qp = tw_qp; t.zr = tw_z;
-        t.icm_c = tw_icm_c; t.tpos = tw_tpos; t.rbase = tw_rbase; t.rows_cap = tw_rows;
+        t.word = tw_word; t.idx = tw_idx; t.rr = tw_r; t.pc = tw_pc; t.qr = tw_q; t.tpos = tw_tpos; t.tlist = tw_list;
+        t.rbase = tw_rbase; t.rows_cap = tw_rows;
         t.exf = tw_exf; t.exb = tw_exb;
         t.tlo = tw_lo; t.thi = tw_hi;
         t.bar = tw_bar;
@@ -957,7 +958,7 @@ struct sdr_solver {
         t.err = &dst->err;
         CK(cudaMemsetAsync(tw_bar, 0, 2 * sizeof(unsigned), st));  // a wound-down launch may leave arrivals
         void* args[] = {&t};
-        CK(cudaLaunchCooperativeKernel((const void*)k_pcg_tiles, dim3((unsigned)tw_grid), dim3(kTwBS), args, 0, st));
+        CK(cudaLaunchCooperativeKernel((const void*)k_pcg_tiles, dim3((unsigned)tw_grid), dim3(kTwBS), args, kTwSmem, st));
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
 
