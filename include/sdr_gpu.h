@@ -240,15 +240,15 @@ int sdr_solver_set_dot_order(sdr_solver* s, int reference_order);
  * the sweeps spread over all of them (large fluid regions). Both run the same
  * per-cell arithmetic (pressure.rs:341-609) and the same dot orders, so they
  * give the same pressure bits (with the reference dot order, the
- * reference's). SDR_PCG_TILES: the whole GPU in one cooperative launch; the
- * grid's (j, k) lines cut into tiles of 16 x 16, one CTA per tile walking the
- * levels of its cells, tiles handing boundary values to their neighbours
- * through exchange entries that mark their own readiness (large fluid regions
- * on a GPU of their own; the cluster kernel if the device cannot launch it).
- * SDR_PCG_AUTO (default): from 200,000 fluid cells in the previous solve
- * (before the first solve: the particle count over particles_per_cell) the
- * tiled solve, or the cluster with SDR_SOLVER_SHARED_GPU; below that one
- * block. */
+ * reference's). SDR_PCG_TILES: the grid's (j, k) lines cut into tiles of
+ * 16 x 16, one CTA per tile walking the levels of its cells, tiles handing
+ * boundary values to their neighbours through entries that mark their own
+ * readiness: one thread-block cluster where the grid has at most 16 tiles, else
+ * the whole GPU in one cooperative launch (the cluster kernel if the device
+ * cannot launch it). SDR_PCG_AUTO (default): the tiled solve on a GPU of its
+ * own; with SDR_SOLVER_SHARED_GPU one block, from 200,000 fluid cells in the
+ * previous solve (before the first solve: the particle count over
+ * particles_per_cell) the cluster. */
 enum { SDR_PCG_AUTO = 0, SDR_PCG_ONE_BLOCK = 1, SDR_PCG_CLUSTER = 2, SDR_PCG_TILES = 3 };
 int sdr_solver_set_pcg_kernel(sdr_solver* s, int kernel);
 /* CTAs of the SDR_PCG_ONE_BLOCK solve's cluster (CTA 0 runs the sweeps).

@@ -7,7 +7,7 @@
 // within a level every line has at most one cell (i = L - j - k), whose -x
 // predecessor is the thread's own previous cell (a register) and whose -y and
 // -z predecessors are the neighbouring lines' cells of level L-1. Those live
-// in a shared-memory window of kTwRing levels, one slot per line plus a halo
+// in a shared-memory window of two levels, one slot per line plus a halo
 // row and column for the cells of the neighbouring tiles. So a level costs one
 // barrier of the tile's threads, and tiles synchronise only with their two
 // upstream neighbours through exchange entries that mark their own readiness:
@@ -27,9 +27,9 @@
 // read. The operands (residual or forward result, factor, z's places) are rows
 // brought to shared memory by the bulk-copy engine, four levels to a copy, and
 // each thread reads its own of level s+1 while it computes level s. The loop is
-// unrolled over a copy's four levels, so most addresses are a constant away
-// from a register (unrolled over the whole window, a step took 700 cycles on
-// sweeps of 15 levels: the instructions themselves had to be fetched).
+// unrolled over a copy's four levels, so that addresses are a constant away
+// from a register (unrolled over 16 levels, a step took 700 cycles on sweeps of
+// 15 levels: the instructions themselves had to be fetched).
 //
 // Per cell the arithmetic is that of k_pcg / k_pcg_cluster (the same operands
 // in the same order), so the factor and both sweeps give the same bits, and so
@@ -40,18 +40,19 @@
 // its row; z goes straight to its place in wavefront order (the cells of a
 // tile row are neighbours there too, so a level's stores are runs of 128 bytes).
 //
-// Synchronisation: one cooperative launch (every CTA resident). Phases are
-// separated by a grid barrier (an arrival counter and a generation word,
-// release/acquire at GPU scope). In a sweep the 8 compute warps of a CTA share
-// a named barrier per level; two more warps, one per upstream face, poll the
-// upstream tiles' exchange entries and copy their values into the window's
-// halo, and one issues the operand copies, so compute threads never wait on a
-// global load. Only tiles with fluid cells take a CTA. Every wait gives up
-// after about a second (2^31 SM cycles) or as soon as another CTA has given
-// up, sets an error bit and lets the kernel wind down. The waits of a level (y
-// values, z values, operands) and the published progress belong to three clerk
-// warps that join its barrier: one release store or one try_wait on a compute
-// warp cost 90 cycles of every other level.
+// Synchronisation, grid form: one cooperative launch (every CTA resident),
+// phases separated by a grid barrier (an arrival counter and a generation word,
+// release/acquire at GPU scope), neighbour values through exchange planes in
+// global memory, polled by a progress warp per face. Cluster form, where the
+// grid has at most 16 tiles: one thread-block cluster, the hardware barrier,
+// neighbour values stored straight into the consumer's shared memory
+// (distributed shared memory, about a third of the hand-off through L2). In a
+// sweep the 8 compute warps share a named barrier per level with three clerk
+// warps, which have the level's y values, z values and operands ready before
+// they join: a release store, a try_wait or a poll on a compute warp cost
+// 90 cycles of every other level. Only tiles with fluid cells take a CTA.
+// Every wait gives up after about a second (2^31 SM cycles) or soon after
+// another CTA has given up, sets an error bit and lets the kernel wind down.
 #pragma once
 #include "pressure.cuh"
 
@@ -60,32 +61,35 @@ namespace sdr {
 constexpr int kTwJ = 16;                     // lines per tile along y
 constexpr int kTwK = 16;                     // lines per tile along z
 constexpr int kTwLines = kTwJ * kTwK;        // compute threads: one per line
-// Threads: the compute warps, a progress warp per upstream face, the operand
-// warp, three clerk warps (kTwBarrier threads share a level's barrier), and
-// more for the grid-wide phases (24 warps per SM keep enough loads in
-// flight; one CTA per SM makes the grid barrier half of what two cost).
+// Threads: the compute warps, three clerk warps (kTwBarrier threads share a
+// level's barrier), the operand warp, on the grid a progress warp per upstream
+// face, and more for
+// the grid-wide phases (24 warps per SM keep enough loads in flight; one CTA
+// per SM makes the grid barrier half of what two cost).
 constexpr int kTwBS = 768;
 constexpr int kTwBarrier = kTwLines + 96;
 constexpr int kTwWarps = kTwBS / 32;
-constexpr int kTwRing = 16;                  // levels the window holds (a power of two)
 constexpr int kTwPitch = kTwJ + 1;           // window slots per line row: the halo, then the tile's lines
 constexpr int kTwSlots = (kTwK + 1) * kTwPitch;  // window slots per level
-constexpr int kTwDepth = kTwRing;            // levels of operands in shared memory
+constexpr int kTwDepth = 16;                 // levels of operands in shared memory
 constexpr int kTwGroup = 4;                  // levels per bulk copy
 constexpr int kTwGroups = kTwDepth / kTwGroup;
+constexpr int kTwRing = 16;                  // levels of neighbour values staged ahead on the grid (a power of two)
 constexpr long long kTwWaitCycles = 1ll << 31;  // ~1.1 s at 1965 MHz
 constexpr uint32_t kTwErrWait = 16u;         // error bit: a sweep or barrier wait gave up
 constexpr uint16_t kTwNoCell = 0xFFFFu;      // a row entry without a fluid cell
 constexpr int kTwFace = 16;                  // lines of a tile face (either face)
 // Levels a progress-warp poll covers: two per load (the half-warps take
 // neighbouring levels), kTwPoll loads in flight.
-constexpr int kTwPoll = 3;
+constexpr int kTwPoll = 2;
 constexpr int kTwThirds = kTwBS / kTwLines;  // 256-thread groups of a CTA in the matvec
 constexpr int kTwBatch = 2 * kTwThirds;      // 256-cell dot tiles of the matvec a CTA has in flight
+constexpr int kTwScratch = 4096;             // doubles of scratch of the grid-wide phases
+constexpr int kTwClusterCtas = 16;           // most tiles the cluster form takes: one per CTA
 static_assert(kTwJ == kTwFace && kTwK == kTwFace, "both tile faces hold kTwFace lines");
-static_assert((kTwRing & (kTwRing - 1)) == 0, "the window's level is taken by a mask");
+static_assert((kTwRing & (kTwRing - 1)) == 0, "the ring's level is taken by a mask");
 static_assert(kTile == kTwLines, "the matvec takes one cell of a dot tile per compute thread");
-static_assert(kTwRing * kTwSlots >= kTwBatch * kTile, "the grid-wide phases use the window as scratch");
+static_assert(kTwScratch >= kTwBatch * kTile && kTwScratch % 32 == 0 && kTwScratch <= kTwDepth * kTwLines, "scratch");
 
 struct TwArgs {
     PcgArgs a;                   // wavefront-order vectors, tables and dots (as k_pcg)
@@ -101,6 +105,7 @@ struct TwArgs {
     uint32_t* tpos;              // wavefront index -> row entry of its cell
     uint32_t* rbase;             // per tile: its first row entry (ntiles + 1 entries)
     int* tlist;                  // the tiles with fluid cells in increasing order, after their number
+    int* trank;                  // per tile: its place in that list (-1: no fluid cell)
     size_t rows_cap;             // row entries allocated
     // Exchange planes, level-major like the rows: a tile's boundary values of
     // its q-th level (sweep order) at rbase[tile] / kTwFace + q * kTwFace + l,
@@ -113,17 +118,10 @@ struct TwArgs {
     unsigned* bar;               // grid barrier: [0] arrivals, [1] generation
     double* gslots;              // 2 x gridDim CTA partials of grid maxima
     uint32_t* err;               // error bits
+    int plane;                   // cluster form: levels of a halo plane (no tile has more)
 };
 
 // ---------------------------------------------------------------- memory-order helpers
-__device__ __forceinline__ unsigned long long ld_acquire_cta_sh(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(smem_addr(p)) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_cta_sh(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.release.cta.shared::cta.u64 [%0], %1;" ::"r"(smem_addr(p)), "l"(v) : "memory");
-}
 // Exchange-plane entries: written and polled with relaxed GPU-scope accesses.
 // kTwEmpty is a signalling-NaN pattern no arithmetic produces (IEEE results
 // are quiet NaNs), so it can mark an entry not yet written.
@@ -160,27 +158,59 @@ __device__ __forceinline__ bool tw_failed(const TwArgs& t) { return *(volatile u
 // Barrier of the compute and clerk warps (named barrier 1).
 __device__ __forceinline__ void tw_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kTwBarrier) : "memory"); }
 
+// A tile and its neighbours (-y, +y, -z, +z): level range, first row entry and
+// place in the tile list; an empty range where there is no fluid cell or no tile.
+struct TwSpan {
+    int lo, hi, rank;
+    uint32_t row0;
+};
 struct TwShared {
-    double win[kTwRing * kTwSlots];   // the last levels' values by window slot; scratch of the grid-wide phases
+    double win[2][kTwSlots];          // the last two levels' values by window slot
     // operand rows by level of the sweep mod kTwDepth (backward: the levels of a
     // group in decreasing place, as they lie in memory):
-    double op_a[kTwDepth][kTwLines];  // residual or forward result,
+    double op_a[kTwDepth][kTwLines];  // residual or forward result (and scratch of the grid-wide phases),
     double op_b[kTwDepth][kTwLines];  // factor,
     uint32_t op_i[kTwDepth][kTwLines];  // and wavefront index (backward)
     uint64_t op_full[kTwGroups];      // mbarriers: the group's rows have arrived
-    unsigned long long avail[2];      // levels (of the sweep) whose y / z neighbour values are in the window
-    long long mine;                   // the last level (of the sweep, from 0) whose barrier this tile has passed
+    double ring[2][kTwRing][kTwFace];  // grid form: the upstream tiles' values by level (kTwEmpty: none yet)
     double red[kTwWarps];
     int ok;
+    int passed;                       // the last level of a group whose barrier this tile has passed
+    int ntile, first;                 // tiles with fluid cells, and the first of this CTA's
+    int tile;                         // the tile `span` describes (-1: none)
+    TwSpan span[5];                   // it, then its -y, +y, -z, +z neighbours
     uint8_t m[2][kTwSlots];           // the factorisation's neighbour masks of the last two levels, by window slot
-    uint8_t ringm[2][kTwRing][kTwFace];  // the upstream neighbours' masks by level (factorisation)
 };
-constexpr size_t kTwSmem = sizeof(TwShared);
+// In the cluster form the upstream tiles write their boundary values straight
+// into this CTA's halo planes, behind TwShared: [direction][face][level][line].
+constexpr size_t kTwSmem = (sizeof(TwShared) + 127) / 128 * 128;
+constexpr size_t kTwMaxSmem = 227 * 1024;
+constexpr size_t tw_cluster_smem(int plane) { return kTwSmem + (size_t)4 * plane * kTwFace * sizeof(double); }
 extern __shared__ __align__(128) unsigned char tw_smem[];
 #define TW_SH (*reinterpret_cast<TwShared*>(tw_smem))
+__device__ __forceinline__ double* tw_plane(const TwArgs& t, int dir, int face) {
+    return reinterpret_cast<double*>(tw_smem + kTwSmem) + (size_t)(dir * 2 + face) * t.plane * kTwFace;
+}
+__device__ __forceinline__ double* tw_scratch() { return &TW_SH.op_a[0][0]; }
+__device__ __forceinline__ double lds_volatile(uint32_t a) {
+    double v;
+    asm volatile("ld.relaxed.cluster.shared::cta.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts_volatile(uint32_t a, unsigned long long v) {
+    asm volatile("st.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+__device__ __forceinline__ bool tw_empty(double v) { return __double_as_longlong(v) == (long long)kTwEmpty; }
 
-// Grid barrier; false if the wait gave up or another CTA has (the error bit is set).
+// Barrier over every CTA of the solve. Grid form: false if the wait gave up or
+// another CTA has (the error bit is set). Cluster form: the hardware barrier;
+// a solve whose sweeps gave up runs on to its end, in step, with the bit set.
+template <bool CL>
 __device__ bool tw_grid_sync(const TwArgs& t) {
+    if (CL) {
+        cluster_sync_all();
+        return true;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
@@ -222,12 +252,13 @@ __device__ __forceinline__ double tw_block_max(double v) {
 }
 
 // Maximum over the grid (order-free): CTA maxima through a double-buffered slot array.
+template <bool CL>
 __device__ bool tw_grid_max(const TwArgs& t, double v, int& parity, double& out) {
     const double bm = tw_block_max(v);
     double* sl = t.gslots + (size_t)parity * gridDim.x;
     parity ^= 1;
     if (threadIdx.x == 0) sl[blockIdx.x] = bm;
-    if (!tw_grid_sync(t)) return false;
+    if (!tw_grid_sync<CL>(t)) return false;
     if (threadIdx.x < 32) {
         double m = 0.0;
         for (unsigned q = threadIdx.x; q < gridDim.x; q += 32) m = fmax(m, __ldcg(sl + q));
@@ -246,8 +277,8 @@ __device__ bool tw_grid_max(const TwArgs& t, double v, int& parity, double& out)
 // One warp loading them from L2 itself took 7 us for the 4,650 sums of a
 // 1.19 M-cell pool, twice per iteration.
 __device__ double tw_tile_total(const TwArgs& t, uint32_t ntile) {
-    double* const scratch = TW_SH.win;
-    constexpr uint32_t kChunk = kTwRing * kTwSlots / 32 * 32;
+    double* const scratch = tw_scratch();
+    constexpr uint32_t kChunk = kTwScratch;
     double s = 0.0;
     for (uint32_t c0 = 0; c0 < ntile; c0 += kChunk) {
         const uint32_t n = min(kChunk, ntile - c0);
@@ -272,9 +303,10 @@ __device__ double tw_tile_total(const TwArgs& t, uint32_t ntile) {
 // The reference's chunked dot (pressure.rs:588-603) over `prod` in cell
 // order: one warp per 4096-cell chunk across the grid, then the chunk sums in
 // chunk order (as pcg_exact_dot).
+template <bool CL>
 __device__ bool tw_exact_dot(const TwArgs& t, double& out) {
     const PcgArgs& a = t.a;
-    if (!tw_grid_sync(t)) return false;  // products complete
+    if (!tw_grid_sync<CL>(t)) return false;  // products complete
     const int lane = threadIdx.x & 31;
     const int gw = blockIdx.x * kTwWarps + (threadIdx.x >> 5), nw = gridDim.x * kTwWarps;
     for (int ch = gw; ch < a.nchunks; ch += nw) {
@@ -300,7 +332,7 @@ __device__ bool tw_exact_dot(const TwArgs& t, double& out) {
         }
         if (lane == 0) a.partials[ch] = acc;
     }
-    if (!tw_grid_sync(t)) return false;
+    if (!tw_grid_sync<CL>(t)) return false;
     if (threadIdx.x == 0) {
         double s = -0.0;
         for (int ch = 0; ch < a.nchunks; ++ch) s = dadd(s, __ldcg(a.partials + ch));
@@ -317,73 +349,70 @@ enum { TW_BUILD = 0, TW_FORWARD = 1, TW_BACKWARD = 2 };
 
 // Line of window slot order `l` of a face: the backward sweep runs mirrored.
 __device__ __forceinline__ int tw_mirror(bool fwd, int l) { return fwd ? l : kTwFace - 1 - l; }
-// Window slots of the sweep's level q.
-__device__ __forceinline__ double* tw_win(int q) { return TW_SH.win + (q & (kTwRing - 1)) * kTwSlots; }
 
-// The progress warp of one face (0: y, 1: z) of a tile's sweep: it brings the
-// upstream tile's boundary values into the window's halo and publishes how
-// many levels are there. The values carry their own readiness: every
+// Which of a tile's levels take values from the upstream tile of a face, and
+// from where: level q (of the sweep, from 0) in [qa, qb) takes the upstream
+// tile's level q + shift.
+struct TwFeed {
+    int qa, qb, shift;
+    const TwSpan* up;
+};
+template <int MODE>
+__device__ __forceinline__ TwFeed tw_feed(int face) {
+    constexpr bool fwd = MODE != TW_BACKWARD;
+    const TwSpan& me = TW_SH.span[0];
+    TwFeed f;
+    f.up = &TW_SH.span[1 + 2 * face + (fwd ? 0 : 1)];
+    f.shift = (fwd ? me.lo - f.up->lo : f.up->hi - me.hi) - 1;
+    const int nlev = me.hi - me.lo + 1, np = f.up->hi - f.up->lo + 1;
+    f.qa = max(0, -f.shift);
+    f.qb = np > 0 ? min(nlev, np - f.shift) : 0;
+    return f;
+}
+
+// Grid form: the progress warp of one face (0: y, 1: z) of a tile's sweep. It
+// brings the upstream tile's boundary values into the shared ring, from which
+// the face's clerk takes them. The values carry their own readiness: every
 // entry of an exchange plane holds kTwEmpty until its producer writes it (the
 // planes are filled when the solve lays out its rows), a lane polls the entries
 // the next levels need (relaxed loads; lane l takes line l % 16, the upper
 // half-warp one level further), and resets each entry it staged to kTwEmpty
 // (the producer writes it again only in the next sweep of this direction,
-// after a grid barrier). So a hand-off costs the producer's store reaching L2
-// and one poll, with no progress flags and no GPU-scope fences. A level needs
-// no entry where the producer tile has no level before it (its range is in
-// tlo/thi) or the line lies outside the grid: the halo gets -0.0 there. The
-// factorisation also stages the upstream cell's neighbour mask from its row.
+// after a grid barrier). Ring entries work the same way: kTwEmpty until staged,
+// and again once the clerk has taken them. So a hand-off costs the producer's
+// store reaching L2 and one poll, with no progress flags and no fences.
 template <int MODE>
-__device__ void tw_progress_warp(const TwArgs& t, int face, int tile, int nb, int s_first, int nlev, int nlevels) {
+__device__ void tw_progress_warp(const TwArgs& t, int face) {
     constexpr bool fwd = MODE != TW_BACKWARD;
-    const int lane = threadIdx.x & 31;
-    const int J = tile % t.tj, K = tile / t.tj;
-    const int j0 = J * kTwJ, k0 = K * kTwK;
-    const int l = lane & 15, half = lane >> 4;
-    // this tile's boundary line
-    const int jl = face == 0 ? (fwd ? j0 : j0 + kTwJ - 1) : j0 + l;
-    const int kl = face == 0 ? k0 + l : (fwd ? k0 : k0 + kTwK - 1);
-    const bool line_ok = jl < t.ny && kl < t.nz;
-    const int lm = tw_mirror(fwd, l);
-    const int slot = face == 0 ? (lm + 1) * kTwPitch : lm + 1;
-    // the producer's entries of this line: level q of its sweep at src + q * kTwFace
-    double* src = (fwd ? t.exf : t.exb) + (face == 0 ? 0 : t.rows_cap / kTwFace) +
-                  (size_t)__ldcg(t.rbase + nb) / kTwFace + (size_t)l;
-    // the producer's levels before this tile's level q: its level q - 1 + shift, if within [0, np)
-    int np = 0, shift = 0;
-    if (line_ok) {
-        const int lo = __ldcg(t.tlo + nb), hi = __ldcg(t.thi + nb);
-        if (hi >= lo) {
-            np = hi - lo + 1;
-            shift = s_first - (fwd ? lo : nlevels - 1 - hi);
-        }
-    }
-    src += (ptrdiff_t)(shift - 1) * kTwFace;  // level q's entry: src + q * kTwFace
-    // and the upstream cell's word (forward: the producer's last line row or column)
-    const uint16_t* const words = t.word + (size_t)__ldcg(t.rbase + nb) + (ptrdiff_t)(shift - 1) * kTwLines +
-                                  (face == 0 ? l * kTwJ + kTwJ - 1 : (kTwK - 1) * kTwJ + l);
-    int next = 0;  // next level to stage
+    const TwFeed f = tw_feed<MODE>(face);
+    const int lane = threadIdx.x & 31, l = lane & 15, half = lane >> 4;
+    const int J = TW_SH.tile % t.tj, K = TW_SH.tile / t.tj;
+    const bool line_ok = face == 0 ? K * kTwK + l < t.nz : J * kTwJ + l < t.ny;
+    // the upstream tile's entries of this line: level q's at src + q * kTwFace
+    double* const src = (fwd ? t.exf : t.exb) + (face == 0 ? 0 : t.rows_cap / kTwFace) + f.up->row0 / kTwFace + l +
+                        (ptrdiff_t)f.shift * kTwFace;
+    const uint32_t ring = smem_addr(&TW_SH.ring[face][0][l]);
+    int next = f.qa;
     const long long t0 = clock64();
-    for (unsigned polls = 1; next < nlev; ++polls) {
-        const int mine = (int)(long long)ld_acquire_cta_sh(reinterpret_cast<unsigned long long*>(&TW_SH.mine));
-        const int lim = min(nlev, mine + kTwRing);  // window room: levels below lim
+    for (unsigned polls = 1; next < f.qb; ++polls) {
         // entries of levels next + half, next + 2 + half, ..., loaded at once
-        double v[kTwPoll];
-        uint16_t mk[kTwPoll];
+        double v[kTwPoll], room[kTwPoll];
         bool need[kTwPoll];
 #pragma unroll
         for (int u = 0; u < kTwPoll; ++u) {
             const int q = next + 2 * u + half;
-            need[u] = q < lim && (unsigned)(q - 1 + shift) < (unsigned)np;
-            if (MODE == TW_BUILD) mk[u] = need[u] ? __ldcg(words + (ptrdiff_t)q * kTwLines) : (uint16_t)0;
+            need[u] = line_ok && q < f.qb;
             v[u] = need[u] ? ld_relaxed_gpu_f64(src + (ptrdiff_t)q * kTwFace) : -0.0;
         }
-        int nr = 0;  // levels that are ready, in order: all 16 lines of each
+#pragma unroll
+        for (int u = 0; u < kTwPoll; ++u)
+            room[u] = lds_volatile(ring + ((next + 2 * u + half) & (kTwRing - 1)) * (kTwFace * 8));
+        int nr = 0;  // levels that are ready and have room, in order: all 16 lines of each
         bool open = true;
 #pragma unroll
         for (int u = 0; u < kTwPoll; ++u) {
-            const bool ok = next + 2 * u + half < lim &&
-                            !(need[u] && __double_as_longlong(v[u]) == (long long)kTwEmpty);
+            const int q = next + 2 * u + half;
+            const bool ok = q < f.qb && (!need[u] || (!tw_empty(v[u]) && tw_empty(room[u])));
             const unsigned b = __ballot_sync(0xffffffffu, ok);
             if (open && (b & 0xffffu) == 0xffffu) {
                 ++nr;
@@ -394,76 +423,89 @@ __device__ void tw_progress_warp(const TwArgs& t, int face, int tile, int nb, in
             }
         }
 #pragma unroll
-        for (int u = 0; u < kTwPoll; ++u) {
-            if (2 * u + half < nr) {
-                const int q = next + 2 * u + half;
-                tw_win(q - 1)[slot] = v[u];
-                if (MODE == TW_BUILD) TW_SH.ringm[face][q & (kTwRing - 1)][l] = (uint8_t)mk[u];
-            }
-        }
-        if (nr) {
-            __syncwarp();
-            if (lane == 0) st_release_cta_sh(&TW_SH.avail[face], (unsigned long long)(next + nr));
+        for (int u = 0; u < kTwPoll; ++u)
+            if (2 * u + half < nr && need[u])
+                sts_volatile(ring + ((next + 2 * u + half) & (kTwRing - 1)) * (kTwFace * 8),
+                             (unsigned long long)__double_as_longlong(v[u]));
 #pragma unroll
-            for (int u = 0; u < kTwPoll; ++u)
-                if (2 * u + half < nr && need[u])
-                    st_relaxed_gpu_u64(src + (ptrdiff_t)(next + 2 * u + half) * kTwFace, kTwEmpty);
-            next += nr;
-        }
+        for (int u = 0; u < kTwPoll; ++u)
+            if (2 * u + half < nr && need[u])
+                st_relaxed_gpu_u64(src + (ptrdiff_t)(next + 2 * u + half) * kTwFace, kTwEmpty);
+        next += nr;
         if ((polls & 63u) == 0u && __shfl_sync(0xffffffffu, (int)(tw_failed(t) || clock64() - t0 > kTwWaitCycles), 0)) {
-            if (lane == 0) {
-                atomicOr(t.err, kTwErrWait);
-                st_release_cta_sh(&TW_SH.avail[face], ~0ull >> 1);  // release this tile's compute warps
-            }
+            if (lane == 0) atomicOr(t.err, kTwErrWait);  // the clerk gives up by itself
             break;
         }
     }
 }
 
-// The operand warp (one lane): the rows of the sweep's levels, a group per
-// bulk copy, completing on the group's mbarrier. A group's place is free once
-// the barrier of its old last level has been passed (those operands were read
-// before it). Every group is issued even while the kernel winds down (groups
-// past the last level arrive without a copy, so that every sweep uses each
-// mbarrier equally often), and the compute threads wait for every group, so no
-// copy is in flight when the sweep ends.
-template <int MODE>
-__device__ void tw_operand_warp(const TwArgs& t, size_t row0, int nlev) {
-    asm volatile("fence.proxy.async;" ::: "memory");  // the rows were written by ordinary stores
+// The clerk of one face: before each level's barrier it puts the upstream
+// tile's values of the level into the window's halo (-0.0 where there are
+// none: beyond the upstream tile's levels or the grid's edge), from the ring or
+// the halo plane, and marks them taken. The wait is bounded; after it has given
+// up the halo gets whatever is there. The factorisation's neighbour masks come
+// from the upstream tile's rows.
+template <int MODE, bool CL>
+__device__ void tw_face_clerk(const TwArgs& t, int face) {
     constexpr bool fwd = MODE != TW_BACKWARD;
-    const long long t0 = clock64();
-    int passed = -1;
-    for (int q = 0; q < nlev || (q & (kTwDepth - 1)) != 0; q += kTwGroup) {
-        const uint32_t bar = smem_addr(&TW_SH.op_full[(q / kTwGroup) % kTwGroups]);
-        // a group past the last level only waits until its old use has been seen
-        const int until = q - kTwDepth + (q < nlev ? kTwGroup - 1 : 0);
-        for (unsigned spin = 1; passed < until; ++spin) {
-            passed = (int)(long long)ld_acquire_cta_sh(reinterpret_cast<unsigned long long*>(&TW_SH.mine));
-            if ((spin & 255u) == 0u && clock64() - t0 > 2 * kTwWaitCycles) {  // cannot happen: every level is passed
-                atomicOr(t.err, kTwErrWait);
-                return;
+    const TwFeed f = tw_feed<MODE>(face);
+    const int nlev = TW_SH.span[0].hi - TW_SH.span[0].lo + 1;
+    const int lane = threadIdx.x & 31, l = lane & 15;
+    const int J = TW_SH.tile % t.tj, K = TW_SH.tile / t.tj;
+    const bool mine = lane < kTwFace && (face == 0 ? K * kTwK + l < t.nz : J * kTwJ + l < t.ny);
+    const int lm = tw_mirror(fwd, l);
+    const int slot = face == 0 ? (lm + 1) * kTwPitch : lm + 1;
+    const uint32_t halo = smem_addr(&TW_SH.win[0][slot]);
+    const uint32_t src = CL ? smem_addr(tw_plane(t, fwd ? 0 : 1, face) + l) : smem_addr(&TW_SH.ring[face][0][l]);
+    const uint16_t* const words = t.word + (size_t)f.up->row0 + (ptrdiff_t)f.shift * kTwLines +
+                                  (face == 0 ? l * kTwJ + kTwJ - 1 : (kTwK - 1) * kTwJ + l);
+    bool given_up = false;
+    uint16_t wd[kTwGroup], wn[kTwGroup];
+    if (MODE == TW_BUILD) {
+#pragma unroll
+        for (int u = 0; u < kTwGroup; ++u) wd[u] = mine && u >= f.qa && u < f.qb ? __ldcg(words + u * kTwLines) : 0;
+    }
+    for (int q0 = 0; q0 < nlev; q0 += kTwGroup) {
+        if (MODE == TW_BUILD) {
+#pragma unroll
+            for (int u = 0; u < kTwGroup; ++u) {
+                const int q = q0 + kTwGroup + u;
+                wn[u] = mine && q >= f.qa && q < f.qb ? __ldcg(words + (ptrdiff_t)q * kTwLines) : 0;
             }
         }
-        if (q >= nlev) {
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-            continue;
+#pragma unroll
+        for (int u = 0; u < kTwGroup; ++u) {
+            const int q = q0 + u;
+            if (u > 0 && q >= nlev) break;
+            double v = -0.0;
+            if (q >= f.qa && q < f.qb) {
+                const uint32_t at = src + (CL ? q : q & (kTwRing - 1)) * (kTwFace * 8);
+                if (mine) v = lds_volatile(at);
+                if (!given_up && __any_sync(0xffffffffu, tw_empty(v))) {
+                    const long long t0 = clock64();
+                    for (unsigned spin = 1;; ++spin) {
+                        if (mine) v = lds_volatile(at);
+                        if (!__any_sync(0xffffffffu, tw_empty(v))) break;
+                        if ((spin & 255u) == 0u &&
+                            __shfl_sync(0xffffffffu, (int)(tw_failed(t) || clock64() - t0 > kTwWaitCycles), 0)) {
+                            if (lane == 0) atomicOr(t.err, kTwErrWait);
+                            given_up = true;
+                            break;
+                        }
+                    }
+                }
+                if (mine) sts_volatile(at, kTwEmpty);
+            }
+            if (lane < kTwFace) {
+                sts_f64(halo + ((u + 1) & 1) * (kTwSlots * 8), v);
+                if (MODE == TW_BUILD) TW_SH.m[(u + 1) & 1][slot] = wd[u] == kTwNoCell ? (uint8_t)0 : (uint8_t)wd[u];
+            }
+            tw_bar();
         }
-        const int n = min(kTwGroup, nlev - q);
-        const int at = (q & (kTwDepth - 1)) + (fwd ? 0 : kTwGroup - n);
-        const size_t e = row0 + (size_t)(fwd ? q : nlev - q - n) * kTwLines;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                     "r"((uint32_t)(n * kTwLines * (fwd ? 16 : 20)))
-                     : "memory");
-        auto copy = [&](void* dst, const void* src, uint32_t bytes) {
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    smem_addr(dst)),
-                "l"(src), "r"(bytes), "r"(bar)
-                : "memory");
-        };
-        copy(TW_SH.op_a[at], (fwd ? t.rr : t.qr) + e, (uint32_t)(n * kTwLines * 8));
-        copy(TW_SH.op_b[at], t.pc + e, (uint32_t)(n * kTwLines * 8));
-        if (!fwd) copy(TW_SH.op_i[at], t.idx + e, (uint32_t)(n * kTwLines * 4));
+        if (MODE == TW_BUILD) {
+#pragma unroll
+            for (int u = 0; u < kTwGroup; ++u) wd[u] = wn[u];
+        }
     }
 }
 
@@ -487,38 +529,65 @@ __device__ __forceinline__ void tw_op_wait(const TwArgs& t, int g, uint32_t pari
     }
 }
 
-// A clerk's wait until the window holds the neighbour values of level s;
-// returns the levels it holds.
-__device__ __forceinline__ int tw_wait(const TwArgs& t, int which, int s) {
-    unsigned long long have = ld_acquire_cta_sh(&TW_SH.avail[which]);
-    if (have <= (unsigned long long)s) {
-        const long long t0 = clock64();
-        for (unsigned spin = 1; (have = ld_acquire_cta_sh(&TW_SH.avail[which])) <= (unsigned long long)s; ++spin) {
-            if ((spin & 255u) == 0u && (tw_failed(t) || clock64() - t0 > kTwWaitCycles)) {
+// The operand warp (one lane): the rows of the sweep's levels, a group per
+// bulk copy, completing on the group's mbarrier. A group's place is free once
+// the barrier of its last level has been passed (those operands were read
+// before it). Groups past the last level arrive without a copy, so that every
+// sweep uses each mbarrier equally often. The compute warps and the operand
+// clerk wait for every group that has a copy, so none is in flight when the
+// sweep ends, also while the kernel winds down.
+template <int MODE>
+__device__ void tw_operand_warp(const TwArgs& t) {
+    constexpr bool fwd = MODE != TW_BACKWARD;
+    const int nlev = TW_SH.span[0].hi - TW_SH.span[0].lo + 1;
+    const size_t row0 = TW_SH.span[0].row0;
+    asm volatile("fence.proxy.async;" ::: "memory");  // the rows were written by ordinary stores
+    const long long t0 = clock64();
+    int passed = -1;  // levels whose barrier has been passed, told by the operand clerk group by group
+    for (int q = 0; q < nlev || (q & (kTwDepth - 1)) != 0; q += kTwGroup) {
+        for (unsigned spin = 1; passed < q - kTwDepth + kTwGroup - 1; ++spin) {
+            asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(passed) : "r"(smem_addr(&TW_SH.passed)) : "memory");
+            if ((spin & 255u) == 0u && clock64() - t0 > 2 * kTwWaitCycles) {  // cannot happen: every level is passed
                 atomicOr(t.err, kTwErrWait);
-                return INT32_MAX;
+                return;
             }
         }
+        const uint32_t bar = smem_addr(&TW_SH.op_full[(q / kTwGroup) % kTwGroups]);
+        if (q >= nlev) {
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+            continue;
+        }
+        const int n = min(kTwGroup, nlev - q);
+        const int at = (q & (kTwDepth - 1)) + (fwd ? 0 : kTwGroup - n);
+        const size_t e = row0 + (size_t)(fwd ? q : nlev - q - n) * kTwLines;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                     "r"((uint32_t)(n * kTwLines * (fwd ? 16 : 20)))
+                     : "memory");
+        auto copy = [&](void* dst, const void* src, uint32_t bytes) {
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                    smem_addr(dst)),
+                "l"(src), "r"(bytes), "r"(bar)
+                : "memory");
+        };
+        copy(TW_SH.op_a[at], (fwd ? t.rr : t.qr) + e, (uint32_t)(n * kTwLines * 8));
+        copy(TW_SH.op_b[at], t.pc + e, (uint32_t)(n * kTwLines * 8));
+        if (!fwd) copy(TW_SH.op_i[at], t.idx + e, (uint32_t)(n * kTwLines * 4));
     }
-    return (int)min(have, (unsigned long long)INT32_MAX);
 }
 
-// A clerk warp: it joins the barrier of every level once the level may begin.
-// Clerk 0 waits for the y neighbour's values, clerk 1 for the z neighbour's
-// and publishes the level passed, clerk 2 waits for the operand group of the
-// level after.
+// The operand clerk: it joins a level's barrier once the operands of the level
+// after it are there, and tells the operand warp of each group passed.
 template <int MODE>
-__device__ void tw_clerk_warp(const TwArgs& t, int clerk, int nb, int nlev, uint32_t parity0) {
-    int have = nb >= 0 ? 0 : INT32_MAX;
+__device__ void tw_operand_clerk(const TwArgs& t, uint32_t parity0) {
+    const int nlev = TW_SH.span[0].hi - TW_SH.span[0].lo + 1;
     for (int q = 0; q < nlev; ++q) {
-        if (clerk < 2) {
-            if (have <= q) have = tw_wait(t, clerk, q);
-        } else if (MODE != TW_BUILD && (q + 1) % kTwGroup == 0 && q + 1 < nlev) {
+        const bool group = MODE != TW_BUILD && (q + 1) % kTwGroup == 0;  // level q ends one
+        if (group && q + 1 < nlev)
             tw_op_wait(t, (q + 1) / kTwGroup % kTwGroups, (parity0 + (uint32_t)(q + 1) / kTwDepth) & 1u);
-        }
         tw_bar();
-        if (clerk == 1 && (threadIdx.x & 31) == 0)
-            st_release_cta_sh(reinterpret_cast<unsigned long long*>(&TW_SH.mine), (unsigned long long)(long long)q);
+        if (group && (threadIdx.x & 31) == 0)
+            asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_addr(&TW_SH.passed)), "r"(q) : "memory");
     }
 }
 
@@ -562,68 +631,109 @@ __device__ __forceinline__ double tw_factor(uint8_t m, double diag, double pxi, 
 // q = L^-1 r into qr. BACKWARD: z = L^-T q, plus the z*r products in cell
 // order for the reference dot order. `uses` counts the rounds of the operand
 // ring this CTA has consumed (the same in every thread).
-template <int MODE>
-__device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, int nlevels, uint32_t& uses) {
+template <int MODE, bool CL>
+__device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, uint32_t& uses) {
     const PcgArgs& a = t.a;
     const int tid = threadIdx.x;
-    const int J = tile % t.tj, K = tile / t.tj;
     constexpr bool fwd = MODE != TW_BACKWARD;
-    // upstream neighbours of this sweep
-    const int nby = fwd ? (J > 0 ? tile - 1 : -1) : (J + 1 < t.tj ? tile + 1 : -1);
-    const int nbz = fwd ? (K > 0 ? tile - t.tj : -1) : (K + 1 < t.tk ? tile + t.tj : -1);
-    const int lo = __ldcg(t.tlo + tile), hi = __ldcg(t.thi + tile);
-    const int s_first = fwd ? lo : nlevels - 1 - hi;  // the sweep's level 0
-    const int nlev = hi - lo + 1;
+    if (TW_SH.tile != tile) {  // the same in every thread; a CTA with one tile comes here once
+        __syncthreads();
+        if (tid < 5) {
+            const int J = tile % t.tj, K = tile / t.tj;
+            const int nb = tid == 0   ? tile
+                           : tid == 1 ? (J > 0 ? tile - 1 : -1)
+                           : tid == 2 ? (J + 1 < t.tj ? tile + 1 : -1)
+                           : tid == 3 ? (K > 0 ? tile - t.tj : -1)
+                                      : (K + 1 < t.tk ? tile + t.tj : -1);
+            TwSpan sp{1, 0, -1, 0u};
+            if (nb >= 0 && __ldcg(t.thi + nb) >= __ldcg(t.tlo + nb))
+                sp = TwSpan{__ldcg(t.tlo + nb), __ldcg(t.thi + nb), __ldcg(t.trank + nb), __ldcg(t.rbase + nb)};
+            TW_SH.span[tid] = sp;
+            if (tid == 0) TW_SH.tile = tile;
+        }
+        __syncthreads();
+    }
+    const int nlev = TW_SH.span[0].hi - TW_SH.span[0].lo + 1;
+    const size_t row0 = TW_SH.span[0].row0;
     // window slot of this thread's line; its predecessors are at slot - 1 and slot - kTwPitch
     const int lj = tid % kTwJ, lk = (tid / kTwJ) & (kTwK - 1);
     const int slot = (lk + 1) * kTwPitch + lj + 1;
-    if (tid == 0) {
-        TW_SH.mine = -1;
-        TW_SH.avail[0] = TW_SH.avail[1] = 0ull;
-    }
-    if (tid < kTwLines) {  // no value before the first level, nor beyond the grid's edge
-        tw_win(-1)[slot] = -0.0;
+    if (tid == 0) TW_SH.passed = -1;
+    if (tid < kTwLines) {  // no value before the first level
+        TW_SH.win[1][slot] = -0.0;
         if (MODE == TW_BUILD) TW_SH.m[1][slot] = 0;
-        if (nby < 0)
-            TW_SH.win[lj * kTwSlots + (lk + 1) * kTwPitch] = -0.0;  // (level, line) of kTwRing x kTwK
-        if (nbz < 0)
-            TW_SH.win[lk * kTwSlots + lj + 1] = -0.0;
     }
     __syncthreads();
-    const size_t row0 = (size_t)__ldcg(t.rbase + tile);
     const uint32_t parity0 = uses & 1u;
     if (MODE != TW_BUILD) uses += (uint32_t)(nlev + kTwDepth - 1) / kTwDepth;
     if (tid >= kTwLines) {
         const int w = (tid - kTwLines) >> 5;
-        if (w < 2) {
-            const int nb = w == 0 ? nby : nbz;
-            if (nb >= 0) tw_progress_warp<MODE>(t, w, tile, nb, s_first, nlev, nlevels);
-        } else if (w == 2) {
-            if (MODE != TW_BUILD && tid == kTwLines + 64) tw_operand_warp<MODE>(t, row0, nlev);
-        } else if (w < 6) {
-            tw_clerk_warp<MODE>(t, w - 3, w == 3 ? nby : w == 4 ? nbz : -1, nlev, parity0);
-        }
+        if (w < 2) tw_face_clerk<MODE, CL>(t, w);
+        else if (w == 2) tw_operand_clerk<MODE>(t, parity0);
+        else if (MODE != TW_BUILD && tid == kTwLines + 96) tw_operand_warp<MODE>(t);
+        else if (!CL && (w == 4 || w == 5)) tw_progress_warp<MODE>(t, w - 4);
         __syncthreads();
         return;
     }
     const int line = fwd ? tid : kTwLines - 1 - tid;  // the line this thread takes
-    const int j = J * kTwJ + line % kTwJ, k = K * kTwK + line / kTwJ;
-    // the lines on the downstream faces write an exchange entry at every level
-    // (-0.0 where the line has no fluid cell), so the downstream tile's
-    // progress warp finds every entry it polls written; level q's entry of
-    // face line l is ex + q * kTwFace
-    double* const ex_own = (fwd ? t.exf : t.exb) + row0 / kTwFace;
+    const int j = TW_SH.tile % t.tj * kTwJ + line % kTwJ, k = TW_SH.tile / t.tj * kTwK + line / kTwJ;
+    // The lines on the downstream faces pass every level's value on where the
+    // downstream tile has the level after it (-0.0 where the line has no fluid
+    // cell, so every entry that is waited for gets written): into their
+    // exchange plane, or into the downstream CTA's halo plane. Level q's entry
+    // of face line l is ex + q * kTwFace, for q in [xa, xa + xn).
     const bool in_grid = j < t.ny && k < t.nz;
-    const bool on_y = in_grid && lj == kTwJ - 1, on_z = in_grid && lk == kTwK - 1;
-    double* ex_y = ex_own + (size_t)(line / kTwJ);
-    double* ex_z = ex_own + t.rows_cap / kTwFace + (size_t)(line % kTwJ);
+    const TwSpan& dy = TW_SH.span[fwd ? 2 : 1];
+    const TwSpan& dz = TW_SH.span[fwd ? 4 : 3];
+    const int sy = fwd ? TW_SH.span[0].lo - dy.lo : dy.hi - TW_SH.span[0].hi;  // level q is its level q + sy
+    const int sz = fwd ? TW_SH.span[0].lo - dz.lo : dz.hi - TW_SH.span[0].hi;
+    const int ya = max(0, -1 - sy), yn = in_grid && lj == kTwJ - 1 ? max(min(nlev, dy.hi - dy.lo - sy) - ya, 0) : 0;
+    const int za = max(0, -1 - sz), zn = in_grid && lk == kTwK - 1 ? max(min(nlev, dz.hi - dz.lo - sz) - za, 0) : 0;
+    double *ex_y = nullptr, *ex_z = nullptr;
+    uint32_t rx_y = 0u, rx_z = 0u;
+    if (CL) {
+        auto remote = [&](const TwSpan& d, int face, int l, int sh) {
+            const uint32_t own = smem_addr(tw_plane(t, fwd ? 0 : 1, face) + l) + (uint32_t)((sh + 1) * (kTwFace * 8));
+            uint32_t r;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(own), "r"(max(d.rank, 0)));
+            return r;
+        };
+        rx_y = remote(dy, 0, line / kTwJ, sy);
+        rx_z = remote(dz, 1, line % kTwJ, sz);
+    } else {
+        double* const ex_own = (fwd ? t.exf : t.exb) + row0 / kTwFace;
+        ex_y = ex_own + (size_t)(line / kTwJ);
+        ex_z = ex_own + t.rows_cap / kTwFace + (size_t)(line % kTwJ);
+    }
+    // bit u of the masks: the group's level u is in the range
+    auto in_range = [](int q0, int first, int n) -> unsigned {
+        const int lo = min(max(first - q0, 0), kTwGroup), hi = min(max(first + n - q0, 0), kTwGroup);
+        return (1u << hi) - (1u << lo);
+    };
+    unsigned my_ = 0u, mz_ = 0u;
+    auto pass_on = [&](int u, double v) {
+        if (my_ >> u & 1u) {
+            if (CL) asm volatile("st.relaxed.cluster.shared::cluster.f64 [%0], %1;" ::"r"(rx_y + u * (kTwFace * 8)), "d"(v) : "memory");
+            else st_relaxed_gpu_f64(ex_y + u * kTwFace, v);
+        }
+        if (mz_ >> u & 1u) {
+            if (CL) asm volatile("st.relaxed.cluster.shared::cluster.f64 [%0], %1;" ::"r"(rx_z + u * (kTwFace * 8)), "d"(v) : "memory");
+            else st_relaxed_gpu_f64(ex_z + u * kTwFace, v);
+        }
+    };
+    auto next_group = [&] {
+        if (CL) {
+            rx_y += kTwGroup * kTwFace * 8;
+            rx_z += kTwGroup * kTwFace * 8;
+        } else {
+            ex_y += kTwGroup * kTwFace;
+            ex_z += kTwGroup * kTwFace;
+        }
+    };
     double carry = -0.0;  // the value of this line's previous cell (the -x / +x predecessor)
     const long long t_loop = a.timing && tid == 0 ? clock64() : 0;
-    // Shared-memory addresses: this line's place in the window by level of the
-    // ring, as byte offsets from one register.
-    constexpr uint32_t kLevel = kTwSlots * 8;
-    const uint32_t w_first = smem_addr(TW_SH.win) + (uint32_t)slot * 8;
-    uint32_t w = w_first, w_prev = w_first + (kTwRing - 1) * kLevel;
+    const uint32_t w0 = smem_addr(&TW_SH.win[0][slot]);
+    constexpr int kWin = kTwSlots * 8;  // level u of a group writes window u % 2 and reads the other
     if (MODE == TW_BUILD) {
         uint8_t carry_m = 0;
         const uint16_t* words = t.word + row0 + line;
@@ -632,6 +742,8 @@ __device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, int nlevels,
 #pragma unroll
         for (int u = 0; u < kTwGroup; ++u) wd[u] = u < nlev ? __ldcg(words + u * kTwLines) : kTwNoCell;
         for (int q0 = 0; q0 < nlev; q0 += kTwGroup) {
+            my_ = in_range(q0, ya, yn);
+            mz_ = in_range(q0, za, zn);
             words += kTwGroup * kTwLines;
 #pragma unroll
             for (int u = 0; u < kTwGroup; ++u)
@@ -642,30 +754,23 @@ __device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, int nlevels,
                 if (q >= nlev) break;  // the same in every thread
                 const uint8_t m = (uint8_t)wd[u];
                 tw_bar();
-                const double vy = lds_f64<-8>(w_prev), vz = lds_f64<-8 * kTwPitch>(w_prev);
+                const uint32_t wr = w0 + ((u + 1) & 1) * kWin;
+                const double vy = lds_f64<-8>(wr), vz = lds_f64<-8 * kTwPitch>(wr);
                 double pc = -0.0;
-                if (wd[u] != kTwNoCell) {
-                    const uint8_t my = lj == 0 ? TW_SH.ringm[0][q & (kTwRing - 1)][lk] : TW_SH.m[(u + 1) & 1][slot - 1];
-                    const uint8_t mz =
-                        lk == 0 ? TW_SH.ringm[1][q & (kTwRing - 1)][lj] : TW_SH.m[(u + 1) & 1][slot - kTwPitch];
-                    pc = tw_factor(m, (double)(wd[u] >> 8), carry, carry_m, vy, my, vz, mz);
-                }
-                sts_f64(w, pc);
+                if (wd[u] != kTwNoCell)
+                    pc = tw_factor(m, (double)(wd[u] >> 8), carry, carry_m, vy, TW_SH.m[(u + 1) & 1][slot - 1], vz,
+                                   TW_SH.m[(u + 1) & 1][slot - kTwPitch]);
+                sts_f64(w0 + (u & 1) * kWin, pc);
                 TW_SH.m[u & 1][slot] = wd[u] != kTwNoCell ? m : (uint8_t)0;
-                if (on_y) st_relaxed_gpu_f64(ex_y + u * kTwFace, pc);
-                if (on_z) st_relaxed_gpu_f64(ex_z + u * kTwFace, pc);
+                pass_on(u, pc);
                 pout[u * kTwLines] = pc;
                 carry = pc;
                 carry_m = m;
-                w_prev = w;
-                w += kLevel;
-                if (u == kTwGroup - 1 && w == w_first + kTwRing * kLevel) w = w_first;
             }
 #pragma unroll
             for (int u = 0; u < kTwGroup; ++u) wd[u] = wn[u];
             pout += kTwGroup * kTwLines;
-            ex_y += kTwGroup * kTwFace;
-            ex_z += kTwGroup * kTwFace;
+            next_group();
         }
     } else {
         tw_op_wait(t, 0, parity0);
@@ -686,11 +791,14 @@ __device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, int nlevels,
             const uint32_t gn = (uint32_t)(q0 / kTwGroup + 1) & (kTwGroups - 1);
             const uint32_t on = o_first + gn * (kTwGroup * kRow), oin = oi_first + gn * (kTwGroup * kRow / 2);
             const int left = nlev - q0;
+            my_ = in_range(q0, ya, yn);
+            mz_ = in_range(q0, za, zn);
 #pragma unroll
             for (int u = 0; u < kTwGroup; ++u) {
                 if (u > 0 && u >= left) break;  // the same in every thread
                 tw_bar();
-                const double vy = lds_f64<-8>(w_prev), vz = lds_f64<-8 * kTwPitch>(w_prev);
+                const uint32_t wr = w0 + ((u + 1) & 1) * kWin;
+                const double vy = lds_f64<-8>(wr), vz = lds_f64<-8 * kTwPitch>(wr);
                 // level q + 1's operands (past the last level: values nobody uses)
                 constexpr int kM = kTwGroup - 1;
                 const uint32_t os = (u < kM ? o : on) + (uint32_t)(((u + 1) & kM) ^ kRev) * kRow;
@@ -719,13 +827,9 @@ __device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, int nlevels,
                     result = zv;
                     at_p = at;
                 }
-                sts_f64(w, out);
+                sts_f64(w0 + (u & 1) * kWin, out);
+                pass_on(u, out);
                 owed = cell;
-                if (on_y) st_relaxed_gpu_f64(ex_y + u * kTwFace, out);
-                if (on_z) st_relaxed_gpu_f64(ex_z + u * kTwFace, out);
-                w_prev = w;
-                w += kLevel;
-                if (u == kTwGroup - 1 && w == w_first + kTwRing * kLevel) w = w_first;
                 carry = out;
                 ra = ra_n;
                 pc = pc_n;
@@ -734,8 +838,7 @@ __device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, int nlevels,
             o = on;
             oi = oin;
             qout += kTwGroup * kTwLines;
-            ex_y += kTwGroup * kTwFace;
-            ex_z += kTwGroup * kTwFace;
+            next_group();
         }
         const int last = (nlev - 1) % kTwGroup - kTwGroup;  // qout is a group past the last level's
         if (owed && MODE == TW_FORWARD) qout[last * kTwLines] = result;
@@ -749,28 +852,33 @@ __device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, int nlevels,
         atomicAdd(a.timing + 9, loop);
         atomicAdd(a.timing + 10, (unsigned long long)nlev);
         atomicAdd(a.timing + 11, 1ull);
-        if (nby < 0 && nbz < 0) {  // a tile that never waits: the bare level step
+        if (TW_SH.span[fwd ? 1 : 2].rank < 0 && TW_SH.span[fwd ? 3 : 4].rank < 0) {  // it never waits: the bare level step
             atomicAdd(a.timing + 12, loop);
             atomicAdd(a.timing + 13, (unsigned long long)nlev);
         }
     }
-    __syncthreads();  // the progress warps have published the final counts and left
+    __syncthreads();  // the clerks and progress warps are done
 }
 
 // Every tile of this CTA: entries blockIdx.x, blockIdx.x + gridDim.x, ... of
 // the tile list, in increasing order forward (each tile after its -y and -z
 // neighbours) and in decreasing order backward, so waits always point to tiles
 // earlier in some CTA's order and the earliest unfinished tile can always run.
-template <int MODE>
-__device__ bool tw_sweep_all(const TwArgs& t, int nlevels, uint32_t& uses) {
-    const int G = (int)gridDim.x, b = (int)blockIdx.x, n = __ldcg(t.tlist);
+template <int MODE, bool CL>
+__device__ bool tw_sweep_all(const TwArgs& t, uint32_t& uses) {
+    const int G = (int)gridDim.x, b = (int)blockIdx.x;
+    if (TW_SH.ntile <= G) {  // at most one tile each (always so in the cluster form)
+        if (b < TW_SH.ntile) tw_sweep<MODE, CL>(t, TW_SH.first, uses);
+        return CL || !tw_failed(t);
+    }
+    const int n = TW_SH.ntile;
     if (MODE == TW_BACKWARD) {
         if (b < n)
-            for (int q = b + ((n - 1 - b) / G) * G; q >= 0; q -= G) tw_sweep<MODE>(t, __ldcg(t.tlist + 1 + q), nlevels, uses);
+            for (int q = b + ((n - 1 - b) / G) * G; q >= 0; q -= G) tw_sweep<MODE, CL>(t, __ldcg(t.tlist + 1 + q), uses);
     } else {
-        for (int q = b; q < n; q += G) tw_sweep<MODE>(t, __ldcg(t.tlist + 1 + q), nlevels, uses);
+        for (int q = b; q < n; q += G) tw_sweep<MODE, CL>(t, __ldcg(t.tlist + 1 + q), uses);
     }
-    return !tw_failed(t);
+    return CL || !tw_failed(t);
 }
 
 // ---------------------------------------------------------------- the solve
@@ -782,7 +890,7 @@ __device__ bool tw_sweep_all(const TwArgs& t, int nlevels, uint32_t& uses) {
 __device__ void tw_matvec(const TwArgs& t, uint32_t nf, uint32_t ntile) {
     constexpr int kPer = kTwBatch / kTwThirds;
     const PcgArgs& a = t.a;
-    double* const scratch = TW_SH.win;
+    double* const scratch = tw_scratch();
     const uint32_t per = (ntile + gridDim.x - 1) / gridDim.x;
     const uint32_t t0 = min(blockIdx.x * per, ntile), t1 = min(t0 + per, ntile);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -855,14 +963,13 @@ __device__ __forceinline__ void tw_dot_zr(const TwArgs& t, uint32_t nf, uint32_t
     }
 }
 
-// Launched cooperatively (every CTA resident at once).
-__global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) {
+template <bool CL>
+__device__ __forceinline__ void tw_solve(const TwArgs& t) {
     const PcgArgs& a = t.a;
     const uint32_t nf = *a.nf;
     const uint32_t ntile = (nf + kTile - 1) / kTile;
     const uint32_t G = gridDim.x * kTwBS, gt = blockIdx.x * kTwBS + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const int nlevels = a.nlevels;
     constexpr int kU = 4;  // cells a thread of the elementwise phases has in flight
     int parity = 0;
     double residual = 0.0, sigma = 0.0, alpha = 0.0;
@@ -883,13 +990,20 @@ __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) {
     if (threadIdx.x < kTwGroups)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&TW_SH.op_full[threadIdx.x])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");  // before the first barrier below
+    if (threadIdx.x == 0) TW_SH.tile = -1;
+    if (CL) {  // nobody's values yet (before the barriers of the set-up)
+        unsigned long long* const pl = reinterpret_cast<unsigned long long*>(tw_plane(t, 0, 0));
+        for (int q = threadIdx.x; q < 4 * t.plane * kTwFace; q += kTwBS) pl[q] = kTwEmpty;
+    } else if (threadIdx.x < 2 * kTwRing * kTwFace) {
+        reinterpret_cast<unsigned long long*>(TW_SH.ring)[threadIdx.x] = kTwEmpty;
+    }
     double mx = 0.0;
     for (uint32_t i = gt; i < nf; i += G) mx = fmax(mx, fabs(a.b[i]));
     for (uint32_t q = gt; q < (uint32_t)t.ntiles; q += G) {
         t.tlo[q] = INT32_MAX;
         t.thi[q] = -1;
     }
-    if (!tw_grid_max(t, mx, parity, residual)) goto out;
+    if (!tw_grid_max<CL>(t, mx, parity, residual)) goto out;
     if (residual > a.tol) {
         // r and p, and the tiles' level ranges
         for (uint32_t i = gt; i < nf; i += G) {
@@ -902,7 +1016,7 @@ __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) {
             atomicMin(t.tlo + tile, ii + jj + kk);
             atomicMax(t.thi + tile, ii + jj + kk);
         }
-        if (!tw_grid_sync(t)) goto out;
+        if (!tw_grid_sync<CL>(t)) goto out;
         // each tile's first row entry: a prefix over the tiles' level counts (one warp)
         if (blockIdx.x == 0 && threadIdx.x < 32) {
             unsigned long long run = 0;
@@ -922,7 +1036,9 @@ __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) {
                 }
                 if (q < t.ntiles) t.rbase[q] = (uint32_t)(run + x - n);
                 const unsigned some = __ballot_sync(0xffffffffu, n > 0);
-                if (n > 0) t.tlist[1 + listed + __popc(some & ((1u << lane) - 1u))] = q;
+                const int at = listed + __popc(some & ((1u << lane) - 1u));
+                if (n > 0) t.tlist[1 + at] = q;
+                if (q < t.ntiles) t.trank[q] = n > 0 ? at : -1;
                 listed += __popc(some);
                 run += __shfl_sync(0xffffffffu, x, 31);
             }
@@ -932,24 +1048,28 @@ __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) {
                 if (run > (unsigned long long)t.rows_cap) atomicOr(t.err, kTwErrWait);  // cannot happen: sized per tile
             }
         }
-        if (!tw_grid_sync(t)) goto out;
+        if (!tw_grid_sync<CL>(t)) goto out;
         {  // rows: every entry without a cell, then every cell's entry; every exchange entry unwritten
             const size_t nrow = __ldcg(t.rbase + t.ntiles);
             {
                 uint32_t* w2 = reinterpret_cast<uint32_t*>(t.word);  // two entries a store; nrow is a multiple of 256
                 for (size_t q = gt; q < nrow / 2; q += G) w2[q] = kTwNoCell | (uint32_t)kTwNoCell << 16;
             }
+            if (threadIdx.x == 0) {
+                TW_SH.ntile = __ldcg(t.tlist);
+                TW_SH.first = (int)blockIdx.x < TW_SH.ntile ? __ldcg(t.tlist + 1 + blockIdx.x) : -1;
+            }
             const size_t nex = nrow / kTwFace, xf = t.rows_cap / kTwFace;
             unsigned long long* ef = reinterpret_cast<unsigned long long*>(t.exf);
             unsigned long long* eb = reinterpret_cast<unsigned long long*>(t.exb);
-            for (size_t q = gt; q < nex; q += G) {
+            for (size_t q = gt; !CL && q < nex; q += G) {
                 ef[q] = kTwEmpty;
                 ef[xf + q] = kTwEmpty;
                 eb[q] = kTwEmpty;
                 eb[xf + q] = kTwEmpty;
             }
         }
-        if (!tw_grid_sync(t)) goto out;
+        if (!tw_grid_sync<CL>(t)) goto out;
         for (uint32_t i = gt; i < nf; i += G) {
             const uint32_t cell = a.lv_cell[i];
             const int ii = (int)(cell % (uint32_t)t.nx), jj = (int)((cell / (uint32_t)t.nx) % (uint32_t)t.ny),
@@ -964,31 +1084,31 @@ __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) {
             t.rr[e] = a.b[i];
             t.tpos[i] = (uint32_t)e;
         }
-        if (!tw_grid_sync(t)) goto out;
-        if (!tw_sweep_all<TW_BUILD>(t, nlevels, uses)) goto out;
-        if (!tw_grid_sync(t)) goto out;  // the factor's exchange planes are reused by the sweeps
+        if (!tw_grid_sync<CL>(t)) goto out;
+        if (!tw_sweep_all<TW_BUILD, CL>(t, uses)) goto out;
+        if (!tw_grid_sync<CL>(t)) goto out;  // the factor's exchange planes are reused by the sweeps
         TW_SECTION(0);
-        if (!tw_sweep_all<TW_FORWARD>(t, nlevels, uses)) goto out;
-        if (!tw_sweep_all<TW_BACKWARD>(t, nlevels, uses)) goto out;
+        if (!tw_sweep_all<TW_FORWARD, CL>(t, uses)) goto out;
+        if (!tw_sweep_all<TW_BACKWARD, CL>(t, uses)) goto out;
         // dot(z, r)
         if (a.exact_dots) {
-            if (!tw_exact_dot(t, sigma)) goto out;
+            if (!tw_exact_dot<CL>(t, sigma)) goto out;
         } else {
-            if (!tw_grid_sync(t)) goto out;
+            if (!tw_grid_sync<CL>(t)) goto out;
             tw_dot_zr(t, nf, ntile);
-            if (!tw_grid_sync(t)) goto out;
+            if (!tw_grid_sync<CL>(t)) goto out;
             sigma = tw_tile_total(t, ntile);
         }
         for (uint32_t i = gt; i < nf; i += G) a.s[i] = __ldcg(a.z + i);
-        if (!tw_grid_sync(t)) goto out;
+        if (!tw_grid_sync<CL>(t)) goto out;
         for (int it = 0; it < a.max_iters; ++it) {
             iters = it + 1;
             tw_matvec(t, nf, ntile);
             double denom;  // dot(s, As)
             if (a.exact_dots) {
-                if (!tw_exact_dot(t, denom)) goto out;
+                if (!tw_exact_dot<CL>(t, denom)) goto out;
             } else {
-                if (!tw_grid_sync(t)) goto out;
+                if (!tw_grid_sync<CL>(t)) goto out;
                 denom = tw_tile_total(t, ntile);
             }
             TW_SECTION(3);
@@ -1016,19 +1136,19 @@ __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) {
                 }
             }
             owed = true;  // p takes alpha * s with the next direction, which reads s too
-            if (!tw_grid_max(t, mr, parity, residual)) goto out;  // also publishes the residual rows
+            if (!tw_grid_max<CL>(t, mr, parity, residual)) goto out;  // also publishes the residual rows
             TW_SECTION(5);
             if (residual <= a.tol) break;
-            if (!tw_sweep_all<TW_FORWARD>(t, nlevels, uses)) goto out;
-            if (!tw_sweep_all<TW_BACKWARD>(t, nlevels, uses)) goto out;
+            if (!tw_sweep_all<TW_FORWARD, CL>(t, uses)) goto out;
+            if (!tw_sweep_all<TW_BACKWARD, CL>(t, uses)) goto out;
             double sigma_new;  // dot(z, r)
             if (a.exact_dots) {
-                if (!tw_exact_dot(t, sigma_new)) goto out;
+                if (!tw_exact_dot<CL>(t, sigma_new)) goto out;
             } else {
-                if (!tw_grid_sync(t)) goto out;
+                if (!tw_grid_sync<CL>(t)) goto out;
                 TW_SECTION(1);  // the sweeps end at this barrier
                 tw_dot_zr(t, nf, ntile);
-                if (!tw_grid_sync(t)) goto out;
+                if (!tw_grid_sync<CL>(t)) goto out;
                 sigma_new = tw_tile_total(t, ntile);
                 TW_SECTION(4);
             }
@@ -1051,7 +1171,7 @@ __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) {
                 }
             }
             owed = false;
-            if (!tw_grid_sync(t)) goto out;  // s complete before the next matvec reads neighbours
+            if (!tw_grid_sync<CL>(t)) goto out;  // s complete before the next matvec reads neighbours
             TW_SECTION(6);
             sigma = sigma_new;
         }
@@ -1066,6 +1186,12 @@ out:
         *a.out_residual = residual;
         if (a.timing) a.timing[14] += 1;
     }
+    if (CL) cluster_sync_all();  // no CTA leaves while another may still write into its planes
 }
+
+// Launched cooperatively (every CTA resident at once), one CTA per SM.
+__global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) { tw_solve<false>(t); }
+// Launched as one cluster with a CTA per tile of the grid.
+__global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles_cluster(TwArgs t) { tw_solve<true>(t); }
 
 }  // namespace sdr

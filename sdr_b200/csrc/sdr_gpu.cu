@@ -77,7 +77,8 @@ struct Fail {
 inline unsigned blocks(size_t n, unsigned bs) { return (unsigned)std::max<size_t>(1, (n + bs - 1) / bs); }
 
 // Fluid cells from which SDR_PCG_AUTO solves on a cluster instead of one block
-// (the fluid count of the previous solve decides).
+// where the tiled solve is not available (shared GPU, or no cooperative
+// launch); the fluid count of the previous solve decides.
 constexpr uint32_t kClusterMinFluidCells = 200000;
 
 // CTAs in the cluster of a one-cluster kernel, once per device and kernel:
@@ -86,7 +87,7 @@ constexpr uint32_t kClusterMinFluidCells = 200000;
 template <class Kern>
 int cluster_ctas(Kern kernel, int slot, int threads, int device, size_t dyn_smem = 0) {
     static std::mutex mu;
-    static int ctas[3][64] = {};
+    static int ctas[4][64] = {};
     if (device < 0 || device >= 64) throw Fail{SDR_ERR_CUDA, "device index out of range"};
     std::lock_guard<std::mutex> lk(mu);
     if (!ctas[slot][device]) {
@@ -456,7 +457,8 @@ struct sdr_solver {
     double* cl_slots = nullptr;     // CTA partials of the cluster kernels
     // whole-GPU tiled solve (k_pcg_tiles), allocated on first use
     uint32_t *tw_idx = nullptr, *tw_tpos = nullptr, *tw_rbase = nullptr;
-    int* tw_list = nullptr;
+    int *tw_list = nullptr, *tw_rank = nullptr;
+    int tw_cluster = 0;  // CTAs of the tiled solve's cluster form (0: the grid form)
     uint16_t* tw_word = nullptr;
     size_t tw_rows = 0;  // row entries of the sweeps' operand rows
     double *tw_r = nullptr, *tw_pc = nullptr, *tw_q = nullptr, *tw_exf = nullptr, *tw_exb = nullptr, *tw_slots = nullptr;
@@ -643,7 +645,7 @@ struct sdr_solver {
         dfree(lines_cnt, st); dfree(lv_cell, st); dfree(cflag, st); dfree(coff, st); dfree(level_start, st); dfree(pos_of_cell, st);
         dfree(nbr, st); dfree(corder, st); dfree(cinv, st); dfree(prod, st); dfree(frec, st); dfree(brec, st); dfree(chunk_start, st); dfree(diag, st); dfree(nmask, st);
         dfree(b, st); dfree(precon, st); dfree(p, st); dfree(r, st); dfree(z, st); dfree(s, st); dfree(as, st); dfree(q, st); dfree(pq, st);
-        dfree(tw_idx, st); dfree(tw_tpos, st); dfree(tw_list, st); dfree(tw_r, st); dfree(tw_word, st); dfree(tw_rbase, st); dfree(tw_pc, st); dfree(tw_q, st); dfree(tw_exf, st); dfree(tw_exb, st); dfree(tw_slots, st); dfree(tw_lo, st);
+        dfree(tw_idx, st); dfree(tw_tpos, st); dfree(tw_list, st); dfree(tw_rank, st); dfree(tw_r, st); dfree(tw_word, st); dfree(tw_rbase, st); dfree(tw_pc, st); dfree(tw_q, st); dfree(tw_exf, st); dfree(tw_exb, st); dfree(tw_slots, st); dfree(tw_lo, st);
         dfree(tw_hi, st); dfree(tw_bar, st);
         dfree(rp_slots, st); dfree(rp_bar, st);
         dfree(partials, st); dfree(p_dense, st); dfree(cl_slots, st); dfree(rclaim, st); dfree(tpart, st); dfree(p2g_list, st);
@@ -843,17 +845,22 @@ struct sdr_solver {
             SLAUNCH(k_pcg, 1, kPcgBS, kPcgSmem, st, a);
             return;
         }
-        // fluid cells of the last solve; before the first one, the cells the
-        // particles fill at particles_per_cell each
-        const uint64_t nf_hint =
-            last_nf ? (uint64_t)last_nf : (uint64_t)n / std::max<uint64_t>(fluid.particles_per_cell, 1);
-        const bool large = pcg_kernel == SDR_PCG_AUTO && nf_hint >= kClusterMinFluidCells && !shared_gpu;
-        if ((pcg_kernel == SDR_PCG_TILES || large) && tiles_ready()) {
+        // A GPU of its own: the tiled solve at every size. Against k_pcg on an
+        // 8-CTA cluster it takes (us per iteration, B200) 16 instead of 22 at
+        // 320 fluid cells of a 21x22x17 grid, 30 instead of 63 at 10,000 cells
+        // (both cluster form), 28 instead of 37 at 340 cells and 58 instead of
+        // 292 at 77,000 cells of a 104x109x81 grid (grid form).
+        const bool tiles = pcg_kernel == SDR_PCG_TILES || (pcg_kernel == SDR_PCG_AUTO && !shared_gpu);
+        if (tiles && tiles_ready()) {
             launch_tiles(a);
             if (profiling) prof.pcg_tile_launches += 1;
             return;
         }
-        const bool cluster = pcg_kernel == SDR_PCG_CLUSTER || pcg_kernel == SDR_PCG_TILES || large ||
+        // fluid cells of the last solve; before the first one, the cells the
+        // particles fill at particles_per_cell each
+        const uint64_t nf_hint =
+            last_nf ? (uint64_t)last_nf : (uint64_t)n / std::max<uint64_t>(fluid.particles_per_cell, 1);
+        const bool cluster = pcg_kernel == SDR_PCG_CLUSTER || pcg_kernel == SDR_PCG_TILES ||
                              (pcg_kernel == SDR_PCG_AUTO && nf_hint >= kClusterMinFluidCells);
         if (cluster) {
             // One cluster of up to 16 CTAs (one per SM); the levels of each
@@ -905,9 +912,10 @@ struct sdr_solver {
         return true;
     }
 
-    // The whole-GPU tiled solve needs a cooperative launch with every CTA
-    // resident; its buffers are allocated on first use. False if the device
-    // cannot run it (then the cluster kernel solves).
+    // The tiled solve needs a cluster with a CTA per tile (grids of up to 16
+    // tiles), else a cooperative launch with every CTA resident; its buffers are
+    // allocated on first use. False if the device cannot run it (then k_pcg or
+    // the cluster kernel solves).
     bool tiles_ready() {
         if (tw_grid < 0) return false;
         if (tw_grid > 0) return true;
@@ -927,6 +935,15 @@ struct sdr_solver {
         tw_tj = (g.ny + kTwJ - 1) / kTwJ;
         tw_tk = (g.nz + kTwK - 1) / kTwK;
         const size_t nt = (size_t)tw_tj * tw_tk;
+        // The cluster form holds a CTA per tile and halo planes of a tile's most
+        // levels in shared memory.
+        const size_t csmem = tw_cluster_smem(tw_plane_levels());
+        if (nt <= (size_t)kTwClusterCtas && csmem <= kTwMaxSmem) {
+            CK(cudaFuncSetAttribute(k_pcg_tiles_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTwMaxSmem));
+            const int most = cluster_ctas(k_pcg_tiles_cluster, 3, kTwBS, device, kTwMaxSmem);
+            const int want = nt <= 8 ? 8 : kTwClusterCtas;
+            tw_cluster = want <= most ? want : 0;
+        }
         // operand rows: a tile's levels span at most nx + kTwJ + kTwK - 2 of them
         tw_rows = nt * (size_t)(g.nx + kTwJ + kTwK) * (size_t)kTwLines;
         if (tw_rows >= (size_t)UINT32_MAX) {  // row entries are 32-bit
@@ -934,7 +951,7 @@ struct sdr_solver {
             return false;
         }
         dalloc(tw_idx, tw_rows, st); dalloc(tw_pc, tw_rows, st); dalloc(tw_q, tw_rows, st);
-        dalloc(tw_r, tw_rows, st); dalloc(tw_tpos, ncell, st); dalloc(tw_list, nt + 1, st);
+        dalloc(tw_r, tw_rows, st); dalloc(tw_tpos, ncell, st); dalloc(tw_list, nt + 1, st); dalloc(tw_rank, nt, st);
         dalloc(tw_word, tw_rows, st); dalloc(tw_rbase, nt + 1, st);
         // exchange planes: two faces of one entry per line and row level
         dalloc(tw_exf, 2 * (tw_rows / kTwFace), st); dalloc(tw_exb, 2 * (tw_rows / kTwFace), st);
@@ -944,18 +961,25 @@ struct sdr_solver {
         return true;
     }
 
+    int tw_plane_levels() const { return g.nx + kTwJ + kTwK; }
+
     void launch_tiles(const PcgArgs& a) {
         TwArgs t{};
         t.a = a;  // a.timing: the section timers of profiling level 2
         t.nx = g.nx; t.ny = g.ny; t.nz = g.nz;
         t.tj = tw_tj; t.tk = tw_tk; t.ntiles = tw_tj * tw_tk;
-        t.word = tw_word; t.idx = tw_idx; t.rr = tw_r; t.pc = tw_pc; t.qr = tw_q; t.tpos = tw_tpos; t.tlist = tw_list;
+        t.word = tw_word; t.idx = tw_idx; t.rr = tw_r; t.pc = tw_pc; t.qr = tw_q; t.tpos = tw_tpos; t.tlist = tw_list; t.trank = tw_rank;
         t.rbase = tw_rbase; t.rows_cap = tw_rows;
         t.exf = tw_exf; t.exb = tw_exb;
         t.tlo = tw_lo; t.thi = tw_hi;
         t.bar = tw_bar;
         t.gslots = tw_slots;
         t.err = &dst->err;
+        t.plane = tw_plane_levels();
+        if (tw_cluster > 0) {
+            launch_one_cluster_smem(k_pcg_tiles_cluster, tw_cluster, kTwBS, tw_cluster_smem(t.plane), st, t);
+            return;
+        }
         CK(cudaMemsetAsync(tw_bar, 0, 2 * sizeof(unsigned), st));  // a wound-down launch may leave arrivals
         void* args[] = {&t};
         CK(cudaLaunchCooperativeKernel((const void*)k_pcg_tiles, dim3((unsigned)tw_grid), dim3(kTwBS), args, kTwSmem, st));
