@@ -2199,9 +2199,10 @@ int sdr_sdf_mesh_grid(const double* tris, size_t ntri, double dx, double padding
         require(tris && ntri && origin && dims && dx > 0, "bad argument");
         double mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
         for (size_t v = 0; v < 3 * ntri; ++v)
-            for (int c = 0; c < 3; ++c) {
-                mn[c] = std::fmin(mn[c], tris[3 * v + c]);
-                mx[c] = std::fmax(mx[c], tris[3 * v + c]);
+            for (int c = 0; c < 3; ++c) {  // as fmin and fmax: a NaN coordinate is passed over
+                const double x = tris[3 * v + c];
+                mn[c] = x < mn[c] ? x : mn[c];
+                mx[c] = x > mx[c] ? x : mx[c];
             }
         for (int c = 0; c < 3; ++c) {
             mn[c] -= padding;
@@ -2221,27 +2222,78 @@ int sdr_sdf_from_mesh(const double* tris, size_t ntri, sdr_vec3 origin, double d
         check_device();
         const uint32_t skip = g_fault == SDR_FAULT_SDF_STAGING ? 0u : kNoSkip;
         g_fault = 0;
-        uint32_t ntiles = (uint32_t)((ntri + kSdfTile - 1) / kSdfTile);
-        size_t padded = (size_t)ntiles * kSdfTile * 9;
-        double *dt = nullptr, *dout = nullptr;
-        uint32_t* derr = nullptr;
+        const uint32_t ntiles = (uint32_t)((ntri + kSdfTile - 1) / kSdfTile);
+        const size_t padded = (size_t)ntiles * kSdfTile * 9;
+        // The closed-mesh path takes three times the memory: up to 2^28 nodes
+        // (6.7 GB), and only where the device has it.
+        bool fast = nn <= (size_t)1 << 28 && skip == kNoSkip;
+        // one block: the triangles, the field and the closed-mesh path's arrays
+        size_t bytes = 0;
+        auto room = [&](size_t n) {
+            const size_t at = bytes;
+            bytes += (n + 255) / 256 * 256;
+            return at;
+        };
+        const size_t o_tri = room(padded * 8), o_out = room(nn * 8), o_flags = room(64);
+        const size_t least = bytes;
+        const size_t ntri_b = (size_t)blocks(ntri, 256) * 256;  // k_sdf_balls writes whole blocks
+        const size_t o_ball = fast ? room(ntri_b * sizeof(float4)) : 0, o_group = fast ? room(ntri_b / 32 * sizeof(float4)) : 0,
+                     o_vert = fast ? room(ntri * 3 * sizeof(float4)) : 0, o_dist = fast ? room(nn * 8) : 0,
+                     o_up = fast ? room(nn * 4) : 0, o_roots = fast ? room((nn + 1) * 4) : 0, o_in = fast ? room(nn) : 0;
+        unsigned char* dev = nullptr;
         cudaStream_t st = nullptr;
         auto cleanup = [&] {
-            if (dt) cudaFree(dt);
-            if (dout) cudaFree(dout);
-            if (derr) cudaFree(derr);
+            if (dev) cudaFreeAsync(dev, st);
             if (st) cudaStreamDestroy(st);
         };
         try {
             CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-            CK(cudaMalloc((void**)&dt, padded * 8));
-            CK(cudaMalloc((void**)&dout, nn * 8));
-            CK(cudaMalloc((void**)&derr, 4));
-            CK(cudaMemsetAsync(dt, 0, padded * 8, st));
-            CK(cudaMemsetAsync(derr, 0, 4, st));
+            try {
+                dalloc(dev, bytes, st);
+            } catch (const Fail& e) {
+                if (!fast || e.code != SDR_ERR_OOM) throw;
+                cudaGetLastError();
+                fast = false;
+                dalloc(dev, least, st);
+            }
+            double *dt = (double*)(dev + o_tri), *dout = (double*)(dev + o_out);
+            // flags: edge sums and extent (24 bytes), error word, gate, number of roots
+            unsigned long long* acc = (unsigned long long*)(dev + o_flags);
+            uint32_t *derr = (uint32_t*)(acc + 3), *gate = derr + 1;
+            if (padded > ntri * 9) CK(cudaMemsetAsync(dt + ntri * 9, 0, (padded - ntri * 9) * 8, st));
+            CK(cudaMemsetAsync(acc, 0, 64, st));
             CK(cudaMemcpyAsync(dt, tris, ntri * 72, cudaMemcpyHostToDevice, st));
+            if (fast) {
+                SdfFast f{};
+                f.tris = dt;
+                f.ntri = (uint32_t)ntri;
+                f.ox = origin.x; f.oy = origin.y; f.oz = origin.z; f.dx = dx;
+                f.nx = (int)dims[0]; f.ny = (int)dims[1]; f.nz = (int)dims[2];
+                f.cx = origin.x + 0.5 * (double)(dims[0] - 1) * dx;
+                f.cy = origin.y + 0.5 * (double)(dims[1] - 1) * dx;
+                f.cz = origin.z + 0.5 * (double)(dims[2] - 1) * dx;
+                f.acc = acc;
+                f.gate = gate;
+                f.ball = (float4*)(dev + o_ball);
+                f.group = (float4*)(dev + o_group);
+                f.vert = (float4*)(dev + o_vert);
+                f.dist = (double*)(dev + o_dist);
+                f.up = (uint32_t*)(dev + o_up);
+                f.roots = (uint32_t*)(dev + o_roots);
+                f.inside = dev + o_in;
+                f.out = dout;
+                CK(cudaMemsetAsync(f.roots, 0, 4, st));
+                const size_t bx = (dims[0] + kSdfB - 1) / kSdfB, by = (dims[1] + kSdfB - 1) / kSdfB,
+                             bz = (dims[2] + kSdfB - 1) / kSdfB;
+                LAUNCH(k_sdf_scan, blocks(ntri, 256), 256, 0, st, f);
+                LAUNCH(k_sdf_balls, blocks(ntri, 256), 256, 0, st, f);
+                LAUNCH(k_sdf_dist, (unsigned)(bx * by * bz), kSdfDistBS, 0, st, f, (int)bx, (int)by);
+                LAUNCH(k_sdf_up, blocks(nn, 256), 256, 0, st, f);
+                LAUNCH(k_sdf_roots, 148, 512, 0, st, f);
+                LAUNCH(k_sdf_sign, blocks(nn, 256), 256, 0, st, f);
+            }
             LAUNCH(k_sdf_mesh, blocks(nn, kSdfBS), kSdfBS, 0, st, dt, (uint32_t)ntri, ntiles, origin.x, origin.y,
-                   origin.z, dx, (int)dims[0], (int)dims[1], (int)dims[2], dout, derr, skip);
+                   origin.z, dx, (int)dims[0], (int)dims[1], (int)dims[2], dout, derr, skip, fast ? gate : nullptr);
             CK(cudaMemcpyAsync(out, dout, nn * 8, cudaMemcpyDeviceToHost, st));
             uint32_t e = 0;
             CK(cudaMemcpyAsync(&e, derr, 4, cudaMemcpyDeviceToHost, st));
