@@ -28,14 +28,7 @@ struct SdfD {
     const double* data;
 };
 
-__device__ __forceinline__ double sdf_sample_d(const SdfD& s, double px, double py, double pz) {
-    double lx = ddiv(dsub(px, s.ox), s.dx), ly = ddiv(dsub(py, s.oy), s.dx),
-           lz = ddiv(dsub(pz, s.oz), s.dx);
-    int i, j, k;
-    double fx, fy, fz;
-    clamp_base_d(lx, s.nx, i, fx);
-    clamp_base_d(ly, s.ny, j, fy);
-    clamp_base_d(lz, s.nz, k, fz);
+__device__ __forceinline__ double sdf_lerp_d(const SdfD& s, int i, int j, int k, double fx, double fy, double fz) {
     auto at = [&](int a, int b, int c) { return s.data[((size_t)c * s.ny + b) * s.nx + a]; };
     double gx = dsub(1.0, fx), gy = dsub(1.0, fy), gz = dsub(1.0, fz);
     double c00 = dadd(dmul(at(i, j, k), gx), dmul(at(i + 1, j, k), fx));
@@ -45,6 +38,16 @@ __device__ __forceinline__ double sdf_sample_d(const SdfD& s, double px, double 
     double c0 = dadd(dmul(c00, gy), dmul(c10, fy));
     double c1 = dadd(dmul(c01, gy), dmul(c11, fy));
     return dadd(dmul(c0, gz), dmul(c1, fz));
+}
+__device__ __forceinline__ double sdf_sample_d(const SdfD& s, double px, double py, double pz) {
+    double lx = ddiv(dsub(px, s.ox), s.dx), ly = ddiv(dsub(py, s.oy), s.dx),
+           lz = ddiv(dsub(pz, s.oz), s.dx);
+    int i, j, k;
+    double fx, fy, fz;
+    clamp_base_d(lx, s.nx, i, fx);
+    clamp_base_d(ly, s.ny, j, fy);
+    clamp_base_d(lz, s.nz, k, fz);
+    return sdf_lerp_d(s, i, j, k, fx, fy, fz);
 }
 
 // cavity_mask (solver.rs:194-199) and the static half of classify

@@ -7,9 +7,9 @@
 //    index + 1, then one colouring pass);
 //  * amber: the coverage update cov += (1 - cov) * a is order-dependent in
 //    f64, so particles are binned by image tile in index order (the stable
-//    counting sort of the particle pipeline) and each pixel merges the nine
-//    neighbouring tiles' lists in index order, applying exactly the
-//    reference's sequence of updates.
+//    counting sort of the particle pipeline) and a block per 8 x 8 pixels
+//    merges the nine neighbouring tiles' lists in index order, each pixel
+//    applying exactly the reference's sequence of updates.
 // The needle overlay is drawn on the host afterwards (a few dozen pixels).
 #pragma once
 #include "grid.cuh"
@@ -60,6 +60,18 @@ __device__ __forceinline__ bool rv_in_slab(const RenderView& v, float4 p) {
 // Background (render.rs:159-178): interior where the SDF is negative on the
 // plane, or at any of 96 depths for a projection.
 __global__ void k_render_bg(RenderView v, SdfD s, uint8_t* __restrict__ rgb) {
+    __shared__ int depth_i[96];
+    __shared__ double depth_f[96];
+    if (v.project && threadIdx.x < 96) {
+        const double lo = v.mn[v.oax], span = fmax(dsub(v.mx[v.oax], v.mn[v.oax]), 1e-9);
+        const double d = dadd(lo, dmul(ddiv((double)threadIdx.x + 0.5, 96.0), span));
+        int i;
+        double f;
+        clamp_base_d(ddiv(dsub(d, rv_comp(s.ox, s.oy, s.oz, v.oax)), s.dx), v.oax == 0 ? s.nx : (v.oax == 1 ? s.ny : s.nz), i, f);
+        depth_i[threadIdx.x] = i;
+        depth_f[threadIdx.x] = f;
+    }
+    __syncthreads();
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= (size_t)v.w * v.h) return;
     const uint32_t px = (uint32_t)(q % v.w), py = (uint32_t)(q / v.w);
@@ -67,17 +79,30 @@ __global__ void k_render_bg(RenderView v, SdfD s, uint8_t* __restrict__ rgb) {
     const double wx = dadd(v.mn[v.hax], dmul(ddiv((double)px + 0.5, (double)v.w), v.wm));
     const double fyv = dmul(ddiv((double)py + 0.5, (double)v.h), v.hm);
     const double wy = v.flip_v ? dsub(v.mx[v.vax], fyv) : dadd(v.mn[v.vax], fyv);
-    double c[3] = {0.0, 0.0, 0.0};
-    c[v.hax] = wx;
-    c[v.vax] = wy;
     bool interior = false;
     if (v.project) {
-        const double lo = v.mn[v.oax], span = fmax(dsub(v.mx[v.oax], v.mn[v.oax]), 1e-9);
+        // The samples of a ray differ along one axis only: the grid places of
+        // the other two are taken once, those of the 96 depths once per block
+        // (shared memory). Sdf::sample with its operations in order
+        // (sdf_sample_d): 103 us per 600 px image before, a quarter of it now.
+        const double p[3] = {v.hax == 0 ? wx : (v.vax == 0 ? wy : 0.0), v.hax == 1 ? wx : (v.vax == 1 ? wy : 0.0),
+                             v.hax == 2 ? wx : (v.vax == 2 ? wy : 0.0)};
+        int ia, ib;
+        double fa, fb;  // the in-plane axes in x, y, z order
+        const int A = v.oax == 0 ? 1 : 0, B = v.oax == 2 ? 1 : 2;
+        clamp_base_d(ddiv(dsub(p[A], A == 0 ? s.ox : s.oy), s.dx), A == 0 ? s.nx : s.ny, ia, fa);
+        clamp_base_d(ddiv(dsub(p[B], B == 1 ? s.oy : s.oz), s.dx), B == 1 ? s.ny : s.nz, ib, fb);
         for (int k = 0; k < 96 && !interior; ++k) {
-            c[v.oax] = dadd(lo, dmul(ddiv((double)k + 0.5, 96.0), span));
-            interior = sdf_sample_d(s, c[0], c[1], c[2]) < 0.0;
+            const int io = depth_i[k];
+            const double fo = depth_f[k];
+            const int i = v.oax == 0 ? io : ia, j = v.oax == 1 ? io : (v.oax == 0 ? ia : ib), l = v.oax == 2 ? io : ib;
+            const double fx = v.oax == 0 ? fo : fa, fy = v.oax == 1 ? fo : (v.oax == 0 ? fa : fb), fz = v.oax == 2 ? fo : fb;
+            interior = sdf_lerp_d(s, i, j, l, fx, fy, fz) < 0.0;
         }
     } else {
+        double c[3] = {0.0, 0.0, 0.0};
+        c[v.hax] = wx;
+        c[v.vax] = wy;
         c[v.oax] = v.slice;
         interior = sdf_sample_d(s, c[0], c[1], c[2]) < 0.0;
     }
@@ -168,7 +193,9 @@ __global__ void k_render_amber_keys(RenderView v, const float4* __restrict__ pos
         }
     }
     key[i] = k;
-    atomicAdd(hist + k, 1u);
+    // particles of a warp are near each other: one add per bin and warp
+    const unsigned same = __match_any_sync(__activemask(), k);
+    if ((int)(threadIdx.x & 31) == __ffs((int)same) - 1) atomicAdd(hist + k, (uint32_t)__popc(same));
 }
 
 __device__ __forceinline__ uint8_t rv_lerp(uint8_t a, uint8_t b, double t) {  // lerp_u8, render.rs:311-316
@@ -179,43 +206,117 @@ __device__ __forceinline__ uint8_t rv_lerp(uint8_t a, uint8_t b, double t) {  //
 }
 
 // Amber pool, compositing (render.rs:261-307): every pixel replays, in
-// particle order, the splats of the particles binned in its 3x3 tiles.
-__global__ void k_render_amber_pixels(RenderView v, int r, int T, int ntx, const uint32_t* __restrict__ start,
-                                      const uint32_t* __restrict__ perm, const int2* __restrict__ cxy,
-                                      uint8_t* __restrict__ rgb) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (size_t)v.w * v.h) return;
-    const int x = (int)(q % v.w), y = (int)(q / v.w);
-    const int tx = x / T + 1, ty = y / T + 1;
-    uint32_t cur[9], end[9];
+// particle order, the splats of the particles binned in its 3x3 tiles. A block
+// takes up to 8 x 8 pixels of a tile: it brings the next kAmTake particles of
+// each of the nine lists to shared memory, those below the least last index of
+// the lists that go on are the next ones in order, each finds its place by
+// binary searches in the other lists, and every pixel walks the merged piece.
+// A pixel is done once no splat can change its coverage any more (the update
+// rounds to the same value even for the largest a, 0.22). Each pixel merging
+// the nine lists by itself from global memory took 18 ms for 2.8 M particles
+// on 600 px and 0.56 ms for 77,000.
+constexpr int kAmPx = 8;              // pixels of a block along each axis
+constexpr int kAmBS = kAmPx * kAmPx;  // 64
+constexpr int kAmTake = 128;          // particles of each list at a time
+constexpr int kAmTable = 1024;        // splat weights by squared distance (radius up to 31 px), else computed
+
+__global__ void __launch_bounds__(kAmBS) k_render_amber_pixels(RenderView v, int r, int T, int ntx,
+                                                               const uint32_t* __restrict__ start,
+                                                               const uint32_t* __restrict__ perm,
+                                                               const int2* __restrict__ cxy, uint8_t* __restrict__ rgb) {
+    __shared__ uint32_t s_idx[9][kAmTake];
+    __shared__ int s_n[9];
+    __shared__ short2 s_xy[9 * kAmTake];
+    __shared__ double s_a[kAmTable];
+    const int tid = threadIdx.x;
+    const int per = (T + kAmPx - 1) / kAmPx;  // blocks of a tile along each axis
+    const int tile = blockIdx.x / (per * per), part = blockIdx.x % (per * per);
+    const int tx = tile % ntx + 1, ty = tile / ntx + 1;  // with the margin tile
+    const int lx = part % per * kAmPx + tid % kAmPx, ly = part / per * kAmPx + tid / kAmPx;
+    const int x0 = (tx - 1) * T, y0 = (ty - 1) * T;
+    const int x = x0 + lx, y = y0 + ly;
+    const bool live = lx < T && ly < T && x < (int)v.w && y < (int)v.h;
+    const int rr_i = r * r;
+    const double rr = (double)((long long)r * r);
+    auto weight = [&](int d2) { return dmul(0.22, dsub(1.0, ddiv((double)d2, rr))); };
+    const bool table = rr_i < kAmTable;
+    if (table)
+        for (int d2 = tid; d2 <= rr_i; d2 += kAmBS) s_a[d2] = weight(d2);
+    uint32_t cur[9], end[9];  // the same in every thread
+#pragma unroll
     for (int b = 0; b < 9; ++b) {
         const uint32_t bin = (uint32_t)(ty + b / 3 - 1) * (uint32_t)(ntx + 2) + (uint32_t)(tx + b % 3 - 1);
         cur[b] = start[bin];
         end[b] = start[bin + 1];
     }
-    const double rr = (double)((long long)r * r);
     double cov = 0.0;
+    bool done = !live;
     for (;;) {
-        uint32_t best = 0xFFFFFFFFu;
-        int bb = -1;
+        uint32_t left = 0, pivot = 0xFFFFFFFFu;
+#pragma unroll
+        for (int b = 0; b < 9; ++b) {
+            left += end[b] - cur[b];
+            for (uint32_t q = tid; q < kAmTake && cur[b] + q < end[b]; q += kAmBS) s_idx[b][q] = perm[cur[b] + q];
+        }
+        if (left == 0) break;
+        __syncthreads();
+#pragma unroll
         for (int b = 0; b < 9; ++b)
-            if (cur[b] < end[b]) {
-                const uint32_t pi = perm[cur[b]];
-                if (pi < best) {
-                    best = pi;
-                    bb = b;
+            if (end[b] - cur[b] > (uint32_t)kAmTake) pivot = min(pivot, s_idx[b][kAmTake - 1]);
+        if (tid < 9) {  // entries of list tid up to the pivot
+            uint32_t c = 0, e = 0;
+#pragma unroll
+            for (int b = 0; b < 9; ++b)
+                if (b == tid) {
+                    c = cur[b];
+                    e = end[b];
                 }
+            int lo = 0, hi = (int)min(e - c, (uint32_t)kAmTake);
+            while (lo < hi) {
+                const int m = (lo + hi) / 2;
+                if (s_idx[tid][m] <= pivot) lo = m + 1;
+                else hi = m;
             }
-        if (bb < 0) break;
-        ++cur[bb];
-        const int2 c = cxy[best];
-        const long long dx = (long long)x - c.x, dy = (long long)y - c.y;
-        if (dx < -r || dx > r || dy < -r || dy > r) continue;
-        const double d2 = (double)(dx * dx + dy * dy);
-        if (d2 > rr) continue;
-        const double a = dmul(0.22, dsub(1.0, ddiv(d2, rr)));
-        cov = dadd(cov, dmul(dsub(1.0, cov), a));
+            s_n[tid] = lo;
+        }
+        __syncthreads();
+        int total = 0;
+#pragma unroll
+        for (int b = 0; b < 9; ++b) {
+            const int n = s_n[b];
+            total += n;
+            for (int q = tid; q < n; q += kAmBS) {
+                const uint32_t p = s_idx[b][q];
+                int at = q;
+                for (int o = 0; o < 9; ++o) {
+                    if (o == b) continue;
+                    int lo = 0, hi = s_n[o];
+                    while (lo < hi) {
+                        const int m = (lo + hi) / 2;
+                        if (s_idx[o][m] < p) lo = m + 1;
+                        else hi = m;
+                    }
+                    at += lo;
+                }
+                const int2 c = cxy[p];
+                s_xy[at] = make_short2((short)(c.x - x0), (short)(c.y - y0));  // within two tiles of this one
+            }
+            cur[b] += (uint32_t)n;
+        }
+        __syncthreads();
+        if (!done) {
+            for (int e = 0; e < total; ++e) {
+                const short2 c = s_xy[e];
+                const int dx = lx - c.x, dy = ly - c.y, d2 = dx * dx + dy * dy;
+                if (d2 > rr_i) continue;
+                cov = dadd(cov, dmul(dsub(1.0, cov), table ? s_a[d2] : weight(d2)));
+            }
+            done = dadd(cov, dmul(dsub(1.0, cov), 0.22)) == cov;
+        }
+        if (__syncthreads_and(done)) break;
     }
+    if (!live) return;
+    const size_t q = (size_t)y * v.w + x;
     const double cc = rv_clamp01(cov);
     if (cc <= 1.0 / 255.0) return;
     uint8_t* o = rgb + 3 * q;

@@ -2103,8 +2103,11 @@ int sdr_render_slice(sdr_solver* s, const sdr_slice_plane* plane, uint32_t targe
             CK(cudaMemcpyAsync(fill, start, nb * 4, cudaMemcpyDeviceToDevice, st));
             if (n) LAUNCH(k_sort_scatter, blocks(n, 256), 256, 0, st, key, n, fill, perm);
             LAUNCH(k_sort_segments, blocks(nb, 256), 256, 0, st, start, nb, perm, longl, lcount);
-            LAUNCH(k_sort_long, 148, 256, 0, st, start, longl, lcount, perm, tmp);
-            LAUNCH(k_render_amber_pixels, blocks(npx, 256), 256, 0, st, v, r, T, ntx, start, perm, cxy, img);
+            // an image has thousands of long bins (hundreds of particles each): eight blocks per SM
+            LAUNCH(k_sort_long, 148 * 8, 256, 0, st, start, longl, lcount, perm, tmp);
+            const unsigned per = (unsigned)((T + kAmPx - 1) / kAmPx);
+            LAUNCH(k_render_amber_pixels, (unsigned)ntx * (unsigned)nty * per * per, kAmBS, 0, st, v, r, T, ntx, start, perm,
+                   cxy, img);
         } else {  // speed-coloured dots (render.rs:201-221)
             dalloc(owner, npx, st);
             dalloc(peak, 1, st);
@@ -2201,7 +2204,7 @@ int sdr_metrics_record(sdr_metrics* m, sdr_solver* s, uint64_t frame, sdr_frame_
         unsigned ncb = blocks(s->ncell, kMetBS);
         LAUNCH(k_metrics_cells, ncb, kMetBS, 0, s->st, s->ncell, s->cells, s->p_dense, m->washed, m->wet, p_cap,
                s->mcell);
-        LAUNCH(k_metrics_final, 1, 32, 0, s->st, s->mcell, (int)ncb, s->mpart, (int)npb, s->mout);
+        LAUNCH(k_metrics_final, 1, kMetFinalBS, 0, s->st, s->mcell, (int)ncb, s->mpart, (int)npb, s->mout);
         copy_dev(s, s->mout, sizeof(MetricsOut), s->h_mout);
         const MetricsOut& o = *s->h_mout;
         double pv = s->particle_volume();
