@@ -200,27 +200,39 @@ struct PcgArgs {
     int exact_dots;              // 1: the reference's chunked sequential dot order (bit-exact); 0: fixed block tree
 };
 
-// Sweep record: the cell's MIC factor and the shared-window slots (index
-// within the neighbouring level, -1 = not fluid) of its three neighbours.
+// Sweep record: the cell's MIC factor and the shared-window places (byte
+// offsets: 8 times the index within the neighbouring level) of its three
+// neighbours, 16 bits each; where one is not fluid the place is kPcgNone, which
+// holds -0.0: t + (-0.0) is t for every t, so a cell adds its three neighbours
+// without a branch.
 struct SweepRec {
     double pc;
-    short s0, s1, s2, pad;
+    unsigned long long at;
 };
+constexpr int kPcgNone = kPcgBS;  // place index
+static_assert(kPcgNone * 8 < 1 << 16, "places are 16-bit byte offsets");
+__device__ __forceinline__ SweepRec lds_rec(uint32_t a) {
+    SweepRec r;
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=d"(r.pc), "=l"(r.at) : "r"(a));
+    return r;
+}
 
-// Shared-memory plan of k_pcg (dynamic): a ring of kStages staged levels
-// (two f64 operands and one record per cell), two level windows of f64 and of
-// neighbour masks and the level starts.
-constexpr int kStages = 4;          // levels in flight ahead of the sweep
+// Shared-memory plan of k_pcg (dynamic): a ring of staged levels (two f64
+// operands and one record per cell), two level windows of f64 and of neighbour
+// masks and the level starts. The ring holds kRingCells cells: as many levels
+// of the widest sweep as fit, 4 to 16 (a level's copies come from L2, which
+// takes as long as two or three level steps).
+constexpr int kRingCells = 4 * kPcgBS;
 constexpr int kMaxLevelsSmem = 2048;
-constexpr int kSweepMax = kPcgBS - 32;  // compute threads; one producer warp stages ahead
-constexpr size_t kPcgSmem = (size_t)kStages * kPcgBS * (8 + 8 + 16) + 2 * kPcgBS * 8 + 2 * kPcgBS * 4 +
+constexpr int kSweepMax = kPcgBS - 32;  // compute threads; up to four producer warps stage ahead
+constexpr size_t kPcgSmem = (size_t)kRingCells * (8 + 8 + 16) + 2 * (kPcgBS + 2) * 8 + 2 * kPcgBS * 4 +
                             (kMaxLevelsSmem + 1) * 4;
 
 struct PcgSmem {
-    double* sa;     // [kStages][BS]
-    double* sb;     // [kStages][BS]
-    SweepRec* sr;   // [kStages][BS]
-    double* w0;     // [BS] level window
+    double* sa;     // [kRingCells]
+    double* sb;     // [kRingCells]
+    SweepRec* sr;   // [kRingCells]
+    double* w0;     // [BS + 1] level window, then -0.0
     double* w1;
     int* m0;        // [BS] neighbour-mask window (MIC build)
     int* m1;
@@ -228,6 +240,23 @@ struct PcgSmem {
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// Shared-memory accesses at a constant offset from a 32-bit address, in program
+// order with the barriers around them.
+template <int OFF>
+__device__ __forceinline__ double lds_f64(uint32_t a) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1+%2];" : "=d"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+template <int OFF>
+__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+__device__ __forceinline__ void sts_f64(uint32_t a, double v) {
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
@@ -235,27 +264,30 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// The producer keeps two levels complete ahead of the one being computed, so
+// The producers keep two levels complete ahead of the one being computed, so
 // compute threads can read level L+1's staged data into registers while level
-// L is in flight.
+// L is in flight; the others of the ring's NS levels are under way.
+template <int NS>
 __device__ __forceinline__ void cp_wait_ahead() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 3) : "memory");
+    asm volatile("cp.async.wait_group %0;" ::"n"(NS - 3) : "memory");
 }
 
 // Barrier over the first `n` threads (named barrier 1): the sweeps run on the
-// compute warps plus one producer warp, sized to the widest level, so the
+// compute warps plus the producer warps, sized to the widest level, so the
 // per-level barrier carries only working warps.
 __device__ __forceinline__ void sweep_bar(int n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); }
 
-// Producer warp: stage every cell of level L (if the level fits the ring)
-// into slot L % kStages: operand A, optional operand B, and the record.
+// Producer warps (np threads): stage every cell of level L (if the level fits
+// the ring) into slot L % NS of `width` cells: operand A, optional operand B,
+// and the record.
+template <int NS>
 __device__ __forceinline__ void produce_level(const PcgSmem& m, int L, int lo, int hi, const double* va,
-                                              const double* vb, const int4* rec, int lane) {
+                                              const double* vb, const int4* rec, int t0, int np, int width) {
     if (L >= lo && L < hi) {
         int ls = m.lvs[L], le = m.lvs[L + 1];
         if (le - ls <= kSweepMax) {
-            int base = (L % kStages) * kPcgBS;
-            for (int t = lane; t < le - ls; t += 32) {
+            int base = (L % NS) * width;
+            for (int t = t0; t < le - ls; t += np) {
                 cp_async8(&m.sa[base + t], &va[ls + t]);
                 if (vb) cp_async8(&m.sb[base + t], &vb[ls + t]);
                 cp_async16(&m.sr[base + t], &rec[ls + t]);
@@ -486,14 +518,12 @@ __device__ void pcg_build_records(const PcgArgs& a, const PcgSmem& m, uint32_t n
         int lsp = L > 0 ? m.lvs[L - 1] : 0, lsn = m.lvs[L + 1];
         SweepRec f, g;
         f.pc = g.pc = a.precon[ps];
-        int mm;
-        f.s0 = (short)((mm = nb[NB_MX]) >= 0 ? mm - lsp : -1);
-        f.s1 = (short)((mm = nb[NB_MY]) >= 0 ? mm - lsp : -1);
-        f.s2 = (short)((mm = nb[NB_MZ]) >= 0 ? mm - lsp : -1);
-        g.s0 = (short)((mm = nb[NB_PX]) >= 0 ? mm - lsn : -1);
-        g.s1 = (short)((mm = nb[NB_PY]) >= 0 ? mm - lsn : -1);
-        g.s2 = (short)((mm = nb[NB_PZ]) >= 0 ? mm - lsn : -1);
-        f.pad = g.pad = 0;
+        auto place = [&](int d, int base) {  // a level wider than the window is not read through its places
+            const int mm = nb[d];
+            return (unsigned long long)(8 * (mm >= 0 ? min(mm - base, kPcgNone) : kPcgNone));
+        };
+        f.at = place(NB_MX, lsp) | place(NB_MY, lsp) << 16 | place(NB_MZ, lsp) << 32;
+        g.at = place(NB_PX, lsn) | place(NB_PY, lsn) << 16 | place(NB_PZ, lsn) << 32;
         a.frec[ps] = *reinterpret_cast<int4*>(&f);
         a.brec[ps] = *reinterpret_cast<int4*>(&g);
     }
@@ -505,36 +535,45 @@ __device__ void pcg_build_records(const PcgArgs& a, const PcgSmem& m, uint32_t n
 //           which is what `t -= plus*precon*q` with plus = -1 adds), q = t*pc.
 // Backward: t = q + pc*z[+x] + pc*z[+y] + pc*z[+z], z = t*pc, plus the z*r
 //           products of the following dot.
-// Compute threads [0, sw) take one cell each per level from the staged ring;
-// the producer warp [sw, sw+32) stages level L + kStages - 1 while level L is
-// computed. Levels wider than the ring use global memory (uniform branch).
-__device__ void pcg_apply_mic0(const PcgArgs& a, const PcgSmem& m, const double* r, double* z, int sw, int l0,
-                               int l1, unsigned long long* lt = nullptr) {
+// Compute threads [0, sw) take one cell each per level from the staged ring of
+// NS levels; the producer warps [sw, sw + np) stage level L + NS - 1 while level
+// L is computed. A level's results go to global memory while the next level's
+// operands are read, off the chain from barrier to barrier. Levels wider than
+// the ring use global memory (uniform branch).
+template <int NS>
+__device__ void pcg_apply_mic0_n(const PcgArgs& a, const PcgSmem& m, const double* r, double* z, int sw, int np,
+                                 int l0, int l1, unsigned long long* lt) {
     const int tid = threadIdx.x;
-    const int nbar = sw + 32;
+    const int nbar = sw + np;
     if (tid >= nbar) {
         __syncthreads();
         return;
     }
     const bool producer = tid >= sw;
-    const int lane = tid - sw;
+    const int pt = tid - sw;
+    const uint32_t a_sa = smem_addr(m.sa) + tid * 8, a_sb = smem_addr(m.sb) + tid * 8, a_sr = smem_addr(m.sr) + tid * 16;
+    const uint32_t a_w0 = smem_addr(m.w0), a_w1 = smem_addr(m.w1);
     // ---------------- forward
     if (producer) {
-        for (int d = 0; d < kStages - 1; ++d) produce_level(m, l0 + d, l0, l1, r, nullptr, a.frec, lane);
-        cp_wait_ahead();
+        for (int d = 0; d < NS - 1; ++d) produce_level<NS>(m, l0 + d, l0, l1, r, nullptr, a.frec, pt, np, sw);
+        cp_wait_ahead<NS>();
     }
+    if (tid == 0) m.w0[kPcgNone] = m.w1[kPcgNone] = -0.0;
     sweep_bar(nbar);
     double* prev = m.w0;
     double* cur = m.w1;
+    uint32_t a_prev = a_w0, a_cur = a_w1;
     int lsP = l0 > 0 ? m.lvs[l0 - 1] : 0, lsA = m.lvs[l0], lsB = m.lvs[l0 + 1];
     // staged operands of this thread's cell in the current level (registers)
     double ct = 0.0;
     SweepRec crc{};
     if (!producer && tid < lsB - lsA && lsB - lsA <= kSweepMax) {
-        int slot = (l0 % kStages) * kPcgBS + tid;
-        ct = m.sa[slot];
-        crc = m.sr[slot];
+        const uint32_t slot = (uint32_t)((l0 % NS) * sw);
+        ct = lds_f64<0>(a_sa + slot * 8);
+        crc = lds_rec(a_sr + slot * 16);
     }
+    double owed = 0.0;  // this thread's result of the level before, and where it goes (-1: none)
+    int owed_at = -1;
     for (int L = l0; L < l1; ++L) {
         int lsC = m.lvs[min(L + 2, a.nlevels)];
         unsigned long long c0 = lt ? clock64() : 0;
@@ -542,54 +581,56 @@ __device__ void pcg_apply_mic0(const PcgArgs& a, const PcgSmem& m, const double*
         double nt_ = 0.0;
         SweepRec nrc{};
         if (producer) {
-            produce_level(m, L + kStages - 1, l0, l1, r, nullptr, a.frec, lane);
-            cp_wait_ahead();
-        } else {
-            if (L + 1 < l1 && tid < wnext && wnext <= kSweepMax) {  // prefetch level L+1
-                int slot = ((L + 1) % kStages) * kPcgBS + tid;
-                nt_ = m.sa[slot];
-                nrc = m.sr[slot];
+            produce_level<NS>(m, L + NS - 1, l0, l1, r, nullptr, a.frec, pt, np, sw);
+            cp_wait_ahead<NS>();
+        } else if (wcur <= kSweepMax && wprev <= kPcgBS) {
+            const bool mine = tid < wcur;
+            double x0 = 0.0, x1 = 0.0, x2 = 0.0;
+            if (mine) {
+                x0 = lds_f64<0>(a_prev + (uint32_t)(crc.at & 0xffffu));
+                x1 = lds_f64<0>(a_prev + (uint32_t)(crc.at >> 16 & 0xffffu));
+                x2 = lds_f64<0>(a_prev + (uint32_t)(crc.at >> 32 & 0xffffu));
             }
-            if (wcur <= kSweepMax) {
-                if (tid < wcur) {
-                    double t = ct;
-                    if (wprev <= kPcgBS) {
-                        if (crc.s0 >= 0) t = dadd(t, prev[crc.s0]);
-                        if (crc.s1 >= 0) t = dadd(t, prev[crc.s1]);
-                        if (crc.s2 >= 0) t = dadd(t, prev[crc.s2]);
-                    } else {
-                        const int* nb = a.nbr + (size_t)(lsA + tid) * 6;
-                        int mm;
-                        if ((mm = nb[NB_MX]) >= 0) t = dadd(t, a.pq[mm]);
-                        if ((mm = nb[NB_MY]) >= 0) t = dadd(t, a.pq[mm]);
-                        if ((mm = nb[NB_MZ]) >= 0) t = dadd(t, a.pq[mm]);
-                    }
-                    double qv = dmul(t, crc.pc);
-                    double pqv = dmul(crc.pc, qv);
-                    cur[tid] = pqv;
-                    a.q[lsA + tid] = qv;
+            if (L + 1 < l1 && tid < wnext && wnext <= kSweepMax) {  // prefetch level L+1
+                const uint32_t slot = (uint32_t)(((L + 1) % NS) * sw);
+                nt_ = lds_f64<0>(a_sa + slot * 8);
+                nrc = lds_rec(a_sr + slot * 16);
+            }
+            if (owed_at >= 0) a.q[owed_at] = owed;
+            owed_at = -1;
+            if (mine) {
+                const double qv = dmul(dadd(dadd(dadd(ct, x0), x1), x2), crc.pc);
+                sts_f64(a_cur + tid * 8, dmul(crc.pc, qv));
+                owed = qv;
+                owed_at = lsA + tid;
+            }
+        } else {
+            if (owed_at >= 0) a.q[owed_at] = owed;
+            owed_at = -1;
+            if (L + 1 < l1 && tid < wnext && wnext <= kSweepMax) {
+                const uint32_t slot = (uint32_t)(((L + 1) % NS) * sw);
+                nt_ = lds_f64<0>(a_sa + slot * 8);
+                nrc = lds_rec(a_sr + slot * 16);
+            }
+            for (int ps = lsA + tid; ps < lsB; ps += sw) {
+                const int* nb = a.nbr + (size_t)ps * 6;
+                double t = r[ps];
+                int mm;
+                if (wprev <= kPcgBS) {
+                    if ((mm = nb[NB_MX]) >= 0) t = dadd(t, prev[mm - lsP]);
+                    if ((mm = nb[NB_MY]) >= 0) t = dadd(t, prev[mm - lsP]);
+                    if ((mm = nb[NB_MZ]) >= 0) t = dadd(t, prev[mm - lsP]);
+                } else {
+                    if ((mm = nb[NB_MX]) >= 0) t = dadd(t, a.pq[mm]);
+                    if ((mm = nb[NB_MY]) >= 0) t = dadd(t, a.pq[mm]);
+                    if ((mm = nb[NB_MZ]) >= 0) t = dadd(t, a.pq[mm]);
                 }
-            } else {
-                for (int ps = lsA + tid; ps < lsB; ps += sw) {
-                    const int* nb = a.nbr + (size_t)ps * 6;
-                    double t = r[ps];
-                    int mm;
-                    if (wprev <= kPcgBS) {
-                        if ((mm = nb[NB_MX]) >= 0) t = dadd(t, prev[mm - lsP]);
-                        if ((mm = nb[NB_MY]) >= 0) t = dadd(t, prev[mm - lsP]);
-                        if ((mm = nb[NB_MZ]) >= 0) t = dadd(t, prev[mm - lsP]);
-                    } else {
-                        if ((mm = nb[NB_MX]) >= 0) t = dadd(t, a.pq[mm]);
-                        if ((mm = nb[NB_MY]) >= 0) t = dadd(t, a.pq[mm]);
-                        if ((mm = nb[NB_MZ]) >= 0) t = dadd(t, a.pq[mm]);
-                    }
-                    double pc = a.precon[ps];
-                    double qv = dmul(t, pc);
-                    double pqv = dmul(pc, qv);
-                    a.q[ps] = qv;
-                    a.pq[ps] = pqv;
-                    if (wcur <= kPcgBS) cur[ps - lsA] = pqv;  // the next level reads the window
-                }
+                double pc = a.precon[ps];
+                double qv = dmul(t, pc);
+                double pqv = dmul(pc, qv);
+                a.q[ps] = qv;
+                a.pq[ps] = pqv;
+                if (wcur <= kPcgBS) cur[ps - lsA] = pqv;  // the next level reads the window
             }
         }
         unsigned long long c1 = lt ? clock64() : 0;
@@ -604,6 +645,9 @@ __device__ void pcg_apply_mic0(const PcgArgs& a, const PcgSmem& m, const double*
             double* tt = prev;
             prev = cur;
             cur = tt;
+            const uint32_t ta = a_prev;
+            a_prev = a_cur;
+            a_cur = ta;
         }
         ct = nt_;
         crc = nrc;
@@ -611,80 +655,94 @@ __device__ void pcg_apply_mic0(const PcgArgs& a, const PcgSmem& m, const double*
         lsA = lsB;
         lsB = lsC;
     }
+    if (owed_at >= 0) a.q[owed_at] = owed;
+    owed_at = -1;
     if (producer) asm volatile("cp.async.wait_all;" ::: "memory");
     sweep_bar(nbar);
     // ---------------- backward
     if (producer) {
-        for (int d = 0; d < kStages - 1; ++d) produce_level(m, l1 - 1 - d, l0, l1, a.q, r, a.brec, lane);
-        cp_wait_ahead();
+        for (int d = 0; d < NS - 1; ++d) produce_level<NS>(m, l1 - 1 - d, l0, l1, a.q, r, a.brec, pt, np, sw);
+        cp_wait_ahead<NS>();
     }
     sweep_bar(nbar);
     double* next = m.w0;
     cur = m.w1;
+    uint32_t a_next = a_w0;
+    a_cur = a_w1;
     int lsN = m.lvs[l1], lsH = m.lvs[min(l1 + 1, a.nlevels)];  // starts of levels L+1, L+2
     lsA = m.lvs[l1 - 1];
-    double cq = 0.0, cr = 0.0;
+    double cq = 0.0, cr = 0.0, owed_p = 0.0;
     crc = SweepRec{};
     if (!producer && tid < lsN - lsA && lsN - lsA <= kSweepMax) {
-        int slot = ((l1 - 1) % kStages) * kPcgBS + tid;
-        cq = m.sa[slot];
-        cr = m.sb[slot];
-        crc = m.sr[slot];
+        const uint32_t slot = (uint32_t)(((l1 - 1) % NS) * sw);
+        cq = lds_f64<0>(a_sa + slot * 8);
+        cr = lds_f64<0>(a_sb + slot * 8);
+        crc = lds_rec(a_sr + slot * 16);
     }
+    auto pay = [&] {
+        if (owed_at >= 0) {
+            z[owed_at] = owed;
+            a.prod[a.exact_dots ? a.cinv[owed_at] : owed_at] = owed_p;
+        }
+        owed_at = -1;
+    };
     for (int L = l1 - 1; L >= l0; --L) {
         int lsQ = L > 0 ? m.lvs[L - 1] : 0;
         const int wnext = lsH - lsN, wcur = lsN - lsA, wlow = lsA - lsQ;
         double nq = 0.0, nr = 0.0;
         SweepRec nrc{};
         if (producer) {
-            produce_level(m, L - (kStages - 1), l0, l1, a.q, r, a.brec, lane);
-            cp_wait_ahead();
-        } else {
-            if (L - 1 >= l0 && tid < wlow && wlow <= kSweepMax) {  // prefetch level L-1
-                int slot = ((L - 1) % kStages) * kPcgBS + tid;
-                nq = m.sa[slot];
-                nr = m.sb[slot];
-                nrc = m.sr[slot];
+            produce_level<NS>(m, L - (NS - 1), l0, l1, a.q, r, a.brec, pt, np, sw);
+            cp_wait_ahead<NS>();
+        } else if (wcur <= kSweepMax && (L + 1 == l1 || wnext <= kPcgBS)) {
+            const bool mine = tid < wcur;
+            double x0 = -0.0, x1 = -0.0, x2 = -0.0;
+            if (mine && L + 1 < l1) {
+                x0 = lds_f64<0>(a_next + (uint32_t)(crc.at & 0xffffu));
+                x1 = lds_f64<0>(a_next + (uint32_t)(crc.at >> 16 & 0xffffu));
+                x2 = lds_f64<0>(a_next + (uint32_t)(crc.at >> 32 & 0xffffu));
             }
-            if (wcur <= kSweepMax) {
-                if (tid < wcur) {
-                    double t = cq, pc = crc.pc;
-                    if (L + 1 < l1 && wnext <= kPcgBS) {
-                        if (crc.s0 >= 0) t = dadd(t, dmul(pc, next[crc.s0]));
-                        if (crc.s1 >= 0) t = dadd(t, dmul(pc, next[crc.s1]));
-                        if (crc.s2 >= 0) t = dadd(t, dmul(pc, next[crc.s2]));
-                    } else {
-                        const int* nb = a.nbr + (size_t)(lsA + tid) * 6;
-                        int mm;
-                        if ((mm = nb[NB_PX]) >= 0) t = dadd(t, dmul(pc, z[mm]));
-                        if ((mm = nb[NB_PY]) >= 0) t = dadd(t, dmul(pc, z[mm]));
-                        if ((mm = nb[NB_PZ]) >= 0) t = dadd(t, dmul(pc, z[mm]));
-                    }
-                    double zv = dmul(t, pc);
-                    cur[tid] = zv;
-                    z[lsA + tid] = zv;
-                    a.prod[a.exact_dots ? a.cinv[lsA + tid] : lsA + tid] = dmul(zv, cr);
+            if (L - 1 >= l0 && tid < wlow && wlow <= kSweepMax) {  // prefetch level L-1
+                const uint32_t slot = (uint32_t)(((L - 1) % NS) * sw);
+                nq = lds_f64<0>(a_sa + slot * 8);
+                nr = lds_f64<0>(a_sb + slot * 8);
+                nrc = lds_rec(a_sr + slot * 16);
+            }
+            pay();
+            if (mine) {
+                const double pc = crc.pc;
+                const double zv = dmul(dadd(dadd(dadd(cq, dmul(pc, x0)), dmul(pc, x1)), dmul(pc, x2)), pc);
+                sts_f64(a_cur + tid * 8, zv);
+                owed = zv;
+                owed_p = dmul(zv, cr);
+                owed_at = lsA + tid;
+            }
+        } else {
+            pay();
+            if (L - 1 >= l0 && tid < wlow && wlow <= kSweepMax) {
+                const uint32_t slot = (uint32_t)(((L - 1) % NS) * sw);
+                nq = lds_f64<0>(a_sa + slot * 8);
+                nr = lds_f64<0>(a_sb + slot * 8);
+                nrc = lds_rec(a_sr + slot * 16);
+            }
+            for (int ps = lsA + tid; ps < lsN; ps += sw) {
+                const int* nb = a.nbr + (size_t)ps * 6;
+                double pc = a.precon[ps];
+                double t = a.q[ps];
+                int mm;
+                if (L + 1 < l1 && wnext <= kPcgBS) {
+                    if ((mm = nb[NB_PX]) >= 0) t = dadd(t, dmul(pc, next[mm - lsN]));
+                    if ((mm = nb[NB_PY]) >= 0) t = dadd(t, dmul(pc, next[mm - lsN]));
+                    if ((mm = nb[NB_PZ]) >= 0) t = dadd(t, dmul(pc, next[mm - lsN]));
+                } else {
+                    if ((mm = nb[NB_PX]) >= 0) t = dadd(t, dmul(pc, z[mm]));
+                    if ((mm = nb[NB_PY]) >= 0) t = dadd(t, dmul(pc, z[mm]));
+                    if ((mm = nb[NB_PZ]) >= 0) t = dadd(t, dmul(pc, z[mm]));
                 }
-            } else {
-                for (int ps = lsA + tid; ps < lsN; ps += sw) {
-                    const int* nb = a.nbr + (size_t)ps * 6;
-                    double pc = a.precon[ps];
-                    double t = a.q[ps];
-                    int mm;
-                    if (L + 1 < l1 && wnext <= kPcgBS) {
-                        if ((mm = nb[NB_PX]) >= 0) t = dadd(t, dmul(pc, next[mm - lsN]));
-                        if ((mm = nb[NB_PY]) >= 0) t = dadd(t, dmul(pc, next[mm - lsN]));
-                        if ((mm = nb[NB_PZ]) >= 0) t = dadd(t, dmul(pc, next[mm - lsN]));
-                    } else {
-                        if ((mm = nb[NB_PX]) >= 0) t = dadd(t, dmul(pc, z[mm]));
-                        if ((mm = nb[NB_PY]) >= 0) t = dadd(t, dmul(pc, z[mm]));
-                        if ((mm = nb[NB_PZ]) >= 0) t = dadd(t, dmul(pc, z[mm]));
-                    }
-                    double zv = dmul(t, pc);
-                    z[ps] = zv;
-                    if (wcur <= kPcgBS) cur[ps - lsA] = zv;  // the next level reads the window
-                    a.prod[a.exact_dots ? a.cinv[ps] : ps] = dmul(zv, r[ps]);
-                }
+                double zv = dmul(t, pc);
+                z[ps] = zv;
+                if (wcur <= kPcgBS) cur[ps - lsA] = zv;  // the next level reads the window
+                a.prod[a.exact_dots ? a.cinv[ps] : ps] = dmul(zv, r[ps]);
             }
         }
         sweep_bar(nbar);
@@ -692,6 +750,9 @@ __device__ void pcg_apply_mic0(const PcgArgs& a, const PcgSmem& m, const double*
             double* tt = next;
             next = cur;
             cur = tt;
+            const uint32_t ta = a_next;
+            a_next = a_cur;
+            a_cur = ta;
         }
         cq = nq;
         cr = nr;
@@ -700,8 +761,20 @@ __device__ void pcg_apply_mic0(const PcgArgs& a, const PcgSmem& m, const double*
         lsN = lsA;
         lsA = lsQ;
     }
+    pay();
     if (producer) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
+}
+
+// The ring's depth and the producers for sweeps of sw threads. A deeper ring
+// hides the copies' latency (a level step at 4 levels was their latency, 450
+// cycles); more producers keep up with wide levels.
+__device__ __forceinline__ void pcg_apply_mic0(const PcgArgs& a, const PcgSmem& m, const double* r, double* z, int sw,
+                                               int l0, int l1, unsigned long long* lt = nullptr) {
+    const int np = min(sw <= 64 ? 32 : (sw <= 256 ? 64 : 128), (kPcgBS - sw) / 32 * 32);
+    if (sw * 16 <= kRingCells) pcg_apply_mic0_n<16>(a, m, r, z, sw, np, l0, l1, lt);
+    else if (sw * 8 <= kRingCells) pcg_apply_mic0_n<8>(a, m, r, z, sw, np, l0, l1, lt);
+    else pcg_apply_mic0_n<4>(a, m, r, z, sw, np, l0, l1, lt);
 }
 
 // pcg (pressure.rs:341-397) as one thread-block cluster of C CTAs (C = 1
@@ -717,11 +790,11 @@ __device__ __forceinline__ void k_pcg_body(VB vb_, PcgArgs a) {
     PcgSmem m;
     {
         unsigned char* q = smem_raw;
-        m.sr = (SweepRec*)q; q += (size_t)kStages * kPcgBS * 16;
-        m.sa = (double*)q; q += (size_t)kStages * kPcgBS * 8;
-        m.sb = (double*)q; q += (size_t)kStages * kPcgBS * 8;
-        m.w0 = (double*)q; q += (size_t)kPcgBS * 8;
-        m.w1 = (double*)q; q += (size_t)kPcgBS * 8;
+        m.sr = (SweepRec*)q; q += (size_t)kRingCells * 16;
+        m.sa = (double*)q; q += (size_t)kRingCells * 8;
+        m.sb = (double*)q; q += (size_t)kRingCells * 8;
+        m.w0 = (double*)q; q += (size_t)(kPcgBS + 2) * 8;
+        m.w1 = (double*)q; q += (size_t)(kPcgBS + 2) * 8;
         m.m0 = (int*)q; q += (size_t)kPcgBS * 4;
         m.m1 = (int*)q; q += (size_t)kPcgBS * 4;
         m.lvs = (int*)q;

@@ -137,23 +137,6 @@ __device__ __forceinline__ void st_relaxed_gpu_f64(double* p, double v) {
 __device__ __forceinline__ void st_relaxed_gpu_u64(double* p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-// Shared-memory accesses at a constant offset from a 32-bit address, in program
-// order with the barriers around them.
-template <int OFF>
-__device__ __forceinline__ double lds_f64(uint32_t a) {
-    double v;
-    asm volatile("ld.shared.f64 %0, [%1+%2];" : "=d"(v) : "r"(a), "n"(OFF));
-    return v;
-}
-template <int OFF>
-__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
-    return v;
-}
-__device__ __forceinline__ void sts_f64(uint32_t a, double v) {
-    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
 __device__ __forceinline__ bool tw_failed(const TwArgs& t) { return *(volatile uint32_t*)t.err != 0u; }
 // Barrier of the compute and clerk warps (named barrier 1).
 __device__ __forceinline__ void tw_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kTwBarrier) : "memory"); }
