@@ -558,9 +558,11 @@ constexpr int kRedistProbes = 64;    // linear probes before a cell counts as no
 constexpr int kRedistBS = 1024;
 constexpr int kRedistSmemCand = 8192;  // candidates sorted and replayed in shared memory
 constexpr uint32_t kResolved = 0x80000000u;  // candidate-list flag: decided (particle indices are < 2^31)
-// A shared-memory round costs about as much as one thread deciding this many
-// candidates in index order: rounds that decide fewer hand the rest to thread 0.
+// A shared-memory round costs about as much as warp 0 deciding this many
+// candidates in index order (4,500 cycles against 150 each): rounds that decide
+// fewer hand the rest to it.
 constexpr uint32_t kRoundsMinDecided = 32;
+constexpr uint32_t kRankSort = 1024;  // lists up to here are sorted by rank, longer ones bitonically
 
 struct RedistArgs {
     Grid g;
@@ -604,11 +606,62 @@ __device__ __forceinline__ void redist_apply_move(const RedistArgs& a, uint32_t 
     a.vel[p] = make_float4(v.x, v.y, v.z, 0.0f);
 }
 
+// The same move by eight lanes: a lane per sample of the distance field (six of
+// the gradient, then the place itself) and per velocity component. Every lane
+// forms the same values in project_inside's order, so the bits are those of
+// redist_apply_move, in a third of its latency (16,700 cycles, chains of
+// lookups).
+__device__ __forceinline__ void redist_apply_move8(const RedistArgs& a, uint32_t p, uint32_t c) {
+    const Grid& g = a.g;
+    const int lane8 = (int)(threadIdx.x & 7);
+    const unsigned team = 0xffu << (threadIdx.x & 24);
+    int i = c % g.nx, j = (c / g.nx) % g.ny, k = c / (g.nx * g.ny);
+    uint64_t key = p;
+    double jx = jitter_mix(key * 3), jy = jitter_mix(key * 3 + 1), jz = jitter_mix(key * 3 + 2);
+    double cx = dadd(g.ox, dmul((double)i + 0.5, g.dx));
+    double cy = dadd(g.oy, dmul((double)j + 0.5, g.dx));
+    double cz = dadd(g.oz, dmul((double)k + 0.5, g.dx));
+    float3 q = make_float3((float)dadd(cx, dmul(jx, g.dx)), (float)dadd(cy, dmul(jy, g.dx)),
+                           (float)dadd(cz, dmul(jz, g.dx)));
+    const float margin = 0.5f * g.dxf, h = a.sdf.dx, d = 2.0f * h;
+    for (int it = 0; it < 3; ++it) {
+        float3 at = q;
+        if (lane8 == 0) at.x = q.x + h;
+        if (lane8 == 1) at.x = q.x - h;
+        if (lane8 == 2) at.y = q.y + h;
+        if (lane8 == 3) at.y = q.y - h;
+        if (lane8 == 4) at.z = q.z + h;
+        if (lane8 == 5) at.z = q.z - h;
+        const float v = sdf_sample(a.sdf, at.x, at.y, at.z);
+        const float phi = __shfl_sync(team, v, 6, 8);
+        const float gx = __shfl_sync(team, v, 0, 8) - __shfl_sync(team, v, 1, 8);
+        const float gy = __shfl_sync(team, v, 2, 8) - __shfl_sync(team, v, 3, 8);
+        const float gz = __shfl_sync(team, v, 4, 8) - __shfl_sync(team, v, 5, 8);
+        if (phi <= -margin) break;  // the same in the eight lanes
+        const float3 n = normalize_or_zero(make_float3(gx / d, gy / d, gz / d));
+        if (sqrtf(n.x * n.x + n.y * n.y + n.z * n.z) == 0.0f) break;
+        const float s = phi + margin;
+        q.x -= n.x * s;
+        q.y -= n.y * s;
+        q.z -= n.z * s;
+    }
+    const float lx = (q.x - g.oxf) / g.dxf, ly = (q.y - g.oyf) / g.dxf, lz = (q.z - g.ozf) / g.dxf;  // velocity_at
+    float v = 0.0f;
+    if (lane8 == 0) v = trilerp(a.f.u, g.nx + 1, g.ny, g.nz, lx, ly - 0.5f, lz - 0.5f);
+    if (lane8 == 1) v = trilerp(a.f.v, g.nx, g.ny + 1, g.nz, lx - 0.5f, ly, lz - 0.5f);
+    if (lane8 == 2) v = trilerp(a.f.w, g.nx, g.ny, g.nz + 1, lx - 0.5f, ly - 0.5f, lz);
+    const float vx = __shfl_sync(team, v, 0, 8), vy = __shfl_sync(team, v, 1, 8), vz = __shfl_sync(team, v, 2, 8);
+    if (lane8 == 0) {
+        a.pos[p] = make_float4(q.x, q.y, q.z, 0.0f);
+        a.vel[p] = make_float4(vx, vy, vz, 0.0f);
+    }
+}
+
 __device__ __forceinline__ uint32_t rd_hash(uint32_t c) { return (c * 2654435761u) & (kRedistTable - 1); }
 
 // One block per sweep: sort the candidates by particle index, insert every
 // referenced cell into a shared hash table, replay the reference's sequential
-// loop (solver.rs:476-555) in rounds and on thread 0, then apply the moves
+// loop (solver.rs:476-555) in rounds and on warp 0, then apply the moves
 // (solver.rs:545-554) with all threads. A list too long for shared memory, or
 // whose cells do not fit the table, goes to k_redist_par (the next launch).
 __device__ __forceinline__ void k_redist_replay_body(VB vb_, RedistArgs a) {
@@ -636,8 +689,23 @@ __device__ __forceinline__ void k_redist_replay_body(VB vb_, RedistArgs a) {
     if (in_smem) {
         uint32_t np2 = 1;
         while (np2 < nc) np2 <<= 1;
-        for (uint32_t t = threadIdx.x; t < np2; t += blockDim.x) scand[t] = t < nc ? a.cand[t] : 0xffffffffu;
-        __syncthreads();
+        if (nc <= kRankSort) {  // one pass: a candidate's place is the number of smaller ones
+            uint32_t* raw = (uint32_t*)slots;  // not in use yet
+            const uint32_t p = threadIdx.x < nc ? a.cand[threadIdx.x] : 0xffffffffu;
+            if (threadIdx.x < nc) raw[threadIdx.x] = p;
+            __syncthreads();
+            if (threadIdx.x < nc) {
+                uint32_t r = 0;
+#pragma unroll 8
+                for (uint32_t t = 0; t < nc; ++t) r += raw[t] < p;
+                scand[r] = p;
+            }
+            __syncthreads();
+            np2 = 1;
+        } else {
+            for (uint32_t t = threadIdx.x; t < np2; t += blockDim.x) scand[t] = t < nc ? a.cand[t] : 0xffffffffu;
+            __syncthreads();
+        }
         for (uint32_t k = 2; k <= np2; k <<= 1)
             for (uint32_t j = k >> 1; j > 0; j >>= 1) {
                 for (uint32_t t = threadIdx.x; t < np2; t += blockDim.x) {
@@ -812,56 +880,82 @@ __device__ __forceinline__ void k_redist_replay_body(VB vb_, RedistArgs a) {
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         uint32_t nm = s_nm;
         if (finish_serial) {
-            // One thread in index order over the candidates no round decided
-            // (all of them without rounds): cheaper than rounds when a few
-            // cells hold most candidates (a fresh jet), whose moves can only
-            // run one per round; the moves are the same.
-            for (uint32_t m = 0; m < nc; ++m) {
-                if (cl[m] & kResolved) continue;
-                const short* sl = slots + (size_t)m * 7;
-                const int s0 = sl[0];
-                if (tcnt[s0] <= cap) continue;
-                int best = -1;
-                double best_down = -INFINITY;
-                uint32_t best_room = 0;
+            // Warp 0 in index order over the candidates no round decided (all of
+            // them without rounds): cheaper than rounds when a few cells hold
+            // most candidates (a fresh jet), whose moves can only run one per
+            // round; the moves are the same. Lanes 1 to 6 look at a candidate's
+            // neighbours. A cell that is back at the cap, or whose neighbours
+            // are full, stays so for the sweep: it is closed (bit 1 of tcav),
+            // and its other candidates are passed over 32 at a time. One thread
+            // looking at every candidate took 100,000 cycles for 800 of them
+            // in a jet, most of closed cells.
+            const int lane = (int)threadIdx.x;
+            double own = 0.0;  // this lane's direction, and how many of the six are less downhill
+            uint32_t rank = 0;
 #pragma unroll
-                for (int q = 1; q < 7; ++q) {
-                    const int sq = sl[q];
-                    if (sq < 0 || !tcav[sq] || tcnt[sq] >= cap) continue;
-                    const uint32_t room = cap - tcnt[sq];
-                    const double dn = a.down[q - 1];
-                    if (best < 0 || dn > best_down || (dn == best_down && room > best_room)) {
-                        best = sq;
-                        best_down = dn;
-                        best_room = room;
+            for (int q = 1; q < 7; ++q)
+                if (q == lane) own = a.down[q - 1];
+#pragma unroll
+            for (int q = 0; q < 6; ++q) rank += a.down[q] < own;
+            for (uint32_t base = 0; base < nc; base += 32) {
+                const uint32_t m = base + lane;
+                const uint32_t p = m < nc ? cl[m] : kResolved;
+                const int s0 = (p & kResolved) ? -1 : (int)slots[(size_t)m * 7];
+                unsigned alive = __ballot_sync(0xffffffffu, s0 >= 0 && !(tcav[max(s0, 0)] & 2));
+                while (alive) {
+                    const int l = __ffs((int)alive) - 1;
+                    const int cell = __shfl_sync(0xffffffffu, s0, l);
+                    const int sq = lane >= 1 && lane <= 6 ? (int)slots[(size_t)(base + l) * 7 + lane] : -1;
+                    const uint32_t c0 = tcnt[cell];
+                    const uint32_t cq = sq >= 0 && (tcav[sq] & 1) ? tcnt[sq] : 0xFFFFFFFFu;
+                    const bool room = cq < cap;
+                    if (c0 <= cap || !__any_sync(0xffffffffu, room)) {
+                        if (lane == 0) tcav[cell] |= 2;
+                        alive &= ~__ballot_sync(0xffffffffu, s0 == cell);
+                        __syncwarp();
+                        continue;
                     }
-                }
-                if (best >= 0) {
-                    tcnt[s0] -= 1;
-                    tcnt[best] += 1;
-                    a.moves[2 * nm] = cl[m];
-                    a.moves[2 * nm + 1] = (uint32_t)tkey[best];
+                    // most downhill, then emptiest, then visit order
+                    const uint32_t top = __reduce_max_sync(0xffffffffu, room ? rank + 1 : 0u);
+                    const bool tied = room && rank + 1 == top;
+                    const uint32_t most = __reduce_max_sync(0xffffffffu, tied ? cap - cq : 0u);
+                    const int best = __ffs((int)__ballot_sync(0xffffffffu, tied && cap - cq == most)) - 1;
+                    const uint32_t who = __shfl_sync(0xffffffffu, p, l);
+                    if (lane == best) {
+                        tcnt[sq] = cq + 1;
+                        a.moves[2 * nm] = who;
+                        a.moves[2 * nm + 1] = (uint32_t)tkey[sq];
+                    }
+                    if (lane == 0) tcnt[cell] = c0 - 1;
                     ++nm;
+                    alive &= alive - 1;
+                    __syncwarp();
                 }
             }
         }
-        s_nm = nm;
-        rs->nmoves = nm;
-        rs->moves_total += nm;
-        rs->cand_total += nc;
-        rs->sweeps_total += 1;
-        rs->long_total += in_smem ? 0 : 1;
-        rs->ncand = 0;
-        if (nm == 0) rs->active = 0;
+        if (threadIdx.x == 0) {
+            s_nm = nm;
+            rs->nmoves = nm;
+            rs->moves_total += nm;
+            rs->cand_total += nc;
+            rs->sweeps_total += 1;
+            rs->long_total += in_smem ? 0 : 1;
+            rs->ncand = 0;
+            if (nm == 0) rs->active = 0;
+        }
     }
     __syncthreads();
     // ---- apply the moves: near the destination centre with the index-keyed
     // jitter, pushed inside, with the local grid velocity.
     const uint32_t nm = s_nm;
-    for (uint32_t mv = threadIdx.x; mv < nm; mv += blockDim.x) redist_apply_move(a, a.moves[2 * mv], a.moves[2 * mv + 1]);
+    if (nm <= 4 * (kRedistBS / 8)) {  // few: the lookups of a move side by side
+        for (uint32_t mv = threadIdx.x / 8; mv < nm; mv += kRedistBS / 8) redist_apply_move8(a, a.moves[2 * mv], a.moves[2 * mv + 1]);
+    } else {
+        for (uint32_t mv = threadIdx.x; mv < nm; mv += blockDim.x) redist_apply_move(a, a.moves[2 * mv], a.moves[2 * mv + 1]);
+    }
 }
 __global__ void __launch_bounds__(kRedistBS, 1) k_redist_replay(RedistArgs a) { k_redist_replay_body(VB{blockIdx.x, gridDim.x}, a); }
 
