@@ -164,14 +164,32 @@ __device__ __forceinline__ bool solid_at(const Grid& g, const uint8_t* cells, in
     return cells[((size_t)k * g.ny + j) * g.nx + i] == SOLID;
 }
 
-// Flat node index -> (i, j, k) over (nx+1) x (ny+1) x (nz+1).
+// Flat node index -> (i, j, k) over (nx+1) x (ny+1) x (nz+1), below 2^31
+// (sdr_solver_create bounds the cells): 32-bit divisions, the 64-bit ones took
+// most of the node kernels' time.
 __device__ __forceinline__ bool node_of(const Grid& g, size_t t, int& i, int& j, int& k) {
-    size_t nxp = (size_t)g.nx + 1, nyp = (size_t)g.ny + 1;
-    if (t >= nxp * nyp * ((size_t)g.nz + 1)) return false;
-    i = (int)(t % nxp);
-    j = (int)((t / nxp) % nyp);
-    k = (int)(t / (nxp * nyp));
+    const uint32_t nxp = (uint32_t)g.nx + 1u, nyp = (uint32_t)g.ny + 1u;
+    const uint32_t q = (uint32_t)t;
+    if (t >= (size_t)nxp * nyp * ((size_t)g.nz + 1)) return false;
+    const uint32_t row = q / nxp, l = row / nyp;
+    i = (int)(q - row * nxp);
+    j = (int)(row - l * nyp);
+    k = (int)l;
     return true;
+}
+
+// Bricks of 8 x 8 x 8 nodes, one per block of kBS threads (two nodes each):
+// work that only the nodes near the liquid have is skipped a brick at a time.
+constexpr int kBrick = 8;
+static_assert(kBS == kBrick * kBrick * 4, "two nodes of a brick per thread");
+struct BrickPos {
+    int i0, j0, k0;  // first node
+};
+__host__ __device__ __forceinline__ int brick_dim(int cells) { return (cells + kBrick) / kBrick; }  // of cells + 1 nodes
+__device__ __forceinline__ BrickPos brick_of(const Grid& g, uint32_t b) {
+    const uint32_t bx = (uint32_t)brick_dim(g.nx), by = (uint32_t)brick_dim(g.ny);
+    const uint32_t row = b / bx, l = row / by;
+    return BrickPos{(int)(b - row * bx) * kBrick, (int)(row - l * by) * kBrick, (int)l * kBrick};
 }
 
 // clamp_base (grid.rs:25-34) in f64 and the weight of node `i` (0 if not a corner).
@@ -225,25 +243,40 @@ __device__ __forceinline__ void p2g_store(const P2GArgs& a, int i, int j, int k,
 }
 
 
-// P2G, first pass: one thread per grid node (i,j,k) in [0,nx]x[0,ny]x[0,nz]
-// (the node owns the u, v and w faces with that index). A node with no
-// particle in the 27 cells around it gets its faces at once (all sums +0);
-// the others are queued for k_p2g.
+// P2G, first pass, a block per brick: every node (i,j,k) in [0,nx]x[0,ny]x[0,nz]
+// owns the u, v and w faces with that index. A node with no particle in the 27
+// cells around it gets its faces at once (all sums +0); the others are queued
+// for k_p2g. A brick with no particle in the 10 x 10 x 10 cells around it asks
+// for nothing per node.
 __device__ __forceinline__ void k_p2g_nodes_body(VB vb_, P2GArgs a, uint32_t* __restrict__ list,
                                                    uint32_t* __restrict__ count) {
     const Grid& g = a.g;
-    const size_t t = (size_t)vb_.bid * blockDim.x + threadIdx.x;
-    int i, j, k;
-    if (!node_of(g, t, i, j, k)) return;
-    uint32_t cnt = 0;
-    const int ci0 = max(i - 1, 0), ci1 = min(i + 1, g.nx - 1);
-    for (int ck = max(k - 1, 0); ck <= min(k + 1, g.nz - 1); ++ck)
-        for (int cj = max(j - 1, 0); cj <= min(j + 1, g.ny - 1); ++cj) {
+    const BrickPos b = brick_of(g, vb_.bid);
+    const int tid = (int)threadIdx.x;
+    uint32_t some = 0;
+    if (tid < 100) {
+        const int cj = b.j0 - 1 + tid % 10, ck = b.k0 - 1 + tid / 10;
+        if (cj >= 0 && cj < g.ny && ck >= 0 && ck < g.nz) {
             const uint32_t c = ((uint32_t)ck * g.ny + cj) * g.nx;
-            cnt += a.start[c + ci1 + 1] - a.start[c + ci0];
+            some = a.start[c + min(b.i0 + kBrick, g.nx - 1) + 1] - a.start[c + max(b.i0 - 1, 0)];
         }
-    if (cnt) list[atomicAdd(count, 1u)] = (uint32_t)t;
-    else p2g_store(a, i, j, k, j < g.ny && k < g.nz, i < g.nx && k < g.nz, i < g.nx && j < g.ny, 0, 0, 0, 0, 0, 0);
+    }
+    const bool any = __syncthreads_or(some != 0);
+    for (int h = 0; h < 2; ++h) {
+        const int i = b.i0 + tid % kBrick, j = b.j0 + tid / kBrick % kBrick, k = b.k0 + tid / (kBrick * kBrick) + 4 * h;
+        if (i > g.nx || j > g.ny || k > g.nz) continue;
+        uint32_t cnt = 0;
+        if (any) {
+            const int ci0 = max(i - 1, 0), ci1 = min(i + 1, g.nx - 1);
+            for (int ck = max(k - 1, 0); ck <= min(k + 1, g.nz - 1); ++ck)
+                for (int cj = max(j - 1, 0); cj <= min(j + 1, g.ny - 1); ++cj) {
+                    const uint32_t c = ((uint32_t)ck * g.ny + cj) * g.nx;
+                    cnt += a.start[c + ci1 + 1] - a.start[c + ci0];
+                }
+        }
+        if (cnt) list[atomicAdd(count, 1u)] = (uint32_t)(((size_t)k * (g.ny + 1) + j) * (g.nx + 1) + i);
+        else p2g_store(a, i, j, k, j < g.ny && k < g.nz, i < g.nx && k < g.nz, i < g.nx && j < g.ny, 0, 0, 0, 0, 0, 0);
+    }
 }
 __global__ void __launch_bounds__(kBS) k_p2g_nodes(P2GArgs a, uint32_t* __restrict__ list,
                                                    uint32_t* __restrict__ count) { k_p2g_nodes_body(VB{blockIdx.x, gridDim.x}, a, list, count); }
@@ -786,7 +819,7 @@ __device__ __forceinline__ void k_redist_replay_body(VB vb_, RedistArgs a) {
     // candidates touch are disjoint, so the moves are the sequential ones.
     // Candidates crowded into a few cells (a fresh jet) decide about one per
     // cell and round: once a round decides fewer than kRoundsMinDecided,
-    // thread 0 decides the pending rest in index order (below). Every
+    // warp 0 decides the pending rest in index order (below). Every
     // candidate decided in a round held its cells against all lower pending
     // ones, so the rest in index order sees the counts the sequential loop sees.
     const uint32_t cap = a.cap;

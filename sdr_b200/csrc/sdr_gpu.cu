@@ -318,7 +318,7 @@ SDR_OP(k_corder, 256)
 SDR_OP(k_pcg, kPcgBS)
 SDR_OP(k_gradient, 256)
 SDR_OP(k_extrap_valid, 256)
-SDR_OP(k_extrap, 256)
+SDR_OP(k_extrap, kBS)
 SDR_OP(k_face_max, 256)
 SDR_OP(k_g2p_advect, kBS)
 SDR_OP(k_bounds_flags, kBS)
@@ -416,6 +416,8 @@ struct sdr_solver {
     float* sdf32 = nullptr;
     float *u = nullptr, *v = nullptr, *w = nullptr, *su = nullptr, *sv = nullptr, *sw = nullptr;
     uint8_t *ku = nullptr, *kv = nullptr, *kw = nullptr;  // extrapolation: when each face became known
+    uint32_t* brick = nullptr;   // per brick of nodes: the last extrapolation in which it had a fluid cell
+    uint32_t extrap_epoch = 0;   // extrapolations so far
     uint8_t *cells = nullptr, *base = nullptr, *cavity = nullptr;
     float4 *pos = nullptr, *vel = nullptr, *pos2 = nullptr, *vel2 = nullptr;
     int* key_cell = nullptr;
@@ -548,6 +550,7 @@ struct sdr_solver {
     SdfD sdf_d() const { return SdfD{snx, sny, snz, sdx, sox, soy, soz, sdf64}; }
     Faces faces() const { return Faces{u, v, w}; }
     size_t nnodes() const { return ((size_t)g.nx + 1) * ((size_t)g.ny + 1) * ((size_t)g.nz + 1); }
+    unsigned nbricks() const { return (unsigned)brick_dim(g.nx) * (unsigned)brick_dim(g.ny) * (unsigned)brick_dim(g.nz); }
     Faces saved() const { return Faces{su, sv, sw}; }
     uint32_t* dn() { return &dst->n; }
 
@@ -611,6 +614,8 @@ struct sdr_solver {
         dalloc(su, nu, st); dalloc(sv, nv, st); dalloc(sw, nw, st);
         dalloc(p2g_list, nnodes(), st);
         dalloc(ku, nu, st); dalloc(kv, nv, st); dalloc(kw, nw, st);
+        dalloc(brick, nbricks(), st);
+        CK(cudaMemsetAsync(brick, 0, nbricks() * 4, st));
         CK(cudaMemsetAsync(u, 0, nu * 4, st));
         CK(cudaMemsetAsync(v, 0, nv * 4, st));
         CK(cudaMemsetAsync(w, 0, nw * 4, st));
@@ -658,7 +663,7 @@ struct sdr_solver {
     void free_all() {
         dfree(sdf64, st); dfree(sdf32, st);
         dfree(u, st); dfree(v, st); dfree(w, st); dfree(su, st); dfree(sv, st); dfree(sw, st);
-        dfree(ku, st); dfree(kv, st); dfree(kw, st);
+        dfree(ku, st); dfree(kv, st); dfree(kw, st); dfree(brick, st);
         dfree(cells, st); dfree(base, st); dfree(cavity, st);
         dfree(pos, st); dfree(vel, st); dfree(pos2, st); dfree(vel2, st);
         dfree(key_cell, st); dfree(key_sort, st); dfree(perm, st); dfree(ptmp, st); dfree(flag, st); dfree(off, st); dfree(drn, st);
@@ -775,7 +780,7 @@ struct sdr_solver {
         // empty nodes at once, the rest queued for the eight-lane gather; its grid
         // follows the last queue length (the loop over the queue covers any length)
         MSET(&dst->p2g_queue, 0, 4);
-        SLAUNCH(k_p2g_nodes, blocks(nnodes(), kBS), kBS, 0, st, a, p2g_list, &dst->p2g_queue);
+        SLAUNCH(k_p2g_nodes, nbricks(), kBS, 0, st, a, p2g_list, &dst->p2g_queue);
         const size_t want = last_p2g_queue ? ((size_t)last_p2g_queue + last_p2g_queue / 4 + 64) * kP2GLanes
                                            : nnodes() * kP2GLanes;  // no history yet: every node
         SLAUNCH(k_p2g, (unsigned)std::min<size_t>(blocks(want, kBS), 148 * 16), kBS, 0, st, a, p2g_list,
@@ -1016,11 +1021,12 @@ struct sdr_solver {
 
     void extrapolate() {  // solver.rs:608-647
         unsigned ngrid = blocks(nnodes(), 256);
-        SLAUNCH(k_extrap_valid, ngrid, 256, 0, st, g, cells, ku, kv, kw);
+        ++extrap_epoch;
+        SLAUNCH(k_extrap_valid, ngrid, 256, 0, st, g, cells, ku, kv, kw, brick, extrap_epoch);
         MSET(dst->maxbits, 0, sizeof(dst->maxbits));
         for (int it = 0; it < 4; ++it) {  // four sweeps, in place
-            ExtrapArgs e{g, u, v, w, ku, kv, kw, it, it == 3 ? dst->maxbits : nullptr};
-            SLAUNCH(k_extrap, ngrid, 256, 0, st, e);
+            ExtrapArgs e{g, u, v, w, ku, kv, kw, it, it == 3 ? dst->maxbits : nullptr, brick, extrap_epoch};
+            SLAUNCH(k_extrap, nbricks(), kBS, 0, st, e);
         }
     }
 
