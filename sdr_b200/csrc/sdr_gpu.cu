@@ -1563,11 +1563,13 @@ int sdr_solver_create(const sdr_sdf_desc* sdf, double sim_dx, const sdr_fluid_pa
         sdr_solver* s = new sdr_solver();
         try {
             CK(cudaGetDevice(&s->device));
-            cudaDeviceProp prop;
-            CK(cudaGetDeviceProperties(&prop, s->device));
-            if (prop.major != 10)
+            // two attributes: the whole property block takes the driver milliseconds, most of a small scene's set-up
+            int major = 0, minor = 0;
+            CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, s->device));
+            CK(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, s->device));
+            if (major != 10)
                 throw Fail{SDR_ERR_NO_DEVICE, "this library is built for sm_100a (B200); device is sm_" +
-                                                  std::to_string(prop.major) + std::to_string(prop.minor)};
+                                                  std::to_string(major) + std::to_string(minor)};
             if (g_engine_stream) {
                 s->st = g_engine_stream;
                 s->own_stream = false;
@@ -2403,7 +2405,6 @@ int sdr_sdf_from_mesh(const double* tris, size_t ntri, sdr_vec3 origin, double d
         cleanup();
     });
 }
-
 int sdr_sdf_from_mesh_noalloc(const double* tris_dev, size_t ntri, sdr_vec3 origin, double dx,
                               const uint64_t dims[3], double* out_dev, void* stream) {
     return guard([&] {
