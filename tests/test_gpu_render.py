@@ -102,3 +102,24 @@ def test_render_dense_pool_matches_oracle():
             diff = int((got != ref).any(axis=2).sum())
             record(f"render_dense_{name}_{px}", {"particles": int(len(pos)), "pixels_differing": diff})
             assert diff == 0, (name, px)
+
+
+@pytest.mark.parametrize("px", [40, 333, 2700])
+def test_render_amber_pixel_blocks(px):
+    """The amber pool where its pixel blocks change shape: splats of 3 px (a
+    tile smaller than a block), 4 px, and 34 px (tiles of several blocks, weights
+    computed instead of tabled), with thousands of particles over a few pixels
+    (lists taken in many pieces, pixels that stop early) beside sparse ones."""
+    from tests.gpu_common import f32
+    gpu, orc, res = make_pair(SHORT_RUN)
+    st = gpu.stats()
+    org = np.array([st.origin.x, st.origin.y, st.origin.z])
+    span = np.array(gpu.grid_dims) * gpu.dx
+    rng = np.random.default_rng(px)
+    clump = org + 0.5 * span + rng.normal(0.0, 0.02, (6000, 3)) * span
+    spread = org + rng.uniform(0.0, 1.0, (400, 3)) * span
+    pos = f32(rng.permutation(np.concatenate([clump, spread])))
+    for s in (gpu, orc):
+        s.set_particles(pos, np.zeros_like(pos))
+    plane = _planes(res)["gravity"]
+    assert np.array_equal(render_slice(gpu, plane, px, 0.0), orc.render_slice(plane.as_dict(), px, 0.0))
