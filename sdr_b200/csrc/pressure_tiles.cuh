@@ -766,9 +766,6 @@ __device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, uint32_t& us
         double ra = lds_f64<kRev * kRow>(o), pc = lds_f64<kRev * kRow + kTwDepth * kRow>(o);
         uint32_t at = fwd ? 0u : lds_u32<kRev * kRow / 2>(oi);
         double* qout = t.qr + row0 + line;
-        double result = 0.0;  // the level before's q or z,
-        bool owed = false;    // if the line had a cell there,
-        uint32_t at_p = 0u;   // and z's place
         for (int q0 = 0; q0 < nlev; q0 += kTwGroup) {
             // the next group's operands
             const uint32_t gn = (uint32_t)(q0 / kTwGroup + 1) & (kTwGroups - 1);
@@ -782,52 +779,41 @@ __device__ __forceinline__ void tw_sweep(const TwArgs& t, int tile, uint32_t& us
                 tw_bar();
                 const uint32_t wr = w0 + ((u + 1) & 1) * kWin;
                 const double vy = lds_f64<-8>(wr), vz = lds_f64<-8 * kTwPitch>(wr);
-                // level q + 1's operands (past the last level: values nobody uses)
-                constexpr int kM = kTwGroup - 1;
-                const uint32_t os = (u < kM ? o : on) + (uint32_t)(((u + 1) & kM) ^ kRev) * kRow;
-                const double ra_n = lds_f64<0>(os), pc_n = lds_f64<kTwDepth * kRow>(os);
-                const uint32_t at_n =
-                    fwd ? 0u : lds_u32<0>((u < kM ? oi : oin) + (uint32_t)(((u + 1) & kM) ^ kRev) * (kRow / 2));
-                // the level before's result goes out while these loads run
-                if (MODE == TW_FORWARD) {
-                    if (owed) qout[(u - 1) * kTwLines] = result;
-                } else if (owed) {
-                    a.z[at_p] = result;
-                    if (a.exact_dots)  // the reference dot order is over cells in cell order
-                        a.prod[a.cinv[at_p]] = dmul(result, __ldcg(a.r + at_p));
-                }
                 const bool cell = __double2hiint(pc) >= 0;
-                double out;
+                double out, result;
                 if (MODE == TW_FORWARD) {
                     // t = r + pq[-x] + pq[-y] + pq[-z]; q = t * pc (pcg_apply_mic0, forward)
-                    const double qv = dmul(dadd(dadd(dadd(ra, carry), vy), vz), pc);
-                    out = cell ? dmul(pc, qv) : -0.0;
-                    result = qv;
+                    result = dmul(dadd(dadd(dadd(ra, carry), vy), vz), pc);
+                    out = cell ? dmul(pc, result) : -0.0;
                 } else {
                     // t = q + pc z[+x] + pc z[+y] + pc z[+z]; z = t * pc (pcg_apply_mic0, backward)
-                    const double zv = dmul(dadd(dadd(dadd(ra, dmul(pc, carry)), dmul(pc, vy)), dmul(pc, vz)), pc);
-                    out = cell ? zv : -0.0;
-                    result = zv;
-                    at_p = at;
+                    result = dmul(dadd(dadd(dadd(ra, dmul(pc, carry)), dmul(pc, vy)), dmul(pc, vz)), pc);
+                    out = cell ? result : -0.0;
                 }
                 sts_f64(w0 + (u & 1) * kWin, out);
                 pass_on(u, out);
-                owed = cell;
                 carry = out;
-                ra = ra_n;
-                pc = pc_n;
-                at = at_n;
+                // off the chain: level q + 1's operands (past the last level values
+                // nobody uses) and the result
+                constexpr int kM = kTwGroup - 1;
+                const uint32_t os = (u < kM ? o : on) + (uint32_t)(((u + 1) & kM) ^ kRev) * kRow;
+                ra = lds_f64<0>(os);
+                pc = lds_f64<kTwDepth * kRow>(os);
+                if (MODE == TW_FORWARD) {
+                    if (cell) qout[u * kTwLines] = result;
+                } else {
+                    if (cell) {
+                        a.z[at] = result;
+                        if (a.exact_dots)  // the reference dot order is over cells in cell order
+                            a.prod[a.cinv[at]] = dmul(result, __ldcg(a.r + at));
+                    }
+                    at = lds_u32<0>((u < kM ? oi : oin) + (uint32_t)(((u + 1) & kM) ^ kRev) * (kRow / 2));
+                }
             }
             o = on;
             oi = oin;
             qout += kTwGroup * kTwLines;
             next_group();
-        }
-        const int last = (nlev - 1) % kTwGroup - kTwGroup;  // qout is a group past the last level's
-        if (owed && MODE == TW_FORWARD) qout[last * kTwLines] = result;
-        if (owed && MODE == TW_BACKWARD) {
-            a.z[at_p] = result;
-            if (a.exact_dots) a.prod[a.cinv[at_p]] = dmul(result, __ldcg(a.r + at_p));
         }
     }
     if (MODE != TW_BUILD && a.timing && tid == 0) {  // per tile: level-loop cycles, levels, sweeps
