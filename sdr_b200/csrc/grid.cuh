@@ -77,8 +77,8 @@ __global__ void k_cavity_and_base(Grid g, SdfD s, int has_outlet, Aabb outlet,
                                   int recompute_cavity) { k_cavity_and_base_body(VB{blockIdx.x, gridDim.x}, g, s, has_outlet, outlet, cavity, base, recompute_cavity); }
 
 // Validity for extrapolation: the face borders a Fluid cell (solver.rs:612-642).
-// Bricks of nodes with a fluid cell get this extrapolation's number: four sweeps
-// reach five nodes from one, so no further than the bricks beside it.
+// Bricks of nodes that four sweeps can reach from a fluid cell (four nodes before
+// it to five behind it, so at most two a direction) get this extrapolation's number.
 __device__ __forceinline__ void k_extrap_valid_body(VB vb_, Grid g, const uint8_t* __restrict__ cells, uint8_t* __restrict__ ku,
                                uint8_t* __restrict__ kv, uint8_t* __restrict__ kw, uint32_t* __restrict__ brick, uint32_t epoch) {
     int i, j, k;
@@ -91,15 +91,22 @@ __device__ __forceinline__ void k_extrap_valid_body(VB vb_, Grid g, const uint8_
     if (i < g.nx && k < g.nz) kv[((size_t)k * (g.ny + 1) + j) * g.nx + i] = own || (j > 0 && fl(i, j - 1, k));
     if (i < g.nx && j < g.ny) kw[((size_t)k * g.ny + j) * g.nx + i] = own || (k > 0 && fl(i, j, k - 1));
     if (own) {
-        uint32_t* const f = brick + ((size_t)(k / kBrick) * brick_dim(g.ny) + j / kBrick) * brick_dim(g.nx) + i / kBrick;
-        if (*f != epoch) *f = epoch;
+        const int bx = brick_dim(g.nx), by = brick_dim(g.ny), bz = brick_dim(g.nz);
+        const int i0 = max(i - 4, 0) / kBrick, j0 = max(j - 4, 0) / kBrick, k0 = max(k - 4, 0) / kBrick;
+        const int i1 = min((i + 5) / kBrick, bx - 1), j1 = min((j + 5) / kBrick, by - 1), k1 = min((k + 5) / kBrick, bz - 1);
+        for (int c = k0; c <= k1; ++c)
+            for (int b = j0; b <= j1; ++b)
+                for (int a = i0; a <= i1; ++a) {
+                    uint32_t* const f = brick + ((size_t)c * by + b) * bx + a;
+                    if (*f != epoch) *f = epoch;
+                }
     }
 }
 __global__ void k_extrap_valid(Grid g, const uint8_t* __restrict__ cells, uint8_t* __restrict__ ku,
                                uint8_t* __restrict__ kv, uint8_t* __restrict__ kw, uint32_t* __restrict__ brick,
                                uint32_t epoch) { k_extrap_valid_body(VB{blockIdx.x, gridDim.x}, g, cells, ku, kv, kw, brick, epoch); }
 
-// One snapshot sweep of extrapolate (solver.rs:964-1007) on one component,
+// One snapshot sweep of extrapolate (solver.rs:964-1007) on one unknown face,
 // in place. kn holds 0 for unknown, 1 for known from the start and s + 2 for
 // a face that became known in sweep s; sweep s reads only faces known before
 // it, whose values no longer change, so every face sees the snapshot the
@@ -109,23 +116,25 @@ __global__ void k_extrap_valid(Grid g, const uint8_t* __restrict__ cells, uint8_
 __device__ __forceinline__ void extrap_one(float* __restrict__ f, uint8_t* __restrict__ kn, int sweep, int nx,
                                            int ny, int nz, int i, int j, int k) {
     const size_t c = ((size_t)k * ny + j) * nx + i;
-    if (kn[c]) return;
-    const int before = sweep + 1;  // kn in [1, before]: known before this sweep
-    auto known = [&](size_t q) {
-        const int v = kn[q];
-        return v != 0 && v <= before;
-    };
-    float sum = 0.0f;
-    int cnt = 0;
+    // The six bytes side by side, then the values: one after another, as the
+    // conditions come, a face is a chain of up to twelve round trips.
     const size_t sy = nx, sz = (size_t)nx * ny;
-    if (i > 0 && known(c - 1)) { sum += f[c - 1]; ++cnt; }
-    if (i + 1 < nx && known(c + 1)) { sum += f[c + 1]; ++cnt; }
-    if (j > 0 && known(c - sy)) { sum += f[c - sy]; ++cnt; }
-    if (j + 1 < ny && known(c + sy)) { sum += f[c + sy]; ++cnt; }
-    if (k > 0 && known(c - sz)) { sum += f[c - sz]; ++cnt; }
-    if (k + 1 < nz && known(c + sz)) { sum += f[c + sz]; ++cnt; }
+    const bool in[6] = {i > 0, i + 1 < nx, j > 0, j + 1 < ny, k > 0, k + 1 < nz};
+    const size_t at[6] = {c - 1, c + 1, c - sy, c + sy, c - sz, c + sz};
+    uint8_t nk[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) nk[q] = in[q] ? kn[at[q]] : (uint8_t)0;
+    float fv[6];
+    int cnt = 0;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        // in [1, sweep + 1]: known before this sweep
+        const bool known = nk[q] != 0 && nk[q] <= sweep + 1;
+        fv[q] = known ? f[at[q]] : 0.0f;  // a sum from +0 is never -0: adding +0 changes no bit
+        cnt += known;
+    }
     if (cnt > 0) {
-        f[c] = sum / (float)cnt;
+        f[c] = (((((0.0f + fv[0]) + fv[1]) + fv[2]) + fv[3]) + fv[4] + fv[5]) / (float)cnt;
         kn[c] = (uint8_t)(sweep + 2);
     }
 }
@@ -140,57 +149,55 @@ struct ExtrapArgs {
     uint8_t* kw;
     int sweep;              // 0..3
     unsigned int* maxbits;  // optional: |u|,|v|,|w| maxima (last sweep)
-    const uint32_t* brick;  // per brick of nodes: the last extrapolation in which it had a fluid cell
+    const uint32_t* brick;  // per brick of nodes: the last extrapolation that reached it
     uint32_t epoch;         // this extrapolation's number
 };
 
-// A block per brick. One without a fluid cell in it or beside it has nothing to
-// extrapolate (its faces only count for the maxima): in a 0.2 mm pool that is
-// two thirds of the nodes, before the jet has filled a cavity nearly all.
+// A block per brick. One out of the liquid's reach has nothing to extrapolate
+// (its faces only count for the maxima): in a 0.2 mm pool that is two thirds of
+// the nodes, before the jet has filled a cavity nearly all. With the gradient,
+// at 2 mm 65 -> 46 us and in the pool 522 -> 359 us against a test of the 27
+// bricks around, two nodes a thread and every warp's maxima in atomics: small
+// scenes wait for round trips, the pool's last sweep queued on the atomics.
 __device__ __forceinline__ void k_extrap_body(VB vb_, ExtrapArgs a) {
     const Grid& g = a.g;
+    const bool near = a.brick[vb_.bid] == a.epoch;
+    if (!near && !a.maxbits) return;
     const BrickPos b = brick_of(g, vb_.bid);
     const int tid = (int)threadIdx.x;
-    bool some = false;
-    if (tid < 27) {
-        const int bi = b.i0 / kBrick + tid % 3 - 1, bj = b.j0 / kBrick + tid / 3 % 3 - 1, bk = b.k0 / kBrick + tid / 9 - 1;
-        const int bx = brick_dim(g.nx), by = brick_dim(g.ny), bz = brick_dim(g.nz);
-        if (bi >= 0 && bj >= 0 && bk >= 0 && bi < bx && bj < by && bk < bz)
-            some = a.brick[((size_t)bk * by + bj) * bx + bi] == a.epoch;
-    }
-    const bool near = __syncthreads_or(some);
-    if (!near && !a.maxbits) return;
-    float mu = 0.f, mv = 0.f, mw = 0.f;
-    for (int h = 0; h < 2; ++h) {
-        const int i = b.i0 + tid % kBrick, j = b.j0 + tid / kBrick % kBrick, k = b.k0 + tid / (kBrick * kBrick) + 4 * h;
-        if (j < g.ny && k < g.nz && i <= g.nx) {
-            if (near) extrap_one(a.u, a.ku, a.sweep, g.nx + 1, g.ny, g.nz, i, j, k);
-            if (a.maxbits) mu = fmaxf(mu, fabsf(a.u[((size_t)k * g.ny + j) * (g.nx + 1) + i]));
-        }
-        if (i < g.nx && k < g.nz && j <= g.ny) {
-            if (near) extrap_one(a.v, a.kv, a.sweep, g.nx, g.ny + 1, g.nz, i, j, k);
-            if (a.maxbits) mv = fmaxf(mv, fabsf(a.v[((size_t)k * (g.ny + 1) + j) * g.nx + i]));
-        }
-        if (i < g.nx && j < g.ny && k <= g.nz) {
-            if (near) extrap_one(a.w, a.kw, a.sweep, g.nx, g.ny, g.nz + 1, i, j, k);
-            if (a.maxbits) mw = fmaxf(mw, fabsf(a.w[((size_t)k * g.ny + j) * g.nx + i]));
-        }
+    const int i = b.i0 + tid % kBrick, j = b.j0 + tid / kBrick % kBrick, k = b.k0 + tid / (kBrick * kBrick);
+    const bool hu = j < g.ny && k < g.nz && i <= g.nx, hv = i < g.nx && k < g.nz && j <= g.ny, hw = i < g.nx && j < g.ny && k <= g.nz;
+    const size_t cu = ((size_t)k * g.ny + j) * (g.nx + 1) + i, cv = ((size_t)k * (g.ny + 1) + j) * g.nx + i,
+                 cw = ((size_t)k * g.ny + j) * g.nx + i;
+    if (near) {
+        const bool du = hu && !a.ku[cu], dv = hv && !a.kv[cv], dw = hw && !a.kw[cw];  // not known yet
+        if (du) extrap_one(a.u, a.ku, a.sweep, g.nx + 1, g.ny, g.nz, i, j, k);
+        if (dv) extrap_one(a.v, a.kv, a.sweep, g.nx, g.ny + 1, g.nz, i, j, k);
+        if (dw) extrap_one(a.w, a.kw, a.sweep, g.nx, g.ny, g.nz + 1, i, j, k);
     }
     if (a.maxbits) {
-        // Non-negative floats order like their bit patterns: exact max via atomicMax.
-        for (int o = 16; o > 0; o >>= 1) {
-            mu = fmaxf(mu, __shfl_xor_sync(0xffffffffu, mu, o));
-            mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-            mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+        // Non-negative floats order like their bit patterns (a NaN counts as 0):
+        // an exact maximum per warp, block and grid. One block's atomics at most,
+        // and only for a larger value: of every warp, they queued on three words.
+        __shared__ uint32_t s_max[3][kBrickBS / 32];
+        const float m[3] = {fmaxf(0.f, hu ? fabsf(a.u[cu]) : 0.f), fmaxf(0.f, hv ? fabsf(a.v[cv]) : 0.f),
+                            fmaxf(0.f, hw ? fabsf(a.w[cw]) : 0.f)};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m[c]));
+            if ((tid & 31) == 0) s_max[c][tid / 32] = w;
         }
-        if ((threadIdx.x & 31) == 0) {
-            atomicMax(&a.maxbits[0], __float_as_uint(mu));
-            atomicMax(&a.maxbits[1], __float_as_uint(mv));
-            atomicMax(&a.maxbits[2], __float_as_uint(mw));
+        __syncthreads();
+        if (tid < 32) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const uint32_t w = __reduce_max_sync(0xffffffffu, s_max[c][tid % (kBrickBS / 32)]);
+                if (tid == 0 && w > __ldcg(a.maxbits + c)) atomicMax(a.maxbits + c, w);
+            }
         }
     }
 }
-__global__ void __launch_bounds__(256) k_extrap(ExtrapArgs a) { k_extrap_body(VB{blockIdx.x, gridDim.x}, a); }
+__global__ void __launch_bounds__(kBrickBS) k_extrap(ExtrapArgs a) { k_extrap_body(VB{blockIdx.x, gridDim.x}, a); }
 
 // Face maxima alone (used when extrapolation did not run, e.g. phase mode).
 __device__ __forceinline__ void k_face_max_body(VB vb_, const float* __restrict__ f, size_t n, unsigned int* __restrict__ out) {

@@ -305,7 +305,7 @@ SDR_OP(k_sort_scatter, kBS)
 SDR_OP(k_sort_segments, 256)
 SDR_OP(k_sort_long, 256)
 SDR_OP(k_sorted_records, kBS)
-SDR_OP(k_p2g_nodes, kBS)
+SDR_OP(k_p2g_nodes, kBrickBS)
 SDR_OP(k_p2g, kBS)
 SDR_OP(k_add_forces, 256)
 SDR_OP(k_enforce_solid, 256)
@@ -318,7 +318,7 @@ SDR_OP(k_corder, 256)
 SDR_OP(k_pcg, kPcgBS)
 SDR_OP(k_gradient, 256)
 SDR_OP(k_extrap_valid, 256)
-SDR_OP(k_extrap, kBS)
+SDR_OP(k_extrap, kBrickBS)
 SDR_OP(k_face_max, 256)
 SDR_OP(k_g2p_advect, kBS)
 SDR_OP(k_bounds_flags, kBS)
@@ -780,7 +780,7 @@ struct sdr_solver {
         // empty nodes at once, the rest queued for the eight-lane gather; its grid
         // follows the last queue length (the loop over the queue covers any length)
         MSET(&dst->p2g_queue, 0, 4);
-        SLAUNCH(k_p2g_nodes, nbricks(), kBS, 0, st, a, p2g_list, &dst->p2g_queue);
+        SLAUNCH(k_p2g_nodes, nbricks(), kBrickBS, 0, st, a, p2g_list, &dst->p2g_queue);
         const size_t want = last_p2g_queue ? ((size_t)last_p2g_queue + last_p2g_queue / 4 + 64) * kP2GLanes
                                            : nnodes() * kP2GLanes;  // no history yet: every node
         SLAUNCH(k_p2g, (unsigned)std::min<size_t>(blocks(want, kBS), 148 * 16), kBS, 0, st, a, p2g_list,
@@ -1026,7 +1026,7 @@ struct sdr_solver {
         MSET(dst->maxbits, 0, sizeof(dst->maxbits));
         for (int it = 0; it < 4; ++it) {  // four sweeps, in place
             ExtrapArgs e{g, u, v, w, ku, kv, kw, it, it == 3 ? dst->maxbits : nullptr, brick, extrap_epoch};
-            SLAUNCH(k_extrap, nbricks(), kBS, 0, st, e);
+            SLAUNCH(k_extrap, nbricks(), kBrickBS, 0, st, e);
         }
     }
 
