@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kScanBS) k_scan_sums(uint32_t* __restrict__ su
 
 __device__ __forceinline__ void k_scan_apply_body(VB vb_, const uint32_t* __restrict__ in, uint32_t n,
                                                        const uint32_t* __restrict__ tile_off,
-                                                       uint32_t* __restrict__ out) {
+                                                       uint32_t* __restrict__ out, uint32_t* __restrict__ out2) {
     __shared__ uint32_t sh[33];
     size_t base = (size_t)vb_.bid * kScanTile + (size_t)threadIdx.x * kScanIPT;
     uint32_t v[kScanIPT];
@@ -87,12 +87,15 @@ __device__ __forceinline__ void k_scan_apply_body(VB vb_, const uint32_t* __rest
     uint32_t run = tile_off[vb_.bid] + ex;
 #pragma unroll
     for (int q = 0; q < kScanIPT; ++q) {
-        if (base + q < n) out[base + q] = run;
+        if (base + q < n) {
+            out[base + q] = run;
+            if (out2) out2[base + q] = run;
+        }
         run += v[q];
     }
 }
 __global__ void __launch_bounds__(kScanBS) k_scan_apply(const uint32_t* __restrict__ in, uint32_t n,
                                                        const uint32_t* __restrict__ tile_off,
-                                                       uint32_t* __restrict__ out) { k_scan_apply_body(VB{blockIdx.x, gridDim.x}, in, n, tile_off, out); }
+                                                       uint32_t* __restrict__ out, uint32_t* __restrict__ out2) { k_scan_apply_body(VB{blockIdx.x, gridDim.x}, in, n, tile_off, out, out2); }
 
 }  // namespace sdr

@@ -272,8 +272,9 @@ __device__ __forceinline__ void k_set_u32_body(VB, uint32_t* p, uint32_t v) {
     if (threadIdx.x == 0) *p = v;
 }
 __global__ void k_set_u32(uint32_t* p, uint32_t v) { k_set_u32_body(VB{blockIdx.x, gridDim.x}, p, v); }
-__device__ __forceinline__ void k_redist_begin_body(VB, RedistState* r) {
+__device__ __forceinline__ void k_redist_begin_body(VB, RedistState* r, unsigned* bar) {
     if (threadIdx.x != 0) return;
+    if (bar) bar[0] = bar[1] = 0u;  // of the long-list rounds: a wound-down launch may leave arrivals
     r->ncand = 0;
     r->active = 1;
     r->nmoves = 0;
@@ -281,7 +282,7 @@ __device__ __forceinline__ void k_redist_begin_body(VB, RedistState* r) {
     r->nmoves_par = 0;
     r->err = 0;
 }
-__global__ void k_redist_begin(RedistState* r) { k_redist_begin_body(VB{blockIdx.x, gridDim.x}, r); }
+__global__ void k_redist_begin(RedistState* r, unsigned* bar) { k_redist_begin_body(VB{blockIdx.x, gridDim.x}, r, bar); }
 __device__ __forceinline__ void k_redist_end_body(VB, const RedistState* r, DevStatus* s) {
     if (threadIdx.x != 0) return;
     s->moves = r->moves_total;
@@ -555,7 +556,8 @@ struct sdr_solver {
     uint32_t* dn() { return &dst->n; }
 
     // Exclusive scan; `site` (the caller's line) keys its kernels in a packed launch.
-    void scan(const uint32_t* in, uint32_t* out, size_t n_, uint32_t* total, int site) {
+    // out2 (optional): the same again.
+    void scan(const uint32_t* in, uint32_t* out, size_t n_, uint32_t* total, int site, uint32_t* out2 = nullptr) {
         const int key = 1000000 + 4 * site;
         if (n_ == 0) {
             if (total) issue<k_set_u32_op>(k_set_u32, key, 1, 1, 0, total, 0u);
@@ -568,7 +570,7 @@ struct sdr_solver {
         }
         issue<k_scan_tiles_op>(k_scan_tiles, key + 1, nt, kScanBS, 0, in, (uint32_t)n_, tsum);
         issue<k_scan_sums_op>(k_scan_sums, key + 2, 1, kScanBS, 0, tsum, nt, total);
-        issue<k_scan_apply_op>(k_scan_apply, key + 3, nt, kScanBS, 0, in, (uint32_t)n_, tsum, out);
+        issue<k_scan_apply_op>(k_scan_apply, key + 3, nt, kScanBS, 0, in, (uint32_t)n_, tsum, out, out2);
     }
 
     void ensure_capacity(size_t need) {
@@ -624,8 +626,8 @@ struct sdr_solver {
         CK(cudaMemsetAsync(sw, 0, nw * 4, st));
         dalloc(cells, nc, st); dalloc(base, nc, st); dalloc(cavity, nc, st);
         CK(cudaMemsetAsync(cells, AIR, nc, st));
-        dalloc(hist_valid, nc + 1, st);
-        dalloc(hist_sort, nc + 1, st);
+        dalloc(hist_valid, 2 * (nc + 1), st);
+        hist_sort = hist_valid + nc + 1;
         dalloc(start, nc + 1, st);
         dalloc(fill, nc + 1, st);
         dalloc(long_list, nc, st);
@@ -667,7 +669,7 @@ struct sdr_solver {
         dfree(cells, st); dfree(base, st); dfree(cavity, st);
         dfree(pos, st); dfree(vel, st); dfree(pos2, st); dfree(vel2, st);
         dfree(key_cell, st); dfree(key_sort, st); dfree(perm, st); dfree(ptmp, st); dfree(flag, st); dfree(off, st); dfree(drn, st);
-        dfree(hist_valid, st); dfree(hist_sort, st); dfree(start, st); dfree(fill, st); dfree(long_list, st); dfree(tsum, st);
+        dfree(hist_valid, st); hist_sort = nullptr; dfree(start, st); dfree(fill, st); dfree(long_list, st); dfree(tsum, st);
         dfree(dst, st);
         dfree(lines_cnt, st); dfree(lv_cell, st); dfree(cflag, st); dfree(coff, st); dfree(level_start, st); dfree(pos_of_cell, st);
         dfree(nbr, st); dfree(corder, st); dfree(cinv, st); dfree(prod, st); dfree(frec, st); dfree(brec, st); dfree(chunk_start, st); dfree(diag, st); dfree(nmask, st);
@@ -743,8 +745,7 @@ struct sdr_solver {
     }
 
     void classify(bool mark) {
-        MSET(hist_valid, 0, (ncell + 1) * 4);
-        MSET(hist_sort, 0, (ncell + 1) * 4);
+        MSET(hist_valid, 0, 2 * (ncell + 1) * 4);  // and hist_sort behind it
         if (mark) SLAUNCH(k_base_labels, blocks(ncell, 256), 256, 0, st, base, cells, ncell);
         if (n)
             SLAUNCH(k_classify_keys, blocks(n, kBS), kBS, 0, st, g, pos, n, (int)has_outlet, outlet,
@@ -752,8 +753,7 @@ struct sdr_solver {
     }
 
     void sort() {  // counting sort by the f32 P2G cell key
-        scan(hist_sort, start, ncell + 1, &dst->total, __LINE__);
-        MCOPY(fill, start, ncell * 4);
+        scan(hist_sort, start, ncell + 1, &dst->total, __LINE__, fill);
         if (n) SLAUNCH(k_sort_scatter, blocks(n, kBS), kBS, 0, st, key_sort, n, fill, perm);
         MSET(&dst->long_count, 0, 4);
         SLAUNCH(k_sort_segments, blocks(ncell, 256), 256, 0, st, start, (uint32_t)ncell, perm, long_list,
@@ -1115,17 +1115,16 @@ struct sdr_solver {
         for (int d = 0; d < 6; ++d) ra.down[d] = dirs[d][0] * gd.x + dirs[d][1] * gd.y + dirs[d][2] * gd.z;
         ra.moves = moves;
         ra.rs = rds;
-        SLAUNCH(k_redist_begin, 1, 1, 0, st, rds);
+        SLAUNCH(k_redist_begin, 1, 32, 0, st, rds, grid_rounds ? rp_bar : nullptr);
+        MSET(hist_valid, 0, ncell * 4);
+        SLAUNCH(k_redist_hist_n, blocks(n_upper, kBS), kBS, 0, st, g, pos, dn(), rds, key_cell, hist_valid);
         for (int sweep = 0; sweep < 4; ++sweep) {
-            MSET(hist_valid, 0, ncell * 4);
-            SLAUNCH(k_redist_hist_n, blocks(n_upper, kBS), kBS, 0, st, g, pos, dn(), rds, key_cell, hist_valid);
             SLAUNCH(k_redist_append, blocks(n_upper, kBS), kBS, 0, st, g, key_cell, hist_valid, cavity, dn(), cap_, rds, cand,
                    (uint32_t)cand_n);
             SLAUNCH(k_redist_replay, 1, kRedistBS, kRedistSmem, st, ra);
             // long lists only (the replay kernel hands over through the state; otherwise it returns at once)
             if (grid_rounds) {
                 // every SM decides the long list (a cooperative launch; it returns at once for short lists)
-                CK(cudaMemsetAsync(rp_bar, 0, 2 * sizeof(unsigned), st));
                 double* sl = rp_slots;
                 unsigned* br = rp_bar;
                 void* args[] = {&ra, &sl, &br};
