@@ -80,7 +80,9 @@ __global__ void k_cavity_and_base(Grid g, SdfD s, int has_outlet, Aabb outlet,
 // Bricks of nodes that four sweeps can reach from a fluid cell (four nodes before
 // it to five behind it, so at most two a direction) get this extrapolation's number.
 __device__ __forceinline__ void k_extrap_valid_body(VB vb_, Grid g, const uint8_t* __restrict__ cells, uint8_t* __restrict__ ku,
-                               uint8_t* __restrict__ kv, uint8_t* __restrict__ kw, uint32_t* __restrict__ brick, uint32_t epoch) {
+                               uint8_t* __restrict__ kv, uint8_t* __restrict__ kw, uint32_t* __restrict__ brick, uint32_t epoch,
+                               unsigned int* __restrict__ maxbits) {
+    if (vb_.bid == 0 && threadIdx.x < 3) maxbits[threadIdx.x] = 0u;  // of the last sweep
     int i, j, k;
     if (!node_of(g, (size_t)vb_.bid * blockDim.x + threadIdx.x, i, j, k)) return;
     auto fl = [&](int a, int b, int c) {
@@ -104,7 +106,7 @@ __device__ __forceinline__ void k_extrap_valid_body(VB vb_, Grid g, const uint8_
 }
 __global__ void k_extrap_valid(Grid g, const uint8_t* __restrict__ cells, uint8_t* __restrict__ ku,
                                uint8_t* __restrict__ kv, uint8_t* __restrict__ kw, uint32_t* __restrict__ brick,
-                               uint32_t epoch) { k_extrap_valid_body(VB{blockIdx.x, gridDim.x}, g, cells, ku, kv, kw, brick, epoch); }
+                               uint32_t epoch, unsigned int* __restrict__ maxbits) { k_extrap_valid_body(VB{blockIdx.x, gridDim.x}, g, cells, ku, kv, kw, brick, epoch, maxbits); }
 
 // One snapshot sweep of extrapolate (solver.rs:964-1007) on one unknown face,
 // in place. kn holds 0 for unknown, 1 for known from the start and s + 2 for

@@ -11,14 +11,32 @@ namespace sdr {
 constexpr int kBS = 256;
 
 // ------------------------------------------------------------------ classify
-// Solver::classify (solver.rs:342-371) first half: static labels per cell.
+// The nozzle's particles from pinned staging behind the others, and the new count.
+__device__ __forceinline__ void k_emit_body(VB vb_, const float4* __restrict__ hpos, const float4* __restrict__ hvel,
+                                            float4* __restrict__ pos, float4* __restrict__ vel, uint32_t n, uint32_t k,
+                                            uint32_t* __restrict__ count) {
+    const uint32_t p = vb_.bid * blockDim.x + threadIdx.x;
+    if (p == 0) *count = n + k;
+    if (p >= k) return;
+    const float4 q = hpos[p], v = hvel[p];
+    pos[n + p] = q;
+    vel[n + p] = v;
+}
+__global__ void k_emit(const float4* __restrict__ hpos, const float4* __restrict__ hvel, float4* __restrict__ pos,
+                       float4* __restrict__ vel, uint32_t n, uint32_t k,
+                       uint32_t* __restrict__ count) { k_emit_body(VB{blockIdx.x, gridDim.x}, hpos, hvel, pos, vel, n, k, count); }
+
+// Solver::classify (solver.rs:342-371) first half: static labels per cell. The
+// cells' two histograms (n + 1 counts each) are cleared on the way.
 __device__ __forceinline__ void k_base_labels_body(VB vb_, const uint8_t* __restrict__ base, uint8_t* __restrict__ cells,
-                              size_t n) {
+                              size_t n, uint32_t* __restrict__ hist_valid, uint32_t* __restrict__ hist_sort) {
     size_t c = (size_t)vb_.bid * blockDim.x + threadIdx.x;
     if (c < n) cells[c] = base[c];
+    if (c <= n) hist_valid[c] = hist_sort[c] = 0u;
 }
-__global__ void k_base_labels(const uint8_t* __restrict__ base, uint8_t* __restrict__ cells,
-                              size_t n) { k_base_labels_body(VB{blockIdx.x, gridDim.x}, base, cells, n); }
+__global__ void k_base_labels(const uint8_t* __restrict__ base, uint8_t* __restrict__ cells, size_t n,
+                              uint32_t* __restrict__ hist_valid,
+                              uint32_t* __restrict__ hist_sort) { k_base_labels_body(VB{blockIdx.x, gridDim.x}, base, cells, n, hist_valid, hist_sort); }
 
 // Per particle: the f64 cell key of Solver::cell_of (labels, histograms) and
 // the clamped cell the P2G gather bins by (from the same f64 grid coordinate
@@ -57,16 +75,19 @@ __global__ void k_classify_keys(Grid g, const float4* __restrict__ pos, uint32_t
                                 uint32_t* __restrict__ hist_sort) { k_classify_keys_body(VB{blockIdx.x, gridDim.x}, g, pos, n, has_outlet, outlet, mark_fluid, cells, key_cell, key_sort, hist_valid, hist_sort); }
 
 // ------------------------------------------------------------------ counting sort
-// Slot assignment within each cell segment (start from the exclusive scan).
+// Slot assignment within each cell segment (start from the exclusive scan). The
+// count of k_sort_segments' long segments is cleared on the way.
 __device__ __forceinline__ void k_sort_scatter_body(VB vb_, const uint32_t* __restrict__ key, uint32_t n,
-                               uint32_t* __restrict__ fill, uint32_t* __restrict__ perm) {
+                               uint32_t* __restrict__ fill, uint32_t* __restrict__ perm, uint32_t* __restrict__ long_count) {
     uint32_t p = vb_.bid * blockDim.x + threadIdx.x;
+    if (p == 0) *long_count = 0u;
     if (p >= n) return;
     uint32_t s = atomicAdd(&fill[key[p]], 1u);
     perm[s] = p;
 }
 __global__ void k_sort_scatter(const uint32_t* __restrict__ key, uint32_t n,
-                               uint32_t* __restrict__ fill, uint32_t* __restrict__ perm) { k_sort_scatter_body(VB{blockIdx.x, gridDim.x}, key, n, fill, perm); }
+                               uint32_t* __restrict__ fill, uint32_t* __restrict__ perm,
+                               uint32_t* __restrict__ long_count) { k_sort_scatter_body(VB{blockIdx.x, gridDim.x}, key, n, fill, perm, long_count); }
 
 // Make each segment ascending in particle index, so the permutation equals a
 // stable counting sort (bit-exact vs a CPU stable sort of the same keys) and
@@ -102,7 +123,8 @@ __global__ void k_sort_segments(const uint32_t* __restrict__ start, uint32_t nce
 // Rank sort of long segments (indices are distinct): one block per segment.
 __device__ __forceinline__ void k_sort_long_body(VB vb_, const uint32_t* __restrict__ start, const uint32_t* __restrict__ long_list,
                             const uint32_t* __restrict__ long_count, uint32_t* __restrict__ perm,
-                            uint32_t* __restrict__ tmp) {
+                            uint32_t* __restrict__ tmp, uint32_t* __restrict__ queue) {
+    if (queue && vb_.bid == 0 && threadIdx.x == 0) *queue = 0u;  // of the nodes that P2G gathers
     uint32_t nl = *long_count;
     for (uint32_t q = vb_.bid; q < nl; q += vb_.nb) {
         uint32_t c = long_list[q];
@@ -120,7 +142,7 @@ __device__ __forceinline__ void k_sort_long_body(VB vb_, const uint32_t* __restr
 }
 __global__ void k_sort_long(const uint32_t* __restrict__ start, const uint32_t* __restrict__ long_list,
                             const uint32_t* __restrict__ long_count, uint32_t* __restrict__ perm,
-                            uint32_t* __restrict__ tmp) { k_sort_long_body(VB{blockIdx.x, gridDim.x}, start, long_list, long_count, perm, tmp); }
+                            uint32_t* __restrict__ tmp, uint32_t* __restrict__ queue) { k_sort_long_body(VB{blockIdx.x, gridDim.x}, start, long_list, long_count, perm, tmp, queue); }
 
 // ------------------------------------------------------------------ P2G gather
 // Sorted particle records for the gather: the f64 grid coordinate

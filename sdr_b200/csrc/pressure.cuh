@@ -30,6 +30,7 @@ enum { NB_MX = 0, NB_PX = 1, NB_MY = 2, NB_PY = 3, NB_MZ = 4, NB_PZ = 5 };
 __device__ __forceinline__ void k_lines_count_body(VB vb_, Grid g, const uint8_t* __restrict__ cells, int nlevels,
                               uint32_t* __restrict__ cnt) {
     int t = vb_.bid * blockDim.x + threadIdx.x;
+    if (t == nlevels * g.nz) cnt[t] = 0;  // behind the last: the scan's total
     if (t >= nlevels * g.nz) return;
     int L = t / g.nz, k = t % g.nz;
     int r = L - k;  // i + j = r
@@ -141,12 +142,17 @@ __device__ __forceinline__ void k_tables_body(VB vb_, TableArgs a) {
 }
 __global__ void k_tables(TableArgs a) { k_tables_body(VB{blockIdx.x, gridDim.x}, a); }
 
-// Fluid cells in cell-index order -> wavefront position, for the chunked dot.
-__device__ __forceinline__ void k_fluid_flags_body(VB vb_, const uint8_t* __restrict__ cells, size_t n, uint32_t* __restrict__ flag) {
+// Fluid cells in cell-index order -> wavefront position, for the chunked dot. The
+// dense pressure is cleared on the way (the solve writes the fluid cells).
+__device__ __forceinline__ void k_fluid_flags_body(VB vb_, const uint8_t* __restrict__ cells, size_t n, uint32_t* __restrict__ flag,
+                                                   double* __restrict__ p_dense) {
     size_t c = (size_t)vb_.bid * blockDim.x + threadIdx.x;
-    if (c < n) flag[c] = cells[c] == FLUID;
+    if (c >= n) return;
+    flag[c] = cells[c] == FLUID;
+    p_dense[c] = 0.0;
 }
-__global__ void k_fluid_flags(const uint8_t* __restrict__ cells, size_t n, uint32_t* __restrict__ flag) { k_fluid_flags_body(VB{blockIdx.x, gridDim.x}, cells, n, flag); }
+__global__ void k_fluid_flags(const uint8_t* __restrict__ cells, size_t n, uint32_t* __restrict__ flag,
+                              double* __restrict__ p_dense) { k_fluid_flags_body(VB{blockIdx.x, gridDim.x}, cells, n, flag, p_dense); }
 
 __device__ __forceinline__ void k_corder_body(VB vb_, const uint8_t* __restrict__ cells, size_t n, const uint32_t* __restrict__ off,
                          const int* __restrict__ pos_of_cell, int* __restrict__ corder, int* __restrict__ cinv,

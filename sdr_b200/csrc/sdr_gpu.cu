@@ -272,8 +272,10 @@ __device__ __forceinline__ void k_set_u32_body(VB, uint32_t* p, uint32_t v) {
     if (threadIdx.x == 0) *p = v;
 }
 __global__ void k_set_u32(uint32_t* p, uint32_t v) { k_set_u32_body(VB{blockIdx.x, gridDim.x}, p, v); }
-__device__ __forceinline__ void k_redist_begin_body(VB, RedistState* r, unsigned* bar) {
-    if (threadIdx.x != 0) return;
+__device__ __forceinline__ void k_redist_begin_body(VB vb_, RedistState* r, unsigned* bar, uint32_t* hist, size_t ncell) {
+    const size_t c = (size_t)vb_.bid * blockDim.x + threadIdx.x;
+    if (c < ncell) hist[c] = 0u;
+    if (c != 0) return;
     if (bar) bar[0] = bar[1] = 0u;  // of the long-list rounds: a wound-down launch may leave arrivals
     r->ncand = 0;
     r->active = 1;
@@ -282,7 +284,7 @@ __device__ __forceinline__ void k_redist_begin_body(VB, RedistState* r, unsigned
     r->nmoves_par = 0;
     r->err = 0;
 }
-__global__ void k_redist_begin(RedistState* r, unsigned* bar) { k_redist_begin_body(VB{blockIdx.x, gridDim.x}, r, bar); }
+__global__ void k_redist_begin(RedistState* r, unsigned* bar, uint32_t* hist, size_t ncell) { k_redist_begin_body(VB{blockIdx.x, gridDim.x}, r, bar, hist, ncell); }
 __device__ __forceinline__ void k_redist_end_body(VB, const RedistState* r, DevStatus* s) {
     if (threadIdx.x != 0) return;
     s->moves = r->moves_total;
@@ -300,6 +302,7 @@ SDR_OP(k_scan_tiles, kScanBS)
 SDR_OP(k_scan_sums, kScanBS)
 SDR_OP(k_scan_apply, kScanBS)
 SDR_OP(k_cavity_and_base, 256)
+SDR_OP(k_emit, kBS)
 SDR_OP(k_base_labels, 256)
 SDR_OP(k_classify_keys, kBS)
 SDR_OP(k_sort_scatter, kBS)
@@ -324,7 +327,7 @@ SDR_OP(k_face_max, 256)
 SDR_OP(k_g2p_advect, kBS)
 SDR_OP(k_bounds_flags, kBS)
 SDR_OP(k_compact, kBS)
-SDR_OP(k_redist_begin, 32)
+SDR_OP(k_redist_begin, 256)
 SDR_OP(k_redist_hist_n, kBS)
 SDR_OP(k_redist_append, kBS)
 SDR_OP(k_redist_replay, kRedistBS)
@@ -733,20 +736,18 @@ struct sdr_solver {
             h_epos[i] = make_float4((float)ps.x, (float)ps.y, (float)ps.z, 0.f);
             h_evel[i] = make_float4((float)vv.x, (float)vv.y, (float)vv.z, 0.f);
         }
-        MCOPY(pos + n, h_epos, k * sizeof(float4));
-        MCOPY(vel + n, h_evel, k * sizeof(float4));
+        SLAUNCH(k_emit, blocks(k, kBS), kBS, 0, st, h_epos, h_evel, pos, vel, n, (uint32_t)k, dn());
         if (profiling) prof.h2d_bytes += 2 * k * sizeof(float4);
         // The staging buffers are reused next substep; the status sync at the
-        // end of this substep orders the copies before any reuse.
+        // end of this substep orders their reads before any reuse.
         n += (uint32_t)k;
         emitted += k;
-        SLAUNCH(k_set_u32, 1, 1, 0, st, dn(), n);
         sorted_valid = false;
     }
 
     void classify(bool mark) {
-        MSET(hist_valid, 0, 2 * (ncell + 1) * 4);  // and hist_sort behind it
-        if (mark) SLAUNCH(k_base_labels, blocks(ncell, 256), 256, 0, st, base, cells, ncell);
+        if (mark) SLAUNCH(k_base_labels, blocks(ncell + 1, 256), 256, 0, st, base, cells, ncell, hist_valid, hist_sort);
+        else MSET(hist_valid, 0, 2 * (ncell + 1) * 4);  // and hist_sort behind it
         if (n)
             SLAUNCH(k_classify_keys, blocks(n, kBS), kBS, 0, st, g, pos, n, (int)has_outlet, outlet,
                    (int)mark, cells, key_cell, key_sort, hist_valid, hist_sort);
@@ -754,16 +755,17 @@ struct sdr_solver {
 
     void sort() {  // counting sort by the f32 P2G cell key
         scan(hist_sort, start, ncell + 1, &dst->total, __LINE__, fill);
-        if (n) SLAUNCH(k_sort_scatter, blocks(n, kBS), kBS, 0, st, key_sort, n, fill, perm);
-        MSET(&dst->long_count, 0, 4);
+        if (n) SLAUNCH(k_sort_scatter, blocks(n, kBS), kBS, 0, st, key_sort, n, fill, perm, &dst->long_count);
+        else MSET(&dst->long_count, 0, 4);
         SLAUNCH(k_sort_segments, blocks(ncell, 256), 256, 0, st, start, (uint32_t)ncell, perm, long_list,
                &dst->long_count);
-        SLAUNCH(k_sort_long, 148, 256, 0, st, start, long_list, &dst->long_count, perm, ptmp);
+        SLAUNCH(k_sort_long, 148, 256, 0, st, start, long_list, &dst->long_count, perm, ptmp,
+               &dst->p2g_queue);
         if (n) SLAUNCH(k_sorted_records, blocks(n, kBS), kBS, 0, st, g, pos, vel, perm, n, lrec, vrec);
         sorted_valid = true;
     }
 
-    void p2g(double dt, bool fused) {
+    void p2g(double dt, bool fused) {  // behind sort(), which clears the queue's length
         P2GArgs a{};
         a.g = g;
         a.lrec = lrec;
@@ -779,7 +781,6 @@ struct sdr_solver {
         a.enforce = fused;
         // empty nodes at once, the rest queued for the eight-lane gather; its grid
         // follows the last queue length (the loop over the queue covers any length)
-        MSET(&dst->p2g_queue, 0, 4);
         SLAUNCH(k_p2g_nodes, nbricks(), kBrickBS, 0, st, a, p2g_list, &dst->p2g_queue);
         const size_t want = last_p2g_queue ? ((size_t)last_p2g_queue + last_p2g_queue / 4 + 64) * kP2GLanes
                                            : nnodes() * kP2GLanes;  // no history yet: every node
@@ -804,8 +805,7 @@ struct sdr_solver {
         unsigned ngrid = blocks(nnodes(), 256);
         if (enforce) SLAUNCH(k_enforce_solid, ngrid, 256, 0, st, g, cells, u, v, w);
         size_t nl = (size_t)nlevels * g.nz;
-        SLAUNCH(k_lines_count, blocks(nl, 256), 256, 0, st, g, cells, nlevels, lines_cnt);
-        MSET(lines_cnt + nl, 0, 4);
+        SLAUNCH(k_lines_count, blocks(nl + 1, 256), 256, 0, st, g, cells, nlevels, lines_cnt);
         scan(lines_cnt, lines_cnt, nl + 1, &dst->nf, __LINE__);
         SLAUNCH(k_lines_assign, blocks(nl, 256), 256, 0, st, g, cells, nlevels, lines_cnt, pos_of_cell, lv_cell);
         SLAUNCH(k_level_starts_dev, blocks(nlevels + 1, 256), 256, 0, st, lines_cnt, nlevels, g.nz, &dst->nf,
@@ -830,11 +830,10 @@ struct sdr_solver {
         t.vs_unit = g.dx / dt;
         t.vs_cap = 0.25 * t.vs_unit;
         SLAUNCH(k_tables, blocks(ncell, 256), 256, 0, st, t);
-        SLAUNCH(k_fluid_flags, blocks(ncell, 256), 256, 0, st, cells, ncell, cflag);
+        SLAUNCH(k_fluid_flags, blocks(ncell, 256), 256, 0, st, cells, ncell, cflag, p_dense);
         scan(cflag, coff, ncell + 1, nullptr, __LINE__);
         SLAUNCH(k_corder, blocks(ncell, 256), 256, 0, st, cells, ncell, coff, pos_of_cell, corder, cinv, chunk_start,
                nchunks, &dst->nf);
-        MSET(p_dense, 0, ncell * 8);
     }
 
     void project_solve(double dt) {
@@ -1022,8 +1021,7 @@ struct sdr_solver {
     void extrapolate() {  // solver.rs:608-647
         unsigned ngrid = blocks(nnodes(), 256);
         ++extrap_epoch;
-        SLAUNCH(k_extrap_valid, ngrid, 256, 0, st, g, cells, ku, kv, kw, brick, extrap_epoch);
-        MSET(dst->maxbits, 0, sizeof(dst->maxbits));
+        SLAUNCH(k_extrap_valid, ngrid, 256, 0, st, g, cells, ku, kv, kw, brick, extrap_epoch, dst->maxbits);
         for (int it = 0; it < 4; ++it) {  // four sweeps, in place
             ExtrapArgs e{g, u, v, w, ku, kv, kw, it, it == 3 ? dst->maxbits : nullptr, brick, extrap_epoch};
             SLAUNCH(k_extrap, nbricks(), kBrickBS, 0, st, e);
@@ -1115,8 +1113,7 @@ struct sdr_solver {
         for (int d = 0; d < 6; ++d) ra.down[d] = dirs[d][0] * gd.x + dirs[d][1] * gd.y + dirs[d][2] * gd.z;
         ra.moves = moves;
         ra.rs = rds;
-        SLAUNCH(k_redist_begin, 1, 32, 0, st, rds, grid_rounds ? rp_bar : nullptr);
-        MSET(hist_valid, 0, ncell * 4);
+        SLAUNCH(k_redist_begin, blocks(ncell, 256), 256, 0, st, rds, grid_rounds ? rp_bar : nullptr, hist_valid, ncell);
         SLAUNCH(k_redist_hist_n, blocks(n_upper, kBS), kBS, 0, st, g, pos, dn(), rds, key_cell, hist_valid);
         for (int sweep = 0; sweep < 4; ++sweep) {
             SLAUNCH(k_redist_append, blocks(n_upper, kBS), kBS, 0, st, g, key_cell, hist_valid, cavity, dn(), cap_, rds, cand,
@@ -2096,7 +2093,7 @@ int sdr_render_slice(sdr_solver* s, const sdr_slice_plane* plane, uint32_t targe
             const uint32_t nb = (uint32_t)(ntx + 2) * (uint32_t)(nty + 2) + 1;  // with the dump bin
             dalloc(hist, nb + 1, st);
             dalloc(start, nb + 1, st);
-            dalloc(fill, nb, st);
+            dalloc(fill, nb + 1, st);
             dalloc(longl, nb, st);
             dalloc(lcount, 1, st);
             dalloc(key, n, st);
@@ -2104,14 +2101,13 @@ int sdr_render_slice(sdr_solver* s, const sdr_slice_plane* plane, uint32_t targe
             dalloc(perm, n, st);
             dalloc(tmp, n, st);
             CK(cudaMemsetAsync(hist, 0, (nb + 1) * 4, st));
-            CK(cudaMemsetAsync(lcount, 0, 4, st));
             if (n) LAUNCH(k_render_amber_keys, blocks(n, 256), 256, 0, st, v, s->pos, n, T, ntx, nty, key, cxy, hist);
-            s->scan(hist, start, nb + 1, nullptr, __LINE__);
-            CK(cudaMemcpyAsync(fill, start, nb * 4, cudaMemcpyDeviceToDevice, st));
-            if (n) LAUNCH(k_sort_scatter, blocks(n, 256), 256, 0, st, key, n, fill, perm);
+            s->scan(hist, start, nb + 1, nullptr, __LINE__, fill);
+            if (n) LAUNCH(k_sort_scatter, blocks(n, 256), 256, 0, st, key, n, fill, perm, lcount);
+            else CK(cudaMemsetAsync(lcount, 0, 4, st));
             LAUNCH(k_sort_segments, blocks(nb, 256), 256, 0, st, start, nb, perm, longl, lcount);
             // an image has thousands of long bins (hundreds of particles each): eight blocks per SM
-            LAUNCH(k_sort_long, 148 * 8, 256, 0, st, start, longl, lcount, perm, tmp);
+            LAUNCH(k_sort_long, 148 * 8, 256, 0, st, start, longl, lcount, perm, tmp, nullptr);
             const unsigned per = (unsigned)((T + kAmPx - 1) / kAmPx);
             LAUNCH(k_render_amber_pixels, (unsigned)ntx * (unsigned)nty * per * per, kAmBS, 0, st, v, r, T, ntx, start, perm,
                    cxy, img);
