@@ -77,6 +77,16 @@ __device__ inline bool grid_sync_bounded(unsigned* bar, uint32_t* err, uint32_t 
     return ok_s != 0;
 }
 
+// Start of every kernel that a substep launches: wait until the kernel before it
+// has finished and its writes are visible, then let the next one's launch begin.
+// Launched with programmatic serialisation, a kernel's blocks are set up while the
+// one before it drains; launched without, both calls return at once. A kernel's
+// end implies the end of all before it, as every one waits.
+__device__ __forceinline__ void pdl_begin() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+
 // The block a kernel body runs as: its index and the block count of its
 // launch. A plain launch passes (blockIdx.x, gridDim.x); a packed launch of
 // many scenes passes the block's place within its own scene's share.

@@ -74,7 +74,7 @@ __device__ __forceinline__ void k_cavity_and_base_body(VB vb_, Grid g, SdfD s, i
 }
 __global__ void k_cavity_and_base(Grid g, SdfD s, int has_outlet, Aabb outlet,
                                   uint8_t* __restrict__ cavity, uint8_t* __restrict__ base,
-                                  int recompute_cavity) { k_cavity_and_base_body(VB{blockIdx.x, gridDim.x}, g, s, has_outlet, outlet, cavity, base, recompute_cavity); }
+                                  int recompute_cavity) { pdl_begin(); k_cavity_and_base_body(VB{blockIdx.x, gridDim.x}, g, s, has_outlet, outlet, cavity, base, recompute_cavity); }
 
 // Validity for extrapolation: the face borders a Fluid cell (solver.rs:612-642).
 // Bricks of nodes that four sweeps can reach from a fluid cell (four nodes before
@@ -106,7 +106,7 @@ __device__ __forceinline__ void k_extrap_valid_body(VB vb_, Grid g, const uint8_
 }
 __global__ void k_extrap_valid(Grid g, const uint8_t* __restrict__ cells, uint8_t* __restrict__ ku,
                                uint8_t* __restrict__ kv, uint8_t* __restrict__ kw, uint32_t* __restrict__ brick,
-                               uint32_t epoch, unsigned int* __restrict__ maxbits) { k_extrap_valid_body(VB{blockIdx.x, gridDim.x}, g, cells, ku, kv, kw, brick, epoch, maxbits); }
+                               uint32_t epoch, unsigned int* __restrict__ maxbits) { pdl_begin(); k_extrap_valid_body(VB{blockIdx.x, gridDim.x}, g, cells, ku, kv, kw, brick, epoch, maxbits); }
 
 // One snapshot sweep of extrapolate (solver.rs:964-1007) on one unknown face,
 // in place. kn holds 0 for unknown, 1 for known from the start and s + 2 for
@@ -199,7 +199,7 @@ __device__ __forceinline__ void k_extrap_body(VB vb_, ExtrapArgs a) {
         }
     }
 }
-__global__ void __launch_bounds__(kBrickBS) k_extrap(ExtrapArgs a) { k_extrap_body(VB{blockIdx.x, gridDim.x}, a); }
+__global__ void __launch_bounds__(kBrickBS) k_extrap(ExtrapArgs a) { pdl_begin(); k_extrap_body(VB{blockIdx.x, gridDim.x}, a); }
 
 // Face maxima alone (used when extrapolation did not run, e.g. phase mode).
 __device__ __forceinline__ void k_face_max_body(VB vb_, const float* __restrict__ f, size_t n, unsigned int* __restrict__ out) {
@@ -209,6 +209,6 @@ __device__ __forceinline__ void k_face_max_body(VB vb_, const float* __restrict_
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
 }
-__global__ void k_face_max(const float* __restrict__ f, size_t n, unsigned int* __restrict__ out) { k_face_max_body(VB{blockIdx.x, gridDim.x}, f, n, out); }
+__global__ void k_face_max(const float* __restrict__ f, size_t n, unsigned int* __restrict__ out) { pdl_begin(); k_face_max_body(VB{blockIdx.x, gridDim.x}, f, n, out); }
 
 }  // namespace sdr

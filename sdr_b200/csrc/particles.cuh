@@ -24,7 +24,7 @@ __device__ __forceinline__ void k_emit_body(VB vb_, const float4* __restrict__ h
 }
 __global__ void k_emit(const float4* __restrict__ hpos, const float4* __restrict__ hvel, float4* __restrict__ pos,
                        float4* __restrict__ vel, uint32_t n, uint32_t k,
-                       uint32_t* __restrict__ count) { k_emit_body(VB{blockIdx.x, gridDim.x}, hpos, hvel, pos, vel, n, k, count); }
+                       uint32_t* __restrict__ count) { pdl_begin(); k_emit_body(VB{blockIdx.x, gridDim.x}, hpos, hvel, pos, vel, n, k, count); }
 
 // Solver::classify (solver.rs:342-371) first half: static labels per cell. The
 // cells' two histograms (n + 1 counts each) are cleared on the way.
@@ -36,7 +36,7 @@ __device__ __forceinline__ void k_base_labels_body(VB vb_, const uint8_t* __rest
 }
 __global__ void k_base_labels(const uint8_t* __restrict__ base, uint8_t* __restrict__ cells, size_t n,
                               uint32_t* __restrict__ hist_valid,
-                              uint32_t* __restrict__ hist_sort) { k_base_labels_body(VB{blockIdx.x, gridDim.x}, base, cells, n, hist_valid, hist_sort); }
+                              uint32_t* __restrict__ hist_sort) { pdl_begin(); k_base_labels_body(VB{blockIdx.x, gridDim.x}, base, cells, n, hist_valid, hist_sort); }
 
 // Per particle: the f64 cell key of Solver::cell_of (labels, histograms) and
 // the clamped cell the P2G gather bins by (from the same f64 grid coordinate
@@ -72,7 +72,7 @@ __global__ void k_classify_keys(Grid g, const float4* __restrict__ pos, uint32_t
                                 int has_outlet, Aabb outlet, int mark_fluid,
                                 uint8_t* __restrict__ cells, int* __restrict__ key_cell,
                                 uint32_t* __restrict__ key_sort, uint32_t* __restrict__ hist_valid,
-                                uint32_t* __restrict__ hist_sort) { k_classify_keys_body(VB{blockIdx.x, gridDim.x}, g, pos, n, has_outlet, outlet, mark_fluid, cells, key_cell, key_sort, hist_valid, hist_sort); }
+                                uint32_t* __restrict__ hist_sort) { pdl_begin(); k_classify_keys_body(VB{blockIdx.x, gridDim.x}, g, pos, n, has_outlet, outlet, mark_fluid, cells, key_cell, key_sort, hist_valid, hist_sort); }
 
 // ------------------------------------------------------------------ counting sort
 // Slot assignment within each cell segment (start from the exclusive scan). The
@@ -87,7 +87,7 @@ __device__ __forceinline__ void k_sort_scatter_body(VB vb_, const uint32_t* __re
 }
 __global__ void k_sort_scatter(const uint32_t* __restrict__ key, uint32_t n,
                                uint32_t* __restrict__ fill, uint32_t* __restrict__ perm,
-                               uint32_t* __restrict__ long_count) { k_sort_scatter_body(VB{blockIdx.x, gridDim.x}, key, n, fill, perm, long_count); }
+                               uint32_t* __restrict__ long_count) { pdl_begin(); k_sort_scatter_body(VB{blockIdx.x, gridDim.x}, key, n, fill, perm, long_count); }
 
 // Make each segment ascending in particle index, so the permutation equals a
 // stable counting sort (bit-exact vs a CPU stable sort of the same keys) and
@@ -118,7 +118,7 @@ __device__ __forceinline__ void k_sort_segments_body(VB vb_, const uint32_t* __r
 }
 __global__ void k_sort_segments(const uint32_t* __restrict__ start, uint32_t ncell,
                                 uint32_t* __restrict__ perm, uint32_t* __restrict__ long_list,
-                                uint32_t* __restrict__ long_count) { k_sort_segments_body(VB{blockIdx.x, gridDim.x}, start, ncell, perm, long_list, long_count); }
+                                uint32_t* __restrict__ long_count) { pdl_begin(); k_sort_segments_body(VB{blockIdx.x, gridDim.x}, start, ncell, perm, long_list, long_count); }
 
 // Rank sort of long segments (indices are distinct): one block per segment.
 __device__ __forceinline__ void k_sort_long_body(VB vb_, const uint32_t* __restrict__ start, const uint32_t* __restrict__ long_list,
@@ -142,7 +142,7 @@ __device__ __forceinline__ void k_sort_long_body(VB vb_, const uint32_t* __restr
 }
 __global__ void k_sort_long(const uint32_t* __restrict__ start, const uint32_t* __restrict__ long_list,
                             const uint32_t* __restrict__ long_count, uint32_t* __restrict__ perm,
-                            uint32_t* __restrict__ tmp, uint32_t* __restrict__ queue) { k_sort_long_body(VB{blockIdx.x, gridDim.x}, start, long_list, long_count, perm, tmp, queue); }
+                            uint32_t* __restrict__ tmp, uint32_t* __restrict__ queue) { pdl_begin(); k_sort_long_body(VB{blockIdx.x, gridDim.x}, start, long_list, long_count, perm, tmp, queue); }
 
 // ------------------------------------------------------------------ P2G gather
 // Sorted particle records for the gather: the f64 grid coordinate
@@ -160,7 +160,7 @@ __device__ __forceinline__ void k_sorted_records_body(VB vb_, Grid g, const floa
 }
 __global__ void k_sorted_records(Grid g, const float4* __restrict__ pos, const float4* __restrict__ vel,
                                  const uint32_t* __restrict__ perm, uint32_t n, double4* __restrict__ lrec,
-                                 float4* __restrict__ vrec) { k_sorted_records_body(VB{blockIdx.x, gridDim.x}, g, pos, vel, perm, n, lrec, vrec); }
+                                 float4* __restrict__ vrec) { pdl_begin(); k_sorted_records_body(VB{blockIdx.x, gridDim.x}, g, pos, vel, perm, n, lrec, vrec); }
 
 struct P2GArgs {
     Grid g;
@@ -299,7 +299,7 @@ __device__ __forceinline__ void k_p2g_nodes_body(VB vb_, P2GArgs a, uint32_t* __
     else p2g_store(a, i, j, k, j < g.ny && k < g.nz, i < g.nx && k < g.nz, i < g.nx && j < g.ny, 0, 0, 0, 0, 0, 0);
 }
 __global__ void __launch_bounds__(kBrickBS) k_p2g_nodes(P2GArgs a, uint32_t* __restrict__ list,
-                                                        uint32_t* __restrict__ count) { k_p2g_nodes_body(VB{blockIdx.x, gridDim.x}, a, list, count); }
+                                                        uint32_t* __restrict__ count) { pdl_begin(); k_p2g_nodes_body(VB{blockIdx.x, gridDim.x}, a, list, count); }
 
 // P2G gather of the queued nodes, eight lanes each. The lanes split the
 // particles of the 27 cells around the node — for each (k, j) the three cells
@@ -376,14 +376,14 @@ __device__ __forceinline__ void k_p2g_body(VB vb_, P2GArgs a, const uint32_t* __
     }
 }
 __global__ void __launch_bounds__(kBS) k_p2g(P2GArgs a, const uint32_t* __restrict__ list,
-                                             const uint32_t* __restrict__ count) { k_p2g_body(VB{blockIdx.x, gridDim.x}, a, list, count); }
+                                             const uint32_t* __restrict__ count) { pdl_begin(); k_p2g_body(VB{blockIdx.x, gridDim.x}, a, list, count); }
 
 // Solver::add_forces (solver.rs:593-604) on its own (phase mode).
 __device__ __forceinline__ void k_add_forces_body(VB vb_, float* __restrict__ f, size_t n, double gdt) {
     size_t q = (size_t)vb_.bid * blockDim.x + threadIdx.x;
     if (q < n) f[q] = (float)dadd((double)f[q], gdt);
 }
-__global__ void k_add_forces(float* __restrict__ f, size_t n, double gdt) { k_add_forces_body(VB{blockIdx.x, gridDim.x}, f, n, gdt); }
+__global__ void k_add_forces(float* __restrict__ f, size_t n, double gdt) { pdl_begin(); k_add_forces_body(VB{blockIdx.x, gridDim.x}, f, n, gdt); }
 
 // enforce_solid_faces (pressure.rs:243-281) on its own (phase mode): one
 // thread per node, owning the u/v/w faces with that index.
@@ -399,7 +399,7 @@ __device__ __forceinline__ void k_enforce_solid_body(VB vb_, Grid g, const uint8
         w[((size_t)k * g.ny + j) * g.nx + i] = 0.0f;
 }
 __global__ void k_enforce_solid(Grid g, const uint8_t* __restrict__ cells, float* __restrict__ u,
-                                float* __restrict__ v, float* __restrict__ w) { k_enforce_solid_body(VB{blockIdx.x, gridDim.x}, g, cells, u, v, w); }
+                                float* __restrict__ v, float* __restrict__ w) { pdl_begin(); k_enforce_solid_body(VB{blockIdx.x, gridDim.x}, g, cells, u, v, w); }
 
 // ------------------------------------------------------------------ G2P + advect
 struct MoveArgs {
@@ -486,7 +486,7 @@ __device__ __forceinline__ void k_g2p_advect_body(VB vb_, MoveArgs a) {
         a.drained[p] = d;
     }
 }
-__global__ void __launch_bounds__(kBS) k_g2p_advect(MoveArgs a) { k_g2p_advect_body(VB{blockIdx.x, gridDim.x}, a); }
+__global__ void __launch_bounds__(kBS) k_g2p_advect(MoveArgs a) { pdl_begin(); k_g2p_advect_body(VB{blockIdx.x, gridDim.x}, a); }
 
 // Bounds flags alone (phase mode, after an external position change).
 __device__ __forceinline__ void k_bounds_flags_body(VB vb_, MoveArgs a) {
@@ -498,7 +498,7 @@ __device__ __forceinline__ void k_bounds_flags_body(VB vb_, MoveArgs a) {
     a.keep[p] = k;
     a.drained[p] = d;
 }
-__global__ void k_bounds_flags(MoveArgs a) { k_bounds_flags_body(VB{blockIdx.x, gridDim.x}, a); }
+__global__ void k_bounds_flags(MoveArgs a) { pdl_begin(); k_bounds_flags_body(VB{blockIdx.x, gridDim.x}, a); }
 
 // Stable scatter of kept particles (ParticleSet::retain, particles.rs:38-49)
 // plus the drained/culled tallies.
@@ -529,7 +529,7 @@ __device__ __forceinline__ void k_compact_body(VB vb_, const float4* __restrict_
 __global__ void k_compact(const float4* __restrict__ pos, const float4* __restrict__ vel,
                           const uint32_t* __restrict__ keep, const uint32_t* __restrict__ drained,
                           const uint32_t* __restrict__ off, uint32_t n, float4* __restrict__ pos2,
-                          float4* __restrict__ vel2, unsigned long long* __restrict__ counters) { k_compact_body(VB{blockIdx.x, gridDim.x}, pos, vel, keep, drained, off, n, pos2, vel2, counters); }
+                          float4* __restrict__ vel2, unsigned long long* __restrict__ counters) { pdl_begin(); k_compact_body(VB{blockIdx.x, gridDim.x}, pos, vel, keep, drained, off, n, pos2, vel2, counters); }
 
 // ------------------------------------------------------------------ redistribute
 // Solver::redistribute (solver.rs:454-557). Facts the GPU form relies on:
@@ -576,7 +576,7 @@ __device__ __forceinline__ void k_redist_hist_n_body(VB vb_, Grid g, const float
 }
 __global__ void k_redist_hist_n(Grid g, const float4* __restrict__ pos, const uint32_t* __restrict__ n_dev,
                                 const RedistState* __restrict__ rs, int* __restrict__ key_cell,
-                                uint32_t* __restrict__ count) { k_redist_hist_n_body(VB{blockIdx.x, gridDim.x}, g, pos, n_dev, rs, key_cell, count); }
+                                uint32_t* __restrict__ count) { pdl_begin(); k_redist_hist_n_body(VB{blockIdx.x, gridDim.x}, g, pos, n_dev, rs, key_cell, count); }
 
 // Particles in over-cap cells, appended in arbitrary order (sorted later).
 // A particle is left out when no face neighbour of its cell is an in-cavity
@@ -607,7 +607,7 @@ __device__ __forceinline__ void k_redist_append_body(VB vb_, Grid g, const int* 
 __global__ void k_redist_append(Grid g, const int* __restrict__ key_cell, const uint32_t* __restrict__ count,
                                 const uint8_t* __restrict__ cavity, const uint32_t* __restrict__ n_dev,
                                 uint32_t cap, RedistState* __restrict__ rs, uint32_t* __restrict__ cand,
-                                uint32_t cand_cap) { k_redist_append_body(VB{blockIdx.x, gridDim.x}, g, key_cell, count, cavity, n_dev, cap, rs, cand, cand_cap); }
+                                uint32_t cand_cap) { pdl_begin(); k_redist_append_body(VB{blockIdx.x, gridDim.x}, g, key_cell, count, cavity, n_dev, cap, rs, cand, cand_cap); }
 
 constexpr int kRedistTable = 4096;   // shared-memory hash slots (power of two)
 constexpr int kRedistProbes = 64;    // linear probes before a cell counts as not fitting the table
@@ -1026,7 +1026,7 @@ __device__ __forceinline__ void k_redist_replay_body(VB vb_, RedistArgs a) {
         for (uint32_t mv = threadIdx.x; mv < nm; mv += blockDim.x) redist_apply_move(a, a.moves[2 * mv], a.moves[2 * mv + 1], false);
     }
 }
-__global__ void __launch_bounds__(kRedistBS, 1) k_redist_replay(RedistArgs a) { k_redist_replay_body(VB{blockIdx.x, gridDim.x}, a); }
+__global__ void __launch_bounds__(kRedistBS, 1) k_redist_replay(RedistArgs a) { pdl_begin(); k_redist_replay_body(VB{blockIdx.x, gridDim.x}, a); }
 
 constexpr size_t kRedistSmem = (size_t)kRedistTable * 8 + (size_t)kRedistTable * 4 * 2 +
                                (size_t)kRedistSmemCand * 4 + (size_t)kRedistSmemCand * 7 * 2 + kRedistTable;
@@ -1334,7 +1334,7 @@ __device__ __forceinline__ void k_redist_par_body(VB, RedistArgs a) {
     t.slots = a.slots;
     redist_par_run(a, t);
 }
-__global__ void __launch_bounds__(kRpBS, 1) k_redist_par(RedistArgs a) { k_redist_par_body(VB{blockIdx.x, gridDim.x}, a); }
+__global__ void __launch_bounds__(kRpBS, 1) k_redist_par(RedistArgs a) { pdl_begin(); k_redist_par_body(VB{blockIdx.x, gridDim.x}, a); }
 
 // The same rounds over every SM: a cooperative launch, one CTA per team rank.
 __global__ void __launch_bounds__(kRpBS, 2) k_redist_par_grid(RedistArgs a, double* slots, unsigned* bar) {

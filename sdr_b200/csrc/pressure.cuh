@@ -43,7 +43,7 @@ __device__ __forceinline__ void k_lines_count_body(VB vb_, Grid g, const uint8_t
     cnt[t] = n;
 }
 __global__ void k_lines_count(Grid g, const uint8_t* __restrict__ cells, int nlevels,
-                              uint32_t* __restrict__ cnt) { k_lines_count_body(VB{blockIdx.x, gridDim.x}, g, cells, nlevels, cnt); }
+                              uint32_t* __restrict__ cnt) { pdl_begin(); k_lines_count_body(VB{blockIdx.x, gridDim.x}, g, cells, nlevels, cnt); }
 
 // Assign wavefront positions: pos = line base + rank along j.
 __device__ __forceinline__ void k_lines_assign_body(VB vb_, Grid g, const uint8_t* __restrict__ cells, int nlevels,
@@ -67,7 +67,7 @@ __device__ __forceinline__ void k_lines_assign_body(VB vb_, Grid g, const uint8_
 }
 __global__ void k_lines_assign(Grid g, const uint8_t* __restrict__ cells, int nlevels,
                                const uint32_t* __restrict__ base, int* __restrict__ pos_of_cell,
-                               uint32_t* __restrict__ lv_cell) { k_lines_assign_body(VB{blockIdx.x, gridDim.x}, g, cells, nlevels, base, pos_of_cell, lv_cell); }
+                               uint32_t* __restrict__ lv_cell) { pdl_begin(); k_lines_assign_body(VB{blockIdx.x, gridDim.x}, g, cells, nlevels, base, pos_of_cell, lv_cell); }
 
 // Level starts from the (level, k) line bases; nf is the device fluid count.
 __device__ __forceinline__ void k_level_starts_dev_body(VB vb_, const uint32_t* __restrict__ base, int nlevels, int nz,
@@ -77,7 +77,7 @@ __device__ __forceinline__ void k_level_starts_dev_body(VB vb_, const uint32_t* 
     if (L == nlevels) level_start[L] = (int)*nf;
 }
 __global__ void k_level_starts_dev(const uint32_t* __restrict__ base, int nlevels, int nz,
-                                   const uint32_t* __restrict__ nf, int* __restrict__ level_start) { k_level_starts_dev_body(VB{blockIdx.x, gridDim.x}, base, nlevels, nz, nf, level_start); }
+                                   const uint32_t* __restrict__ nf, int* __restrict__ level_start) { pdl_begin(); k_level_starts_dev_body(VB{blockIdx.x, gridDim.x}, base, nlevels, nz, nf, level_start); }
 
 struct TableArgs {
     Grid g;
@@ -140,7 +140,7 @@ __device__ __forceinline__ void k_tables_body(VB vb_, TableArgs a) {
     }
     a.b[pos] = dmul(-a.inv_scale, dsub(div, s));
 }
-__global__ void k_tables(TableArgs a) { k_tables_body(VB{blockIdx.x, gridDim.x}, a); }
+__global__ void k_tables(TableArgs a) { pdl_begin(); k_tables_body(VB{blockIdx.x, gridDim.x}, a); }
 
 // Fluid cells in cell-index order -> wavefront position, for the chunked dot. The
 // dense pressure is cleared on the way (the solve writes the fluid cells).
@@ -152,7 +152,7 @@ __device__ __forceinline__ void k_fluid_flags_body(VB vb_, const uint8_t* __rest
     p_dense[c] = 0.0;
 }
 __global__ void k_fluid_flags(const uint8_t* __restrict__ cells, size_t n, uint32_t* __restrict__ flag,
-                              double* __restrict__ p_dense) { k_fluid_flags_body(VB{blockIdx.x, gridDim.x}, cells, n, flag, p_dense); }
+                              double* __restrict__ p_dense) { pdl_begin(); k_fluid_flags_body(VB{blockIdx.x, gridDim.x}, cells, n, flag, p_dense); }
 
 __device__ __forceinline__ void k_corder_body(VB vb_, const uint8_t* __restrict__ cells, size_t n, const uint32_t* __restrict__ off,
                          const int* __restrict__ pos_of_cell, int* __restrict__ corder, int* __restrict__ cinv,
@@ -167,7 +167,7 @@ __device__ __forceinline__ void k_corder_body(VB vb_, const uint8_t* __restrict_
 }
 __global__ void k_corder(const uint8_t* __restrict__ cells, size_t n, const uint32_t* __restrict__ off,
                          const int* __restrict__ pos_of_cell, int* __restrict__ corder, int* __restrict__ cinv,
-                         int* __restrict__ chunk_start, int nchunks, const uint32_t* __restrict__ nf) { k_corder_body(VB{blockIdx.x, gridDim.x}, cells, n, off, pos_of_cell, corder, cinv, chunk_start, nchunks, nf); }
+                         int* __restrict__ chunk_start, int nchunks, const uint32_t* __restrict__ nf) { pdl_begin(); k_corder_body(VB{blockIdx.x, gridDim.x}, cells, n, off, pos_of_cell, corder, cinv, chunk_start, nchunks, nf); }
 
 struct PcgArgs {
     const uint32_t* nf;  // device fluid count
@@ -955,7 +955,7 @@ __device__ __forceinline__ void k_pcg_body(VB vb_, PcgArgs a) {
         }
     }
 }
-__global__ void __launch_bounds__(kPcgBS, 1) k_pcg(PcgArgs a) { k_pcg_body(VB{blockIdx.x, gridDim.x}, a); }
+__global__ void __launch_bounds__(kPcgBS, 1) k_pcg(PcgArgs a) { pdl_begin(); k_pcg_body(VB{blockIdx.x, gridDim.x}, a); }
 
 // apply_pressure_gradient (pressure.rs:285-332): one thread per node owning
 // its u/v/w faces; f64 update rounded back to the f32 face.
@@ -989,6 +989,6 @@ __device__ __forceinline__ void k_gradient_body(VB vb_, Grid g, const uint8_t* _
 }
 __global__ void k_gradient(Grid g, const uint8_t* __restrict__ cells, const double* __restrict__ p,
                            double coef, float* __restrict__ u, float* __restrict__ v,
-                           float* __restrict__ w) { k_gradient_body(VB{blockIdx.x, gridDim.x}, g, cells, p, coef, u, v, w); }
+                           float* __restrict__ w) { pdl_begin(); k_gradient_body(VB{blockIdx.x, gridDim.x}, g, cells, p, coef, u, v, w); }
 
 }  // namespace sdr

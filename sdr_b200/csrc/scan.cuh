@@ -50,7 +50,7 @@ __device__ __forceinline__ void k_scan_tiles_body(VB vb_, const uint32_t* __rest
     if (threadIdx.x == 0) tile_sums[vb_.bid] = tot;
 }
 __global__ void __launch_bounds__(kScanBS) k_scan_tiles(const uint32_t* __restrict__ in, uint32_t n,
-                                                       uint32_t* __restrict__ tile_sums) { k_scan_tiles_body(VB{blockIdx.x, gridDim.x}, in, n, tile_sums); }
+                                                       uint32_t* __restrict__ tile_sums) { pdl_begin(); k_scan_tiles_body(VB{blockIdx.x, gridDim.x}, in, n, tile_sums); }
 
 // One block scans all tile sums (exclusive) in order; writes the grand total.
 __device__ __forceinline__ void k_scan_sums_body(VB vb_, uint32_t* __restrict__ sums, uint32_t nt,
@@ -68,7 +68,7 @@ __device__ __forceinline__ void k_scan_sums_body(VB vb_, uint32_t* __restrict__ 
     if (threadIdx.x == 0 && total) *total = carry;
 }
 __global__ void __launch_bounds__(kScanBS) k_scan_sums(uint32_t* __restrict__ sums, uint32_t nt,
-                                                      uint32_t* __restrict__ total) { k_scan_sums_body(VB{blockIdx.x, gridDim.x}, sums, nt, total); }
+                                                      uint32_t* __restrict__ total) { pdl_begin(); k_scan_sums_body(VB{blockIdx.x, gridDim.x}, sums, nt, total); }
 
 __device__ __forceinline__ void k_scan_apply_body(VB vb_, const uint32_t* __restrict__ in, uint32_t n,
                                                        const uint32_t* __restrict__ tile_off,
@@ -96,6 +96,6 @@ __device__ __forceinline__ void k_scan_apply_body(VB vb_, const uint32_t* __rest
 }
 __global__ void __launch_bounds__(kScanBS) k_scan_apply(const uint32_t* __restrict__ in, uint32_t n,
                                                        const uint32_t* __restrict__ tile_off,
-                                                       uint32_t* __restrict__ out, uint32_t* __restrict__ out2) { k_scan_apply_body(VB{blockIdx.x, gridDim.x}, in, n, tile_off, out, out2); }
+                                                       uint32_t* __restrict__ out, uint32_t* __restrict__ out2) { pdl_begin(); k_scan_apply_body(VB{blockIdx.x, gridDim.x}, in, n, tile_off, out, out2); }
 
 }  // namespace sdr

@@ -271,7 +271,7 @@ struct DevStatus {
 __device__ __forceinline__ void k_set_u32_body(VB, uint32_t* p, uint32_t v) {
     if (threadIdx.x == 0) *p = v;
 }
-__global__ void k_set_u32(uint32_t* p, uint32_t v) { k_set_u32_body(VB{blockIdx.x, gridDim.x}, p, v); }
+__global__ void k_set_u32(uint32_t* p, uint32_t v) { pdl_begin(); k_set_u32_body(VB{blockIdx.x, gridDim.x}, p, v); }
 __device__ __forceinline__ void k_redist_begin_body(VB vb_, RedistState* r, unsigned* bar, uint32_t* hist, size_t ncell) {
     const size_t c = (size_t)vb_.bid * blockDim.x + threadIdx.x;
     if (c < ncell) hist[c] = 0u;
@@ -284,7 +284,7 @@ __device__ __forceinline__ void k_redist_begin_body(VB vb_, RedistState* r, unsi
     r->nmoves_par = 0;
     r->err = 0;
 }
-__global__ void k_redist_begin(RedistState* r, unsigned* bar, uint32_t* hist, size_t ncell) { k_redist_begin_body(VB{blockIdx.x, gridDim.x}, r, bar, hist, ncell); }
+__global__ void k_redist_begin(RedistState* r, unsigned* bar, uint32_t* hist, size_t ncell) { pdl_begin(); k_redist_begin_body(VB{blockIdx.x, gridDim.x}, r, bar, hist, ncell); }
 __device__ __forceinline__ void k_redist_end_body(VB, const RedistState* r, DevStatus* s) {
     if (threadIdx.x != 0) return;
     s->moves = r->moves_total;
@@ -294,7 +294,7 @@ __device__ __forceinline__ void k_redist_end_body(VB, const RedistState* r, DevS
     s->redist_long = r->long_total;
     s->redist_rounds = r->rounds_total;
 }
-__global__ void k_redist_end(const RedistState* r, DevStatus* s) { k_redist_end_body(VB{blockIdx.x, gridDim.x}, r, s); }
+__global__ void k_redist_end(const RedistState* r, DevStatus* s) { pdl_begin(); k_redist_end_body(VB{blockIdx.x, gridDim.x}, r, s); }
 
 // The kernels of a substep as packable operations (largest block of their call sites).
 SDR_OP(k_set_u32, 32)
@@ -506,9 +506,19 @@ struct sdr_solver {
             pk->record<Op>(line, grid, block, smem, args...);
             return;
         }
-        kern<<<grid, block, smem, st>>>(args...);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(block);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        // Not beside other scenes: blocks that wait would hold places the others' could use.
+        cfg.numAttrs = shared_gpu ? 0 : 1;
+        CK(cudaLaunchKernelEx(&cfg, kern, args...));
         g_launches.fetch_add(1, std::memory_order_relaxed);
-        CK(cudaGetLastError());
     }
     void mset(int line, void* p, int v, size_t bytes) {
         if (!bytes) return;
