@@ -1161,6 +1161,9 @@ out:
 // Launched cooperatively (every CTA resident at once), one CTA per SM.
 __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) { tw_solve<false>(t); }
 // Launched as one cluster with a CTA per tile of the grid.
-__global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles_cluster(TwArgs t) { tw_solve<true>(t); }
+__global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles_cluster(TwArgs t) {
+    pdl_begin();
+    tw_solve<true>(t);
+}
 
 }  // namespace sdr

@@ -111,26 +111,28 @@ int cluster_ctas(Kern kernel, int slot, int threads, int device, size_t dyn_smem
 
 // Launch a kernel as exactly one cluster of `ctas` CTAs on `st`.
 template <class Kern, class... Args>
-void launch_one_cluster_smem(Kern kernel, int ctas, int threads, size_t dyn_smem, cudaStream_t st, Args... args) {
+void launch_one_cluster_smem(Kern kernel, int ctas, int threads, size_t dyn_smem, bool pdl, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = dyn_smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)ctas;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl ? 2 : 1;  // pdl: the kernel begins with pdl_begin()
     CK(cudaLaunchKernelEx(&cfg, kernel, args...));
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
 template <class Kern, class... Args>
 void launch_one_cluster(Kern kernel, int ctas, int threads, cudaStream_t st, Args... args) {
-    launch_one_cluster_smem(kernel, ctas, threads, 0, st, args...);
+    launch_one_cluster_smem(kernel, ctas, threads, 0, false, st, args...);
 }
 
 // Solver-owned device buffers come from one library memory pool per device,
@@ -922,7 +924,7 @@ struct sdr_solver {
                 // launch overlaps other streams' kernels like any other
                 SLAUNCH(k_pcg, 1, kPcgBS, kPcgSmem, st, a);
             } else {
-                launch_one_cluster_smem(k_pcg, ctas, kPcgBS, kPcgSmem, st, a);
+                launch_one_cluster_smem(k_pcg, ctas, kPcgBS, kPcgSmem, false, st, a);
             }
         }
     }
@@ -1013,7 +1015,7 @@ struct sdr_solver {
         t.err = &dst->err;
         t.plane = tw_plane_levels();
         if (tw_cluster > 0) {
-            launch_one_cluster_smem(k_pcg_tiles_cluster, tw_cluster, kTwBS, tw_cluster_smem(t.plane), st, t);
+            launch_one_cluster_smem(k_pcg_tiles_cluster, tw_cluster, kTwBS, tw_cluster_smem(t.plane), true, st, t);
             return;
         }
         CK(cudaMemsetAsync(tw_bar, 0, 2 * sizeof(unsigned), st));  // a wound-down launch may leave arrivals
