@@ -212,6 +212,7 @@ struct SdfFast {
     uint32_t* gate;         // 1: k_sdf_mesh writes the field
     float4* ball;           // per triangle: bounding sphere (padded to whole groups of 32)
     float4* group;          // per 32 triangles: their bounding sphere
+    float4* norm;           // per triangle: unit normal
     float4* vert;           // per triangle: three vertices; vert[3 t].w: the f32 distance holds up to this distance squared
     double* dist;           // per node
     uint32_t* up;           // per node: the neighbour it follows, or itself; later its root
@@ -309,6 +310,8 @@ __global__ void __launch_bounds__(256) k_sdf_balls(SdfFast a) {
         if (!(nn > 1e-10 * (double)ext * (double)ext * l2)) *a.gate = 1u;
         ball = make_float4((float)(g[0] - a.cx), (float)(g[1] - a.cy), (float)(g[2] - a.cz),
                            __double2float_ru(sqrt(r2)) * 1.000001f + 2e-6f * ext);
+        const double rn = 1.0 / sqrt(nn);
+        a.norm[t] = make_float4((float)(n0 * rn), (float)(n1 * rn), (float)(n2 * rn), 0.0f);
         for (int q = 0; q < 3; ++q)
             a.vert[3 * (size_t)t + q] = make_float4((float)(v[3 * q] - a.cx), (float)(v[3 * q + 1] - a.cy),
                                                     (float)(v[3 * q + 2] - a.cz), (float)(0.02 / (64.0 * 6e-8) * nn / l2));
@@ -365,11 +368,24 @@ __device__ __forceinline__ float sdf_dist_f(float px, float py, float pz, float4
     return sq(apx - (v * abx + w * acx), apy - (v * aby + w * acy), apz - (v * abz + w * acz));
 }
 
+// Is a triangle further than `near` from a point at (x, y, z) from its sphere's
+// centre c? Its points are c + s with s in its plane and |s| <= w, so their
+// distance squared is at least f^2 - 2 t w for a point f from c whose offset has
+// the length t along the plane: tight where the triangle faces the point, as the
+// candidates for its nearest one mostly do (the sphere alone leaves a shell of
+// its radius). f and the height over the plane are off by less than `slack`.
+__device__ __forceinline__ bool sdf_beyond(float x, float y, float z, float w, float4 nrm, float near, float slack) {
+    const float f = sqrtf(x * x + y * y + z * z), h = fmaxf(fabsf(x * nrm.x + y * nrm.y + z * nrm.z) - slack, 0.0f);
+    const float hi = f + slack, lo = f - slack;
+    const float t = sqrtf(fmaxf(hi * hi - h * h, 0.0f) + 1e-6f * hi * hi);
+    return lo * lo * 0.99999f - 2.002f * t * w > near * near;
+}
+
 constexpr int kSdfB = 4;                               // nodes of a brick along each axis
 constexpr int kSdfNodes = kSdfB * kSdfB * kSdfB;       // 64
 constexpr int kSdfSplit = 4;                           // threads per node
 constexpr int kSdfDistBS = kSdfNodes * kSdfSplit;      // 256
-constexpr int kSdfList = 608;                          // triangles a brick considers at a time
+constexpr int kSdfList = 512;                          // triangles a brick considers at a time
 constexpr int kSdfWarpList = 256;                      // and a warp's eight nodes
 static_assert(kSdfWarpList / kSdfSplit <= 64, "a bit per entry of a lane");
 static_assert(kSdfB == 4 && kSdfSplit == 4 && kSdfDistBS == 256, "eight warps of 2 x 2 x 2 nodes");
@@ -380,14 +396,20 @@ static_assert(kSdfB == 4 && kSdfSplit == 4 && kSdfDistBS == 256, "eight warps of
 // the brick), then the same again per warp for its eight nodes. Then per node,
 // four lanes sharing the list: the f32 distances give an upper bound of the
 // node's own, and the triangles that may be nearer than it within the error
-// bounds are evaluated in f64. The margins (1e-3 and
-// 2e-6 of the extent) cover the rounding of the f32 and f64 distances
-// (k_sdf_balls), so no triangle that could give the minimum is left out.
-__global__ void __launch_bounds__(kSdfDistBS) k_sdf_dist(SdfFast a, int bx, int by) {
+// bounds are evaluated in f64. Deep inside a smooth cavity the spheres leave
+// hundreds of triangles a node: the bound by the normal (sdf_beyond) and the
+// distance of a vertex as upper bound leave a few (20,480 triangles, 0.8 M nodes:
+// 4.6 -> 3.0 ms a field). Three blocks an SM take 3.0 ms, two 3.5, four 3.0 to
+// 3.8 (spilling). The margins (1e-3 and 2e-6 of the extent) cover the rounding of
+// the f32 and f64 distances (k_sdf_balls), so no triangle that could give the
+// minimum is left out.
+__global__ void __launch_bounds__(kSdfDistBS, 3) k_sdf_dist(SdfFast a, int bx, int by) {
     __shared__ float4 s_ball[kSdfList];
     __shared__ float4 s_vert[kSdfList * 3];
+    __shared__ float4 s_norm[kSdfList];
     __shared__ uint32_t s_tri[kSdfList];
-    __shared__ uint32_t s_n;
+    __shared__ uint32_t s_n, s_ng;
+    __shared__ uint32_t s_group[kSdfDistBS];  // of the groups looked at together: those within reach
     __shared__ float s_u[kSdfDistBS / 32];
     __shared__ uint16_t s_w[kSdfDistBS / 32][kSdfWarpList];
     if (*a.gate) return;
@@ -425,12 +447,32 @@ __global__ void __launch_bounds__(kSdfDistBS) k_sdf_dist(SdfFast a, int bx, int 
         u = fminf(u, far_of(q) + q.w);
     }
     u = block_min(u) * 1.0001f;
+    // the groups from g0 on, one per thread, within r of the brick's centre
+    auto groups_within = [&](uint32_t g0, float r) {
+        const uint32_t g = g0 + tid;
+        bool in = false;
+        if (g < ngroup) {
+            const float4 q = a.group[g];
+            in = far_of(q) * 0.9999f <= r + q.w;
+        }
+        __syncthreads();  // the list before has been used
+        if (tid == 0) s_ng = 0u;
+        __syncthreads();
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        uint32_t at = 0;
+        if (lane == 0 && m) at = atomicAdd(&s_ng, (uint32_t)__popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (in) s_group[at] = g;
+        __syncthreads();
+        return s_ng;
+    };
     float u2 = u;  // the same from the triangles of the groups that can hold the nearest one
-    for (uint32_t g = wid; g < ngroup; g += kWarps) {
-        const float4 q = a.group[g];
-        if (far_of(q) * 0.9999f > u + q.w) continue;
-        const float4 t = a.ball[(size_t)g * 32 + lane];
-        if (t.w >= 0.0f) u2 = fminf(u2, far_of(t) + t.w);
+    for (uint32_t g0 = 0; g0 < ngroup; g0 += kSdfDistBS) {
+        const uint32_t ng = groups_within(g0, u);
+        for (uint32_t e = wid; e < ng; e += kWarps) {
+            const float4 t = a.ball[(size_t)s_group[e] * 32 + lane];
+            if (t.w >= 0.0f) u2 = fminf(u2, far_of(t) + t.w);
+        }
     }
     u = block_min(u2) * 1.0001f;
     const float reach = u * 1.001f + 2.0f * rad;  // a triangle of the brick: centre within reach + its radius
@@ -445,35 +487,39 @@ __global__ void __launch_bounds__(kSdfDistBS) k_sdf_dist(SdfFast a, int bx, int 
     double min_d2 = INFINITY;
     if (tid == 0) s_n = 0u;
     __syncthreads();
-    for (uint32_t g0 = 0; g0 < ngroup; g0 += kWarps) {
-        const uint32_t g = g0 + wid;
-        if (g < ngroup) {
-            const float4 q = a.group[g];
-            if (far_of(q) * 0.9999f <= reach + q.w) {
-                const float4 t = a.ball[(size_t)g * 32 + lane];
-                const bool in = t.w >= 0.0f && far_of(t) * 0.9999f <= reach + t.w;
-                const unsigned m = __ballot_sync(0xffffffffu, in);
-                uint32_t at = 0;
-                if (lane == 0 && m) at = atomicAdd(&s_n, (uint32_t)__popc(m));
-                at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
-                if (in) {
-                    const float4* v = a.vert + 3 * ((size_t)g * 32 + lane);
-                    s_ball[at] = t;
-                    for (int c = 0; c < 3; ++c) s_vert[3 * at + c] = v[c];
-                    s_tri[at] = g * 32 + lane;
-                }
+    for (uint32_t g0 = 0, e0 = 0, ng = 0;; e0 += kWarps) {
+        if (e0 >= ng) {  // the next groups
+            ng = groups_within(g0, reach);
+            g0 += kSdfDistBS;
+            e0 = 0;
+        }
+        const uint32_t e1 = e0 + wid;
+        if (e1 < ng) {
+            const uint32_t tri = s_group[e1] * 32 + lane;
+            const float4 t = a.ball[tri];
+            const bool in = t.w >= 0.0f && far_of(t) * 0.9999f <= reach + t.w;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            uint32_t at = 0;
+            if (lane == 0 && m) at = atomicAdd(&s_n, (uint32_t)__popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+            if (in) {
+                const float4* v = a.vert + 3 * (size_t)tri;
+                s_ball[at] = t;
+                s_norm[at] = a.norm[tri];
+                for (int c = 0; c < 3; ++c) s_vert[3 * at + c] = v[c];
+                s_tri[at] = tri;
             }
         }
         // a round adds at most kWarps * 32 triangles
-        const bool last = g0 + kWarps >= ngroup;
+        const bool last = g0 >= ngroup && e0 + kWarps >= ng;
         __syncthreads();
         const uint32_t n = s_n;
         __syncthreads();
         if (!last && n + kWarps * 32 <= kSdfList) continue;  // room for another
         for (uint32_t c = lane; c < n; c += 32) {
-            const float4 q = s_ball[c];
+            const float4 q = s_vert[3 * c];  // any point of the triangle bounds its distance
             const float x = q.x - wx, y = q.y - wy, z = q.z - wz;
-            uw = fminf(uw, (sqrtf(x * x + y * y + z * z) + q.w) * 1.0001f);
+            uw = fminf(uw, sqrtf(x * x + y * y + z * z) * 1.0001f + slack);
         }
         for (int o = 16; o > 0; o >>= 1) uw = fminf(uw, __shfl_xor_sync(0xffffffffu, uw, o));
         ub = fminf(ub, (uw + wrad) * 1.0001f);
@@ -485,7 +531,7 @@ __global__ void __launch_bounds__(kSdfDistBS) k_sdf_dist(SdfFast a, int bx, int 
             if (c < n) {
                 const float4 q = s_ball[c];
                 const float x = q.x - wx, y = q.y - wy, z = q.z - wz;
-                in = sqrtf(x * x + y * y + z * z) * 0.9999f <= wreach + q.w;
+                in = !sdf_beyond(x, y, z, q.w, s_norm[c], wreach, slack);
             }
             const unsigned m = __ballot_sync(0xffffffffu, in);
             if (in) s_w[wid][cnt + __popc(m & ((1u << lane) - 1u))] = (uint16_t)c;
@@ -498,7 +544,7 @@ __global__ void __launch_bounds__(kSdfDistBS) k_sdf_dist(SdfFast a, int bx, int 
                 const uint32_t at = s_w[wid][e];
                 const float4 q = s_ball[at];
                 const float x = q.x - px, y = q.y - py, z = q.z - pz, r = ub * 1.001f + q.w, f2 = x * x + y * y + z * z;
-                if (f2 > r * r * 1.0002f) continue;
+                if (f2 > r * r * 1.0002f || sdf_beyond(x, y, z, q.w, s_norm[at], ub * 1.001f, slack)) continue;
                 const float4 A = s_vert[3 * at];
                 float least = 0.0f;
                 if (f2 > A.w) {
@@ -531,6 +577,7 @@ __global__ void __launch_bounds__(kSdfDistBS) k_sdf_dist(SdfFast a, int bx, int 
             __syncwarp();
         }
         __syncthreads();
+        if (last) break;
         if (tid == 0) s_n = 0u;
         __syncthreads();
     }

@@ -2344,7 +2344,7 @@ int sdr_sdf_from_mesh(const double* tris, size_t ntri, sdr_vec3 origin, double d
         const size_t least = bytes;
         const size_t ntri_b = (size_t)blocks(ntri, 256) * 256;  // k_sdf_balls writes whole blocks
         const size_t o_ball = fast ? room(ntri_b * sizeof(float4)) : 0, o_group = fast ? room(ntri_b / 32 * sizeof(float4)) : 0,
-                     o_vert = fast ? room(ntri * 3 * sizeof(float4)) : 0, o_dist = fast ? room(nn * 8) : 0,
+                     o_norm = fast ? room(ntri * sizeof(float4)) : 0, o_vert = fast ? room(ntri * 3 * sizeof(float4)) : 0, o_dist = fast ? room(nn * 8) : 0,
                      o_up = fast ? room(nn * 4) : 0, o_roots = fast ? room((nn + 1) * 4) : 0, o_in = fast ? room(nn) : 0;
         unsigned char* dev = nullptr;
         cudaStream_t st = nullptr;
@@ -2382,6 +2382,7 @@ int sdr_sdf_from_mesh(const double* tris, size_t ntri, sdr_vec3 origin, double d
                 f.gate = gate;
                 f.ball = (float4*)(dev + o_ball);
                 f.group = (float4*)(dev + o_group);
+                f.norm = (float4*)(dev + o_norm);
                 f.vert = (float4*)(dev + o_vert);
                 f.dist = (double*)(dev + o_dist);
                 f.up = (uint32_t*)(dev + o_up);
