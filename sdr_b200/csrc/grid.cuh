@@ -82,7 +82,7 @@ __global__ void k_cavity_and_base(Grid g, SdfD s, int has_outlet, Aabb outlet,
 __device__ __forceinline__ void k_extrap_valid_body(VB vb_, Grid g, const uint8_t* __restrict__ cells, uint8_t* __restrict__ ku,
                                uint8_t* __restrict__ kv, uint8_t* __restrict__ kw, uint32_t* __restrict__ brick, uint32_t epoch,
                                unsigned int* __restrict__ maxbits) {
-    if (vb_.bid == 0 && threadIdx.x < 3) maxbits[threadIdx.x] = 0u;  // of the last sweep
+    if (vb_.bid == 0 && threadIdx.x < 3) maxbits[threadIdx.x] = 0u;  // of k_face_max
     int i, j, k;
     if (!node_of(g, (size_t)vb_.bid * blockDim.x + threadIdx.x, i, j, k)) return;
     auto fl = [&](int a, int b, int c) {
@@ -150,65 +150,74 @@ struct ExtrapArgs {
     uint8_t* kv;
     uint8_t* kw;
     int sweep;              // 0..3
-    unsigned int* maxbits;  // optional: |u|,|v|,|w| maxima (last sweep)
     const uint32_t* brick;  // per brick of nodes: the last extrapolation that reached it
+    uint32_t nbricks;
     uint32_t epoch;         // this extrapolation's number
 };
 
-// A block per brick. One out of the liquid's reach has nothing to extrapolate
-// (its faces only count for the maxima): in a 0.2 mm pool that is two thirds of
-// the nodes, before the jet has filled a cavity nearly all. With the gradient,
-// at 2 mm 65 -> 46 us and in the pool 522 -> 359 us against a test of the 27
-// bricks around, two nodes a thread and every warp's maxima in atomics: small
-// scenes wait for round trips, the pool's last sweep queued on the atomics.
-__device__ __forceinline__ void k_extrap_body(VB vb_, ExtrapArgs a) {
+// The faces of one brick's nodes, a node per thread.
+__device__ __forceinline__ void extrap_brick(const ExtrapArgs& a, const BrickPos& b, int tid) {
     const Grid& g = a.g;
-    const bool near = a.brick[vb_.bid] == a.epoch;
-    if (!near && !a.maxbits) return;
-    const BrickPos b = brick_of(g, vb_.bid);
-    const int tid = (int)threadIdx.x;
     const int i = b.i0 + tid % kBrick, j = b.j0 + tid / kBrick % kBrick, k = b.k0 + tid / (kBrick * kBrick);
     const bool hu = j < g.ny && k < g.nz && i <= g.nx, hv = i < g.nx && k < g.nz && j <= g.ny, hw = i < g.nx && j < g.ny && k <= g.nz;
     const size_t cu = ((size_t)k * g.ny + j) * (g.nx + 1) + i, cv = ((size_t)k * (g.ny + 1) + j) * g.nx + i,
                  cw = ((size_t)k * g.ny + j) * g.nx + i;
-    if (near) {
-        const bool du = hu && !a.ku[cu], dv = hv && !a.kv[cv], dw = hw && !a.kw[cw];  // not known yet
-        if (du) extrap_one(a.u, a.ku, a.sweep, g.nx + 1, g.ny, g.nz, i, j, k);
-        if (dv) extrap_one(a.v, a.kv, a.sweep, g.nx, g.ny + 1, g.nz, i, j, k);
-        if (dw) extrap_one(a.w, a.kw, a.sweep, g.nx, g.ny, g.nz + 1, i, j, k);
-    }
-    if (a.maxbits) {
-        // Non-negative floats order like their bit patterns (a NaN counts as 0):
-        // an exact maximum per warp, block and grid. One block's atomics at most,
-        // and only for a larger value: of every warp, they queued on three words.
-        __shared__ uint32_t s_max[3][kBrickBS / 32];
-        const float m[3] = {fmaxf(0.f, hu ? fabsf(a.u[cu]) : 0.f), fmaxf(0.f, hv ? fabsf(a.v[cv]) : 0.f),
-                            fmaxf(0.f, hw ? fabsf(a.w[cw]) : 0.f)};
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m[c]));
-            if ((tid & 31) == 0) s_max[c][tid / 32] = w;
-        }
+    const bool du = hu && !a.ku[cu], dv = hv && !a.kv[cv], dw = hw && !a.kw[cw];  // not known yet
+    if (du) extrap_one(a.u, a.ku, a.sweep, g.nx + 1, g.ny, g.nz, i, j, k);
+    if (dv) extrap_one(a.v, a.kv, a.sweep, g.nx, g.ny + 1, g.nz, i, j, k);
+    if (dw) extrap_one(a.w, a.kw, a.sweep, g.nx, g.ny, g.nz + 1, i, j, k);
+}
+
+// A block takes every vb_.nb-th brick; those out of the liquid's reach have nothing
+// to extrapolate (in a 0.2 mm pool two thirds of the nodes, before the jet has
+// filled a cavity nearly all). Small scenes wait for round trips: with the gradient,
+// at 2 mm 65 -> 34 us against a test of the 27 bricks around, two nodes a thread
+// and conditional loads one after another. In the pool 522 -> 294 us: there the
+// blocks of empty bricks and every warp's atomics for the maxima cost the time.
+__device__ __forceinline__ void k_extrap_body(VB vb_, ExtrapArgs a) {
+    const Grid& g = a.g;
+    const int tid = (int)threadIdx.x;
+    __shared__ uint32_t s_list[kBrickBS], s_n;
+    // the block's bricks, kBrickBS at a time, a thread each: those within reach
+    for (uint32_t base = vb_.bid; base < a.nbricks; base += vb_.nb * kBrickBS) {
+        const uint32_t mine = base + (uint32_t)tid * vb_.nb;
+        const bool in = mine < a.nbricks && a.brick[mine] == a.epoch;
+        if (!__syncthreads_or(in)) continue;
+        if (tid == 0) s_n = 0u;
         __syncthreads();
-        if (tid < 32) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const uint32_t w = __reduce_max_sync(0xffffffffu, s_max[c][tid % (kBrickBS / 32)]);
-                if (tid == 0 && w > __ldcg(a.maxbits + c)) atomicMax(a.maxbits + c, w);
-            }
-        }
+        if (in) s_list[atomicAdd(&s_n, 1u)] = mine;
+        __syncthreads();
+        const uint32_t n = s_n;
+        for (uint32_t q = 0; q < n; ++q) extrap_brick(a, brick_of(g, s_list[q]), tid);
     }
 }
 __global__ void __launch_bounds__(kBrickBS) k_extrap(ExtrapArgs a) { pdl_begin(); k_extrap_body(VB{blockIdx.x, gridDim.x}, a); }
 
-// Face maxima alone (used when extrapolation did not run, e.g. phase mode).
-__device__ __forceinline__ void k_face_max_body(VB vb_, const float* __restrict__ f, size_t n, unsigned int* __restrict__ out) {
+// The faces' maxima |u|, |v|, |w|, a third of the grid's blocks (at least one)
+// each. Non-negative floats order like their bit patterns (a NaN counts as 0):
+// an exact maximum per warp, block and grid, with an atomic for a larger value only.
+constexpr int kFaceMaxBS = 256;
+__device__ __forceinline__ void k_face_max_body(VB vb_, Faces f, size_t nu, size_t nv, size_t nw, unsigned int* __restrict__ out) {
+    __shared__ uint32_t s_max[kFaceMaxBS / 32];
+    const int c = (int)(vb_.bid % 3), tid = (int)threadIdx.x;
+    const float* const p = c == 0 ? f.u : c == 1 ? f.v : f.w;
+    const size_t n = c == 0 ? nu : c == 1 ? nv : nw;
+    const size_t step = (size_t)(vb_.nb / 3) * kFaceMaxBS;
+    const float4* const p4 = reinterpret_cast<const float4*>(p);
     float m = 0.f;
-    for (size_t q = (size_t)vb_.bid * blockDim.x + threadIdx.x; q < n; q += (size_t)vb_.nb * blockDim.x)
-        m = fmaxf(m, fabsf(f[q]));
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+#pragma unroll 4
+    for (size_t q = (size_t)(vb_.bid / 3) * kFaceMaxBS + tid; q < n / 4; q += step) {
+        const float4 x = p4[q];
+        m = fmaxf(fmaxf(fmaxf(fmaxf(m, fabsf(x.x)), fabsf(x.y)), fabsf(x.z)), fabsf(x.w));
+    }
+    if (vb_.bid < 3 && tid < (int)(n % 4)) m = fmaxf(m, fabsf(p[n / 4 * 4 + tid]));
+    uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((tid & 31) == 0) s_max[tid / 32] = w;
+    __syncthreads();
+    if (tid >= 32) return;
+    w = __reduce_max_sync(0xffffffffu, s_max[tid % (kFaceMaxBS / 32)]);
+    if (tid == 0 && w > __ldcg(out + c)) atomicMax(out + c, w);
 }
-__global__ void k_face_max(const float* __restrict__ f, size_t n, unsigned int* __restrict__ out) { pdl_begin(); k_face_max_body(VB{blockIdx.x, gridDim.x}, f, n, out); }
+__global__ void __launch_bounds__(kFaceMaxBS) k_face_max(Faces f, size_t nu, size_t nv, size_t nw, unsigned int* __restrict__ out) { pdl_begin(); k_face_max_body(VB{blockIdx.x, gridDim.x}, f, nu, nv, nw, out); }
 
 }  // namespace sdr

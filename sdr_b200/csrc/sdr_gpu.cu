@@ -325,7 +325,7 @@ SDR_OP(k_pcg, kPcgBS)
 SDR_OP(k_gradient, 256)
 SDR_OP(k_extrap_valid, 256)
 SDR_OP(k_extrap, kBrickBS)
-SDR_OP(k_face_max, 256)
+SDR_OP(k_face_max, kFaceMaxBS)
 SDR_OP(k_g2p_advect, kBS)
 SDR_OP(k_bounds_flags, kBS)
 SDR_OP(k_compact, kBS)
@@ -422,7 +422,7 @@ struct sdr_solver {
     float* sdf32 = nullptr;
     float *u = nullptr, *v = nullptr, *w = nullptr, *su = nullptr, *sv = nullptr, *sw = nullptr;
     uint8_t *ku = nullptr, *kv = nullptr, *kw = nullptr;  // extrapolation: when each face became known
-    uint32_t* brick = nullptr;   // per brick of nodes: the last extrapolation in which it had a fluid cell
+    uint32_t* brick = nullptr;   // per brick of nodes: the last extrapolation that reached it
     uint32_t extrap_epoch = 0;   // extrapolations so far
     uint8_t *cells = nullptr, *base = nullptr, *cavity = nullptr;
     float4 *pos = nullptr, *vel = nullptr, *pos2 = nullptr, *vel2 = nullptr;
@@ -1035,16 +1035,21 @@ struct sdr_solver {
         ++extrap_epoch;
         SLAUNCH(k_extrap_valid, ngrid, 256, 0, st, g, cells, ku, kv, kw, brick, extrap_epoch, dst->maxbits);
         for (int it = 0; it < 4; ++it) {  // four sweeps, in place
-            ExtrapArgs e{g, u, v, w, ku, kv, kw, it, it == 3 ? dst->maxbits : nullptr, brick, extrap_epoch};
-            SLAUNCH(k_extrap, nbricks(), kBrickBS, 0, st, e);
+            // three blocks an SM; of a scene beside others one
+            ExtrapArgs e{g, u, v, w, ku, kv, kw, it, brick, nbricks(), extrap_epoch};
+            SLAUNCH(k_extrap, std::min(nbricks(), pk ? 148u : 148u * 3u), kBrickBS, 0, st, e);
         }
+        issue_face_max();
+    }
+
+    void issue_face_max() {
+        const unsigned per = (unsigned)std::min<size_t>(blocks(std::max({nu, nv, nw}) / 4, kFaceMaxBS), 148);
+        SLAUNCH(k_face_max, 3 * per, kFaceMaxBS, 0, st, faces(), nu, nv, nw, dst->maxbits);
     }
 
     void face_max() {
         MSET(dst->maxbits, 0, sizeof(dst->maxbits));
-        SLAUNCH(k_face_max, 296, 256, 0, st, u, nu, &dst->maxbits[0]);
-        SLAUNCH(k_face_max, 296, 256, 0, st, v, nv, &dst->maxbits[1]);
-        SLAUNCH(k_face_max, 296, 256, 0, st, w, nw, &dst->maxbits[2]);
+        issue_face_max();
     }
 
     MoveArgs move_args(double dt) {
