@@ -569,6 +569,7 @@ struct sdr_solver {
     unsigned nbricks() const { return (unsigned)brick_dim(g.nx) * (unsigned)brick_dim(g.ny) * (unsigned)brick_dim(g.nz); }
     Faces saved() const { return Faces{su, sv, sw}; }
     uint32_t* dn() { return &dst->n; }
+    size_t hist_room() const { return (ncell + 1 + 3) / 4 * 4; }  // of a histogram: the scans read 16 bytes at a time
 
     // Exclusive scan; `site` (the caller's line) keys its kernels in a packed launch.
     // out2 (optional): the same again.
@@ -583,9 +584,13 @@ struct sdr_solver {
             dalloc(tsum, nt, st);
             tsum_cap = nt;
         }
-        issue<k_scan_tiles_op>(k_scan_tiles, key + 1, nt, kScanBS, 0, in, (uint32_t)n_, tsum);
-        issue<k_scan_sums_op>(k_scan_sums, key + 2, 1, kScanBS, 0, tsum, nt, total);
-        issue<k_scan_apply_op>(k_scan_apply, key + 3, nt, kScanBS, 0, in, (uint32_t)n_, tsum, out, out2);
+        // of scenes packed together each has the same kernels, whatever its size
+        const bool direct = !pk && (nt == 1 || (nt <= kScanFewTiles && in != out));
+        const int scanned = nt > kScanManyTiles;
+        if (!direct) issue<k_scan_tiles_op>(k_scan_tiles, key + 1, nt, kScanBS, 0, in, (uint32_t)n_, tsum);
+        if (scanned) issue<k_scan_sums_op>(k_scan_sums, key + 2, 1, kScanBS, 0, tsum, nt);
+        issue<k_scan_apply_op>(k_scan_apply, key + 3, nt, kScanBS, 0, in, (uint32_t)n_, (const uint32_t*)(direct ? nullptr : tsum),
+                               scanned, out, out2, total);
     }
 
     void ensure_capacity(size_t need) {
@@ -641,8 +646,8 @@ struct sdr_solver {
         CK(cudaMemsetAsync(sw, 0, nw * 4, st));
         dalloc(cells, nc, st); dalloc(base, nc, st); dalloc(cavity, nc, st);
         CK(cudaMemsetAsync(cells, AIR, nc, st));
-        dalloc(hist_valid, 2 * (nc + 1), st);
-        hist_sort = hist_valid + nc + 1;
+        dalloc(hist_valid, 2 * hist_room(), st);
+        hist_sort = hist_valid + hist_room();
         dalloc(start, nc + 1, st);
         dalloc(fill, nc + 1, st);
         dalloc(long_list, nc, st);
@@ -759,7 +764,7 @@ struct sdr_solver {
 
     void classify(bool mark) {
         if (mark) SLAUNCH(k_base_labels, blocks(ncell + 1, 256), 256, 0, st, base, cells, ncell, hist_valid, hist_sort);
-        else MSET(hist_valid, 0, 2 * (ncell + 1) * 4);  // and hist_sort behind it
+        else MSET(hist_valid, 0, 2 * hist_room() * 4);  // and hist_sort behind it
         if (n)
             SLAUNCH(k_classify_keys, blocks(n, kBS), kBS, 0, st, g, pos, n, (int)has_outlet, outlet,
                    (int)mark, cells, key_cell, key_sort, hist_valid, hist_sort);
