@@ -613,6 +613,10 @@ constexpr int kRedistTable = 4096;   // shared-memory hash slots (power of two)
 constexpr int kRedistProbes = 64;    // linear probes before a cell counts as not fitting the table
 constexpr int kRedistBS = 1024;
 constexpr int kRedistSmemCand = 8192;  // candidates sorted and replayed in shared memory
+// The same where the whole GPU can take longer lists: one block decides 1,100
+// candidates (a 0.8 mm jet) in 142 us a substep against 210, but 4,700 (a 0.5 mm
+// jet) in 404 against 332.
+constexpr uint32_t kRedistReplayGrid = 2048;
 constexpr uint32_t kResolved = 0x80000000u;  // candidate-list flag: decided (particle indices are < 2^31)
 // A shared-memory round costs about as much as warp 0 deciding this many
 // candidates in index order (4,500 cycles against 150 each): rounds that decide
@@ -637,6 +641,7 @@ struct RedistArgs {
     uint32_t* moves;         // pairs (particle, destination cell)
     RedistState* rs;
     unsigned long long* claim;  // per cell: the latest claim stamp (k_redist_par); zero at allocation
+    uint32_t replay_max;        // lists up to here are replayed by one block (at most kRedistSmemCand)
     int rounds;                 // short lists: parallel rounds (1) or warp 0 alone in index order (0)
     double* slots;              // unused by the rounds (kept for the launch layout)
     uint32_t* pend;             // 2 x cand_cap: the rounds' pending unit heads, double-buffered
@@ -753,7 +758,7 @@ __device__ __forceinline__ void k_redist_replay_body(VB vb_, RedistArgs a) {
     }
     const uint32_t nc = nc_all;
     const Grid& g = a.g;
-    const bool in_smem = nc <= (uint32_t)kRedistSmemCand;
+    const bool in_smem = nc <= a.replay_max;
     // ---- sort candidates ascending (indices are distinct)
     if (in_smem) {
         uint32_t np2 = 1;
@@ -1052,7 +1057,11 @@ constexpr size_t kRedistSmem = (size_t)kRedistTable * 8 + (size_t)kRedistTable *
 // The long-list form (redist_par_run) decides units of one cell's consecutive
 // candidates the same way.
 constexpr int kRpBS = 512;
-constexpr uint32_t kRpSoloList = 4 * kRpBS;  // pending units CTA 0 decides alone on the grid form
+// Pending units CTA 0 decides alone on the grid form: one a thread, as a unit is a
+// chain of ten L2 round trips and two grid barriers cost fewer. Redistribution of a
+// 0.5 mm jet / a 0.4 mm / a 0.2 mm pool: from 128 303 / 959 / 1691 us, from 512
+// 293 / 926 / 1647, from 1,024 301 / 954 / 1693, from 2,048 334 / 1059 / 1833.
+constexpr uint32_t kRpSoloList = kRpBS;
 
 // The CTAs that decide one long list: one thread-block cluster (barrier in
 // hardware), or every CTA of a cooperative launch (a bounded grid barrier;

@@ -1131,6 +1131,7 @@ struct sdr_solver {
         if (!shared_gpu && !ctas_rp) ctas_rp = cluster_ctas(k_redist_par, 1, kRpBS, device);
         const int rp_ctas = shared_gpu ? 1 : ctas_rp;
         ra.cap = cap_;
+        ra.replay_max = grid_rounds ? kRedistReplayGrid : (uint32_t)kRedistSmemCand;
         const double dirs[6][3] = {{-1, 0, 0}, {1, 0, 0}, {0, -1, 0}, {0, 1, 0}, {0, 0, -1}, {0, 0, 1}};
         for (int d = 0; d < 6; ++d) ra.down[d] = dirs[d][0] * gd.x + dirs[d][1] * gd.y + dirs[d][2] * gd.z;
         ra.moves = moves;

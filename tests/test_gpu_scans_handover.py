@@ -36,3 +36,31 @@ def test_scans_at_tile_edges(dims, n):
     for w in range(3):
         a, b = gpu.face(w), orc.face(w)
         assert float(np.max(np.abs(a - b))) <= 2 * EPS * float(np.max(np.abs(b)))
+
+
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 4500])
+def test_redistribution_handover_exact(n):
+    gpu, orc, _ = make_pair()
+    nx, ny, nz = gpu.grid_dims
+    st = gpu.stats()
+    cav = gpu.cavity_mask().reshape(nz, ny, nx).astype(bool)
+    inner = cav.copy()
+    for ax in range(3):
+        for sh in (-1, 1):
+            inner &= np.roll(cav, sh, axis=ax)
+    k, j, i = (int(x) for x in np.argwhere(inner)[len(np.argwhere(inner)) // 2])
+    rng = np.random.default_rng(n)
+    pos = f32(np.array([st.origin.x, st.origin.y, st.origin.z]) +
+              (np.array([i, j, k]) + 0.5 + rng.uniform(-0.3, 0.3, (n, 3))) * gpu.dx)
+    vel = np.zeros_like(pos)
+    for s in (gpu, orc):
+        s.set_particles(pos, vel)
+    sync_faces(gpu, orc)
+    gpu.set_profiling(True)
+    gpu.run_phase(_lib.PHASE_REDISTRIBUTE)
+    orc.phase(oracle.PHASE_REDISTRIBUTE)
+    pg, po = gpu.particles()[0], orc.particles()[0]
+    assert (gpu.profile()["redist_long_sweeps"] >= 1) == (n > 2048)
+    moved = np.any(po != pos, axis=1)
+    assert moved.sum() > 20
+    assert np.array_equal(np.any(pg != pos, axis=1), moved)
