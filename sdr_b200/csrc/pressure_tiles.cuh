@@ -223,31 +223,37 @@ __device__ bool tw_grid_sync(const TwArgs& t) {
     return TW_SH.ok != 0;
 }
 
-__device__ __forceinline__ double tw_block_max(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) TW_SH.red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double m = TW_SH.red[0];
-    for (int w = 1; w < kTwWarps; ++w) m = fmax(m, TW_SH.red[w]);
-    __syncthreads();
-    return m;
+// Maximum over a warp of values that are not negative (so ordered like their bits).
+__device__ __forceinline__ double tw_warp_max(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)__double2loint(v) : 0u);
+    return __hiloint2double((int)mh, (int)ml);
 }
 
-// Maximum over the grid (order-free): CTA maxima through a double-buffered slot array.
+// Maximum over the grid (order-free) of values that are not negative: CTA maxima
+// through a double-buffered slot array.
 template <bool CL>
 __device__ bool tw_grid_max(const TwArgs& t, double v, int& parity, double& out) {
-    const double bm = tw_block_max(v);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    v = tw_warp_max(v);
+    if (lane == 0) TW_SH.red[w] = v;
+    __syncthreads();
     double* sl = t.gslots + (size_t)parity * gridDim.x;
     parity ^= 1;
-    if (threadIdx.x == 0) sl[blockIdx.x] = bm;
+    if (w == 0) {
+        v = tw_warp_max(lane < kTwWarps ? TW_SH.red[lane] : 0.0);
+        if (lane == 0) sl[blockIdx.x] = v;
+    }
     if (!tw_grid_sync<CL>(t)) return false;
-    if (threadIdx.x < 32) {
+    if (CL) {  // at most 16: every warp reads them itself
+        out = tw_warp_max(lane < (int)gridDim.x ? __ldcg(sl + lane) : 0.0);
+        return true;
+    }
+    if (w == 0) {
         double m = 0.0;
-        for (unsigned q = threadIdx.x; q < gridDim.x; q += 32) m = fmax(m, __ldcg(sl + q));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (threadIdx.x == 0) TW_SH.red[0] = m;
+        for (unsigned q = lane; q < gridDim.x; q += 32) m = fmax(m, __ldcg(sl + q));
+        m = tw_warp_max(m);
+        if (lane == 0) TW_SH.red[0] = m;
     }
     __syncthreads();
     out = TW_SH.red[0];
@@ -258,8 +264,15 @@ __device__ bool tw_grid_max(const TwArgs& t, double v, int& parity, double& out)
 // Total of the tree-order tile sums (the lane pattern and xor tree of
 // pcg_tile_total): the CTA brings them to shared memory, warp 0 adds them.
 // One warp loading them from L2 itself took 7 us for the 4,650 sums of a
-// 1.19 M-cell pool, twice per iteration.
+// 1.19 M-cell pool, twice per iteration. Where the loads of every warp are few
+// (the cluster form's scenes) each adds them itself, without the CTA's barriers.
 __device__ double tw_tile_total(const TwArgs& t, uint32_t ntile) {
+    if (gridDim.x * ntile <= 4096) {
+        double s = 0.0;
+#pragma unroll 4
+        for (uint32_t q = threadIdx.x & 31; q < ntile; q += 32) s = dadd(s, __ldcg(t.a.tpart + q));
+        return warp_tree_sum(s);
+    }
     double* const scratch = tw_scratch();
     constexpr uint32_t kChunk = kTwScratch;
     double s = 0.0;
@@ -856,15 +869,18 @@ __device__ bool tw_sweep_all(const TwArgs& t, uint32_t& uses) {
 // kTwBatch / 3 of them, a thread one cell of each (their loads are
 // independent); the products meet in shared memory and a warp per tile adds
 // them in the tree order (lane l: cells l, l+32, ...; then the xor tree).
-__device__ void tw_matvec(const TwArgs& t, uint32_t nf, uint32_t ntile) {
-    constexpr int kPer = kTwBatch / kTwThirds;
+// kPer: tiles of a third at a time; of a share of a tile per third one, as the
+// places without a tile cost their instructions too.
+template <int kPer>
+__device__ __forceinline__ void tw_matvec_by(const TwArgs& t, uint32_t nf, uint32_t ntile) {
+    constexpr int kBatch = kPer * kTwThirds;
     const PcgArgs& a = t.a;
     double* const scratch = tw_scratch();
     const uint32_t per = (ntile + gridDim.x - 1) / gridDim.x;
     const uint32_t t0 = min(blockIdx.x * per, ntile), t1 = min(t0 + per, ntile);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int third = threadIdx.x / kTile, tc = threadIdx.x % kTile;
-    for (uint32_t tb = t0; tb < t1; tb += kTwBatch) {
+    for (uint32_t tb = t0; tb < t1; tb += kBatch) {
         int2 nb[kPer][3];
         double sv[kPer], dg[kPer];
 #pragma unroll
@@ -899,7 +915,7 @@ __device__ void tw_matvec(const TwArgs& t, uint32_t nf, uint32_t ntile) {
         }
         if (a.exact_dots) continue;
         __syncthreads();
-        if (w < kTwBatch && tb + w < t1) {
+        if (w < kBatch && tb + w < t1) {
             double acc = 0.0;
 #pragma unroll
             for (int u = 0; u < kTile / 32; ++u)
@@ -909,6 +925,11 @@ __device__ void tw_matvec(const TwArgs& t, uint32_t nf, uint32_t ntile) {
         }
         __syncthreads();
     }
+}
+
+__device__ void tw_matvec(const TwArgs& t, uint32_t nf, uint32_t ntile) {
+    if (ntile <= kTwThirds * gridDim.x) tw_matvec_by<1>(t, nf, ntile);
+    else tw_matvec_by<kTwBatch / kTwThirds>(t, nf, ntile);
 }
 
 // dot(z, r) by the tiles of the tree order, a warp per tile.
