@@ -140,12 +140,16 @@ typedef struct {
     uint64_t particles;         /* sum over substeps of particles advanced */
     /* SM cycles inside the pressure-solve kernel by section: MIC(0) build,
      * forward+backward preconditioner sweeps, (unused), matvec, dot products,
-     * update of p and r with the residual norm, search direction, setup/exit;
-     * then per forward-sweep level: staging wait, compute, barrier, level
-     * count; then the sum of sweep widths, of non-empty level ranges, and solves. */
+     * update of r with the residual norm (one-block kernel: and of p), search
+     * direction (tiled kernel: and p), setup/exit. One-block kernel: then per
+     * forward-sweep level staging wait, compute, barrier, level count; the sum
+     * of sweep widths and of non-empty level ranges. Tiled kernel: unused; level
+     * loops' cycles over all tiles, their levels and their number; the same
+     * cycles and levels of the tiles that wait for no other. Last: solves. */
     uint64_t pcg_section_cycles[16];
     /* redistribution: candidates (particles in over-cap cells) replayed, replay
-     * sweeps run, and sweeps whose list was longer than the shared-memory one */
+     * sweeps run, and sweeps whose list one block's shared memory did not take
+     * (too long, or too many cells) */
     uint64_t redist_candidates;
     uint64_t redist_sweeps;
     uint64_t redist_long_sweeps;
@@ -154,7 +158,7 @@ typedef struct {
      * -> host (the per-substep status block) */
     uint64_t h2d_bytes;
     uint64_t d2h_bytes;
-    uint64_t pcg_tile_launches; /* solves that ran on the whole-GPU tiled kernel */
+    uint64_t pcg_tile_launches; /* solves that ran on the tiled kernel (cluster or whole GPU) */
     uint64_t redist_rounds;     /* decision rounds of long redistribution lists */
 } sdr_profile;
 

@@ -177,7 +177,7 @@ class Solver:
         check(_lib.load().sdr_solver_set_dot_order(self._h, 1 if reference_order else 0))
 
     def set_pcg_kernel(self, kernel: int) -> None:
-        """_lib.PCG_AUTO, PCG_ONE_BLOCK (one SM) or PCG_CLUSTER (up to 16 SMs)."""
+        """_lib.PCG_AUTO, PCG_ONE_BLOCK (one SM), PCG_CLUSTER (up to 16 SMs) or PCG_TILES (a CTA per tile of lines)."""
         check(_lib.load().sdr_solver_set_pcg_kernel(self._h, int(kernel)))
 
     def set_pcg_ctas(self, ctas: int) -> None:
