@@ -1188,6 +1188,9 @@ __device__ void redist_par_run(const RedistArgs& a, const Team& team) {
     uint32_t na = __ldcg(&rs->pend_n[0]);
     uint32_t round = 0;
     bool solo = false;
+    // CTA 0's counts of its own rounds: the grid's keep the value at which the
+    // others leave, which they may read after CTA 0 has gone on.
+    __shared__ uint32_t s_pend[2];
     uint32_t gt_ = gt, G_ = G;
     while (na > 0 && ok) {
         if (Team::kGrid && !solo && na <= kRpSoloList) {  // the same decision in every CTA
@@ -1195,6 +1198,7 @@ __device__ void redist_par_run(const RedistArgs& a, const Team& team) {
             if (rank != 0) break;
             gt_ = threadIdx.x;
             G_ = kRpBS;
+            if (threadIdx.x < 2) s_pend[threadIdx.x] = 0u;  // before the appends by the barrier after the claims
         }
         ++round;
         const int cur = (int)(round & 1u);
@@ -1248,7 +1252,7 @@ __device__ void redist_par_run(const RedistArgs& a, const Team& team) {
                 if (n >= 0 && a.cavity[n] && __ldcg(a.count + n) < cap && __ldcg(a.claim + n) != key) ready = false;
             }
             if (!ready) {
-                pb[atomicAdd(&rs->pend_n[cur], 1u)] = m;
+                pb[atomicAdd(solo ? &s_pend[cur] : &rs->pend_n[cur], 1u)] = m;
                 continue;
             }
             // The unit's candidates in index order, on its counts held in
@@ -1309,10 +1313,14 @@ __device__ void redist_par_run(const RedistArgs& a, const Team& team) {
         }
         if (solo) __syncthreads();
         else ok = team.sync() && ok;
-        na = __ldcg(&rs->pend_n[cur]);
+        na = solo ? s_pend[cur] : __ldcg(&rs->pend_n[cur]);
         // the other counter was last read after the previous round: clear it
         // for the next round's appends (ordered before them by its first barrier)
-        if (rank == 0 && threadIdx.x == 0) rs->pend_n[cur ^ 1] = 0u;
+        if (solo) {
+            if (threadIdx.x == 0) s_pend[cur ^ 1] = 0u;
+        } else if (rank == 0 && threadIdx.x == 0) {
+            rs->pend_n[cur ^ 1] = 0u;
+        }
         pa = pb;
         pb = (pb == a.pend) ? a.pend + a.cand_cap : a.pend;
         if (na > 0 && round > nc) {  // cannot happen: the lowest pending unit always runs
