@@ -117,6 +117,9 @@ struct TwArgs {
     int* thi;
     unsigned* bar;               // grid barrier: [0] arrivals, [1] generation
     double* gslots;              // 2 x gridDim CTA partials of grid maxima
+    // Tile sums of the tree-order dots, an array for each of the two dots:
+    double* sums_as;             // s*As, written by the matvec
+    double* sums_zr;             // z*r, written behind the sweeps
     uint32_t* err;               // error bits
     int plane;                   // cluster form: levels of a halo plane (no tile has more)
 };
@@ -266,11 +269,18 @@ __device__ bool tw_grid_max(const TwArgs& t, double v, int& parity, double& out)
 // One warp loading them from L2 itself took 7 us for the 4,650 sums of a
 // 1.19 M-cell pool, twice per iteration. Where the loads of every warp are few
 // (the cluster form's scenes) each adds them itself, without the CTA's barriers.
-__device__ double tw_tile_total(const TwArgs& t, uint32_t ntile) {
+// Every CTA reads all of the sums, and may be late: between its read and the
+// next write of the same array there has to be a barrier of all CTAs. With an
+// array per dot the barriers of the other dot are that: sums_as is written by
+// the next matvec, behind the barriers of the residual's maximum and around
+// the z*r sums; sums_zr behind the next sweeps, after the barrier of the s*As
+// sums. (In one array, the cluster form, whose direction has no barrier of its
+// own, stored a matvec's sums while a late CTA still read those of z*r.)
+__device__ double tw_tile_total(const double* sums, uint32_t ntile) {
     if (gridDim.x * ntile <= 4096) {
         double s = 0.0;
 #pragma unroll 4
-        for (uint32_t q = threadIdx.x & 31; q < ntile; q += 32) s = dadd(s, __ldcg(t.a.tpart + q));
+        for (uint32_t q = threadIdx.x & 31; q < ntile; q += 32) s = dadd(s, __ldcg(sums + q));
         return warp_tree_sum(s);
     }
     double* const scratch = tw_scratch();
@@ -279,7 +289,7 @@ __device__ double tw_tile_total(const TwArgs& t, uint32_t ntile) {
     for (uint32_t c0 = 0; c0 < ntile; c0 += kChunk) {
         const uint32_t n = min(kChunk, ntile - c0);
         __syncthreads();
-        for (uint32_t q = threadIdx.x; q < n; q += kTwBS) scratch[q] = __ldcg(t.a.tpart + c0 + q);
+        for (uint32_t q = threadIdx.x; q < n; q += kTwBS) scratch[q] = __ldcg(sums + c0 + q);
         __syncthreads();
         if (threadIdx.x < 32) {
 #pragma unroll 8
@@ -941,7 +951,7 @@ __device__ __forceinline__ void tw_matvec_by(const TwArgs& t, uint32_t nf, uint3
             for (int u = 0; u < kTile / 32; ++u)
                 if ((tb + w) * kTile + u * 32 + lane < nf) acc = dadd(acc, scratch[w * kTile + u * 32 + lane]);
             acc = warp_tree_sum(acc);
-            if (lane == 0) a.tpart[tb + w] = acc;
+            if (lane == 0) t.sums_as[tb + w] = acc;
         }
         __syncthreads();
     }
@@ -971,7 +981,7 @@ __device__ __forceinline__ void tw_dot_zr(const TwArgs& t, uint32_t nf, uint32_t
         for (int u = 0; u < kTile / 32; ++u)
             if (tl * kTile + lane + 32u * u < nf) acc = dadd(acc, dmul(zv[u], rv[u]));
         acc = warp_tree_sum(acc);
-        if (lane == 0) a.tpart[tl] = acc;
+        if (lane == 0) t.sums_zr[tl] = acc;
     }
 }
 
@@ -1110,7 +1120,7 @@ __device__ __forceinline__ void tw_solve(const TwArgs& t) {
             if (!tw_grid_sync<CL>(t)) goto out;
             tw_dot_zr(t, nf, ntile);
             if (!tw_grid_sync<CL>(t)) goto out;
-            sigma = tw_tile_total(t, ntile);
+            sigma = tw_tile_total(t.sums_zr, ntile);
         }
         for (uint32_t i = gt; i < nf; i += G) a.s[i] = __ldcg(a.z + i);
         if (!tw_grid_sync<CL>(t)) goto out;
@@ -1130,7 +1140,7 @@ __device__ __forceinline__ void tw_solve(const TwArgs& t) {
                 if (!tw_exact_dot<CL>(t, denom)) goto out;
             } else {
                 if (!tw_grid_sync<CL>(t)) goto out;
-                denom = tw_tile_total(t, ntile);
+                denom = tw_tile_total(t.sums_as, ntile);
             }
             TW_SECTION(3);
             if (fabs(denom) < 1e-30) break;
@@ -1170,7 +1180,7 @@ __device__ __forceinline__ void tw_solve(const TwArgs& t) {
                 TW_SECTION(1);  // the sweeps end at this barrier
                 tw_dot_zr(t, nf, ntile);
                 if (!tw_grid_sync<CL>(t)) goto out;
-                sigma_new = tw_tile_total(t, ntile);
+                sigma_new = tw_tile_total(t.sums_zr, ntile);
                 TW_SECTION(4);
             }
             beta = ddiv(sigma_new, sigma);

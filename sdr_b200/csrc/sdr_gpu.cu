@@ -480,7 +480,7 @@ struct sdr_solver {
     int pcg_ctas = 0;               // CTAs of k_pcg's cluster (0: 1 on a shared GPU, else the device's largest)
     bool shared_gpu = false;        // SDR_SOLVER_SHARED_GPU
     int ctas_pcg = 0, ctas_pcgc = 0, ctas_rp = 0;  // largest clusters the device schedules (asked once)
-    double* tpart = nullptr;        // tile sums of the tree-order dots
+    double* tpart = nullptr;        // tile sums of the tree-order dots: dot_room() each for the tiled solve's two
     uint32_t* p2g_list = nullptr;   // grid nodes with particles around them (P2G queue)
     uint32_t last_p2g_queue = 0;    // its length at the last status read
     uint32_t last_nf = 0;           // fluid cells of the last solve (picks the kernel under SDR_PCG_AUTO)
@@ -569,6 +569,7 @@ struct sdr_solver {
     unsigned nbricks() const { return (unsigned)brick_dim(g.nx) * (unsigned)brick_dim(g.ny) * (unsigned)brick_dim(g.nz); }
     Faces saved() const { return Faces{su, sv, sw}; }
     uint32_t* dn() { return &dst->n; }
+    size_t dot_room() const { return ncell / kTile + 2; }  // of a dot's tile sums
     size_t hist_room() const { return (ncell + 1 + 3) / 4 * 4; }  // of a histogram: the scans read 16 bytes at a time
 
     // Exclusive scan; `site` (the caller's line) keys its kernels in a packed launch.
@@ -664,7 +665,7 @@ struct sdr_solver {
         dalloc(s, nc, st); dalloc(as, nc, st); dalloc(q, nc, st); dalloc(pq, nc, st);
         dalloc(partials, nchunks + 1, st);
         if (!cl_slots) dalloc(cl_slots, 2 * kClMaxCtas, st);
-        dalloc(tpart, ncell / kTile + 2, st);
+        dalloc(tpart, 2 * dot_room(), st);
         dalloc(rclaim, ncell, st);
         CK(cudaMemsetAsync(rclaim, 0, ncell * sizeof(unsigned long long), st));
         dalloc(corder, nc, st);
@@ -1017,6 +1018,8 @@ struct sdr_solver {
         t.tlo = tw_lo; t.thi = tw_hi;
         t.bar = tw_bar;
         t.gslots = tw_slots;
+        t.sums_as = tpart;
+        t.sums_zr = tpart + dot_room();
         t.err = &dst->err;
         t.plane = tw_plane_levels();
         if (tw_cluster > 0) {
