@@ -412,7 +412,9 @@ __global__ void __launch_bounds__(kSdfDistBS, 3) k_sdf_dist(SdfFast a, int bx, i
     __shared__ uint32_t s_group[kSdfDistBS];  // of the groups looked at together: those within reach
     __shared__ float s_u[kSdfDistBS / 32];
     __shared__ uint16_t s_w[kSdfDistBS / 32][kSdfWarpList];
-    if (*a.gate) return;
+    // Other blocks of this launch may open the gate meanwhile, so a block leaves
+    // as one: warps that went on alone would take unset list lengths.
+    if (__syncthreads_or(*a.gate != 0u)) return;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     constexpr int kWarps = kSdfDistBS / 32;
     const int b = blockIdx.x, sub = tid % kSdfSplit;
@@ -619,7 +621,7 @@ __global__ void __launch_bounds__(256) k_sdf_up(SdfFast a) {
 // number up to rounding, whatever the order of the sum.
 __global__ void __launch_bounds__(512) k_sdf_roots(SdfFast a) {
     __shared__ double sh[33];
-    if (*a.gate) return;
+    if (__syncthreads_or(*a.gate != 0u)) return;  // as one block: others may open it meanwhile
     const uint32_t nr = a.roots[0];
     for (uint32_t q = blockIdx.x; q < nr; q += gridDim.x) {
         const uint32_t n = a.roots[1 + q];
