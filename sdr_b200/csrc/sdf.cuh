@@ -213,7 +213,7 @@ struct SdfFast {
     float4* ball;           // per triangle: bounding sphere (padded to whole groups of 32)
     float4* group;          // per 32 triangles: their bounding sphere
     float4* norm;           // per triangle: unit normal
-    float4* vert;           // per triangle: three vertices; vert[3 t].w: the f32 distance holds up to this distance squared
+    float4* vert;           // per triangle: three vertices; vert[3 t].w: the f32 distance holds up to this distance squared (-1: nowhere)
     double* dist;           // per node
     uint32_t* up;           // per node: the neighbour it follows, or itself; later its root
     uint32_t* roots;        // [0] their number, then the nodes
@@ -281,7 +281,11 @@ __device__ __forceinline__ float sdf_extent(const SdfFast& a) {
 // coordinates of the point nearest to p are off by about 64 eps D^2 l^2 / |n|^2
 // (differences of products of dot products of size l D, over the squared
 // normal): a triangle is too thin if that is over a thousandth in f64 two
-// extents away, and its f32 distance holds while it is under a fiftieth.
+// extents away, and its f32 distance holds while it is under a fiftieth. That
+// distance forms products of four lengths (up to 1e4 l^4 within its reach) and
+// divides by |n|^2: only where both are normal numbers of f32 with room to spare.
+// Other triangles are told apart by their spheres alone (squares of lengths, which
+// f32 holds over all extents that pass here).
 __global__ void __launch_bounds__(256) k_sdf_balls(SdfFast a) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const float ext = sdf_extent(a);
@@ -311,10 +315,11 @@ __global__ void __launch_bounds__(256) k_sdf_balls(SdfFast a) {
         ball = make_float4((float)(g[0] - a.cx), (float)(g[1] - a.cy), (float)(g[2] - a.cz),
                            __double2float_ru(sqrt(r2)) * 1.000001f + 2e-6f * ext);
         const double rn = 1.0 / sqrt(nn);
+        const float holds = nn > 1e-30 && l2 < 1e16 ? (float)(0.02 / (64.0 * 6e-8) * nn / l2) : -1.0f;
         a.norm[t] = make_float4((float)(n0 * rn), (float)(n1 * rn), (float)(n2 * rn), 0.0f);
         for (int q = 0; q < 3; ++q)
             a.vert[3 * (size_t)t + q] = make_float4((float)(v[3 * q] - a.cx), (float)(v[3 * q + 1] - a.cy),
-                                                    (float)(v[3 * q + 2] - a.cz), (float)(0.02 / (64.0 * 6e-8) * nn / l2));
+                                                    (float)(v[3 * q + 2] - a.cz), holds);
     }
     a.ball[t] = ball;
     // the group's sphere, around the mean of its centres
