@@ -249,7 +249,7 @@ int sdr_solver_set_dot_order(sdr_solver* s, int reference_order);
  * boundary values to their neighbours through entries that mark their own
  * readiness: one thread-block cluster where the grid has at most 16 tiles, else
  * the whole GPU in one cooperative launch (the cluster kernel if the device
- * cannot launch it). SDR_PCG_AUTO (default): the tiled solve on a GPU of its
+ * cannot launch it or its buffers do not fit). SDR_PCG_AUTO (default): the tiled solve on a GPU of its
  * own; with SDR_SOLVER_SHARED_GPU one block, from 200,000 fluid cells in the
  * previous solve (before the first solve: the particle count over
  * particles_per_cell) the cluster. */
@@ -333,13 +333,15 @@ int sdr_sdf_mesh_grid(const double* tris, size_t ntri, double dx, double padding
  * sign and closest-point distance per node, on the device. */
 int sdr_sdf_from_mesh(const double* tris, size_t ntri, sdr_vec3 origin, double dx,
                       const uint64_t dims[3], double* out);
-/* Test hook: the next sdr_sdf_from_mesh call on the calling thread makes one
- * bounded device wait run out on purpose, so that its error path runs without
- * any GPU fault. SDR_FAULT_SDF_STAGING: the bulk copy of the first triangle
- * tile is not issued, the staging wait gives up after its limit (about one
- * second), the kernel waits for its other copies in flight and reports, and
- * the call returns SDR_ERR_DEVICE_TIMEOUT. 0 clears a pending fault. */
-enum { SDR_FAULT_NONE = 0, SDR_FAULT_SDF_STAGING = 1 };
+/* Test hook: runs an error path of the calling thread's next call on purpose,
+ * without any GPU fault. SDR_FAULT_SDF_STAGING (the next sdr_sdf_from_mesh):
+ * the bulk copy of the first triangle tile is not issued, the staging wait
+ * gives up after its limit (about one second), the kernel waits for its other
+ * copies in flight and reports, and the call returns SDR_ERR_DEVICE_TIMEOUT.
+ * SDR_FAULT_LAZY_BUFFERS (the next solver that allocates the tiled solve's
+ * buffers, at its first solve): the last of them counts as one that did not
+ * fit, and the solver takes the other kernels. 0 clears a pending fault. */
+enum { SDR_FAULT_NONE = 0, SDR_FAULT_SDF_STAGING = 1, SDR_FAULT_LAZY_BUFFERS = 2 };
 int sdr_debug_inject(int fault);
 /* Largest mesh sdr_sdf_from_mesh_noalloc accepts. */
 #define SDR_NOALLOC_MAX_TRIANGLES 32768

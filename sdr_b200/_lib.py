@@ -151,7 +151,7 @@ class ServerStats(C.Structure):
 
 REQ_QUEUED, REQ_RUNNING, REQ_DONE, REQ_FAILED = 0, 1, 2, 3
 FORMAT_VTK, FORMAT_XYZ = 0, 1
-FAULT_NONE, FAULT_SDF_STAGING = 0, 1
+FAULT_NONE, FAULT_SDF_STAGING, FAULT_LAZY_BUFFERS = 0, 1, 2
 
 P = C.POINTER
 d, u64, i32, vp, sz = C.c_double, C.c_uint64, C.c_int, C.c_void_p, C.c_size_t

@@ -695,8 +695,7 @@ struct sdr_solver {
         dfree(lines_cnt, st); dfree(lv_cell, st); dfree(cflag, st); dfree(coff, st); dfree(level_start, st); dfree(pos_of_cell, st);
         dfree(nbr, st); dfree(corder, st); dfree(cinv, st); dfree(prod, st); dfree(frec, st); dfree(brec, st); dfree(chunk_start, st); dfree(diag, st); dfree(nmask, st);
         dfree(b, st); dfree(precon, st); dfree(p, st); dfree(r, st); dfree(z, st); dfree(s, st); dfree(as, st); dfree(q, st); dfree(pq, st);
-        dfree(tw_idx, st); dfree(tw_tpos, st); dfree(tw_list, st); dfree(tw_rank, st); dfree(tw_r, st); dfree(tw_word, st); dfree(tw_rbase, st); dfree(tw_pc, st); dfree(tw_q, st); dfree(tw_exf, st); dfree(tw_exb, st); dfree(tw_slots, st); dfree(tw_lo, st);
-        dfree(tw_hi, st); dfree(tw_bar, st);
+        tw_free();
         dfree(rp_slots, st); dfree(rp_bar, st);
         dfree(partials, st); dfree(p_dense, st); dfree(cl_slots, st); dfree(rclaim, st); dfree(tpart, st); dfree(p2g_list, st);
         dfree(cand, st); dfree(rpend, st); dfree(rbits, st); dfree(moves, st); dfree(rds, st); dfree(lrec, st); dfree(vrec, st);
@@ -958,8 +957,8 @@ struct sdr_solver {
 
     // The tiled solve needs a cluster with a CTA per tile (grids of up to 16
     // tiles), else a cooperative launch with every CTA resident; its buffers are
-    // allocated on first use. False if the device cannot run it (then k_pcg or
-    // the cluster kernel solves).
+    // allocated on first use. False if the device cannot run it or has no room
+    // for them (then k_pcg or the cluster kernel solves, for good).
     bool tiles_ready() {
         if (tw_grid < 0) return false;
         if (tw_grid > 0) return true;
@@ -975,18 +974,18 @@ struct sdr_solver {
             tw_grid = -1;
             return false;
         }
-        tw_grid = nsm;
         tw_tj = (g.ny + kTwJ - 1) / kTwJ;
         tw_tk = (g.nz + kTwK - 1) / kTwK;
         const size_t nt = (size_t)tw_tj * tw_tk;
         // The cluster form holds a CTA per tile and halo planes of a tile's most
         // levels in shared memory.
         const size_t csmem = tw_cluster_smem(tw_plane_levels());
+        int ctas = 0;
         if (nt <= (size_t)kTwClusterCtas && csmem <= kTwMaxSmem) {
             CK(cudaFuncSetAttribute(k_pcg_tiles_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTwMaxSmem));
             const int most = cluster_ctas(k_pcg_tiles_cluster, 3, kTwBS, device, kTwMaxSmem);
             const int want = nt <= 8 ? 8 : kTwClusterCtas;
-            tw_cluster = want <= most ? want : 0;
+            ctas = want <= most ? want : 0;
         }
         // operand rows: a tile's levels span at most nx + kTwJ + kTwK - 2 of them
         tw_rows = nt * (size_t)(g.nx + kTwJ + kTwK) * (size_t)kTwLines;
@@ -994,15 +993,37 @@ struct sdr_solver {
             tw_grid = -1;
             return false;
         }
-        dalloc(tw_idx, tw_rows, st); dalloc(tw_pc, tw_rows, st); dalloc(tw_q, tw_rows, st);
-        dalloc(tw_r, tw_rows, st); dalloc(tw_tpos, ncell, st); dalloc(tw_list, nt + 1, st); dalloc(tw_rank, nt, st);
-        dalloc(tw_word, tw_rows, st); dalloc(tw_rbase, nt + 1, st);
-        // exchange planes: two faces of one entry per line and row level
-        dalloc(tw_exf, 2 * (tw_rows / kTwFace), st); dalloc(tw_exb, 2 * (tw_rows / kTwFace), st);
-        dalloc(tw_lo, nt, st); dalloc(tw_hi, nt, st);
-        dalloc(tw_bar, 2, st);
-        dalloc(tw_slots, 2 * (size_t)tw_grid, st);
+        // About 32 B per row entry, 73 B per cell of a grid 25 cells wide: not
+        // every grid that k_pcg solves leaves room for them.
+        try {
+            dalloc(tw_idx, tw_rows, st); dalloc(tw_pc, tw_rows, st); dalloc(tw_q, tw_rows, st);
+            dalloc(tw_r, tw_rows, st); dalloc(tw_tpos, ncell, st); dalloc(tw_list, nt + 1, st); dalloc(tw_rank, nt, st);
+            dalloc(tw_word, tw_rows, st); dalloc(tw_rbase, nt + 1, st);
+            // exchange planes: two faces of one entry per line and row level
+            dalloc(tw_exf, 2 * (tw_rows / kTwFace), st); dalloc(tw_exb, 2 * (tw_rows / kTwFace), st);
+            dalloc(tw_lo, nt, st); dalloc(tw_hi, nt, st);
+            dalloc(tw_bar, 2, st);
+            if (g_fault == SDR_FAULT_LAZY_BUFFERS) {
+                g_fault = 0;
+                throw Fail{SDR_ERR_OOM, "tiled solve's buffers (test hook)"};
+            }
+            dalloc(tw_slots, 2 * (size_t)nsm, st);
+        } catch (const Fail& e) {
+            tw_free();
+            if (e.code != SDR_ERR_OOM) throw;
+            cudaGetLastError();  // reported here; the call goes on
+            tw_grid = -1;
+            return false;
+        }
+        tw_cluster = ctas;
+        tw_grid = nsm;  // last: from here on every buffer is there
         return true;
+    }
+
+    void tw_free() {
+        dfree(tw_idx, st); dfree(tw_tpos, st); dfree(tw_list, st); dfree(tw_rank, st); dfree(tw_r, st); dfree(tw_word, st);
+        dfree(tw_rbase, st); dfree(tw_pc, st); dfree(tw_q, st); dfree(tw_exf, st); dfree(tw_exb, st); dfree(tw_slots, st);
+        dfree(tw_lo, st); dfree(tw_hi, st); dfree(tw_bar, st);
     }
 
     int tw_plane_levels() const { return g.nx + kTwJ + kTwK; }
@@ -1764,7 +1785,7 @@ int sdr_solver_set_candidate_capacity(sdr_solver* s, uint64_t candidates) {
 
 int sdr_debug_inject(int fault) {
     return guard([&] {
-        require(fault == 0 || fault == SDR_FAULT_SDF_STAGING, "unknown fault");
+        require(fault == 0 || fault == SDR_FAULT_SDF_STAGING || fault == SDR_FAULT_LAZY_BUFFERS, "unknown fault");
         g_fault = fault;
     });
 }
