@@ -338,9 +338,10 @@ int sdr_sdf_from_mesh(const double* tris, size_t ntri, sdr_vec3 origin, double d
  * the bulk copy of the first triangle tile is not issued, the staging wait
  * gives up after its limit (about one second), the kernel waits for its other
  * copies in flight and reports, and the call returns SDR_ERR_DEVICE_TIMEOUT.
- * SDR_FAULT_LAZY_BUFFERS (the next solver that allocates the tiled solve's
- * buffers, at its first solve): the last of them counts as one that did not
- * fit, and the solver takes the other kernels. 0 clears a pending fault. */
+ * SDR_FAULT_LAZY_BUFFERS (the next solver that allocates the buffers of the
+ * tiled solve, at its first solve, or of the long lists' rounds over the whole
+ * GPU, at its first redistribution): they count as not fitting, and the solver
+ * takes the other kernels. 0 clears a pending fault. */
 enum { SDR_FAULT_NONE = 0, SDR_FAULT_SDF_STAGING = 1, SDR_FAULT_LAZY_BUFFERS = 2 };
 int sdr_debug_inject(int fault);
 /* Largest mesh sdr_sdf_from_mesh_noalloc accepts. */

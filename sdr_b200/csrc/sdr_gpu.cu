@@ -935,7 +935,8 @@ struct sdr_solver {
     }
 
     // Cooperative launch of k_redist_par_grid (every CTA resident): false if
-    // the device cannot run it (then the cluster decides long lists).
+    // the device cannot run it or has no room for its buffers (then the cluster
+    // decides long lists, for good).
     bool rounds_grid_ready() {
         if (rp_grid != 0) return rp_grid > 0;
         int coop = 0, nsm = 0, occ = 0;
@@ -949,9 +950,32 @@ struct sdr_solver {
             rp_grid = -1;
             return false;
         }
-        rp_grid = nsm * std::min(occ, 2);
-        dalloc(rp_slots, 2 * (size_t)rp_grid, st);
-        dalloc(rp_bar, 2, st);
+        const int ctas = nsm * std::min(occ, 2);
+        if (!lazily([&] { dalloc(rp_slots, 2 * (size_t)ctas, st); dalloc(rp_bar, 2, st); },
+                    [&] { dfree(rp_slots, st); dfree(rp_bar, st); })) {
+            rp_grid = -1;
+            return false;
+        }
+        rp_grid = ctas;  // last: from here on both buffers are there
+        return true;
+    }
+
+    // Buffers of one of several kernels, allocated on first use. False, with
+    // nothing kept, if they do not fit: another kernel takes the work.
+    template <class Alloc, class Free>
+    bool lazily(Alloc alloc, Free release) {
+        try {
+            alloc();
+            if (g_fault == SDR_FAULT_LAZY_BUFFERS) {
+                g_fault = 0;
+                throw Fail{SDR_ERR_OOM, "buffers of a kernel (test hook)"};
+            }
+        } catch (const Fail& e) {
+            release();
+            if (e.code != SDR_ERR_OOM) throw;
+            cudaGetLastError();  // reported here; the call goes on
+            return false;
+        }
         return true;
     }
 
@@ -995,23 +1019,19 @@ struct sdr_solver {
         }
         // About 32 B per row entry, 73 B per cell of a grid 25 cells wide: not
         // every grid that k_pcg solves leaves room for them.
-        try {
-            dalloc(tw_idx, tw_rows, st); dalloc(tw_pc, tw_rows, st); dalloc(tw_q, tw_rows, st);
-            dalloc(tw_r, tw_rows, st); dalloc(tw_tpos, ncell, st); dalloc(tw_list, nt + 1, st); dalloc(tw_rank, nt, st);
-            dalloc(tw_word, tw_rows, st); dalloc(tw_rbase, nt + 1, st);
-            // exchange planes: two faces of one entry per line and row level
-            dalloc(tw_exf, 2 * (tw_rows / kTwFace), st); dalloc(tw_exb, 2 * (tw_rows / kTwFace), st);
-            dalloc(tw_lo, nt, st); dalloc(tw_hi, nt, st);
-            dalloc(tw_bar, 2, st);
-            if (g_fault == SDR_FAULT_LAZY_BUFFERS) {
-                g_fault = 0;
-                throw Fail{SDR_ERR_OOM, "tiled solve's buffers (test hook)"};
-            }
-            dalloc(tw_slots, 2 * (size_t)nsm, st);
-        } catch (const Fail& e) {
-            tw_free();
-            if (e.code != SDR_ERR_OOM) throw;
-            cudaGetLastError();  // reported here; the call goes on
+        const bool fit = lazily(
+            [&] {
+                dalloc(tw_idx, tw_rows, st); dalloc(tw_pc, tw_rows, st); dalloc(tw_q, tw_rows, st);
+                dalloc(tw_r, tw_rows, st); dalloc(tw_tpos, ncell, st); dalloc(tw_list, nt + 1, st); dalloc(tw_rank, nt, st);
+                dalloc(tw_word, tw_rows, st); dalloc(tw_rbase, nt + 1, st);
+                // exchange planes: two faces of one entry per line and row level
+                dalloc(tw_exf, 2 * (tw_rows / kTwFace), st); dalloc(tw_exb, 2 * (tw_rows / kTwFace), st);
+                dalloc(tw_lo, nt, st); dalloc(tw_hi, nt, st);
+                dalloc(tw_bar, 2, st);
+                dalloc(tw_slots, 2 * (size_t)nsm, st);
+            },
+            [&] { tw_free(); });
+        if (!fit) {
             tw_grid = -1;
             return false;
         }

@@ -1,7 +1,7 @@
-"""A solver whose tiled-solve buffers do not fit (the test hook lets the last of
-them fail): it frees the others, solves with the other kernels from then on, and
-never launches the tiled kernel on what it has not got. Against the oracle's
-solve with the reference dot order, bit for bit."""
+"""A solver whose tiled-solve buffers do not fit (by the test hook): it frees
+them, solves with the other kernels from then on, and never launches the tiled
+kernel on what it has not got. Against the oracle's solve with the reference dot
+order, bit for bit."""
 import numpy as np
 import pytest
 
