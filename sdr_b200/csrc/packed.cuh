@@ -43,10 +43,8 @@ __device__ __forceinline__ void pack_call(VB vb, const Tup& t, cuda::std::index_
 // One slot of a packed substep: CTAs take virtual blocks in turn; each finds
 // its scene in the offset table (binary search) and runs the body with that
 // scene's arguments.
-// Two blocks of 512 threads an SM: without the bound the brick kernels took 67 to
-// 72 registers and one block had an SM to itself.
 template <class Op, class Tup>
-__global__ void __launch_bounds__(Op::kThreads, Op::kThreads == 512 ? 2 : 1) k_packed(const unsigned char* __restrict__ hdr_p) {
+__global__ void __launch_bounds__(Op::kThreads, Op::kBlocks) k_packed(const unsigned char* __restrict__ hdr_p) {
     const PackHdr h = *reinterpret_cast<const PackHdr*>(hdr_p);
     const uint32_t* off = reinterpret_cast<const uint32_t*>(hdr_p + h.off_at);
     for (uint32_t v = blockIdx.x; v < h.total; v += gridDim.x) {
@@ -65,10 +63,12 @@ __global__ void __launch_bounds__(Op::kThreads, Op::kThreads == 512 ? 2 : 1) k_p
 
 // The body of a kernel as a packable operation: SDR_OP(k_name, threads)
 // declares k_name_op, whose run() calls k_name_body; `threads` is the largest
-// block the call sites use.
-#define SDR_OP(kern, threads)                                                   \
+// block the call sites use. SDR_OP_BLOCKS: with at least `blocks` of them an SM.
+#define SDR_OP(kern, threads) SDR_OP_BLOCKS(kern, threads, 1)
+#define SDR_OP_BLOCKS(kern, threads, blocks)                                    \
     struct kern##_op {                                                          \
         static constexpr int kThreads = (threads);                              \
+        static constexpr int kBlocks = (blocks);                                \
         template <class... A>                                                   \
         __device__ __forceinline__ static void run(VB vb, A... a) {             \
             kern##_body(vb, a...);                                              \

@@ -311,7 +311,9 @@ SDR_OP(k_sort_scatter, kBS)
 SDR_OP(k_sort_segments, 256)
 SDR_OP(k_sort_long, 256)
 SDR_OP(k_sorted_records, kBS)
-SDR_OP(k_p2g_nodes, kBrickBS)
+// two blocks an SM: without the bound the brick kernels took 67 to 72 registers,
+// and one block of 512 threads had an SM to itself
+SDR_OP_BLOCKS(k_p2g_nodes, kBrickBS, 2)
 SDR_OP(k_p2g, kBS)
 SDR_OP(k_add_forces, 256)
 SDR_OP(k_enforce_solid, 256)
@@ -324,7 +326,7 @@ SDR_OP(k_corder, 256)
 SDR_OP(k_pcg, kPcgBS)
 SDR_OP(k_gradient, 256)
 SDR_OP(k_extrap_valid, 256)
-SDR_OP(k_extrap, kBrickBS)
+SDR_OP_BLOCKS(k_extrap, kBrickBS, 2)  // as k_p2g_nodes
 SDR_OP(k_face_max, kFaceMaxBS)
 SDR_OP(k_g2p_advect, kBS)
 SDR_OP(k_bounds_flags, kBS)
