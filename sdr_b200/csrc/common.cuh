@@ -78,13 +78,20 @@ __device__ inline bool grid_sync_bounded(unsigned* bar, uint32_t* err, uint32_t 
 }
 
 // Start of every kernel that a substep launches: wait until the kernel before it
-// has finished and its writes are visible, then let the next one's launch begin.
-// Launched with programmatic serialisation, a kernel's blocks are set up while the
-// one before it drains; launched without, both calls return at once. A kernel's
-// end implies the end of all before it, as every one waits.
+// has finished and its writes are visible (pdl_wait), then let the next one's
+// launch begin (pdl_next). Launched with programmatic serialisation, a kernel's
+// blocks are set up while the one before it drains; launched without, both calls
+// return at once. A kernel's end implies the end of all before it, as every one
+// waits. The blocks set up hold their places while they wait: short kernels call
+// both at once, the pressure solves, which run for a millisecond on a few SMs,
+// pdl_next once their iterations are over, or the next kernel's blocks would keep
+// other solvers' work off the other SMs meanwhile (two threads with a solver of
+// 2,800 fluid cells each: a solve took 1.81 ms beside the other, 1.24 ms alone).
+__device__ __forceinline__ void pdl_wait() { cudaGridDependencySynchronize(); }
+__device__ __forceinline__ void pdl_next() { cudaTriggerProgrammaticLaunchCompletion(); }
 __device__ __forceinline__ void pdl_begin() {
-    cudaGridDependencySynchronize();
-    cudaTriggerProgrammaticLaunchCompletion();
+    pdl_wait();
+    pdl_next();
 }
 
 // The block a kernel body runs as: its index and the block count of its

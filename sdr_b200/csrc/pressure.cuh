@@ -939,6 +939,7 @@ __device__ __forceinline__ void k_pcg_body(VB vb_, PcgArgs a) {
             SECTION(6);
             sigma = sigma_new;
         }
+        pdl_next();
         for (uint32_t i = c.gt; i < nf; i += c.G) a.p_dense[a.lv_cell[i]] = a.p[i];
     }
     SECTION(7);
@@ -955,7 +956,7 @@ __device__ __forceinline__ void k_pcg_body(VB vb_, PcgArgs a) {
         }
     }
 }
-__global__ void __launch_bounds__(kPcgBS, 1) k_pcg(PcgArgs a) { pdl_begin(); k_pcg_body(VB{blockIdx.x, gridDim.x}, a); }
+__global__ void __launch_bounds__(kPcgBS, 1) k_pcg(PcgArgs a) { pdl_wait(); k_pcg_body(VB{blockIdx.x, gridDim.x}, a); }
 
 // apply_pressure_gradient (pressure.rs:285-332): one thread per node owning
 // its u/v/w faces; f64 update rounded back to the f32 face.

@@ -1208,6 +1208,7 @@ __device__ __forceinline__ void tw_solve(const TwArgs& t) {
                 TW_SECTION(6);
             }
         }
+        if (CL) pdl_next();
         for (uint32_t i = gt; i < nf; i += G)
             a.p_dense[a.lv_cell[i]] = owed ? dadd(__ldcg(a.p + i), dmul(alpha, __ldcg(s + i))) : __ldcg(a.p + i);
     }
@@ -1226,7 +1227,7 @@ out:
 __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) { tw_solve<false>(t); }
 // Launched as one cluster with a CTA per tile of the grid.
 __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles_cluster(TwArgs t) {
-    pdl_begin();
+    pdl_wait();
     tw_solve<true>(t);
 }
 

@@ -125,7 +125,7 @@ void launch_one_cluster_smem(Kern kernel, int ctas, int threads, size_t dyn_smem
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl ? 2 : 1;  // pdl: the kernel begins with pdl_begin()
+    cfg.numAttrs = pdl ? 2 : 1;  // pdl: the kernel begins with pdl_wait()
     CK(cudaLaunchKernelEx(&cfg, kernel, args...));
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
