@@ -121,6 +121,7 @@ struct TwArgs {
     double* sums_as;             // s*As, written by the matvec
     double* sums_zr;             // z*r, written behind the sweeps
     uint32_t* err;               // error bits
+    uint32_t* out_tiles;         // number of tiles with fluid cells
     int plane;                   // cluster form: levels of a halo plane (no tile has more)
 };
 
@@ -1067,6 +1068,7 @@ __device__ __forceinline__ void tw_solve(const TwArgs& t) {
             }
             if (lane == 0) {
                 t.tlist[0] = listed;
+                *t.out_tiles = (uint32_t)listed;
                 t.rbase[t.ntiles] = (uint32_t)min(run, (unsigned long long)t.rows_cap);
                 if (run > (unsigned long long)t.rows_cap) atomicOr(t.err, kTwErrWait);  // cannot happen: sized per tile
             }
@@ -1223,7 +1225,7 @@ out:
     if (CL) cluster_sync_all();  // no CTA leaves while another may still write into its planes
 }
 
-// Launched cooperatively (every CTA resident at once), one CTA per SM.
+// Launched cooperatively (every CTA resident at once), at most one CTA per SM.
 __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles(TwArgs t) { tw_solve<false>(t); }
 // Launched as one cluster with a CTA per tile of the grid.
 __global__ void __launch_bounds__(kTwBS, 1) k_pcg_tiles_cluster(TwArgs t) {

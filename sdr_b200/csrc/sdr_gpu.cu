@@ -257,6 +257,7 @@ struct DevStatus {
     double residual;
     unsigned long long drained, culled, moves;
     uint32_t nf;            // fluid cells of the last solve
+    uint32_t tiles;         // tiles with fluid cells of the last tiled solve that iterated
     uint32_t ncand;
     uint32_t nmoves;
     uint32_t long_count;
@@ -486,6 +487,7 @@ struct sdr_solver {
     uint32_t* p2g_list = nullptr;   // grid nodes with particles around them (P2G queue)
     uint32_t last_p2g_queue = 0;    // its length at the last status read
     uint32_t last_nf = 0;           // fluid cells of the last solve (picks the kernel under SDR_PCG_AUTO)
+    uint32_t last_tiles = 0;        // and its tiles with fluid cells (0: not known)
     double* cl_slots = nullptr;     // CTA partials of the cluster kernels
     // whole-GPU tiled solve (k_pcg_tiles), allocated on first use
     uint32_t *tw_idx = nullptr, *tw_tpos = nullptr, *tw_rbase = nullptr;
@@ -1050,6 +1052,20 @@ struct sdr_solver {
 
     int tw_plane_levels() const { return g.nx + kTwJ + kTwK; }
 
+    // CTAs of the grid form: one for every 512 fluid cells and for every tile
+    // with fluid cells of the last solve (a few more, as liquid spreads), at most
+    // one per SM; all of them while those are not known. More gain nothing: on
+    // 148, 48, 16 and 8 CTAs 744 cells of a 104x109x81 grid take 1.42, 1.30, 1.27
+    // and 1.17 ms, 7,400 cells 2.68, 2.60, 2.64 and 2.49, 74,000 cells 6.0, 6.2,
+    // 7.0 and 8.6. And CTAs that a solve does not need keep other solvers' solves
+    // waiting: four threads with 744 cells each take 4.2 to 4.9 ms a solve on 148,
+    // 1.4 this way (alone 1.2).
+    int tw_ctas() const {
+        if (!last_tiles) return tw_grid;
+        const uint64_t nf = std::max<uint64_t>(last_nf, n / std::max<uint64_t>(fluid.particles_per_cell, 1));
+        return (int)std::min<uint64_t>((uint64_t)tw_grid, std::max<uint64_t>({8, last_tiles + 4ull, nf / 512}));
+    }
+
     void launch_tiles(const PcgArgs& a) {
         TwArgs t{};
         t.a = a;  // a.timing: the section timers of profiling level 2
@@ -1064,6 +1080,7 @@ struct sdr_solver {
         t.sums_as = tpart;
         t.sums_zr = tpart + dot_room();
         t.err = &dst->err;
+        t.out_tiles = &dst->tiles;
         t.plane = tw_plane_levels();
         if (tw_cluster > 0) {
             launch_one_cluster_smem(k_pcg_tiles_cluster, tw_cluster, kTwBS, tw_cluster_smem(t.plane), true, st, t);
@@ -1071,7 +1088,7 @@ struct sdr_solver {
         }
         CK(cudaMemsetAsync(tw_bar, 0, 2 * sizeof(unsigned), st));  // a wound-down launch may leave arrivals
         void* args[] = {&t};
-        CK(cudaLaunchCooperativeKernel((const void*)k_pcg_tiles, dim3((unsigned)tw_grid), dim3(kTwBS), args, kTwSmem, st));
+        CK(cudaLaunchCooperativeKernel((const void*)k_pcg_tiles, dim3((unsigned)tw_ctas()), dim3(kTwBS), args, kTwSmem, st));
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
 
@@ -1292,6 +1309,7 @@ struct sdr_solver {
         last_pcg_iters = (uint64_t)hst->iters;
         last_residual = hst->residual;
         last_nf = hst->nf;
+        last_tiles = hst->tiles;
         last_p2g_queue = hst->p2g_queue;
         read_grid_speed();
         if (pending_timed) device_ms += elapsed(0, 9);
@@ -1388,6 +1406,7 @@ struct sdr_solver {
                 last_pcg_iters = (uint64_t)hst->iters;
                 last_residual = hst->residual;
                 last_nf = hst->nf;
+                last_tiles = hst->tiles;
                 if (profiling)
                     for (int q = 0; q < 16; ++q) prof.pcg_section_cycles[q] = hst->pcg_cycles[q];
             }
@@ -1920,6 +1939,7 @@ int sdr_solver_set_particles(sdr_solver* s, const double* pos_xyz, const double*
         }
         s->n = (uint32_t)n;
         LAUNCH(k_set_u32, 1, 1, 0, s->st, s->dn(), s->n);
+        s->last_tiles = 0;
         s->sorted_valid = false;
         CK(cudaStreamSynchronize(s->st));
     });
