@@ -95,7 +95,7 @@ typedef struct {
  * spinning): for many solvers driven by more host threads than cores. */
 #define SDR_SOLVER_BLOCKING_SYNC 1
 /* The GPU is shared with other scenes (batches, the request server): every
- * pressure solve holds one SM instead of a cluster of them. Results are the
+ * pressure solve holds one SM instead of 8 to all of them. Results are the
  * same either way. */
 #define SDR_SOLVER_SHARED_GPU 2
 
@@ -247,12 +247,16 @@ int sdr_solver_set_dot_order(sdr_solver* s, int reference_order);
  * reference's). SDR_PCG_TILES: the grid's (j, k) lines cut into tiles of
  * 16 x 16, one CTA per tile walking the levels of its cells, tiles handing
  * boundary values to their neighbours through entries that mark their own
- * readiness: one thread-block cluster where the grid has at most 16 tiles, else
- * the whole GPU in one cooperative launch (the cluster kernel if the device
- * cannot launch it or its buffers do not fit). SDR_PCG_AUTO (default): the tiled solve on a GPU of its
- * own; with SDR_SOLVER_SHARED_GPU one block, from 200,000 fluid cells in the
- * previous solve (before the first solve: the particle count over
- * particles_per_cell) the cluster. */
+ * readiness: one thread-block cluster of 8 or 16 CTAs where the grid has at
+ * most 16 tiles, else a cooperative launch of as many CTAs as the fluid of the
+ * last solve asks for (all of the GPU's from 75,000 fluid cells, and at the
+ * first solve; the cluster kernel if the device cannot launch it or its
+ * buffers do not fit). SDR_PCG_AUTO (default): the tiled solve; with
+ * SDR_SOLVER_SHARED_GPU one block, from 200,000 fluid cells in the previous
+ * solve (before the first solve: the particle count over particles_per_cell)
+ * the cluster. A few solvers on threads of their own run side by side without
+ * that flag: a solve of 7,400 cells takes 2.7 ms alone and 2.8 ms on four
+ * threads at once, one of 74,000, which fills the GPU, 6 and 18 ms. */
 enum { SDR_PCG_AUTO = 0, SDR_PCG_ONE_BLOCK = 1, SDR_PCG_CLUSTER = 2, SDR_PCG_TILES = 3 };
 int sdr_solver_set_pcg_kernel(sdr_solver* s, int kernel);
 /* CTAs of the SDR_PCG_ONE_BLOCK solve's cluster (CTA 0 runs the sweeps).

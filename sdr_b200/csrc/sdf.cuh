@@ -215,7 +215,7 @@ struct SdfFast {
     float4* norm;           // per triangle: unit normal
     float4* vert;           // per triangle: three vertices; vert[3 t].w: the f32 distance holds up to this distance squared (-1: nowhere)
     double* dist;           // per node
-    uint32_t* up;           // per node: the neighbour it follows, or itself; later its root
+    uint32_t* up;           // per node: the neighbour it follows, or itself (a root)
     uint32_t* roots;        // [0] their number, then the nodes
     uint8_t* inside;        // per node that is a root
     double* out;
@@ -404,8 +404,8 @@ static_assert(kSdfB == 4 && kSdfSplit == 4 && kSdfDistBS == 256, "eight warps of
 // bounds are evaluated in f64. Deep inside a smooth cavity the spheres leave
 // hundreds of triangles a node: the bound by the normal (sdf_beyond) and the
 // distance of a vertex as upper bound leave a few (20,480 triangles, 0.8 M nodes:
-// 4.6 -> 3.0 ms a field). Three blocks an SM take 3.0 ms, two 3.5, four 3.0 to
-// 3.8 (spilling). The margins (1e-3 and 2e-6 of the extent) cover the rounding of
+// 4.6 -> 3.0 ms a field). Three blocks an SM take 3.0 ms (with a little spilling,
+// 80 B of stores), two 3.5, four 3.0 to 3.8 (with more). The margins (1e-3 and 2e-6 of the extent) cover the rounding of
 // the f32 and f64 distances (k_sdf_balls), so no triangle that could give the
 // minimum is left out.
 __global__ void __launch_bounds__(kSdfDistBS, 3) k_sdf_dist(SdfFast a, int bx, int by) {

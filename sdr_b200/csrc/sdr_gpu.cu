@@ -895,7 +895,7 @@ struct sdr_solver {
         // A GPU of its own: the tiled solve at every size. Against k_pcg on an
         // 8-CTA cluster it takes (us per iteration, B200) 16 instead of 22 at
         // 320 fluid cells of a 21x22x17 grid, 30 instead of 63 at 10,000 cells
-        // (both cluster form), 28 instead of 37 at 340 cells and 58 instead of
+        // (both cluster form), 23 instead of 28 at 740 cells and 58 instead of
         // 292 at 77,000 cells of a 104x109x81 grid (grid form).
         const bool tiles = pcg_kernel == SDR_PCG_TILES || (pcg_kernel == SDR_PCG_AUTO && !shared_gpu);
         if (tiles && tiles_ready()) {
@@ -2440,7 +2440,7 @@ int sdr_sdf_from_mesh(const double* tris, size_t ntri, sdr_vec3 origin, double d
                 dalloc(dev, least, st);
             }
             double *dt = (double*)(dev + o_tri), *dout = (double*)(dev + o_out);
-            // flags: edge sums and extent (24 bytes), error word, gate, number of roots
+            // flags: edge sums and extent (24 bytes), error word, gate
             unsigned long long* acc = (unsigned long long*)(dev + o_flags);
             uint32_t *derr = (uint32_t*)(acc + 3), *gate = derr + 1;
             if (padded > ntri * 9) CK(cudaMemsetAsync(dt + ntri * 9, 0, (padded - ntri * 9) * 8, st));

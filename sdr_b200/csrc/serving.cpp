@@ -93,7 +93,11 @@ uint64_t footprint(const sdr_scene_desc& s) {
     // per cell: labels, histograms, wavefront tables, PCG vectors (f64), pressure;
     // per node: the six face arrays and their scratch copies (f32); per
     // particle: positions and velocities (double-buffered float4), sort keys,
-    // gather records; the SDF in f64 and f32; a fixed workspace.
+    // gather records; the SDF in f64 and f32; a fixed workspace. The solver has
+    // 201 B a cell and 31 B a node of it; a scene alone also the tiled solve's
+    // rows, 32 B (nx + 32) / nx a cell and whole tiles of 16 lines: within the
+    // rest from about 12 cells of width on. (A scene without room for the rows is
+    // solved without them.)
     return 320 * cells + 64 * nodes + 160 * particle_capacity(s) + 12 * sdf_nodes + (16ull << 20);
 }
 
